@@ -65,15 +65,21 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // of the block has given up, so that one lost signal costs one time limit, not one
 // per waiter.
 // Not inlined on purpose: the kernels wait in dozens of places and their instruction footprint
-// already exceeds the instruction cache.
-static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
+// already exceeds the instruction cache.  (A kernel that moves registers between its warpgroups cannot call
+// functions; it defines TTT_WAIT_INLINE before including this file.)
+#ifdef TTT_WAIT_INLINE
+#define TTT_WAIT_FN __forceinline__
+#else
+#define TTT_WAIT_FN __noinline__
+#endif
+static __device__ TTT_WAIT_FN bool mbar_wait_slow(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
                                             uint64_t limit_ns);
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity,
                                                   volatile uint32_t* abort_flag, uint64_t limit_ns) {
   if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait_slow(bar, parity, abort_flag, limit_ns);
 }
-static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
+static __device__ TTT_WAIT_FN bool mbar_wait_slow(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
                                             uint64_t limit_ns) {
   const uint64_t t0 = globaltimer_ns();
   uint32_t spins = 0;
@@ -102,6 +108,70 @@ __device__ __forceinline__ void tc_fence_after_sync() {
 }
 __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+
+// named barrier with an OR over the predicate of all its threads (a decision all of them take alike)
+__device__ __forceinline__ bool named_bar_or(uint32_t id, uint32_t nthreads, bool pred) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %3, 0;\n\t"
+      "barrier.cta.red.or.pred q, %1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(id), "r"(nthreads), "r"(pred ? 1u : 0u)
+      : "memory");
+  return r != 0;
+}
+
+// ------------------------------------------------------------------ packed fp32 pairs
+// One instruction of the fp32 pipe works on two values (add / mul / fma .f32x2, each half rounded like its
+// scalar form): the epilogues are bound by instruction issue, and most of their arithmetic pairs up.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ f32x2 pk(uint32_t lo, uint32_t hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+  return r;
+}
+__device__ __forceinline__ f32x2 pk1(float v) { return pk(v, v); }
+__device__ __forceinline__ void upk(f32x2 a, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a));
+}
+__device__ __forceinline__ float hsum(f32x2 a) {
+  float lo, hi;
+  upk(a, lo, hi);
+  return lo + hi;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// Registers per thread of this warpgroup from here on (all four warps execute it).  What one warpgroup takes,
+// another of the block must have given back: the shares add up to the block's registers at launch.
+template <int N>
+__device__ __forceinline__ void reg_take() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void reg_give() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
 // ------------------------------------------------------------------ TMA (tiled, 2-D)
@@ -204,6 +274,15 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
       "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr)
       : "memory");
 }
+// 16-column variant of tmem_st32
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::"r"(r[0]),
+      "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+      : "memory");
+}
 // tcgen05.ld, shape 16x256b, 4 repetitions: the warp reads 16 TMEM lanes (base lane .. +15) x 32
 // columns.  Thread i holds, for repetition j (8 columns each): r[4j], r[4j+1] = lane i/4, columns
 // 8j + 2(i%4), +1;  r[4j+2], r[4j+3] = lane i/4 + 8, same columns (the m16n8 accumulator pattern).
@@ -283,5 +362,12 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+
+__device__ __forceinline__ f32x2 bf16x2_to_f32x2(uint32_t w) { return pk(w << 16, w & 0xffff0000u); }
+__device__ __forceinline__ uint32_t f32x2_to_bf16x2(f32x2 a) {
+  float lo, hi;
+  upk(a, lo, hi);
+  return pack_bf16(lo, hi);
+}
 
 }  // namespace sm100

@@ -37,6 +37,26 @@ __device__ __forceinline__ float gelu_only(float x) {
   const float t = tanh_fast(x * fmaf(kG01, x * x, kG0));
   return x * fmaf(0.5f, t, 0.5f);
 }
+// The same on two elements at a time in packed fp32.  The epilogues that evaluate it are bound by the fp32 pipe, so
+// the forms below have the fewest operations and no negation (which packed operands do not have): gelu and gelu'
+// from t' = -t = tanh(-u) as h = (1 - t') / 2, g = x h, gelu' = h + (g + g t') q; gelu alone from y = x / 2 as y + y t.
+__device__ __forceinline__ f32x2 tanh2(f32x2 u) {
+  float lo, hi;
+  upk(u, lo, hi);
+  return pk(tanh_fast(lo), tanh_fast(hi));
+}
+__device__ __forceinline__ void gelu_pair2(f32x2 x, f32x2& g, f32x2& gp) {
+  const f32x2 x2 = mul2(x, x);
+  const f32x2 t = tanh2(mul2(x, fma2(x2, pk1(-kG01), pk1(-kG0))));       // -tanh(u)
+  const f32x2 h = fma2(t, pk1(-0.5f), pk1(0.5f));
+  g = mul2(x, h);
+  gp = fma2(fma2(g, t, g), fma2(x2, pk1(kG2), pk1(kG0)), h);
+}
+// gelu(2 y)
+__device__ __forceinline__ f32x2 gelu_half2(f32x2 y) {
+  const f32x2 t = tanh2(mul2(y, fma2(mul2(y, y), pk1(8.f * kG01), pk1(2.f * kG0))));
+  return fma2(y, t, y);
+}
 // gelu'(x) and gelu''(x)
 __device__ __forceinline__ void gelu_grad_pair(float x, float& gp, float& gpp) {
   const float x2 = x * x;
@@ -254,6 +274,65 @@ TTT_MMA_LOOP
 #endif
 }
 
+// ---- The same products issued by a whole warp under a predicate: the warp runs the code uniformly, so that the
+// descriptors are computed in uniform registers, and only the elected lane's tcgen05.mma is enabled (`lead`).
+// Inside an `if (elect_one())` block the operands pass through vector registers instead: 8 MMAs took 390 cycles
+// to issue there and take 182 here (16: 537 and 397), against 376 (512) that the tensor pipe needs for them.
+template <bool kAccumulate>
+__device__ __forceinline__ void mma_lead(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %4};\n\t"
+      "mov.b64 db, {%2, %4};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kDescHi), "n"(kAccumulate ? 1 : 0), "r"(lead)
+      : "memory");
+}
+// one 128-row block: D[128 x 64] (+)= A[128][64] B
+template <bool kBMn, bool kAccumulate>
+__device__ __forceinline__ void mma_hidden_lead(uint32_t tmem_d, uint32_t a_smem, uint32_t b_smem, int blk, uint32_t lead) {
+  constexpr uint32_t idesc = umma_idesc_bf16(128, 64, false, kBMn, false);
+  const uint32_t a0 = desc_lo(a_smem, 16) + blk * (16384u >> 4);
+  const uint32_t b0 = desc_lo(b_smem, kBMn ? 8192 : 16);
+  constexpr uint32_t bstep = kBMn ? (2048u >> 4) : (32u >> 4);
+  const uint32_t d = tmem_d + blk * 64;
+  mma_lead<kAccumulate>(d, a0, b0, idesc, lead);
+#pragma unroll
+  for (int j = 1; j < 4; ++j) mma_lead<true>(d, a0 + j * 2, b0 + j * bstep, idesc, lead);
+}
+// The same block with A in tensor memory: bf16 pairs, row = lane, 32 columns for the 64 elements along K.  The MMA
+// then reads 2 KB of shared memory instead of 6 KB (32 cycles instead of 47, the tensor pipe's own rate).
+template <bool kAccumulate>
+__device__ __forceinline__ void mma_lead_ta(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
+      "mov.b64 db, {%2, %4};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(kDescHi), "n"(kAccumulate ? 1 : 0), "r"(lead)
+      : "memory");
+}
+template <bool kBMn, bool kAccumulate>
+__device__ __forceinline__ void mma_hidden_ta(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_smem, uint32_t lead) {
+  constexpr uint32_t idesc = umma_idesc_bf16(128, 64, false, kBMn, false);
+  const uint32_t b0 = desc_lo(b_smem, kBMn ? 8192 : 16);
+  constexpr uint32_t bstep = kBMn ? (2048u >> 4) : (32u >> 4);
+  mma_lead_ta<kAccumulate>(tmem_d, tmem_a, b0, idesc, lead);
+#pragma unroll
+  for (int j = 1; j < 4; ++j) mma_lead_ta<true>(tmem_d, tmem_a + j * 8, b0 + j * bstep, idesc, lead);
+}
+__device__ __forceinline__ void mma_token_lead(uint32_t tmem_d, uint32_t x_smem, uint32_t w_smem, uint32_t lead) {
+  constexpr uint32_t idesc = umma_idesc_bf16(64, 64, true, true, false);
+  const uint32_t a0 = desc_lo(x_smem, BIG);
+  const uint32_t b0 = desc_lo(w_smem, BIG);
+  mma_lead<false>(tmem_d, a0, b0, idesc, lead);
+#pragma unroll
+  for (int j = 1; j < 16; ++j) mma_lead<true>(tmem_d, a0 + j * (2048u >> 4), b0 + j * (2048u >> 4), idesc, lead);
+}
+
 // ---- A warp's 32 rows x 32 fp32 columns (lane = row, v = the row's 32 values) -> a row-major global
 // matrix with `ld` floats per row, as whole 128-byte lines: written straight from the registers the
 // 16-byte stores of a warp would land in 32 different lines (measured: the fp32 W2 checkpoint written
@@ -395,6 +474,111 @@ __device__ __forceinline__ void tok_layernorm(const TokMap& m, float (&z)[16], f
   tok_row_allreduce<1, 1>(m, s0, s1, xch);
   rstd0 = rsqrtf(s0[0] * (1.f / 64.f) + eps);
   rstd1 = rsqrtf(s1[0] * (1.f / 64.f) + eps);
+}
+
+// ---- The same fragments as packed fp32 pairs, for kernels whose CTA runs several groups of 8 warps: a[j] is
+// the column pair col(j), col(j) + 1 of row r0, b[j] that of row r1.  `bar` = the group's first of four named
+// barriers (one per warp pair), `xch` the group's exchange area (kXchBytes).
+constexpr uint32_t kXchBytes = 2 * 2 * 64 * 2 * 4;      // two exchanges x two column halves x 64 rows x two values
+struct TokFrag {
+  f32x2 a[4], b[4];
+};
+__device__ __forceinline__ void frag_ld(const TokMap& m, uint32_t tmem_acc, TokFrag& f) {
+  uint32_t u[16];
+  tmem_ld_16x256b_x4(tmem_acc + m.taddr, u);
+  tmem_wait_ld();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    f.a[j] = pk(u[4 * j], u[4 * j + 1]);
+    f.b[j] = pk(u[4 * j + 2], u[4 * j + 3]);
+  }
+}
+// the raw bf16 pairs of a swizzled tile: w[2j] row r0, w[2j + 1] row r1
+__device__ __forceinline__ void frag_ld_raw(const TokMap& m, const uint8_t* tile, uint32_t (&w)[8]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    w[2 * j] = *reinterpret_cast<const uint32_t*>(tile + m.off(m.r0, j));
+    w[2 * j + 1] = *reinterpret_cast<const uint32_t*>(tile + m.off(m.r1, j));
+  }
+}
+__device__ __forceinline__ void frag_st_tile(const TokMap& m, uint8_t* tile, const TokFrag& f) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    *reinterpret_cast<uint32_t*>(tile + m.off(m.r0, j)) = f32x2_to_bf16x2(f.a[j]);
+    *reinterpret_cast<uint32_t*>(tile + m.off(m.r1, j)) = f32x2_to_bf16x2(f.b[j]);
+  }
+}
+// per-column vector (fp32[64] in shared memory): the thread's four column pairs
+__device__ __forceinline__ f32x2 frag_col(const TokMap& m, const float* vec, int j) {
+  return *reinterpret_cast<const f32x2*>(vec + m.col(j));
+}
+// two sums per row over the row's 8 threads; kSlot = 0 or 1 picks the exchange (each once per phase)
+template <int kSlot>
+__device__ __forceinline__ void frag_allreduce2(const TokMap& m, float (&a)[2], float (&b)[2], float* xch, uint32_t bar) {
+#pragma unroll
+  for (int s = 1; s <= 2; s <<= 1) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      a[i] += __shfl_xor_sync(0xffffffffu, a[i], s);
+      b[i] += __shfl_xor_sync(0xffffffffu, b[i], s);
+    }
+  }
+  float2* x = reinterpret_cast<float2*>(xch) + kSlot * 128;
+  if (m.l3 == 0) {
+    x[m.colhalf * 64 + m.r0] = make_float2(a[0], a[1]);
+    x[m.colhalf * 64 + m.r1] = make_float2(b[0], b[1]);
+  }
+  named_bar_sync(bar + m.quad, 64);
+  const float2 oa = x[(m.colhalf ^ 1) * 64 + m.r0], ob = x[(m.colhalf ^ 1) * 64 + m.r1];
+  a[0] += oa.x; a[1] += oa.y;
+  b[0] += ob.x; b[1] += ob.y;
+}
+// LayerNorm of the thread's two rows in place (x -> (x - mean) / std), returns 1/std per row.  Mean and sum of
+// squared deviations are merged pairwise (Chan, Golub and LeVeque's update for equal counts): as accurate as a
+// second pass about the mean, with one exchange between the warp pair instead of two.  Uses exchange 0.
+__device__ __forceinline__ void frag_layernorm(const TokMap& m, TokFrag& f, float eps, float* xch, uint32_t bar,
+                                               float& rs0, float& rs1) {
+  float m0 = hsum(add2(add2(f.a[0], f.a[1]), add2(f.a[2], f.a[3]))) * 0.125f;
+  float m1 = hsum(add2(add2(f.b[0], f.b[1]), add2(f.b[2], f.b[3]))) * 0.125f;
+  f32x2 q0 = 0ull, q1 = 0ull;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const f32x2 d0 = add2(f.a[j], pk1(-m0)), d1 = add2(f.b[j], pk1(-m1));
+    q0 = fma2(d0, d0, q0);
+    q1 = fma2(d1, d1, q1);
+  }
+  float s0 = hsum(q0), s1 = hsum(q1);
+#pragma unroll
+  for (int s = 1; s <= 2; s <<= 1) {
+    const float n0 = __shfl_xor_sync(0xffffffffu, m0, s), n1 = __shfl_xor_sync(0xffffffffu, m1, s);
+    const float t0 = __shfl_xor_sync(0xffffffffu, s0, s), t1 = __shfl_xor_sync(0xffffffffu, s1, s);
+    const float d0 = n0 - m0, d1 = n1 - m1;
+    m0 = 0.5f * (m0 + n0);
+    m1 = 0.5f * (m1 + n1);
+    s0 = fmaf(d0 * d0, 4.f * s, s0 + t0);
+    s1 = fmaf(d1 * d1, 4.f * s, s1 + t1);
+  }
+  float2* x = reinterpret_cast<float2*>(xch);
+  if (m.l3 == 0) {
+    x[m.colhalf * 64 + m.r0] = make_float2(m0, s0);
+    x[m.colhalf * 64 + m.r1] = make_float2(m1, s1);
+  }
+  named_bar_sync(bar + m.quad, 64);
+  const float2 o0 = x[(m.colhalf ^ 1) * 64 + m.r0], o1 = x[(m.colhalf ^ 1) * 64 + m.r1];
+  {
+    const float d0 = o0.x - m0, d1 = o1.x - m1;
+    m0 = 0.5f * (m0 + o0.x);
+    m1 = 0.5f * (m1 + o1.x);
+    s0 = fmaf(d0 * d0, 16.f, s0 + o0.y);
+    s1 = fmaf(d1 * d1, 16.f, s1 + o1.y);
+  }
+  rs0 = rsqrtf(s0 * (1.f / 64.f) + eps);
+  rs1 = rsqrtf(s1 * (1.f / 64.f) + eps);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    f.a[j] = mul2(add2(f.a[j], pk1(-m0)), pk1(rs0));
+    f.b[j] = mul2(add2(f.b[j], pk1(-m1)), pk1(rs1));
+  }
 }
 
 }  // namespace tttdev

@@ -11,22 +11,45 @@
 // memory, refreshed once per mini-batch, feeds the other MMAs.  b1 lives in registers (one
 // hidden unit per thread), b2 in shared memory.
 //
-// Per mini-batch (K, V, Q: 64x64 bf16 tiles brought in by TMA, eta: 64 bf16):
-//   MMA1  Z1^T  = W1^T K^T                    [256 x 64 tok]   (2 x M128, N64, K64)
-//   EPI1  X2^T = gelu(Z1^T + b1), G' = gelu'(.)  -> smem bf16
-//   MMA2  Z2    = X2 W2                       [64 tok x 64]    (M64, N64, K256)
-//   LN    fused LayerNorm + L2-gradient: U2 = -eta * dl/dZ2    -> smem bf16;  b2 += colsum(U2)
-//   MMA3  R^T   = W2 U2^T                     [256 x 64 tok]
-//   EPI3  U1^T = R^T * G'  (= -eta * dl/dZ1)   -> smem bf16;  b1 += rowsum
-//   MMA4  W1^T += U1^T K ;  W2 += X2^T U2     (accumulate into the TMEM state)
-//   EPI4  bf16 copies of the new W1^T, W2     -> smem
-//   MMA5  Z1b^T = W1^T Q^T ;  EPI5  X2b^T = gelu(. + b1)
-//   MMA6  Z2b   = X2b W2   ;  OUT   Out = Q + gamma * LN(Z2b + b2) + beta  -> TMA store
+// A mini-batch is a chain of dependent MMA -> epilogue round trips, and only a part of it is needed by the
+// next mini-batch: the output pass (the post-update product with Q, GELU, LayerNorm) is not.  So the CTA runs two
+// groups of eight warps, each with its own accumulator in tensor memory, one MMA issuer and its own barriers:
+//
+//   chain group                                        output group
+//   MMA1  Z1^T = W1^T K^T        [256 x 64 tok]        (W2 updated:)  bf16 copy of the new W2 -> smem
+//   EPI1  X2^T = gelu(Z1^T + b1), G' = gelu'(.)                       b2 += colsum(U2); checkpoints
+//   MMA2  Z2 = X2 W2             [64 tok x 64]         (W1 copied:)   MMA5  Z1b^T = W1^T Q^T
+//   LN    U2 = -eta * dl/dZ2 (fused LN + L2 gradient)  EPI5  X2b^T = gelu(Z1b^T + b1)
+//   MMA3  R^T = W2 U2^T                                MMA6  Z2b = X2b W2
+//   EPI3  U1^T = R^T * G';  b1 += rowsum               OUT   Q + gamma * LN(Z2b + b2) + beta -> TMA store
+//   MMA4  W1^T += U1^T K ;  W2 += X2^T U2
+//   EPI4  bf16 copy of the new W1^T -> smem
+//
+// The output group works one step behind, on the state the chain group has just left: the chain is four round
+// trips per mini-batch instead of six, and each group's MMA latencies are filled with the other's epilogues (four
+// warps per scheduler).
+//
+// What bounds it: instruction issue and the fp32 / MUFU pipes (EPI1 alone is 1300 cycles of fp32 pipe per mini-batch
+// at 9 packed operations and 2 conversions per pair of elements) and shared-memory bandwidth.  So the arithmetic
+// runs on packed fp32 pairs; what only one thread needs stays out of shared memory (G' in registers from EPI1 to
+// EPI3, U1 and the bf16 W1 in tensor memory as A operands of their MMAs, which then read 2 KB of shared memory
+// instead of 6); and the MMAs are issued from warp-uniform code.  Measured (B200, 128 streams, one checkpoint in 8
+// mini-batches): 8.0 us per mini-batch before, one group of 8 warps, 6.0 with the two groups, 5.3 now; 1536 streams of
+// 64 mini-batches 5.43 -> 3.68 ms.
+//
+// Hand-over between the groups (mbarriers, each completed once per mini-batch):
+//   w2upd   MMA4's W2 update has completed                     chain's tensor work -> output group
+//   w2rdy   bf16 W2 and b2 are refreshed                       output group -> chain (MMA2, LN)
+//   sread   the output group has read the state columns and
+//           taken note of w1rdy                                output group -> chain (MMA4)
+//   w1rdy   bf16 W1 and the shared copy of b1 are refreshed    chain -> output group (MMA5)
+//   accb[1] MMA5 has completed: the bf16 W1 may be rewritten   output's tensor work -> chain (EPI4)
 //
 // All waits are bounded (see sm100_ptx.cuh); on expiry the CTA reports through the status
 // word, drains its own copies, frees its tensor memory and returns.
 #include <mutex>
 
+#define TTT_WAIT_INLINE
 #include "ttt_device.cuh"
 #include "ttt_internal.h"
 
@@ -34,37 +57,53 @@ using namespace tttdev;
 
 namespace {
 
-constexpr int kStages = 3;
-constexpr int kThreads = 256;
-// The thread that issues the bulk copies and waits for their completion is not one of the four MMA issuers
-// (lane 0 of warps 0..3): its bookkeeping between a barrier and the next MMA group stays off the issue path.
-constexpr int kProd = 128;
+constexpr int kStages = 2;
+constexpr int kGroup = 256;          // threads of one group
+constexpr int kThreads = 2 * kGroup;
+// registers per thread: EPI1 leaves G' in 32 of the chain group's
+constexpr int kRegsChain = 152, kRegsOut = 104;
+static_assert(kRegsChain + kRegsOut <= 2 * 128, "the block is launched with 128 registers per thread");
+// named barriers: one per warp pair of each group, then one per group
+constexpr uint32_t kBarPairC = 1, kBarPairO = 5, kBarC = 9, kBarO = 10;
 
 constexpr uint32_t OFF_K = 0;
 constexpr uint32_t OFF_V = OFF_K + kStages * TILE;
-constexpr uint32_t OFF_Q = OFF_V + kStages * TILE;
-constexpr uint32_t OFF_OUT = OFF_Q + kStages * TILE;
-constexpr uint32_t OFF_W1 = OFF_OUT + TILE;
-constexpr uint32_t OFF_W2 = OFF_W1 + BIG;
+constexpr uint32_t OFF_Q = OFF_V + kStages * TILE;      // Q, then Out on its way to global memory
+constexpr uint32_t OFF_W2 = OFF_Q + kStages * TILE;
 constexpr uint32_t OFF_X2 = OFF_W2 + BIG;
-constexpr uint32_t OFF_GP = OFF_X2 + BIG;
-constexpr uint32_t OFF_U2 = OFF_GP + BIG;
+constexpr uint32_t OFF_X2B = OFF_X2 + BIG;
+constexpr uint32_t OFF_STG = OFF_X2B + BIG;             // 4 KB per warp of the output group: W2 checkpoints on their way out
+constexpr uint32_t OFF_U2 = OFF_STG + BIG;
 constexpr uint32_t OFF_ETA = OFF_U2 + TILE;
-constexpr uint32_t OFF_B2 = OFF_ETA + kStages * 128;
-constexpr uint32_t OFF_GAMMA = OFF_B2 + 256;
+constexpr uint32_t OFF_B1 = OFF_ETA + kStages * 128;    // fp32[2][256]: b1 as of odd / even mini-batches
+constexpr uint32_t OFF_B2 = OFF_B1 + 2048;              // fp32[2][64]
+constexpr uint32_t OFF_GAMMA = OFF_B2 + 512;
 constexpr uint32_t OFF_BETA = OFF_GAMMA + 256;
-constexpr uint32_t OFF_BAR = OFF_BETA + 256;
-constexpr uint32_t OFF_MISC = OFF_BAR + 64;
-constexpr uint32_t OFF_XCH = OFF_MISC + 64;       // fp32[2][64][8] row-sum exchange between warp pairs
-constexpr uint32_t SMEM_USED = OFF_XCH + 4096;
-constexpr uint32_t SMEM_BYTES = SMEM_USED + 1024;  // slack for the 1024-byte alignment
+constexpr uint32_t OFF_XCHC = OFF_BETA + 256;           // row-sum exchange of each group
+constexpr uint32_t OFF_XCHO = OFF_XCHC + kXchBytes;     // also the partial column sums: fp32[8][64]
+constexpr uint32_t OFF_BAR = OFF_XCHO + kXchBytes;
+constexpr uint32_t OFF_MISC = OFF_BAR + 192;
+constexpr uint32_t SMEM_USED = OFF_MISC + 16;
+constexpr uint32_t SMEM_BYTES = SMEM_USED + 1024;       // slack for the 1024-byte alignment
 static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB per-CTA shared memory of sm_100");
+static_assert(kXchBytes >= 8 * 64 * 4, "the partial column sums fit the exchange area");
 
-// tensor-memory columns (fp32): two 128-lane blocks of 64 columns per 256-row matrix
+// barrier indices
+constexpr int BAR_K = 0, BAR_V = 2, BAR_Q = 4;          // + stage
+constexpr int BAR_ACCA = 6;                             // + block (the two 128-row halves of the accumulator)
+constexpr int BAR_Z = 8;
+constexpr int BAR_ACCB = 9;                             // two uses per mini-batch
+constexpr int BAR_ZB = 11;
+constexpr int BAR_W2UPD = 12, BAR_W2RDY = 13, BAR_SREAD = 14, BAR_W1RDY = 15;
+constexpr int BAR_DRAIN = 16;                           // abort path only
+constexpr int kBars = 17;
+
+// tensor-memory columns: two 128-lane blocks of 64 fp32 (32 bf16-pair) columns per 256-row matrix
 constexpr uint32_t TM_W1 = 0;
 constexpr uint32_t TM_W2 = 128;
-constexpr uint32_t TM_A = 256;
-constexpr uint32_t TM_Z = 384;
+constexpr uint32_t TM_A = 256;       // chain: Z1; Z2 in its first 64 columns; R; U1 (bf16) in the first half of each block
+constexpr uint32_t TM_W1B = 384;     // bf16 operand copy of W1^T
+constexpr uint32_t TM_B = 448;       // output: Z1b, one block after the other; Z2b
 constexpr uint32_t TM_COLS = 512;
 
 struct FwdParams {
@@ -89,21 +128,43 @@ struct FwdParams {
   uint64_t wait_limit_ns;
 };
 
-// The MMAs of one phase are issued by lane 0 of warps 0..3: four instruction streams on four
-// schedulers instead of one.  Every issuer commits (an issuer without work too), so the MMA
-// barrier counts four arrivals per phase.
-#define TTT_ISSUE(W0, W1, W2, W3)   \
-  if (warp < 4) {                   \
-    if (elect_one()) {              \
-      tc_fence_after_sync();        \
-      if (warp == 0) { W0; }        \
-      else if (warp == 1) { W1; }   \
-      else if (warp == 2) { W2; }   \
-      else { W3; }                  \
-      umma_commit(mma_bar);         \
-    }                               \
-    __syncwarp();                   \
+// A warp's 32 rows x 32 fp32 columns (lane = row) -> a row-major global matrix with 64 floats per row, as whole
+// 128-byte lines, turned through the warp's own 4 KB of a hidden-major tile (16-byte chunks XOR-swizzled by row:
+// both directions conflict-free).
+__device__ __forceinline__ void store_rows_own(float* dst, const uint32_t (&v)[32], uint8_t* stage, int lane) {
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    *reinterpret_cast<uint4*>(stage + sw128_off(lane, c)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = 4 * i + (lane >> 3), ch = lane & 7;
+    *reinterpret_cast<uint4*>(dst + r * 64 + ch * 4) = *reinterpret_cast<const uint4*>(stage + sw128_off(r, ch));
   }
+  __syncwarp();
+}
+
+// the four 16-byte chunks of 32 fp32 accumulator columns as bf16, to row `row` of a swizzled tile
+__device__ __forceinline__ void st_cols32(uint8_t* tile, int row, int half, const uint32_t (&v)[32]) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint4 w;
+    w.x = pack_bf16(__uint_as_float(v[c * 8 + 0]), __uint_as_float(v[c * 8 + 1]));
+    w.y = pack_bf16(__uint_as_float(v[c * 8 + 2]), __uint_as_float(v[c * 8 + 3]));
+    w.z = pack_bf16(__uint_as_float(v[c * 8 + 4]), __uint_as_float(v[c * 8 + 5]));
+    w.w = pack_bf16(__uint_as_float(v[c * 8 + 6]), __uint_as_float(v[c * 8 + 7]));
+    *reinterpret_cast<uint4*>(tile + sw128_off(row, half * 4 + c)) = w;
+  }
+}
+
+// 32 fp32 accumulator columns as bf16 pairs to 16 columns of tensor memory (an A operand of the MMAs)
+__device__ __forceinline__ void st_cols32_tmem(uint32_t taddr, const uint32_t (&v)[32]) {
+  uint32_t w[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) w[k] = pack_bf16(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
+  tmem_st16(taddr, w);
+}
 
 __global__ void __launch_bounds__(kThreads, 1)
 ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -113,27 +174,25 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
   const int tid = threadIdx.x, lane = tid & 31;
-  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // same value, known to be warp-uniform
+  const int cta_warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // same value, known to be warp-uniform
+  const int warp = cta_warp & 7;                         // within the group
   const int quad = warp & 3, wg = warp >> 2;
+  const int gtid = tid & (kGroup - 1);
   const int hrow = wg * 128 + quad * 32 + lane;          // hidden unit owned in the 256-row epilogues
   const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
   const TokMap tm(warp, lane);                           // fragment of the 64 x 64 token-major tiles
   const long stream_id = blockIdx.x;
   const int head = static_cast<int>(stream_id % p.H);
 
-  uint8_t* sW1 = smem + OFF_W1;
   uint8_t* sW2 = smem + OFF_W2;
   uint8_t* sX2 = smem + OFF_X2;
-  uint8_t* sGP = smem + OFF_GP;
+  uint8_t* sX2b = smem + OFF_X2B;
   uint8_t* sU2 = smem + OFF_U2;
-  uint8_t* sOut = smem + OFF_OUT;
+  float* sB1 = reinterpret_cast<float*>(smem + OFF_B1);
   float* sB2 = reinterpret_cast<float*>(smem + OFF_B2);
   float* sGamma = reinterpret_cast<float*>(smem + OFF_GAMMA);
   float* sBeta = reinterpret_cast<float*>(smem + OFF_BETA);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + OFF_BAR);   // [kStages]
-  uint64_t* mma_bar = full + kStages;
-  uint64_t* drain_bar = mma_bar + 1;        // abort path only
-  float* sXch = reinterpret_cast<float*>(smem + OFF_XCH);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_MISC);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + OFF_MISC + 4);
   volatile uint32_t* never_flag = reinterpret_cast<volatile uint32_t*>(smem + OFF_MISC + 8);   // stays 0
@@ -141,10 +200,9 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   const uint64_t limit = p.wait_limit_ns;
   const int NC = p.NC;
 
-  if (tid == kProd) {
-    for (int s = 0; s < kStages; ++s) mbar_init(&full[s], 1);
-    mbar_init(mma_bar, 4);
-    mbar_init(drain_bar, 4);
+  if (tid == 0) {
+    for (int i = 0; i < kBars; ++i)
+      mbar_init(&bars[i], i == BAR_SREAD ? 8 : i == BAR_W2RDY ? 3 : i == BAR_DRAIN ? 2 : 1);
     fence_mbar_init();
     *abort_flag = 0;
     *never_flag = 0;
@@ -153,7 +211,7 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     prefetch_tmap(&tmV);
     prefetch_tmap(&tmOut);
   }
-  if (warp == 0) {
+  if (cta_warp == 0) {
     tmem_alloc(tmem_slot, TM_COLS);
     tmem_relinquish();
   }
@@ -167,368 +225,472 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
 
-  auto issue_loads = [&](int i) {   // thread 0 only
-    if (i == p.drop_load && stream_id == 0) return;
-    const int s = i % kStages;
-    const int row0 = static_cast<int>((stream_id * NC + i) * 64);
-    mbar_expect_tx(&full[s], 3 * TILE + 128);
-    tma_load_2d(smem + OFF_K + s * TILE, &tmK, &full[s], 0, row0);
-    tma_load_2d(smem + OFF_V + s * TILE, &tmV, &full[s], 0, row0);
-    tma_load_2d(smem + OFF_Q + s * TILE, &tmQ, &full[s], 0, row0);
-    bulk_load_1d(smem + OFF_ETA + s * 128, p.eta + (stream_id * NC + i) * 64, 128, &full[s]);
+  auto wait_bar = [&](int b, uint32_t parity) { mbar_wait_bounded(&bars[b], parity & 1u, abort_flag, limit); };
+  // Loads, by one thread of the group that consumes them: K with eta, V (chain group), Q (output group).  Stream
+  // 0's loads of mini-batch drop_load are never issued (test of the failure path).
+  auto dropped = [&](int i) { return i == p.drop_load && stream_id == 0; };
+  auto row_of = [&](int i) { return static_cast<int>((stream_id * NC + i) * 64); };
+  auto load_k = [&](int i) {
+    if (i >= NC || dropped(i)) return;
+    const int s = i & 1;
+    mbar_expect_tx(&bars[BAR_K + s], TILE + 128);
+    tma_load_2d(smem + OFF_K + s * TILE, &tmK, &bars[BAR_K + s], 0, row_of(i));
+    bulk_load_1d(smem + OFF_ETA + s * 128, p.eta + (stream_id * NC + i) * 64, 128, &bars[BAR_K + s]);
   };
-  int loads_issued = 0;
-  if (tid == kProd) {
-    for (; loads_issued < kStages && loads_issued < NC; ++loads_issued) issue_loads(loads_issued);
-  }
-
-  // ---- initial state: global fp32 -> tensor memory (master) + shared memory (bf16 operand copy)
-  float b1v = p.b1[stream_id * 256 + hrow];
-  {
-    const float* W1g = p.W1 + stream_id * (64 * 256);
-    const float* W2g = p.W2 + stream_id * (256 * 64) + hrow * 64;
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-      uint32_t v[32];
-      float f[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        f[j] = W1g[(half * 32 + j) * 256 + hrow];
-        v[j] = __float_as_uint(f[j]);
-      }
-      tmem_st32(tmem + lane_base + TM_W1 + wg * 64 + half * 32, v);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) st_chunk(sW1, hrow, half * 4 + c, f + c * 8);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float4 q4 = reinterpret_cast<const float4*>(W2g)[half * 8 + j];
-        f[j * 4 + 0] = q4.x; f[j * 4 + 1] = q4.y; f[j * 4 + 2] = q4.z; f[j * 4 + 3] = q4.w;
-      }
-#pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(f[j]);
-      tmem_st32(tmem + lane_base + TM_W2 + wg * 64 + half * 32, v);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) st_chunk(sW2, hrow, half * 4 + c, f + c * 8);
-    }
-    tmem_wait_st();
-  }
-  fence_proxy_async_smem();
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-
-  // fp32 state (tensor memory, registers, shared memory) -> global, reference layouts
-  // Quarter q of the state: 0, 2 = the two 32-column halves of W1^T; 1, 3 = those of W2.
-  auto store_state_quarter = [&](int q, float* W1o, float* W2o) {
-    const int half = q >> 1;
-    uint32_t v[32];
-    __syncwarp();
-    if ((q & 1) == 0) {
-      tmem_ld32(tmem + lane_base + TM_W1 + wg * 64 + half * 32, v);
-      tmem_wait_ld();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) W1o[(half * 32 + j) * 256 + hrow] = __uint_as_float(v[j]);
-    } else {
-      // through a staging area in the X2 / G' buffers: only called while those are free (before EPI1
-      // writes them: the first MMA window of a mini-batch, or after the last mini-batch)
-      tmem_ld32(tmem + lane_base + TM_W2 + wg * 64 + half * 32, v);
-      tmem_wait_ld();
-      store_rows_coalesced(W2o + (hrow - lane) * 64 + half * 32, 64, v, sX2 + warp * kRowStageBytes, lane);
-    }
+  auto load_tile = [&](int i, const CUtensorMap* map, uint32_t off, int bar) {
+    if (i >= NC || dropped(i)) return;
+    const int s = i & 1;
+    mbar_expect_tx(&bars[bar + s], TILE);
+    tma_load_2d(smem + off + s * TILE, map, &bars[bar + s], 0, row_of(i));
   };
-  auto store_state = [&](float* W1o, float* b1o, float* W2o, float* b2o) {
-#pragma unroll 1
-    for (int q = 0; q < 4; ++q) store_state_quarter(q, W1o, W2o);
-    b1o[hrow] = b1v;
-    if (tid < 64) b2o[tid] = sB2[tid];
+  // abort path: the loads of mini-batches i and i + 1 or before that may still be in flight, one per stage
+  auto drain_loads = [&](int bar, int issued) {
+    for (int i = issued > kStages ? issued - kStages : 0; i < issued && i < NC; ++i)
+      if (!dropped(i)) mbar_wait_bounded(&bars[bar + (i & 1)], (i >> 1) & 1, never_flag, limit);
   };
-
-  uint32_t mma_phase = 0;
-  auto wait_mma = [&]() {
-    mbar_wait_bounded(mma_bar, mma_phase, abort_flag, limit);
-    mma_phase ^= 1;
-    __syncwarp();
-    tc_fence_after_sync();
-  };
-  // generic-proxy smem writes + TMEM reads done -> next MMA may be issued
-  auto publish = [&]() {
-    fence_proxy_async_smem();
-    tc_fence_before_sync();
-    __syncthreads();
-  };
-
+  const long st_w = stream_id * (64 * 256);
+  const bool chain = cta_warp < 8;
+  const uint32_t lead = elect_one() ? 1u : 0u;      // the lane that issues the MMAs (warp 0 of each group)
   int it = 0;
-  for (; it < NC; ++it) {
-    const int s = it % kStages;
-    const uint8_t* sK = smem + OFF_K + s * TILE;
-    const uint8_t* sV = smem + OFF_V + s * TILE;
-    const uint8_t* sQ = smem + OFF_Q + s * TILE;
-    const __nv_bfloat16* sEta = reinterpret_cast<const __nv_bfloat16*>(smem + OFF_ETA + s * 128);
+  int issued = 0;       // loads of this group issued so far (its loading thread), for the abort path
 
-    // A checkpoint (the state before this mini-batch) is written while the first three MMA groups of the
-    // mini-batch run: they leave the state columns alone (the update is the fourth), and the stores use
-    // neither shared memory nor the tensor pipe.
-    const bool ckpt = it % p.cgs == 0;
-    const long ckc = stream_id * p.nck + it / p.cgs;
-    float* ckW1 = p.W1c + ckc * (64 * 256);
-    float* ckW2 = p.W2c + ckc * (256 * 64);
-    mbar_wait_bounded(&full[s], (it / kStages) & 1, abort_flag, limit);
-
-    // ---- MMA1: Z1^T = W1^T K^T
-    TTT_ISSUE(mma_hidden_half(tmem + TM_A, smem_u32(sW1), smem_u32(sK), false, false, 0),
-              mma_hidden_half(tmem + TM_A, smem_u32(sW1), smem_u32(sK), false, false, 1),
-              ,
-              )
-    if (ckpt) {
-      store_state_quarter(1, ckW1, ckW2);
-      store_state_quarter(3, ckW1, ckW2);
-      p.b1c[ckc * 256 + hrow] = b1v;
-      if (tid < 64) p.b2c[ckc * 64 + tid] = sB2[tid];     // before this mini-batch's column sums reach b2
-      // a warp's staging area reaches into the X2 rows its neighbour writes in EPI1: nobody goes on to EPI1
-      // before every warp is done with its area
-      __syncthreads();
-    }
-    wait_mma();
-    // ---- EPI1: X2^T = gelu(Z1^T + b1), G' = gelu'(Z1^T + b1)
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-      uint32_t v[32];
-      tmem_ld32(tmem + lane_base + TM_A + wg * 64 + half * 32, v);
-      tmem_wait_ld();
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float g[8], gp[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) gelu_pair(__uint_as_float(v[c * 8 + k]) + b1v, g[k], gp[k]);
-        st_chunk(sX2, hrow, half * 4 + c, g);
-        st_chunk(sGP, hrow, half * 4 + c, gp);
+  if (chain) {
+    // ================================================================================== chain group
+    reg_take<kRegsChain>();
+    const bool loader = gtid == 128;      // not the MMA issuer: its bookkeeping stays off the issue path
+    if (loader) {
+      for (; issued < kStages; ++issued) {
+        load_k(issued);
+        load_tile(issued, &tmV, OFF_V, BAR_V);
       }
     }
-    publish();
-
-    // ---- MMA2: Z2 = X2 W2
-    TTT_ISSUE(mma_token_major(tmem + TM_Z, smem_u32(sX2), smem_u32(sW2)),
-              ,
-              ,
-              )
-    if (ckpt) store_state_quarter(0, ckW1, ckW2);
-    wait_mma();
-    // ---- LN: fused LayerNorm + L2 gradient, U2 = -eta * dl/dZ2 (all 8 warps, 16 values each)
+    auto publish = [&]() {     // shared-memory writes and tensor-memory reads done -> the next MMA may be issued
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      named_bar_sync(kBarC, kGroup);
+    };
+    // ---- initial W1, b1: global fp32 -> tensor memory (master), shared memory (bf16 operand copy), checkpoint 0
+    float b1v = p.b1[stream_id * 256 + hrow];
     {
-      float xh[16], b2c[8], gam[8], bet[8];
-      tok_ld(tm, tmem + TM_Z, xh);
-      tok_ld_cols(tm, sB2, b2c);
-      tok_ld_cols(tm, sGamma, gam);
-      tok_ld_cols(tm, sBeta, bet);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        xh[4 * j] += b2c[2 * j]; xh[4 * j + 1] += b2c[2 * j + 1];
-        xh[4 * j + 2] += b2c[2 * j]; xh[4 * j + 3] += b2c[2 * j + 1];
-      }
-      float rs0, rs1;
-      float kk[16], vv[16], g[16];
-      tok_ld_tile(tm, sK, kk);          // requested before the all-reduces of the LayerNorm, used after them
-      tok_ld_tile(tm, sV, vv);
-      tok_layernorm(tm, xh, TTT_LN_EPS, sXch, rs0, rs1);
-      float a[2] = {0.f, 0.f}, b[2] = {0.f, 0.f};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i0 = 4 * j + e, i1 = 4 * j + 2 + e, c = 2 * j + e;
-          xh[i0] *= rs0;
-          xh[i1] *= rs1;
-          g[i0] = (fmaf(gam[c], xh[i0], bet[c]) - (vv[i0] - kk[i0])) * gam[c];
-          g[i1] = (fmaf(gam[c], xh[i1], bet[c]) - (vv[i1] - kk[i1])) * gam[c];
-          a[0] += g[i0]; a[1] = fmaf(g[i0], xh[i0], a[1]);
-          b[0] += g[i1]; b[1] = fmaf(g[i1], xh[i1], b[1]);
-        }
-      }
-      tok_row_allreduce<2, 2>(tm, a, b, sXch);
-      const float sc0 = -__bfloat162float(sEta[tm.r0]) * rs0 * (1.f / 64.f);
-      const float sc1 = -__bfloat162float(sEta[tm.r1]) * rs1 * (1.f / 64.f);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i0 = 4 * j + e, i1 = 4 * j + 2 + e;
-          g[i0] = (64.f * g[i0] - a[0] - xh[i0] * a[1]) * sc0;
-          g[i1] = (64.f * g[i1] - b[0] - xh[i1] * b[1]) * sc1;
-        }
-      }
-      tok_st_tile(tm, sU2, g);
-    }
-    publish();
-
-    // ---- MMA3: R^T = W2 U2^T
-    TTT_ISSUE(mma_hidden_half(tmem + TM_A, smem_u32(sW2), smem_u32(sU2), false, false, 0),
-              mma_hidden_half(tmem + TM_A, smem_u32(sW2), smem_u32(sU2), false, false, 1),
-              ,
-              )
-    // b2 += column sums of U2 (bf16 values, the operand the W2 update sees), fp32 accumulate: every
-    // thread sums 16 rows of one column while the MMA runs, threads 0..63 add the four parts
-    {
-      const int q = tid >> 6, f = tid & 63;
-      float acc = 0.f;
-#pragma unroll 8
-      for (int t = q * 16; t < q * 16 + 16; ++t) acc += ld_elem(sU2, t, f);
-      sXch[tid] = acc;     // the exchange buffer of the token-major epilogues is idle here
-      __syncthreads();
-      if (tid < 64) sB2[tid] += (sXch[tid] + sXch[64 + tid]) + (sXch[128 + tid] + sXch[192 + tid]);
-    }
-    if (ckpt) {
-      store_state_quarter(2, ckW1, ckW2);
-      tc_fence_before_sync();      // the state columns are written by the next MMA group
-    }
-    wait_mma();
-    // ---- EPI3: U1^T = R^T * G' (= -eta dl/dZ1), b1 += row sum
-    {
-      float bsum = 0.f;
+      const float* W1g = p.W1 + st_w + hrow;
+      float* W1k = p.W1c + stream_id * p.nck * (64 * 256) + hrow;
 #pragma unroll 1
       for (int half = 0; half < 2; ++half) {
         uint32_t v[32];
-        tmem_ld32(tmem + lane_base + TM_A + wg * 64 + half * 32, v);
-        const uint4 gr[4] = {ld_chunk_raw(sGP, hrow, half * 4), ld_chunk_raw(sGP, hrow, half * 4 + 1),
-                             ld_chunk_raw(sGP, hrow, half * 4 + 2), ld_chunk_raw(sGP, hrow, half * 4 + 3)};
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(W1g[(half * 32 + j) * 256]);
+        tmem_st32(tmem + lane_base + TM_W1 + wg * 64 + half * 32, v);
+        st_cols32_tmem(tmem + lane_base + TM_W1B + wg * 32 + half * 16, v);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) W1k[(half * 32 + j) * 256] = __uint_as_float(v[j]);
+      }
+      p.b1c[stream_id * p.nck * 256 + hrow] = b1v;
+      if (gtid < 64) p.b2c[stream_id * p.nck * 64 + gtid] = sB2[gtid];
+      tmem_wait_st();
+    }
+    publish();
+
+    uint32_t pa = 0;      // parity of the accumulator barriers: three uses per mini-batch
+    auto wait_acca = [&]() {
+      wait_bar(BAR_ACCA + wg, pa);
+      pa ^= 1u;
+      __syncwarp();
+      tc_fence_after_sync();
+    };
+    // The two 128-row blocks of a product are committed one by one: the warps of a block start when theirs is
+    // complete.
+    for (; it < NC; ++it) {
+      const int s = it & 1;
+      const uint8_t* sK = smem + OFF_K + s * TILE;
+      const uint8_t* sV = smem + OFF_V + s * TILE;
+      const __nv_bfloat16* sEta = reinterpret_cast<const __nv_bfloat16*>(smem + OFF_ETA + s * 128);
+      const uint32_t par = it & 1, prev = par ^ 1u;      // parity of this / the last mini-batch's hand-overs
+      wait_bar(BAR_K + s, it >> 1);
+
+      // ---- MMA1: Z1^T = W1^T K^T
+      if (cta_warp == 0) {
+        tc_fence_after_sync();
+#pragma unroll
+        for (int blk = 0; blk < 2; ++blk) {
+          mma_hidden_ta<false, false>(tmem + TM_A + blk * 64, tmem + TM_W1B + blk * 32, smem_u32(sK), lead);
+          if (lead) umma_commit(&bars[BAR_ACCA + blk]);
+        }
+      }
+      wait_acca();
+      // ---- EPI1: X2^T = gelu(Z1^T + b1) -> smem; G' = gelu'(Z1^T + b1) stays in registers (the thread that needs it
+      // in EPI3 is this one).  The next 16 columns are requested before these are processed.
+      uint32_t gp[32];
+      {
+        const f32x2 bb = pk1(b1v);
+        const uint32_t acc = tmem + lane_base + TM_A + wg * 64;
+        uint32_t v[2][16];
+        tmem_ld16(acc, v[0]);
         tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float gp[8];
-          unpack_chunk(gr[c], gp);
+        for (int q = 0; q < 4; ++q) {
+          if (q < 3) tmem_ld16(acc + q * 16 + 16, v[(q + 1) & 1]);
+          uint32_t g[8];
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
-            gp[k] *= __uint_as_float(v[c * 8 + k]);
-            bsum += gp[k];
+            f32x2 x, y;
+            gelu_pair2(add2(pk(v[q & 1][2 * k], v[q & 1][2 * k + 1]), bb), x, y);
+            g[k] = f32x2_to_bf16x2(x);
+            gp[q * 8 + k] = f32x2_to_bf16x2(y);
           }
-          st_chunk(sGP, hrow, half * 4 + c, gp);
+          *reinterpret_cast<uint4*>(sX2 + sw128_off(hrow, q * 2)) = make_uint4(g[0], g[1], g[2], g[3]);
+          *reinterpret_cast<uint4*>(sX2 + sw128_off(hrow, q * 2 + 1)) = make_uint4(g[4], g[5], g[6], g[7]);
+          tmem_wait_ld();
         }
       }
-      b1v += bsum;
-    }
-    publish();
+      publish();
 
-    // ---- MMA4: W1^T += U1^T K ;  W2 += X2^T U2
-    TTT_ISSUE(mma_hidden_half(tmem + TM_W1, smem_u32(sGP), smem_u32(sK), true, true, 0),
-              mma_hidden_half(tmem + TM_W1, smem_u32(sGP), smem_u32(sK), true, true, 1),
-              mma_hidden_half(tmem + TM_W2, smem_u32(sX2), smem_u32(sU2), true, true, 0),
-              mma_hidden_half(tmem + TM_W2, smem_u32(sX2), smem_u32(sU2), true, true, 1))
-    wait_mma();
-    // ---- EPI4: refresh the bf16 operand copies of the state
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-      uint32_t v[32];
-      float f[32];
-      tmem_ld32(tmem + lane_base + TM_W1 + wg * 64 + half * 32, v);
-      tmem_wait_ld();
+      // ---- MMA2: Z2 = X2 W2
+      wait_bar(BAR_W2RDY, par);                          // also b2, written with it
+      if (cta_warp == 0) {
+        __syncwarp();
+        tc_fence_after_sync();
+        mma_token_lead(tmem + TM_A, smem_u32(sX2), smem_u32(sW2), lead);
+        if (lead) umma_commit(&bars[BAR_Z]);
+      }
+      wait_bar(BAR_V + s, it >> 1);
+      wait_bar(BAR_Z, par);
+      __syncwarp();
+      tc_fence_after_sync();
+      // ---- LN: fused LayerNorm + L2 gradient, U2 = -eta * dl/dZ2 (all 8 warps, 16 values each)
+      {
+        float* xch = reinterpret_cast<float*>(smem + OFF_XCHC);
+        const float* b2 = sB2 + par * 64;
+        TokFrag x;
+        uint32_t kk[8], vv[8];
+        frag_ld(tm, tmem + TM_A, x);
+        frag_ld_raw(tm, sK, kk);         // requested before the all-reduces of the LayerNorm, used after them
+        frag_ld_raw(tm, sV, vv);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
+        for (int j = 0; j < 4; ++j) {
+          const f32x2 b = frag_col(tm, b2, j);
+          x.a[j] = add2(x.a[j], b);
+          x.b[j] = add2(x.b[j], b);
+        }
+        float rs0, rs1;
+        frag_layernorm(tm, x, TTT_LN_EPS, xch, kBarPairC, rs0, rs1);
+        TokFrag g;
+        f32x2 a0 = 0ull, a1 = 0ull, c0 = 0ull, c1 = 0ull;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) st_chunk(sW1, hrow, half * 4 + c, f + c * 8);
-      tmem_ld32(tmem + lane_base + TM_W2 + wg * 64 + half * 32, v);
-      tmem_wait_ld();
+        for (int j = 0; j < 4; ++j) {
+          const f32x2 gam = frag_col(tm, sGamma, j), bet = frag_col(tm, sBeta, j), neg = pk1(-1.f);
+          const f32x2 t0 = fma2(bf16x2_to_f32x2(vv[2 * j]), neg, bf16x2_to_f32x2(kk[2 * j]));          // K - V
+          const f32x2 t1 = fma2(bf16x2_to_f32x2(vv[2 * j + 1]), neg, bf16x2_to_f32x2(kk[2 * j + 1]));
+          g.a[j] = mul2(fma2(gam, x.a[j], add2(t0, bet)), gam);
+          g.b[j] = mul2(fma2(gam, x.b[j], add2(t1, bet)), gam);
+          a0 = add2(a0, g.a[j]); a1 = fma2(g.a[j], x.a[j], a1);
+          c0 = add2(c0, g.b[j]); c1 = fma2(g.b[j], x.b[j], c1);
+        }
+        float a[2] = {hsum(a0), hsum(a1)}, b[2] = {hsum(c0), hsum(c1)};
+        frag_allreduce2<1>(tm, a, b, xch, kBarPairC);
+        const f32x2 sc0 = pk1(-__bfloat162float(sEta[tm.r0]) * rs0 * (1.f / 64.f));
+        const f32x2 sc1 = pk1(-__bfloat162float(sEta[tm.r1]) * rs1 * (1.f / 64.f));
 #pragma unroll
-      for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) st_chunk(sW2, hrow, half * 4 + c, f + c * 8);
-    }
-    publish();
+        for (int j = 0; j < 4; ++j) {
+          g.a[j] = mul2(fma2(x.a[j], pk1(-a[1]), fma2(g.a[j], pk1(64.f), pk1(-a[0]))), sc0);
+          g.b[j] = mul2(fma2(x.b[j], pk1(-b[1]), fma2(g.b[j], pk1(64.f), pk1(-b[0]))), sc1);
+        }
+        frag_st_tile(tm, sU2, g);
+      }
+      publish();
 
-    // ---- MMA5: Z1b^T = W1^T Q^T
-    TTT_ISSUE(mma_hidden_half(tmem + TM_A, smem_u32(sW1), smem_u32(sQ), false, false, 0),
-              mma_hidden_half(tmem + TM_A, smem_u32(sW1), smem_u32(sQ), false, false, 1),
-              ,
-              )
-    wait_mma();
-    // ---- EPI5: X2b^T = gelu(Z1b^T + b1)
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-      uint32_t v[32];
-      tmem_ld32(tmem + lane_base + TM_A + wg * 64 + half * 32, v);
-      tmem_wait_ld();
+      // ---- MMA3: R^T = W2 U2^T
+      if (cta_warp == 0) {
+        tc_fence_after_sync();
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float g[8];
+        for (int blk = 0; blk < 2; ++blk) {
+          mma_hidden_lead<false, false>(tmem + TM_A, smem_u32(sW2), smem_u32(sU2), blk, lead);
+          if (lead) umma_commit(&bars[BAR_ACCA + blk]);
+        }
+      }
+      if (loader) load_tile(it + kStages, &tmV, OFF_V, BAR_V);      // V has been read
+      wait_acca();
+      // ---- EPI3: U1^T = R^T * G' (= -eta dl/dZ1), as bf16 over R in tensor memory; b1 += row sum
+      {
+        f32x2 bsum = 0ull;
+        const uint32_t acc = tmem + lane_base + TM_A + wg * 64;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) g[k] = gelu_only(__uint_as_float(v[c * 8 + k]) + b1v);
-        st_chunk(sX2, hrow, half * 4 + c, g);
+        for (int half = 0; half < 2; ++half) {
+          uint32_t v[32], u[16];
+          tmem_ld32(acc + half * 32, v);
+          tmem_wait_ld();
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            const f32x2 w = mul2(bf16x2_to_f32x2(gp[half * 16 + k]), pk(v[2 * k], v[2 * k + 1]));
+            bsum = add2(bsum, w);
+            u[k] = f32x2_to_bf16x2(w);
+          }
+          tmem_st16(acc + half * 16, u);
+        }
+        b1v += hsum(bsum);
+        sB1[prev * 256 + hrow] = b1v;      // b1 after this mini-batch
+        tmem_wait_st();
+      }
+      publish();
+
+      // ---- MMA4: W1^T += U1^T K ;  W2 += X2^T U2
+      if (cta_warp == 0) {
+        if (it > 0) wait_bar(BAR_SREAD, prev);
+        __syncwarp();
+        tc_fence_after_sync();
+#pragma unroll
+        for (int blk = 0; blk < 2; ++blk) {
+          mma_hidden_ta<true, true>(tmem + TM_W1 + blk * 64, tmem + TM_A + blk * 64, smem_u32(sK), lead);
+          if (lead) umma_commit(&bars[BAR_ACCA + blk]);
+        }
+        mma_hidden_lead<true, true>(tmem + TM_W2, smem_u32(sX2), smem_u32(sU2), 0, lead);
+        mma_hidden_lead<true, true>(tmem + TM_W2, smem_u32(sX2), smem_u32(sU2), 1, lead);
+        if (lead) umma_commit(&bars[BAR_W2UPD]);
+      }
+      if (it > 0) wait_bar(BAR_ACCB, 1);              // the last mini-batch's MMA5 has read the bf16 W1 (second use)
+      wait_acca();
+      // ---- EPI4: bf16 operand copy of the new W1
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t v[32];
+        tmem_ld32(tmem + lane_base + TM_W1 + wg * 64 + half * 32, v);
+        tmem_wait_ld();
+        st_cols32_tmem(tmem + lane_base + TM_W1B + wg * 32 + half * 16, v);
+      }
+      tmem_wait_st();
+      tc_fence_before_sync();
+      const bool stop = named_bar_or(kBarC, kGroup, *abort_flag != 0);
+      if (gtid == 0) mbar_arrive(&bars[BAR_W1RDY]);
+      if (stop) break;
+      if (loader) {          // MMA4 has read K
+        load_k(it + kStages);
+        issued = it + kStages + 1;
       }
     }
-    // the Out tile stored earlier has long left shared memory: confirmed here, off the critical path,
-    // before the barrier after which the tile is written again
-    if (tid == kProd) tma_wait_group_read<0>();
-    publish();
-
-    // ---- MMA6: Z2b = X2b W2
-    TTT_ISSUE(mma_token_major(tmem + TM_Z, smem_u32(sX2), smem_u32(sW2)),
-              ,
-              ,
-              )
-    wait_mma();
-    // ---- OUT: Q + gamma * LN(Z2b + b2) + beta
+    if (loader && *abort_flag) {
+      drain_loads(BAR_K, issued);
+      drain_loads(BAR_V, it + kStages + 1);
+    }
+  } else {
+    // ================================================================================= output group
+    reg_give<kRegsOut>();
+    const bool loader = gtid == 128;
+    if (loader)
+      for (; issued < kStages; ++issued) load_tile(issued, &tmQ, OFF_Q, BAR_Q);
+    auto publish = [&]() {
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      named_bar_sync(kBarO, kGroup);
+    };
+    uint8_t* stage = smem + OFF_STG + warp * 4096;
+    // ---- initial W2: global fp32 -> tensor memory (master), shared memory (bf16 operand copy), checkpoint 0
     {
-      float z[16], b2c[8], gam[8], bet[8], q[16];
-      tok_ld(tm, tmem + TM_Z, z);
-      tok_ld_cols(tm, sB2, b2c);
-      tok_ld_cols(tm, sGamma, gam);
-      tok_ld_cols(tm, sBeta, bet);
+      const float4* W2g = reinterpret_cast<const float4*>(p.W2 + st_w + hrow * 64);
+      float* W2k = p.W2c + stream_id * p.nck * (64 * 256) + (hrow - lane) * 64;
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        uint32_t v[32];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        z[4 * j] += b2c[2 * j]; z[4 * j + 1] += b2c[2 * j + 1];
-        z[4 * j + 2] += b2c[2 * j]; z[4 * j + 3] += b2c[2 * j + 1];
-      }
-      float rs0, rs1;
-      tok_ld_tile(tm, sQ, q);           // requested before the all-reduces of the LayerNorm, used after them
-      tok_layernorm(tm, z, TTT_LN_EPS, sXch, rs0, rs1);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i0 = 4 * j + e, i1 = 4 * j + 2 + e, c = 2 * j + e;
-          q[i0] += fmaf(gam[c], z[i0] * rs0, bet[c]);
-          q[i1] += fmaf(gam[c], z[i1] * rs1, bet[c]);
+        for (int j = 0; j < 8; ++j) {
+          const float4 q4 = W2g[half * 8 + j];
+          v[4 * j] = __float_as_uint(q4.x); v[4 * j + 1] = __float_as_uint(q4.y);
+          v[4 * j + 2] = __float_as_uint(q4.z); v[4 * j + 3] = __float_as_uint(q4.w);
         }
+        tmem_st32(tmem + lane_base + TM_W2 + wg * 64 + half * 32, v);
+        st_cols32(sW2, hrow, half, v);
+        store_rows_own(W2k + half * 32, v, stage, lane);
       }
-      tok_st_tile(tm, sOut, q);
+      tmem_wait_st();
     }
     publish();
-    if (tid == kProd) {
-      tma_store_2d(&tmOut, sOut, 0, static_cast<int>((stream_id * NC + it) * 64));
-      tma_commit_group();
-      if (!*abort_flag && loads_issued < NC && loads_issued == it + kStages) {
-        issue_loads(loads_issued);
-        ++loads_issued;
+    if (gtid < 3) mbar_arrive(&bars[BAR_W2RDY]);
+
+    for (; it < NC; ++it) {
+      const int s = it & 1;
+      uint8_t* sQ = smem + OFF_Q + s * TILE;
+      const uint32_t par = it & 1, next = par ^ 1u;
+      wait_bar(BAR_W2UPD, par);
+      __syncwarp();
+      tc_fence_after_sync();
+      // ---- b2 += column sums of U2 (bf16 values, the operand the W2 update sees), fp32 accumulate: a thread
+      // sums 8 rows of a column pair, threads 0..63 add the eight parts.  bf16 operand copy of the new W2.
+      float* part = reinterpret_cast<float*>(smem + OFF_XCHO);
+      {
+        const int pr = gtid & 31;
+        f32x2 acc = 0ull;
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+          acc = add2(acc, bf16x2_to_f32x2(*reinterpret_cast<const uint32_t*>(
+                              sU2 + sw128_off(warp * 8 + r, pr >> 2) + (pr & 3) * 4)));
+        *reinterpret_cast<f32x2*>(part + warp * 64 + 2 * pr) = acc;
       }
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        uint32_t v[32];
+        tmem_ld32(tmem + lane_base + TM_W2 + wg * 64 + half * 32, v);
+        tmem_wait_ld();
+        st_cols32(sW2, hrow, half, v);
+      }
+      publish();
+      if (gtid == 128) mbar_arrive(&bars[BAR_W2RDY]);
+      if (gtid < 64) {
+        float b = sB2[par * 64 + gtid];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) b += part[k * 64 + gtid];
+        sB2[next * 64 + gtid] = b;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[BAR_W2RDY]);
+      }
+      wait_bar(BAR_W1RDY, par);
+      __syncwarp();
+      // ---- the state after this mini-batch is a checkpoint if the next one starts a group
+      if (it + 1 < NC && (it + 1) % p.cgs == 0) {
+        const long ckc = stream_id * p.nck + (it + 1) / p.cgs;
+        float* W1k = p.W1c + ckc * (64 * 256) + hrow;
+        float* W2k = p.W2c + ckc * (256 * 64) + (hrow - lane) * 64;
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+          uint32_t v[32];
+          tmem_ld32(tmem + lane_base + TM_W1 + wg * 64 + half * 32, v);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) W1k[(half * 32 + j) * 256] = __uint_as_float(v[j]);
+          tmem_ld32(tmem + lane_base + TM_W2 + wg * 64 + half * 32, v);
+          tmem_wait_ld();
+          store_rows_own(W2k + half * 32, v, stage, lane);
+        }
+        p.b1c[ckc * 256 + hrow] = sB1[next * 256 + hrow];
+        if (gtid < 64) p.b2c[ckc * 64 + gtid] = sB2[next * 64 + gtid];
+      }
+      tc_fence_before_sync();
+      if (lane == 0) mbar_arrive(&bars[BAR_SREAD]);
+      if (loader && it > 0) {      // the last Out tile has left its stage: Q of the next mini-batch comes in
+        tma_wait_group_read<0>();
+        load_tile(it + 1, &tmQ, OFF_Q, BAR_Q);
+        issued = it + 2;
+      }
+      wait_bar(BAR_Q + s, it >> 1);
+
+      // ---- MMA5, EPI5: X2b^T = gelu(W1^T Q^T + b1), one 128-row block after the other; the two warps of a quadrant
+      // take 32 tokens each.  (Holding EPI5 back until the next mini-batch's EPI1, with which it shares the fp32 and
+      // MUFU pipes, has led to MMA2 was 1.5 % slower: it then meets the LayerNorm.)
+      auto issue_mma5 = [&](int blk) {
+        tc_fence_after_sync();
+        mma_hidden_ta<false, false>(tmem + TM_B, tmem + TM_W1B + blk * 32, smem_u32(sQ), lead);
+        if (lead) umma_commit(&bars[BAR_ACCB]);
+      };
+      __syncwarp();
+      if (warp == 0) issue_mma5(0);
+#pragma unroll
+      for (int blk = 0; blk < 2; ++blk) {
+        const int row = blk * 128 + quad * 32 + lane;
+        const f32x2 bb = pk1(0.5f * sB1[next * 256 + row]);
+        wait_bar(BAR_ACCB, blk);
+        __syncwarp();
+        tc_fence_after_sync();
+        uint32_t v[32];
+        tmem_ld32(tmem + lane_base + TM_B + wg * 32, v);
+        tmem_wait_ld();
+        if (blk == 0) {
+          tc_fence_before_sync();
+          named_bar_sync(kBarO, kGroup);       // the accumulator has been read
+          if (warp == 0) issue_mma5(1);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t g[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            g[k] = f32x2_to_bf16x2(gelu_half2(fma2(pk(v[c * 8 + 2 * k], v[c * 8 + 2 * k + 1]), pk1(0.5f), bb)));
+          *reinterpret_cast<uint4*>(sX2b + sw128_off(row, wg * 4 + c)) = make_uint4(g[0], g[1], g[2], g[3]);
+        }
+      }
+      publish();
+
+      // ---- MMA6: Z2b = X2b W2
+      if (warp == 0) {
+        tc_fence_after_sync();
+        mma_token_lead(tmem + TM_B, smem_u32(sX2b), smem_u32(sW2), lead);
+        if (lead) umma_commit(&bars[BAR_ZB]);
+      }
+      wait_bar(BAR_ZB, par);
+      __syncwarp();
+      tc_fence_after_sync();
+      // ---- OUT: Q + gamma * LN(Z2b + b2) + beta, over the Q tile (every thread rewrites what it has read)
+      {
+        TokFrag x;
+        uint32_t q[8];
+        frag_ld(tm, tmem + TM_B, x);
+        frag_ld_raw(tm, sQ, q);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const f32x2 b = frag_col(tm, sB2 + next * 64, j);
+          x.a[j] = add2(x.a[j], b);
+          x.b[j] = add2(x.b[j], b);
+        }
+        float rs0, rs1;
+        frag_layernorm(tm, x, TTT_LN_EPS, part, kBarPairO, rs0, rs1);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const f32x2 gam = frag_col(tm, sGamma, j), bet = frag_col(tm, sBeta, j);
+          x.a[j] = add2(bf16x2_to_f32x2(q[2 * j]), fma2(gam, x.a[j], bet));
+          x.b[j] = add2(bf16x2_to_f32x2(q[2 * j + 1]), fma2(gam, x.b[j], bet));
+        }
+        frag_st_tile(tm, sQ, x);
+      }
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      const bool stop = named_bar_or(kBarO, kGroup, *abort_flag != 0);
+      if (loader) {
+        tma_store_2d(&tmOut, sQ, 0, row_of(it));
+        tma_commit_group();
+      }
+      if (stop) break;
     }
-    if (*abort_flag) break;
+    if (loader) {
+      if (*abort_flag) drain_loads(BAR_Q, issued);
+      tma_wait_group<0>();
+    }
   }
 
   // ---- epilogue: optional final state, then teardown
-  const bool aborted = *abort_flag != 0;
+  tc_fence_before_sync();
+  const bool aborted = __syncthreads_or(*abort_flag != 0) != 0;
+  tc_fence_after_sync();
   if (!aborted && p.W1f != nullptr) {
-    store_state(p.W1f + stream_id * (64 * 256), p.b1f + stream_id * 256, p.W2f + stream_id * (256 * 64),
-                p.b2f + stream_id * 64);
+    uint32_t v[32];
+    if (chain) {
+      float* W1o = p.W1f + st_w + hrow;
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        tmem_ld32(tmem + lane_base + TM_W1 + wg * 64 + half * 32, v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) W1o[(half * 32 + j) * 256] = __uint_as_float(v[j]);
+      }
+      p.b1f[stream_id * 256 + hrow] = sB1[(NC & 1) * 256 + hrow];
+      if (gtid < 64) p.b2f[stream_id * 64 + gtid] = sB2[(NC & 1) * 64 + gtid];
+    } else {
+      float* W2o = p.W2f + st_w + (hrow - lane) * 64;
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        tmem_ld32(tmem + lane_base + TM_W2 + wg * 64 + half * 32, v);
+        tmem_wait_ld();
+        store_rows_own(W2o + half * 32, v, smem + OFF_STG + warp * 4096, lane);
+      }
+    }
   }
   if (aborted) {
     // everything this CTA still has in flight is waited for (bounded, not cut short by the abort flag)
-    // before its shared and tensor memory go away: the tensor-core work of the four issuers ...
-    if (warp < 4) {
-      if (elect_one()) umma_commit(drain_bar);
-      __syncwarp();
-    }
-    if (tid == kProd) {
-      mbar_wait_bounded(drain_bar, 0, never_flag, limit);
-      // ... and its own loads
-      for (int j = it; j < loads_issued; ++j) {
-        if (j == p.drop_load && stream_id == 0) continue;
-        mbar_wait_bounded(&full[j % kStages], (j / kStages) & 1, never_flag, limit);
-      }
+    // before its shared and tensor memory go away: the loads above, and the tensor-core work of both issuers
+    if (warp == 0 && lead) umma_commit(&bars[BAR_DRAIN]);
+    if (tid == 0) {
+      mbar_wait_bounded(&bars[BAR_DRAIN], 0, never_flag, limit);
       atomicExch(p.status, static_cast<uint32_t>(TTT_B200_ERR_TIMEOUT));
     }
   }
-  if (tid == kProd) tma_wait_group<0>();
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, TM_COLS);
+  if (cta_warp == 0) tmem_dealloc(tmem, TM_COLS);
 }
 
 }  // namespace
