@@ -52,10 +52,6 @@ def build(force=False, verbose=False):
     return LIB_PATH
 
 
-if __name__ == "__main__":
-    print(build(force="--force" in sys.argv, verbose=True))
-
-
 # ---------------------------------------------------------------------------------------------
 # The PyTorch extension module `test_time_training` (the reference's module name): a C++ shim
 # over the C ABI, built in-tree next to the library it links against.
@@ -63,16 +59,23 @@ EXT_NAME = "test_time_training"
 EXT_SOURCE = os.path.join(CSRC, "test_time_training.cpp")
 
 
-def extension_path():
+HOST_NAME = "_ttt_host"                      # validation and launch for ttt_tk_b200.ops
+HOST_SOURCE = os.path.join(CSRC, "ttt_host.cpp")
+
+
+def _module_path(name):
     import sysconfig
-    return os.path.join(LIB_DIR, EXT_NAME + sysconfig.get_config_var("EXT_SUFFIX"))
+    return os.path.join(LIB_DIR, name + sysconfig.get_config_var("EXT_SUFFIX"))
 
 
-def build_extension(force=False, verbose=False):
-    """Compile ttt_tk_b200/lib/test_time_training*.so with g++ against the installed torch."""
+def extension_path():
+    return _module_path(EXT_NAME)
+
+
+def _build_torch_module(name, source, out, force, verbose):
+    """Compile one C++ module against the installed torch and the C-ABI library, with g++, in-tree."""
     build(force=False, verbose=verbose)
-    out = extension_path()
-    deps = [EXT_SOURCE, os.path.join(CSRC, "..", "..", "include", "ttt_mlp_b200.h")]
+    deps = [source, os.path.join(CSRC, "..", "..", "include", "ttt_mlp_b200.h")]
     if not force and os.path.exists(out) and all(os.path.getmtime(d) <= os.path.getmtime(out) for d in deps):
         return out
     import sysconfig
@@ -84,28 +87,51 @@ def build_extension(force=False, verbose=False):
         else ce.library_paths(cuda=True)
     cxx = os.environ.get("CXX", "g++")
     cmd = [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-w",
-           f"-DTORCH_EXTENSION_NAME={EXT_NAME}", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f"-DTORCH_EXTENSION_NAME={name}", "-DTORCH_API_INCLUDE_EXTENSION_H",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            "-I" + sysconfig.get_path("include")]
     cmd += ["-I" + p for p in inc]
-    cmd += [EXT_SOURCE, "-o", out, "-L" + LIB_DIR, "-lttt_mlp_b200", "-Wl,-rpath,$ORIGIN"]
+    cmd += [source, "-o", out, "-L" + LIB_DIR, "-lttt_mlp_b200", "-Wl,-rpath,$ORIGIN"]
     cmd += ["-L" + p for p in libdirs] + ["-Wl,-rpath," + p for p in libdirs if "torch" in p]
     cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-lcudart"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or res.returncode != 0:
         sys.stderr.write(" ".join(cmd) + "\n" + res.stdout + res.stderr)
     if res.returncode != 0:
-        raise RuntimeError("building the test_time_training extension failed")
+        raise RuntimeError(f"building the {name} extension failed")
     return out
+
+
+def build_extension(force=False, verbose=False):
+    """Compile ttt_tk_b200/lib/test_time_training*.so and ttt_tk_b200/lib/_ttt_host*.so."""
+    _build_torch_module(HOST_NAME, HOST_SOURCE, _module_path(HOST_NAME), force, verbose)
+    return _build_torch_module(EXT_NAME, EXT_SOURCE, extension_path(), force, verbose)
+
+
+def _load(name, path):
+    import importlib.util
+    import torch  # noqa: F401  (libtorch must be loaded before the extension)
+    spec = importlib.util.spec_from_file_location(name, path)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod
 
 
 def load_extension():
     """Import and return the `test_time_training` module (building it if needed)."""
-    import importlib.util
-    import torch  # noqa: F401  (libtorch must be loaded before the extension)
-    path = build_extension()
-    spec = importlib.util.spec_from_file_location(EXT_NAME, path)
-    mod = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(mod)
+    mod = _load(EXT_NAME, build_extension())
     sys.modules.setdefault(EXT_NAME, mod)
     return mod
+
+
+def load_host():
+    """Import and return the operators' native host side (building it if it is missing)."""
+    path = _module_path(HOST_NAME)
+    if not os.path.exists(path):
+        _build_torch_module(HOST_NAME, HOST_SOURCE, path, False, False)
+    return _load(HOST_NAME, path)
+
+
+if __name__ == "__main__":
+    print(build(force="--force" in sys.argv, verbose=True))
+    print(build_extension())
