@@ -11,7 +11,6 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <initializer_list>
-#include <sstream>
 #include <stdexcept>
 #include <string>
 
@@ -25,11 +24,9 @@ constexpr at::ScalarType kBf = at::kBFloat16, kF32 = at::kFloat;
 [[noreturn]] void fail(const std::string& msg) { throw std::runtime_error(msg); }
 
 std::string shape_text(at::IntArrayRef s) {
-  std::ostringstream o;
-  o << '(';
-  for (size_t i = 0; i < s.size(); ++i) o << (i ? ", " : "") << s[i];
-  o << (s.size() == 1 ? ",)" : ")");
-  return o.str();
+  std::string o = "(";
+  for (size_t i = 0; i < s.size(); ++i) o += (i ? ", " : "") + std::to_string(s[i]);
+  return o + (s.size() == 1 ? ",)" : ")");
 }
 
 const char* dtype_text(at::ScalarType t) {
