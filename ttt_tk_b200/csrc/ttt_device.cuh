@@ -356,6 +356,54 @@ __device__ __forceinline__ void store_rows_coalesced(float* dst, int ld, const u
 }
 constexpr uint32_t kRowStageBytes = 32 * 144;     // per warp
 
+// ---- 64 x 64 x 64 products on M = 64 accumulators, issued likewise.  A is a [64][64] tile read K-major (row = M index),
+// B one read K-major (row = N index) or MN-major (row = contraction index).
+template <bool kBMn, bool kAccumulate>
+__device__ __forceinline__ void mma_64_lead(uint32_t tmem_d, uint32_t a_smem, uint32_t b_smem, uint32_t lead) {
+  constexpr uint32_t idesc = umma_idesc_bf16(64, 64, false, kBMn, false);
+  const uint32_t a0 = desc_lo(a_smem, 16);
+  const uint32_t b0 = desc_lo(b_smem, kBMn ? 8192 : 16);
+  constexpr uint32_t bstep = kBMn ? (2048u >> 4) : (32u >> 4);
+  mma_lead<kAccumulate>(tmem_d, a0, b0, idesc, lead);
+#pragma unroll
+  for (int j = 1; j < 4; ++j) mma_lead<true>(tmem_d, a0 + j * 2, b0 + j * bstep, idesc, lead);
+}
+// D += A^T B, both tiles read MN-major (row = contraction index)
+__device__ __forceinline__ void mma_64_tn_lead(uint32_t tmem_d, uint32_t a_smem, uint32_t b_smem, uint32_t lead) {
+  constexpr uint32_t idesc = umma_idesc_bf16(64, 64, true, true, false);
+  const uint32_t a0 = desc_lo(a_smem, TILE);
+  const uint32_t b0 = desc_lo(b_smem, TILE);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) mma_lead<true>(tmem_d, a0 + j * (2048u >> 4), b0 + j * (2048u >> 4), idesc, lead);
+}
+// column sums of a [64 tok][64] tile: D[64 feat x 8] = T^T * ones (8 rows of bf16 ones)
+__device__ __forceinline__ void mma_colsum_lead(uint32_t tmem_d, uint32_t tile_smem, uint32_t ones_smem, uint32_t lead) {
+  constexpr uint32_t idesc = umma_idesc_bf16(64, 8, true, false, false);
+  const uint32_t a0 = desc_lo(tile_smem, TILE);
+  const uint32_t b0 = desc_lo(ones_smem, 16);
+  mma_lead<false>(tmem_d, a0, b0, idesc, lead);
+#pragma unroll
+  for (int j = 1; j < 4; ++j) mma_lead<true>(tmem_d, a0 + j * (2048u >> 4), b0 + j * (32u >> 4), idesc, lead);
+}
+
+// A warp's 32 rows x 32 fp32 columns (lane = row) -> a row-major global matrix with 64 floats per row, as whole
+// 128-byte lines, turned through the warp's own 4 KB of a hidden-major tile (16-byte chunks XOR-swizzled by row:
+// both directions conflict-free).
+__device__ __forceinline__ void store_rows_own(float* dst, const uint32_t (&v)[32], uint8_t* stage, int lane) {
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    *reinterpret_cast<uint4*>(stage + sw128_off(lane, c)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = 4 * i + (lane >> 3), ch = lane & 7;
+    *reinterpret_cast<uint4*>(dst + r * 64 + ch * 4) = *reinterpret_cast<const uint4*>(stage + sw128_off(r, ch));
+  }
+  __syncwarp();
+}
+
+
 // ---- Token-major 64 x 64 accumulators spread over 8 warps (256 threads).
 // A token-major accumulator (M = 64) keeps row r in TMEM lane (r % 16) + 32 * (r / 16): quadrant q
 // holds rows 16q .. 16q+15 in its first 16 lanes.  The two warps that may touch quadrant q (q and
@@ -579,6 +627,87 @@ __device__ __forceinline__ void frag_layernorm(const TokMap& m, TokFrag& f, floa
     f.a[j] = mul2(add2(f.a[j], pk1(-m0)), pk1(rs0));
     f.b[j] = mul2(add2(f.b[j], pk1(-m1)), pk1(rs1));
   }
+}
+
+// Column sums of fragments over a warp's 16 rows: v[2j], v[2j + 1] hold this lane's sums over its own rows for the
+// column pair j.  The eight lanes that share a pair halve the set at every exchange, so that seven shuffles leave every
+// lane with the total of one column: col(2 * bit4 + bit3 of the lane) + bit2.
+__device__ __forceinline__ float frag_colsum(const f32x2 (&v)[4], int lane) {
+  float k[8];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) upk(v[j], k[2 * j], k[2 * j + 1]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const bool up = lane & 16;
+    const float send = up ? k[i] : k[4 + i], keep = up ? k[4 + i] : k[i];
+    k[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const bool up = lane & 8;
+    const float send = up ? k[i] : k[2 + i], keep = up ? k[2 + i] : k[i];
+    k[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+  }
+  const bool up = lane & 4;
+  return (up ? k[1] : k[0]) + __shfl_xor_sync(0xffffffffu, up ? k[0] : k[1], 4);
+}
+__device__ __forceinline__ int frag_colsum_col(const TokMap& m, int lane) {
+  return m.colhalf * 32 + (lane >> 3) * 8 + m.l3 * 2 + ((lane >> 2) & 1);
+}
+
+// ---- A 64 x 64 token-major accumulator over 16 warps: the four warps of a quadrant take 16 columns each, every
+// thread holds 8 values: column pairs j = 0, 1 (col(j) = 16 cq + 8 j + 2 (lane % 4)) of rows r0 and r1.
+struct TokMap16 {
+  int quad, cq, l3, r0, r1;
+  uint32_t taddr;
+  __device__ __forceinline__ TokMap16(int warp, int lane)
+      : quad(warp & 3), cq(warp >> 2), l3(lane & 3), r0((warp & 3) * 16 + (lane >> 2)), r1((warp & 3) * 16 + (lane >> 2) + 8),
+        taddr((static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>((warp >> 2) * 16)) {}
+  __device__ __forceinline__ int col(int j) const { return cq * 16 + j * 8 + l3 * 2; }
+  __device__ __forceinline__ uint32_t off(int r, int j) const { return sw128_off(r, cq * 2 + j) + l3 * 4; }
+};
+struct Frag16 {
+  f32x2 a[2], b[2];
+};
+__device__ __forceinline__ void frag_set(Frag16& f, const uint32_t (&u)[8]) {
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    f.a[j] = pk(u[4 * j], u[4 * j + 1]);
+    f.b[j] = pk(u[4 * j + 2], u[4 * j + 3]);
+  }
+}
+__device__ __forceinline__ void frag_ld_raw(const TokMap16& m, const uint8_t* tile, uint32_t (&w)[4]) {
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    w[2 * j] = *reinterpret_cast<const uint32_t*>(tile + m.off(m.r0, j));
+    w[2 * j + 1] = *reinterpret_cast<const uint32_t*>(tile + m.off(m.r1, j));
+  }
+}
+__device__ __forceinline__ void frag_st_tile(const TokMap16& m, uint8_t* tile, const Frag16& f) {
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    *reinterpret_cast<uint32_t*>(tile + m.off(m.r0, j)) = f32x2_to_bf16x2(f.a[j]);
+    *reinterpret_cast<uint32_t*>(tile + m.off(m.r1, j)) = f32x2_to_bf16x2(f.b[j]);
+  }
+}
+// column sums over the warp's 16 rows, as frag_colsum: four shuffles, the total of column col(bit4) + bit3 of the lane
+// (the lanes that differ in bit 2 hold the same)
+__device__ __forceinline__ float frag_colsum(f32x2 v0, f32x2 v1, int lane) {
+  float k[4];
+  upk(v0, k[0], k[1]);
+  upk(v1, k[2], k[3]);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const bool up = lane & 16;
+    const float send = up ? k[i] : k[2 + i], keep = up ? k[2 + i] : k[i];
+    k[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+  const bool up = lane & 8;
+  float r = (up ? k[1] : k[0]) + __shfl_xor_sync(0xffffffffu, up ? k[0] : k[1], 8);
+  return r + __shfl_xor_sync(0xffffffffu, r, 4);
+}
+__device__ __forceinline__ int frag_colsum_col(const TokMap16& m, int lane) {
+  return m.cq * 16 + (lane >> 4) * 8 + m.l3 * 2 + ((lane >> 3) & 1);
 }
 
 }  // namespace tttdev

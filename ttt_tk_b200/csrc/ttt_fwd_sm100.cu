@@ -128,23 +128,6 @@ struct FwdParams {
   uint64_t wait_limit_ns;
 };
 
-// A warp's 32 rows x 32 fp32 columns (lane = row) -> a row-major global matrix with 64 floats per row, as whole
-// 128-byte lines, turned through the warp's own 4 KB of a hidden-major tile (16-byte chunks XOR-swizzled by row:
-// both directions conflict-free).
-__device__ __forceinline__ void store_rows_own(float* dst, const uint32_t (&v)[32], uint8_t* stage, int lane) {
-  __syncwarp();
-#pragma unroll
-  for (int c = 0; c < 8; ++c)
-    *reinterpret_cast<uint4*>(stage + sw128_off(lane, c)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = 4 * i + (lane >> 3), ch = lane & 7;
-    *reinterpret_cast<uint4*>(dst + r * 64 + ch * 4) = *reinterpret_cast<const uint4*>(stage + sw128_off(r, ch));
-  }
-  __syncwarp();
-}
-
 // the four 16-byte chunks of 32 fp32 accumulator columns as bf16, to row `row` of a swizzled tile
 __device__ __forceinline__ void st_cols32(uint8_t* tile, int row, int half, const uint32_t (&v)[32]) {
 #pragma unroll

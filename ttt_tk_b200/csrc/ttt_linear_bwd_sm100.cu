@@ -1,31 +1,37 @@
 // TTT-Linear backward for sm_100a: gradients of the TTT-Linear forward (ttt_linear_fwd_sm100.cu) from its
-// checkpoints, one persistent CTA of 256 threads per (batch, head) stream.
+// checkpoints, one persistent CTA of 16 warps per (batch, head) stream.
 //
 // The reference has no counterpart (it ships the TTT-MLP operator only, README.md:18); the structure is its
 // backward's (kernels/ttt_backward/ttt.cu:453-1424, math kernels/ttt_backward/matching.py:173-342) with the
 // hidden layer removed: per checkpoint group, last to first, recompute the group's mini-batches from the
 // checkpoint, keeping what the reverse sweep needs in the caller's scratch buffer, then sweep the group in
 // reverse.  Every tile is 64 x 64: token-major tiles and the 64 x 64 state alike are M = 64 accumulators read
-// with the 16x256b fragments of TokMap by all eight warps.  The state W^T and the gradient state
-// G^T = (dL/dW)^T live side by side in tensor memory as the accumulators of their own update MMAs (the MLP
-// kernel has to park one of them: here both fit), b and dL/db in shared memory.
+// with the 16x256b fragments of TokMap by eight warps.  The state W^T and the gradient state
+// G^T = (dL/dW)^T live side by side in tensor memory as the accumulators of their own update MMAs, b and dL/db in
+// shared memory.
 //
-// Recompute of mini-batch j (3 MMA phases, the forward's):
-//   Z = K W;  x_f = LN(Z + b), e = gamma x_f + beta - (V - K), gZ = LNbwd(e gamma), U = -eta gZ;
-//   W^T += U^T K, b += colsum U;  Zb = Q W+;  x_ln = LN(Zb + b+)
-//   slot j of the scratch buffer <- bf16 W^T before the update, x_f, gZ, x_ln (raw images of the swizzled
-//   shared-memory tiles, stored and read back with bulk copies), 1/std of both LayerNorms.
-// Reverse step of mini-batch j (3 MMA phases), with go = dL/dOut and the state after j's update W+ = the
-// pre-update state of j + 1 (or the group's last state):
-//   S4   gZb = LNbwd(go gamma; x_ln);  d_beta += colsum go;  d_gamma += colsum go x_ln;  G_b += colsum gZb
-//   A    dQ = go + gZb W+^T;  G^T += gZb^T Q
-//   B    A1 = -eta (K G + G_b);  T1 = gZ G^T;  d_eta = -rowsum(T1 K) - rowsum(G_b gZ)
-//   E4   second order through the fused LayerNorm + L2 gradient: Bt, d_gamma, d_beta, dV = -gamma Bt,
-//        gZin (the formulas of the MLP kernel's E4 with A1 in the place of A2 and gZ in the place of dl/dZ2)
-//   C    dK = gamma Bt - eta T1 + gZin W^T;  G^T += gZin^T K;  G_b += colsum gZin
-// All waits are bounded; on expiry the CTA reports through the status word, drains its own copies, frees its
-// tensor memory and returns.
-#include <cstdlib>
+// The recompute of one group does not depend on the sweep of another, so the two run side by side: eight warps
+// recompute group g - 1 while the other eight sweep group g, each a chain of short MMA -> epilogue round trips that
+// alone would leave the SM idle most of the time.  One slot of scratch per mini-batch of a group is enough for both:
+// the sweep frees the slots of its group from the last mini-batch to the first, so every other group numbers its
+// slots backwards and the recompute fills them in the order in which they become free.
+//
+//   recompute of mini-batch j                              reverse step of mini-batch j, go = dL/dOut
+//   MMA1  Z = K W                                          P1  dK(j+1) += gZin W^T;  G^T += gZin^T K   (of step j + 1)
+//   LN    x_f = LN(Z + b), e = gamma x_f + beta - (V - K)      G^T += gZb^T Q;  G_b += column sums of gZb
+//         gZ = LNbwd(e gamma), U = -eta gZ                 E2  bf16 copy of G^T
+//   MMA2  W^T += U^T K, b += colsum U                      P2  K G, T1 = gZ G^T
+//   EPI   bf16 copy of W+^T                                E4  A1 = -eta (K G + G_b), second order through the fused
+//   MMA3  Zb = Q W+                                            LayerNorm + L2 gradient: Bt, d_gamma, d_beta,
+//   LNB   x_l = LN(Zb + b+), gZb = LNbwd(go gamma; x_l),       dV = -gamma Bt, gZin, d_eta; G_b += column sums of gZin
+//         d_beta += colsum go, d_gamma += colsum go x_l
+//   MMA4  gZb W+^T;  dQ = go + .
+//   slot <- bf16 W^T before the update, x_f, gZ, gZb (raw images of the swizzled shared-memory tiles, stored and read
+//   back with bulk copies), 1/std of the fused LayerNorm, the column sums of gZb.
+//
+// What bounds it: instruction issue (15 k warp-instructions per mini-batch in token-major epilogues) and the latency
+// of the two chains.  Measured: see the launcher.  All waits are bounded; on expiry the CTA reports through the status
+// word, drains its own copies, frees its tensor memory and returns.
 #include <mutex>
 
 #include "ttt_cluster.cuh"
@@ -35,66 +41,79 @@ using namespace tttcl;
 
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kProd = 128;     // issues the bulk copies; not the MMA issuer (lane 0 of warp 0)
+constexpr int kGroup = 256;
+constexpr int kThreads = 2 * kGroup;
+constexpr uint32_t kBarPairR = 1, kBarPairS = 5, kBarR = 9, kBarS = 10;     // named barriers
 
 // scratch slot (one per mini-batch of a checkpoint group and stream)
 constexpr uint32_t SL_W = 0;
 constexpr uint32_t SL_XF = TILE;
 constexpr uint32_t SL_GZ = 2 * TILE;
-constexpr uint32_t SL_XL = 3 * TILE;
-constexpr uint32_t SL_SIG = 4 * TILE;          // fp32[64] 1/std of the fused LayerNorm, fp32[64] of the output one
+constexpr uint32_t SL_GZB = 3 * TILE;
+constexpr uint32_t SL_VEC = 4 * TILE;          // fp32[64] 1/std of the fused LayerNorm, fp32[64] column sums of gZb
 constexpr uint32_t SLOT_BYTES = 4 * TILE + 512;
 
-// Shared memory.  kStages = 2: every per-mini-batch tile has two stages, the next mini-batch's loads are issued a
-// whole step ahead, one CTA per SM (for launches with no more streams than SMs, where nothing else could hide
-// the load latency).  kStages = 1: single tiles, loads issued when the step before has ended, half the shared
-// memory and a 128-register budget: two CTAs per SM, which hide each other's latencies (for launches with more
-// streams than SMs).  Tiles that are never live at the same time share their place: the bf16 copy of G^T with the
-// state copy W^T (read as the post-update state by the first reverse step only, before G^T is first copied), gZin
-// with gZb / U, the d_gamma addends with dL/dOut.
-template <int kStages>
-struct Lay {
-  static constexpr uint32_t OFF_K = 0;
-  static constexpr uint32_t OFF_Q = OFF_K + kStages * TILE;
-  static constexpr uint32_t OFF_V = OFF_Q + kStages * TILE;
-  static constexpr uint32_t OFF_GO = OFF_V + kStages * TILE;
-  static constexpr uint32_t OFF_XL = OFF_GO + kStages * TILE;
-  static constexpr uint32_t OFF_XF = OFF_XL + kStages * TILE;
-  static constexpr uint32_t OFF_GZ = OFF_XF + kStages * TILE;
-  static constexpr uint32_t OFF_WP = OFF_GZ + kStages * TILE;   // pre-update W^T of the sweep's mini-batch (always two)
-  static constexpr uint32_t OFF_W = OFF_WP + 2 * TILE;          // bf16 operand copy of the current state W^T / of G^T
-  static constexpr uint32_t OFF_A = OFF_W + TILE;               // U (recompute) / gZb, then gZin (sweep)
-  static constexpr uint32_t OFF_ETA = OFF_A + TILE;             // bf16[kStages][64]
-  static constexpr uint32_t OFF_SIG = OFF_ETA + 256;            // fp32[kStages][128]: both 1/std vectors of the sweep's mini-batch
-  static constexpr uint32_t OFF_B = OFF_SIG + 1024;
-  static constexpr uint32_t OFF_GB = OFF_B + 256;
-  static constexpr uint32_t OFF_GAMMA = OFF_GB + 256;
-  static constexpr uint32_t OFF_BETA = OFF_GAMMA + 256;
-  static constexpr uint32_t OFF_DG = OFF_BETA + 256;
-  static constexpr uint32_t OFF_DB = OFF_DG + 256;
-  static constexpr uint32_t OFF_PART = OFF_DB + 256;            // fp32[3][4][64] column-sum partials
-  static constexpr uint32_t OFF_BAR = OFF_PART + 3072;
-  static constexpr uint32_t OFF_MISC = OFF_BAR + 64;
-  static constexpr uint32_t OFF_XCH = OFF_MISC + 64;            // fp32[2][64][8] row-sum exchange between warp pairs
-  static constexpr uint32_t OFF_ONES = (OFF_XCH + 4096 + 1023) & ~1023u;   // bf16[8][64] ones: B operand of the column sums
-  static constexpr uint32_t SMEM_USED = OFF_ONES + 1024;
-  static constexpr uint32_t SMEM_BYTES = SMEM_USED + 1024;
-  static constexpr int kCtasPerSm = kStages == 1 ? 2 : 1;
-  static_assert(kCtasPerSm * (SMEM_BYTES + 1024) <= 233472, "exceeds the shared memory of an SM of sm_100");
-};
+// shared memory
+constexpr uint32_t OFF_RK = 0;                          // recompute: + stage
+constexpr uint32_t OFF_RQ = OFF_RK + 2 * TILE;
+constexpr uint32_t OFF_RV = OFF_RQ + 2 * TILE;          // V, then x_f on its way out
+constexpr uint32_t OFF_RGO = OFF_RV + 2 * TILE;         // dL/dOut, then dQ on its way out
+constexpr uint32_t OFF_RW = OFF_RGO + 2 * TILE;         // bf16 W^T before / after the update
+constexpr uint32_t OFF_RGZ = OFF_RW + 2 * TILE;
+constexpr uint32_t OFF_RU = OFF_RGZ + TILE;
+constexpr uint32_t OFF_RGZB = OFF_RU + TILE;
+constexpr uint32_t OFF_SK = OFF_RGZB + TILE;            // sweep: + stage
+constexpr uint32_t OFF_SQ = OFF_SK + 2 * TILE;
+constexpr uint32_t OFF_SV = OFF_SQ + TILE;              // V, then dV on its way out
+constexpr uint32_t OFF_SXF = OFF_SV + TILE;
+constexpr uint32_t OFF_SGZ = OFF_SXF + TILE;
+constexpr uint32_t OFF_SGZB = OFF_SGZ + TILE;
+constexpr uint32_t OFF_SWP = OFF_SGZB + TILE;           // bf16 W^T before the update
+constexpr uint32_t OFF_SG = OFF_SWP + TILE;             // bf16 G^T
+constexpr uint32_t OFF_SZIN = OFF_SG + TILE;
+constexpr uint32_t OFF_SDK = OFF_SZIN + TILE;           // dK on its way out
+constexpr uint32_t OFF_ONES = OFF_SDK + TILE;           // bf16[8][64] ones: B operand of the column sums
+constexpr uint32_t OFF_RETA = OFF_ONES + 1024;          // bf16[2][64]
+constexpr uint32_t OFF_SETA = OFF_RETA + 256;           // bf16[2][64]
+constexpr uint32_t OFF_RVEC = OFF_SETA + 256;           // fp32[2][128]: the slot's vectors on their way out
+constexpr uint32_t OFF_SVEC = OFF_RVEC + 1024;          // fp32[128]
+constexpr uint32_t OFF_B = OFF_SVEC + 512;
+constexpr uint32_t OFF_GB = OFF_B + 256;
+constexpr uint32_t OFF_GAMMA = OFF_GB + 256;
+constexpr uint32_t OFF_BETA = OFF_GAMMA + 256;
+constexpr uint32_t OFF_CSR = OFF_BETA + 256;            // fp32[4][64] column sums, one row per quadrant
+constexpr uint32_t OFF_CSS = OFF_CSR + 1024;
+constexpr uint32_t OFF_XR = OFF_CSS + 1024;             // row-sum exchange of each group
+constexpr uint32_t OFF_XS = OFF_XR + 4096;
+constexpr uint32_t OFF_BAR = OFF_XS + 4096;
+constexpr uint32_t OFF_MISC = OFF_BAR + 192;
+constexpr uint32_t SMEM_USED = OFF_MISC + 64;
+constexpr uint32_t SMEM_BYTES = SMEM_USED + 1024;       // slack for the 1024-byte alignment
+static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB per-CTA shared memory of sm_100");
 
-constexpr int BAR_IN = 0;      // +stage: K, Q, V, eta (and dL/dOut in the sweep)
-constexpr int BAR_SC = 2;      // +stage: scratch tiles of the sweep
-constexpr int BAR_MMA = 4;
-constexpr int BAR_DRAIN = 5;
-constexpr int NUM_BARS = 6;
+// barriers: loads first (their completion is what an aborting CTA still waits for)
+constexpr int BAR_RIN = 0;                              // recompute, + stage: K, eta, Q, V, dL/dOut
+constexpr int BAR_SK = 2;                               // sweep, + stage: K, eta
+constexpr int BAR_SQB = 4;                              // Q, gZb, vectors
+constexpr int BAR_SGZ = 5;                              // gZ, x_f
+constexpr int BAR_SV = 6;
+constexpr int BAR_SWP = 7;
+constexpr int kLoadBars = 8;
+constexpr int BAR_RM = 8;                               // the recompute's products: four uses per mini-batch
+constexpr int BAR_DK = 9, BAR_P1 = 10, BAR_P2 = 11;     // the sweep's
+constexpr int BAR_GROUP = 12;                           // a group's slots are written
+constexpr int BAR_TAIL = 13;
+constexpr int BAR_DRAIN = 14;                           // abort path only
+constexpr int kBars = 15;
 
+// tensor-memory columns
 constexpr uint32_t TM_W = 0;
 constexpr uint32_t TM_G = 64;
-constexpr uint32_t TM_A = 128;
-constexpr uint32_t TM_B = 192;
-constexpr uint32_t TM_COLS = 256;
+constexpr uint32_t TM_R = 128;        // recompute accumulator
+constexpr uint32_t TM_RC = 192;       // its column sums
+constexpr uint32_t TM_SA = 256;       // sweep accumulators
+constexpr uint32_t TM_SB = 320;
+constexpr uint32_t TM_COLS = 512;
 
 struct LinBwdParams {
   const __nv_bfloat16* eta;
@@ -110,86 +129,64 @@ struct LinBwdParams {
   float* gW;
   float* gb;
   __nv_bfloat16* d_eta;
-  __nv_bfloat16* dXQ;
-  __nv_bfloat16* dXK;
-  __nv_bfloat16* dXV;
   int H, NC, cgs, nck;
   int drop_load;            // test only: mini-batch whose recompute inputs stream 0 never loads (-1: none)
   uint32_t* status;
   uint64_t wait_limit_ns;
 };
 
-// D[64 x 64] += A^T B with both operands [64 k][64] tiles read MN-major (row = contraction index)
-__device__ __forceinline__ void mma_mn_accumulate(uint32_t tmem_d, uint32_t a_smem, uint32_t b_smem) {
-  constexpr uint32_t idesc = umma_idesc_bf16(64, 64, true, true, false);
-  const uint32_t a0 = desc_lo(a_smem, TILE);
-  const uint32_t b0 = desc_lo(b_smem, TILE);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) mma_issue_rt(tmem_d, a0 + j * (2048u >> 4), b0 + j * (2048u >> 4), idesc, 1u);
-}
-
-template <int kStages>
-__global__ void __launch_bounds__(kThreads, Lay<kStages>::kCtasPerSm)
+__global__ void __launch_bounds__(kThreads, 1)
 ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmGo,
-                      const LinBwdParams p) {
-  using L = Lay<kStages>;
-  constexpr uint32_t OFF_K = L::OFF_K, OFF_Q = L::OFF_Q, OFF_V = L::OFF_V, OFF_GO = L::OFF_GO, OFF_XL = L::OFF_XL,
-                     OFF_XF = L::OFF_XF, OFF_GZ = L::OFF_GZ, OFF_WP = L::OFF_WP, OFF_W = L::OFF_W, OFF_A = L::OFF_A,
-                     OFF_ETA = L::OFF_ETA, OFF_SIG = L::OFF_SIG, OFF_B = L::OFF_B, OFF_GB = L::OFF_GB,
-                     OFF_GAMMA = L::OFF_GAMMA, OFF_BETA = L::OFF_BETA, OFF_DG = L::OFF_DG, OFF_DB = L::OFF_DB,
-                     OFF_PART = L::OFF_PART, OFF_BAR = L::OFF_BAR, OFF_MISC = L::OFF_MISC, OFF_XCH = L::OFF_XCH;
-  constexpr int kSt = kStages - 1;            // stage of mini-batch j: j & kSt
+                      const __grid_constant__ CUtensorMap tmDQ, const __grid_constant__ CUtensorMap tmDK,
+                      const __grid_constant__ CUtensorMap tmDV, const LinBwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
   const int tid = threadIdx.x, lane = tid & 31;
-  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int cta_warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int warp = cta_warp & 7;                       // within the group
+  const bool recompute = cta_warp < 8;
+  const int gtid = tid & (kGroup - 1);
+  const bool loader = gtid == 128;                     // issues its group's bulk copies; not its MMA issuer (warp 0)
   const TokMap tm(warp, lane);
+  const int quad = tm.quad;
   const long sid = blockIdx.x;
   const int head = static_cast<int>(sid % p.H);
   const int NC = p.NC, cgs = p.cgs;
   const bool row_writer = tm.colhalf == 0 && tm.l3 == 0;   // of the 8 threads that share a row, the one that stores per-row values
 
-  auto tK = [&](int s) { return smem + OFF_K + s * TILE; };
-  auto tQ = [&](int s) { return smem + OFF_Q + s * TILE; };
-  auto tV = [&](int s) { return smem + OFF_V + s * TILE; };
-  auto tGo = [&](int s) { return smem + OFF_GO + s * TILE; };
-  auto tXL = [&](int s) { return smem + OFF_XL + s * TILE; };
-  auto tXF = [&](int s) { return smem + OFF_XF + s * TILE; };
-  auto tGZ = [&](int s) { return smem + OFF_GZ + s * TILE; };
-  auto tWP = [&](int s) { return smem + OFF_WP + s * TILE; };
-  uint8_t* sW = smem + OFF_W;
-  uint8_t* sA = smem + OFF_A;
-  uint8_t* sG = sW;        // see Lay
-  uint8_t* sZin = sA;
-  __nv_bfloat16* sEta = reinterpret_cast<__nv_bfloat16*>(smem + OFF_ETA);
-  float* sSig = reinterpret_cast<float*>(smem + OFF_SIG);
-  float* sB = reinterpret_cast<float*>(smem + OFF_B);
-  float* sGb = reinterpret_cast<float*>(smem + OFF_GB);
-  float* sGamma = reinterpret_cast<float*>(smem + OFF_GAMMA);
-  float* sBeta = reinterpret_cast<float*>(smem + OFF_BETA);
-  float* sDG = reinterpret_cast<float*>(smem + OFF_DG);
-  float* sDB = reinterpret_cast<float*>(smem + OFF_DB);
-  float* part = reinterpret_cast<float*>(smem + OFF_PART);
+  auto tile = [&](uint32_t off, int s = 0) { return smem + off + s * TILE; };
+  auto vec = [&](uint32_t off) { return reinterpret_cast<float*>(smem + off); };
+  float* sGamma = vec(OFF_GAMMA);
+  float* sBeta = vec(OFF_BETA);
+  float* sB = vec(OFF_B);
+  float* sGb = vec(OFF_GB);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
-  float* sXch = reinterpret_cast<float*>(smem + OFF_XCH);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_MISC);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + OFF_MISC + 4);
   volatile uint32_t* never_flag = reinterpret_cast<volatile uint32_t*>(smem + OFF_MISC + 8);   // stays 0
+  volatile uint32_t* freed = reinterpret_cast<volatile uint32_t*>(smem + OFF_MISC + 12);       // slots the sweep has read so far
+  // loads issued so far, for the abort path: bit b of word 0 = parity of barrier b's next load, of word 1 = there was one
+  uint32_t* loads = reinterpret_cast<uint32_t*>(smem + OFF_MISC + 16);
   const uint64_t limit = p.wait_limit_ns;
 
-  if (tid == kProd) {
-    for (int i = 0; i < NUM_BARS; ++i) mbar_init(&bars[i], 1);
+  if (tid == 0) {
+    for (int i = 0; i < kBars; ++i) mbar_init(&bars[i], i == BAR_DRAIN ? 2 : 1);
     fence_mbar_init();
     *abort_flag = 0;
     *never_flag = 0;
+    *freed = 0;
+    loads[0] = loads[1] = 0;
     prefetch_tmap(&tmQ);
     prefetch_tmap(&tmK);
     prefetch_tmap(&tmV);
     prefetch_tmap(&tmGo);
+    prefetch_tmap(&tmDQ);
+    prefetch_tmap(&tmDK);
+    prefetch_tmap(&tmDV);
   }
-  if (warp == 0) {
+  if (cta_warp == 0) {
     tmem_alloc(tmem_slot, TM_COLS);
     tmem_relinquish();
   }
@@ -197,72 +194,35 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     sGamma[tid] = p.gamma[head * 64 + tid];
     sBeta[tid] = p.beta[head * 64 + tid];
     sGb[tid] = p.gb_last[sid * 64 + tid];
-    sDG[tid] = 0.f;
-    sDB[tid] = 0.f;
   }
-  reinterpret_cast<uint32_t*>(smem + L::OFF_ONES)[tid] = 0x3F803F80u;     // 256 x two bf16 ones
+  if (tid < 256) reinterpret_cast<uint32_t*>(smem + OFF_ONES)[tid] = 0x3F803F80u;     // 256 x two bf16 ones
+  fence_proxy_async_smem();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t sOnes = smem_u32(smem + L::OFF_ONES);
-  // Column sums over the tokens of a bf16 tile are taken by the tensor pipe (mma_colsum: the MMA windows of
-  // these 64 x 64 products are too short to hide a pass over the tile by the warps), into accumulator columns
-  // that are free in that phase; warps 0..3 read them back after the phase (16 sums per warp).
-  auto add_colsum = [&](float* vec, uint32_t tm_cols, float sign) {
-    if (warp < 4) {
-      const float cs = colsum_read(tmem + tm_cols, warp);
-      if (lane < 16) vec[16 * warp + lane] += sign * cs;
-    }
-  };
+  const uint32_t lead = elect_one() ? 1u : 0u;         // the lane that issues the MMAs (warp 0 of each group)
 
-  // ---- barrier bookkeeping: every thread waits on every barrier use, in program order
-  uint32_t ph = 0;        // expected parity per barrier
-  uint32_t pending = 0;   // kProd: loads issued and not yet waited for
-  auto wait_bar = [&](int b) {
-    if (mbar_wait_bounded(&bars[b], (ph >> b) & 1u, abort_flag, limit)) {
-      ph ^= 1u << b;
-      pending &= ~(1u << b);
-    }
-  };
-  auto wait_mma = [&]() {
-    wait_bar(BAR_MMA);
+  auto wait_bar = [&](int b, uint32_t parity) { mbar_wait_bounded(&bars[b], parity & 1u, abort_flag, limit); };
+  auto mma_seen = [&]() {
     __syncwarp();
     tc_fence_after_sync();
   };
-  auto publish = [&]() {
-    fence_proxy_async_smem();
-    tc_fence_before_sync();
-    __syncthreads();
+  auto commit = [&](int b) { if (lead) umma_commit(&bars[b]); };
+  auto expect = [&](int b, uint32_t bytes) {
+    mbar_expect_tx(&bars[b], bytes);
+    atomicXor(loads, 1u << b);
+    atomicOr(loads + 1, 1u << b);
   };
-  auto publish_vote = [&]() -> bool {
-    fence_proxy_async_smem();
-    tc_fence_before_sync();
-    return __syncthreads_or(*abort_flag != 0) != 0;
-  };
-#define TTT_ISSUE1(WORK)            \
-  if (warp == 0) {                  \
-    if (elect_one()) {              \
-      tc_fence_after_sync();        \
-      WORK;                         \
-      umma_commit(&bars[BAR_MMA]);  \
-    }                               \
-    __syncwarp();                   \
-  }
-
-  const int cs_q = tid >> 6, cs_f = tid & 63;
-  auto colsum16 = [&](const uint8_t* t) {
-    float acc = 0.f;
-#pragma unroll 8
-    for (int r = cs_q * 16; r < cs_q * 16 + 16; ++r) acc += ld_elem(t, r, cs_f);
-    return acc;
-  };
-  auto part_sum = [&](int k) {
-    return (part[k * 256 + tid] + part[k * 256 + 64 + tid]) + (part[k * 256 + 128 + tid] + part[k * 256 + 192 + tid]);
-  };
-
-  // ---- state <-> global memory.  W-shaped matrices are [64 in][64 out] in global memory; the fragment of the
-  // transposed matrix holds output features r0 / r1 (rows) and the input-feature pairs col(j), col(j) + 1.
+  const long tok_rows0 = sid * NC * 64;
+  auto row_of = [&](int i) { return static_cast<int>(tok_rows0 + static_cast<long>(i) * 64); };
+  uint8_t* slots = p.scratch + sid * cgs * static_cast<long>(SLOT_BYTES);
+  // group g (0 = the last of the sequence, the first to be processed): its first mini-batch, size, slot of mini-batch j
+  auto first_of = [&](int g) { return (p.nck - 1 - g) * cgs; };
+  auto size_of = [&](int g) { return g == 0 ? NC - (p.nck - 1) * cgs : cgs; };
+  auto slot_of = [&](int g, int j) { return slots + static_cast<long>(g & 1 ? cgs - 1 - j : j) * SLOT_BYTES; };
+  // W-shaped matrices are [64 in][64 out] in global memory; the fragment of the transposed matrix holds output features
+  // r0 / r1 (rows) and the input-feature pairs col(j), col(j) + 1.
   auto load_frag = [&](const float* Wg, float (&w)[16]) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -273,443 +233,602 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       w[4 * j + 3] = Wg[(c + 1) * 64 + tm.r1];
     }
   };
-  {   // the gradient state starts as dL/d(final state)
-    float w[16];
-    load_frag(p.gW_last + sid * 4096, w);
-    tok_st_tmem(tm, tmem + TM_G, w);
-    tmem_wait_st();
-  }
+  // column sums left by the four quadrants of a group's warps
+  auto quad_sum = [&](const float* cs, int f) { return (cs[f] + cs[64 + f]) + (cs[128 + f] + cs[192 + f]); };
+  float dgam = 0.f, dbet = 0.f;      // this lane's column (frag_colsum_col) of what its group adds to d_gamma / d_beta
+  bool stop = false;
 
-  const long tok_rows0 = sid * NC * 64;
-  bool aborted = false;
-
-  for (int ck = p.nck - 1; ck >= 0 && !aborted; --ck) {
-    const int i0 = ck * cgs;
-    const int gsz = min(cgs, NC - i0);
-    uint8_t* slots = p.scratch + sid * cgs * static_cast<long>(SLOT_BYTES);
-
-    auto issue_inputs = [&](int j, bool with_go) {   // kProd
-      if (!with_go && i0 + j == p.drop_load && sid == 0) return;
-      const int s = j & kSt;
-      const int row0 = static_cast<int>(tok_rows0 + (long)(i0 + j) * 64);
-      mbar_expect_tx(&bars[BAR_IN + s], (with_go ? 4 : 3) * TILE + 128);
-      tma_load_2d(tK(s), &tmK, &bars[BAR_IN + s], 0, row0);
-      tma_load_2d(tQ(s), &tmQ, &bars[BAR_IN + s], 0, row0);
-      tma_load_2d(tV(s), &tmV, &bars[BAR_IN + s], 0, row0);
-      if (with_go) tma_load_2d(tGo(s), &tmGo, &bars[BAR_IN + s], 0, row0);
-      bulk_load_1d(sEta + s * 64, p.eta + (sid * NC + i0 + j) * 64, 128, &bars[BAR_IN + s]);
-      pending |= 1u << (BAR_IN + s);
+  if (recompute) {
+    // ======================================================================================= recompute
+    auto publish = [&]() {
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      named_bar_sync(kBarR, kGroup);
     };
-    // The barrier is armed with all the bytes of the slot; the pre-update state copy follows separately
-    // (issue_wp) when its tile, which holds the post-update state of the step before, is free.
-    auto issue_wp = [&](int j) {                     // kProd
-      bulk_load_1d(tWP(j & 1), slots + static_cast<long>(j) * SLOT_BYTES + SL_W, TILE, &bars[BAR_SC + (j & kSt)]);
+    uint32_t n = 0, pm = 0;
+    auto wait_mma = [&]() {
+      wait_bar(BAR_RM, pm);
+      pm ^= 1u;
+      mma_seen();
     };
-    auto issue_scratch = [&](int j) {                // kProd
-      const int s = j & kSt;
-      const uint8_t* sl = slots + static_cast<long>(j) * SLOT_BYTES;
-      mbar_expect_tx(&bars[BAR_SC + s], 4 * TILE + 512);
-      bulk_load_1d(tXF(s), sl + SL_XF, TILE, &bars[BAR_SC + s]);
-      bulk_load_1d(tGZ(s), sl + SL_GZ, TILE, &bars[BAR_SC + s]);
-      bulk_load_1d(tXL(s), sl + SL_XL, TILE, &bars[BAR_SC + s]);
-      bulk_load_1d(sSig + s * 128, sl + SL_SIG, 512, &bars[BAR_SC + s]);
-      pending |= 1u << (BAR_SC + s);
+    auto issue_inputs = [&](int i, uint32_t cnt) {     // loader
+      if (i == p.drop_load && sid == 0) return;
+      const int s = cnt & 1;
+      expect(BAR_RIN + s, 4 * TILE + 128);
+      tma_load_2d(tile(OFF_RK, s), &tmK, &bars[BAR_RIN + s], 0, row_of(i));
+      tma_load_2d(tile(OFF_RV, s), &tmV, &bars[BAR_RIN + s], 0, row_of(i));
+      tma_load_2d(tile(OFF_RQ, s), &tmQ, &bars[BAR_RIN + s], 0, row_of(i));
+      tma_load_2d(tile(OFF_RGO, s), &tmGo, &bars[BAR_RIN + s], 0, row_of(i));
+      bulk_load_1d(smem + OFF_RETA + s * 128, p.eta + (sid * NC + i) * 64, 128, &bars[BAR_RIN + s]);
     };
-    if (tid == kProd) {
-      issue_inputs(0, false);
-      if (kStages == 2 && gsz > 1) issue_inputs(1, false);
-    }
-    // ---- checkpoint -> tensor memory (fp32) + shared memory (bf16)
-    {
-      float w[16];
-      load_frag(p.Wc + (sid * p.nck + ck) * 4096, w);
-      tok_st_tmem(tm, tmem + TM_W, w);
-      tok_st_tile(tm, sW, w);
-      tmem_wait_st();
-      if (tid < 64) sB[tid] = p.bc[(sid * p.nck + ck) * 64 + tid];
-    }
-    publish();
-
-    // ================================================================== recompute the group
-    for (int j = 0; j < gsz; ++j) {
-      const int s = j & kSt;
-      uint8_t* sl = slots + static_cast<long>(j) * SLOT_BYTES;
-      float* sig = reinterpret_cast<float*>(sl + SL_SIG);
-      const __nv_bfloat16* eta = sEta + s * 64;
-      wait_bar(BAR_IN + s);
-
-      // MMA1: Z = K W
-      TTT_ISSUE1(mma_hid64<false>(tmem + TM_A, smem_u32(tK(s)), smem_u32(sW), 0u))
-      wait_mma();
-      {
-        float xh[16], bc[8], gam[8], bet[8];
-        tok_ld(tm, tmem + TM_A, xh);
-        tok_ld_cols(tm, sB, bc);
-        tok_ld_cols(tm, sGamma, gam);
-        tok_ld_cols(tm, sBeta, bet);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          xh[4 * q] += bc[2 * q]; xh[4 * q + 1] += bc[2 * q + 1];
-          xh[4 * q + 2] += bc[2 * q]; xh[4 * q + 3] += bc[2 * q + 1];
-        }
-        float rs0, rs1;
-        float kk[16], vv[16], g[16];
-        tok_ld_tile(tm, tK(s), kk);
-        tok_ld_tile(tm, tV(s), vv);
-        tok_layernorm(tm, xh, TTT_LN_EPS, sXch, rs0, rs1);
-        float a[2] = {0.f, 0.f}, b[2] = {0.f, 0.f};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h, c = 2 * q + h;
-            xh[x0] *= rs0;
-            xh[x1] *= rs1;
-            g[x0] = (fmaf(gam[c], xh[x0], bet[c]) - (vv[x0] - kk[x0])) * gam[c];
-            g[x1] = (fmaf(gam[c], xh[x1], bet[c]) - (vv[x1] - kk[x1])) * gam[c];
-            a[0] += g[x0]; a[1] = fmaf(g[x0], xh[x0], a[1]);
-            b[0] += g[x1]; b[1] = fmaf(g[x1], xh[x1], b[1]);
-          }
-        }
-        tok_st_tile(tm, tXF(s), xh);
-        tok_row_allreduce<2, 2>(tm, a, b, sXch);
-        const float sc0 = rs0 * (1.f / 64.f), sc1 = rs1 * (1.f / 64.f);
-        const float ne0 = -__bfloat162float(eta[tm.r0]), ne1 = -__bfloat162float(eta[tm.r1]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h;
-            // dl/dZ, rounded to bf16 once: the update below uses -eta times the rounded value
-            g[x0] = __bfloat162float(__float2bfloat16((64.f * g[x0] - a[0] - xh[x0] * a[1]) * sc0));
-            g[x1] = __bfloat162float(__float2bfloat16((64.f * g[x1] - b[0] - xh[x1] * b[1]) * sc1));
-          }
-        }
-        tok_st_tile(tm, tGZ(s), g);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          g[4 * q] *= ne0; g[4 * q + 1] *= ne0;
-          g[4 * q + 2] *= ne1; g[4 * q + 3] *= ne1;
-        }
-        tok_st_tile(tm, sA, g);
-        if (row_writer) {
-          sig[tm.r0] = rs0;
-          sig[tm.r1] = rs1;
+    // The slots of group g that group g - 1 used as well are free once the sweep has read them: wait (bounded) for its count.
+    auto wait_slot = [&](int g, int j) {               // loader
+      if (g == 0) return;
+      const int before = g == 1 ? 0 : size_of(0) + (g - 2) * cgs;       // steps of the groups before g - 1
+      const int own = j - (cgs - size_of(g - 1));                       // step of group g - 1 that reads this slot
+      if (own < 0) return;
+      const uint32_t need = static_cast<uint32_t>(before + own + 1);
+      if (*freed >= need) return;
+      const uint64_t t0 = globaltimer_ns();
+      while (*freed < need) {
+        if (*abort_flag) return;
+        if (globaltimer_ns() - t0 > limit) {
+          *abort_flag = 1;
+          return;
         }
       }
-      publish();
-      if (tid == kProd) {   // the pre-update state and the fused-LayerNorm tiles of this mini-batch leave for its slot
-        bulk_store_1d(sl + SL_W, sW, TILE);
-        bulk_store_1d(sl + SL_XF, tXF(s), TILE);
-        bulk_store_1d(sl + SL_GZ, tGZ(s), TILE);
-        tma_commit_group();
+    };
+    for (int g = 0; g < p.nck && !stop; ++g) {
+      const int i0 = first_of(g), gsz = size_of(g);
+      if (loader) {
+        if (g > 0) tma_wait_group_read<0>();
+        issue_inputs(i0, n);
+        if (gsz > 1) issue_inputs(i0 + 1, n + 1);
       }
-
-      // MMA2: W^T += U^T K;  b += column sums of U
-      TTT_ISSUE1(mma_mn_accumulate(tmem + TM_W, smem_u32(sA), smem_u32(tK(s)));
-                 mma_colsum(tmem + TM_B, smem_u32(sA), sOnes))
-      if (tid == kProd) tma_wait_group_read<0>();   // the state copy has left shared memory: the refresh below may overwrite it
-      __syncthreads();
-      wait_mma();
-      add_colsum(sB, TM_B, 1.f);
-      {
+      {   // checkpoint -> tensor memory (fp32) + shared memory (bf16)
         float w[16];
-        tok_ld(tm, tmem + TM_W, w);
-        tok_st_tile(tm, sW, w);
+        load_frag(p.Wc + (sid * p.nck + p.nck - 1 - g) * 4096, w);
+        tok_st_tmem(tm, tmem + TM_W, w);
+        tok_st_tile(tm, tile(OFF_RW, n & 1), w);
+        tmem_wait_st();
+        if (gtid < 64) sB[gtid] = p.bc[(sid * p.nck + p.nck - 1 - g) * 64 + gtid];
       }
       publish();
+      for (int j = 0; j < gsz; ++j, ++n) {
+        const int s = n & 1;
+        uint8_t* tK = tile(OFF_RK, s);
+        uint8_t* tV = tile(OFF_RV, s);
+        uint8_t* tGo = tile(OFF_RGO, s);
+        uint8_t* tW = tile(OFF_RW, s);
+        uint8_t* tWn = tile(OFF_RW, s ^ 1);
+        uint8_t* tGZ = tile(OFF_RGZ);
+        uint8_t* tU = tile(OFF_RU);
+        uint8_t* tGZB = tile(OFF_RGZB);
+        float* sVec = vec(OFF_RVEC) + s * 128;
+        float* xch = vec(OFF_XR);
+        const __nv_bfloat16* eta = reinterpret_cast<const __nv_bfloat16*>(smem + OFF_RETA) + s * 64;
+        uint8_t* sl = slot_of(g, j);
+        wait_bar(BAR_RIN + s, n >> 1);
 
-      // MMA3: Zb = Q W+;  output LayerNorm statistics
-      TTT_ISSUE1(mma_hid64<false>(tmem + TM_A, smem_u32(tQ(s)), smem_u32(sW), 0u))
-      wait_mma();
-      {
-        float z[16], bc[8];
-        tok_ld(tm, tmem + TM_A, z);
-        tok_ld_cols(tm, sB, bc);
+        // ---- MMA1: Z = K W
+        if (cta_warp == 0) {
+          tc_fence_after_sync();
+          mma_64_lead<false, false>(tmem + TM_R, smem_u32(tK), smem_u32(tW), lead);
+          commit(BAR_RM);
+        }
+        if (loader && j > 0) {         // the last mini-batch's tiles have left: its stage takes the next inputs
+          tma_wait_group_read<0>();
+          if (j + 1 < gsz) issue_inputs(i0 + j + 1, n + 1);
+        }
+        wait_mma();
+        // ---- LN.  x_f leaves through the V tile (every thread overwrites exactly the elements it has read); dl/dZ is
+        // rounded to bf16 once, the update uses -eta times the rounded value.
+        {
+          TokFrag x, gr;
+          uint32_t kk[8], vv[8];
+          frag_ld(tm, tmem + TM_R, x);
+          frag_ld_raw(tm, tK, kk);
+          frag_ld_raw(tm, tV, vv);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          z[4 * q] += bc[2 * q]; z[4 * q + 1] += bc[2 * q + 1];
-          z[4 * q + 2] += bc[2 * q]; z[4 * q + 3] += bc[2 * q + 1];
-        }
-        float rs0, rs1;
-        tok_layernorm(tm, z, TTT_LN_EPS, sXch, rs0, rs1);
+          for (int q = 0; q < 4; ++q) {
+            const f32x2 b = frag_col(tm, sB, q);
+            x.a[q] = add2(x.a[q], b);
+            x.b[q] = add2(x.b[q], b);
+          }
+          float rs0, rs1;
+          frag_layernorm(tm, x, TTT_LN_EPS, xch, kBarPairR, rs0, rs1);
+          f32x2 a0 = 0ull, a1 = 0ull, c0 = 0ull, c1 = 0ull;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          z[4 * q] *= rs0; z[4 * q + 1] *= rs0;
-          z[4 * q + 2] *= rs1; z[4 * q + 3] *= rs1;
+          for (int q = 0; q < 4; ++q) {
+            const f32x2 gam = frag_col(tm, sGamma, q), bet = frag_col(tm, sBeta, q), neg = pk1(-1.f);
+            const f32x2 t0 = fma2(bf16x2_to_f32x2(vv[2 * q]), neg, bf16x2_to_f32x2(kk[2 * q]));          // K - V
+            const f32x2 t1 = fma2(bf16x2_to_f32x2(vv[2 * q + 1]), neg, bf16x2_to_f32x2(kk[2 * q + 1]));
+            gr.a[q] = mul2(fma2(gam, x.a[q], add2(t0, bet)), gam);
+            gr.b[q] = mul2(fma2(gam, x.b[q], add2(t1, bet)), gam);
+            a0 = add2(a0, gr.a[q]); a1 = fma2(gr.a[q], x.a[q], a1);
+            c0 = add2(c0, gr.b[q]); c1 = fma2(gr.b[q], x.b[q], c1);
+          }
+          frag_st_tile(tm, tV, x);
+          float a[2] = {hsum(a0), hsum(a1)}, b[2] = {hsum(c0), hsum(c1)};
+          frag_allreduce2<1>(tm, a, b, xch, kBarPairR);
+          const f32x2 sc0 = pk1(rs0 * (1.f / 64.f)), sc1 = pk1(rs1 * (1.f / 64.f));
+          const f32x2 ne0 = pk1(-__bfloat162float(eta[tm.r0])), ne1 = pk1(-__bfloat162float(eta[tm.r1]));
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t w0 = f32x2_to_bf16x2(mul2(fma2(x.a[q], pk1(-a[1]), fma2(gr.a[q], pk1(64.f), pk1(-a[0]))), sc0));
+            const uint32_t w1 = f32x2_to_bf16x2(mul2(fma2(x.b[q], pk1(-b[1]), fma2(gr.b[q], pk1(64.f), pk1(-b[0]))), sc1));
+            *reinterpret_cast<uint32_t*>(tGZ + tm.off(tm.r0, q)) = w0;
+            *reinterpret_cast<uint32_t*>(tGZ + tm.off(tm.r1, q)) = w1;
+            gr.a[q] = mul2(bf16x2_to_f32x2(w0), ne0);
+            gr.b[q] = mul2(bf16x2_to_f32x2(w1), ne1);
+          }
+          frag_st_tile(tm, tU, gr);
+          if (row_writer) {
+            sVec[tm.r0] = rs0;
+            sVec[tm.r1] = rs1;
+          }
         }
-        tok_st_tile(tm, tXL(s), z);
-        if (row_writer) {
-          sig[64 + tm.r0] = rs0;
-          sig[64 + tm.r1] = rs1;
+        publish();
+
+        // ---- MMA2: W^T += U^T K;  b += column sums of U
+        if (cta_warp == 0) {
+          tc_fence_after_sync();
+          mma_64_tn_lead(tmem + TM_W, smem_u32(tU), smem_u32(tK), lead);
+          mma_colsum_lead(tmem + TM_RC, smem_u32(tU), smem_u32(smem + OFF_ONES), lead);
+          commit(BAR_RM);
         }
+        if (loader) {
+          wait_slot(g, j);
+          bulk_store_1d(sl + SL_W, tW, TILE);
+          bulk_store_1d(sl + SL_XF, tV, TILE);
+          bulk_store_1d(sl + SL_GZ, tGZ, TILE);
+          tma_commit_group();
+        }
+        __syncwarp();
+        wait_mma();
+        if (warp < 4) {
+          const float cs = colsum_read(tmem + TM_RC, warp);
+          if (lane < 16) sB[16 * warp + lane] += cs;       // its next reader comes after the barrier below
+        }
+        // ---- EPI: bf16 copy of the new W^T
+        {
+          TokFrag w;
+          frag_ld(tm, tmem + TM_W, w);
+          frag_st_tile(tm, tWn, w);
+        }
+        publish();
+
+        // ---- MMA3: Zb = Q W+
+        if (cta_warp == 0) {
+          tc_fence_after_sync();
+          mma_64_lead<false, false>(tmem + TM_R, smem_u32(tile(OFF_RQ, s)), smem_u32(tWn), lead);
+          commit(BAR_RM);
+        }
+        wait_mma();
+        // ---- LNB: output LayerNorm and its backward, gZb; its column sums; d_beta += sum go, d_gamma += sum go x_l
+        {
+          TokFrag x, gr;
+          uint32_t go[8];
+          frag_ld(tm, tmem + TM_R, x);
+          frag_ld_raw(tm, tGo, go);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const f32x2 b = frag_col(tm, sB, q);
+            x.a[q] = add2(x.a[q], b);
+            x.b[q] = add2(x.b[q], b);
+          }
+          float rs0, rs1;
+          frag_layernorm(tm, x, TTT_LN_EPS, xch, kBarPairR, rs0, rs1);
+          f32x2 a0 = 0ull, a1 = 0ull, c0 = 0ull, c1 = 0ull, sb[4], sg[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const f32x2 gam = frag_col(tm, sGamma, q);
+            const f32x2 o0 = bf16x2_to_f32x2(go[2 * q]), o1 = bf16x2_to_f32x2(go[2 * q + 1]);
+            sb[q] = add2(o0, o1);
+            sg[q] = fma2(o0, x.a[q], mul2(o1, x.b[q]));
+            gr.a[q] = mul2(o0, gam);
+            gr.b[q] = mul2(o1, gam);
+            a0 = add2(a0, gr.a[q]); a1 = fma2(gr.a[q], x.a[q], a1);
+            c0 = add2(c0, gr.b[q]); c1 = fma2(gr.b[q], x.b[q], c1);
+          }
+          dbet += frag_colsum(sb, lane);
+          dgam += frag_colsum(sg, lane);
+          float a[2] = {hsum(a0), hsum(a1)}, b[2] = {hsum(c0), hsum(c1)};
+          frag_allreduce2<1>(tm, a, b, xch, kBarPairR);
+          const f32x2 q0 = pk1(rs0 * (1.f / 64.f)), q1 = pk1(rs1 * (1.f / 64.f));
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            gr.a[q] = mul2(fma2(x.a[q], pk1(-a[1]), fma2(gr.a[q], pk1(64.f), pk1(-a[0]))), q0);
+            gr.b[q] = mul2(fma2(x.b[q], pk1(-b[1]), fma2(gr.b[q], pk1(64.f), pk1(-b[0]))), q1);
+            sb[q] = add2(gr.a[q], gr.b[q]);
+          }
+          frag_st_tile(tm, tGZB, gr);
+          vec(OFF_CSR)[quad * 64 + frag_colsum_col(tm, lane)] = frag_colsum(sb, lane);
+        }
+        publish();
+
+        // ---- MMA4: gZb W+^T
+        if (cta_warp == 0) {
+          tc_fence_after_sync();
+          mma_64_lead<true, false>(tmem + TM_R, smem_u32(tGZB), smem_u32(tWn), lead);
+          commit(BAR_RM);
+        }
+        if (gtid < 64) sVec[64 + gtid] = quad_sum(vec(OFF_CSR), gtid);
+        wait_mma();
+        // ---- dQ = go + gZb W+^T, over the dL/dOut tile
+        {
+          TokFrag x;
+          uint32_t go[8];
+          frag_ld(tm, tmem + TM_R, x);
+          frag_ld_raw(tm, tGo, go);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            x.a[q] = add2(x.a[q], bf16x2_to_f32x2(go[2 * q]));
+            x.b[q] = add2(x.b[q], bf16x2_to_f32x2(go[2 * q + 1]));
+          }
+          frag_st_tile(tm, tGo, x);
+        }
+        if (loader) tma_wait_group_read<0>();        // W, x_f and gZ have left their tiles
+        fence_proxy_async_smem();
+        tc_fence_before_sync();
+        stop = named_bar_or(kBarR, kGroup, *abort_flag != 0);
+        if (loader) {
+          tma_store_2d(&tmDQ, tGo, 0, row_of(i0 + j));
+          bulk_store_1d(sl + SL_GZB, tGZB, TILE);
+          bulk_store_1d(sl + SL_VEC, sVec, 512);
+          tma_commit_group();
+        }
+        if (stop) break;
       }
-      aborted = publish_vote();
-      if (tid == kProd && !aborted) {
-        bulk_store_1d(sl + SL_XL, tXL(s), TILE);
+      if (loader && !stop) {       // the group's slots are complete
+        tma_wait_group<0>();
+        mbar_arrive(&bars[BAR_GROUP]);
+      }
+    }
+    if (loader) tma_wait_group<0>();
+  } else {
+    // =========================================================================================== sweep
+    auto publish = [&]() {
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      named_bar_sync(kBarS, kGroup);
+    };
+    uint8_t* tQ = tile(OFF_SQ);
+    uint8_t* tV = tile(OFF_SV);
+    uint8_t* tXF = tile(OFF_SXF);
+    uint8_t* tGZ = tile(OFF_SGZ);
+    uint8_t* tGZB = tile(OFF_SGZB);
+    uint8_t* tWP = tile(OFF_SWP);
+    uint8_t* tG = tile(OFF_SG);
+    uint8_t* tZin = tile(OFF_SZIN);
+    uint8_t* tDK = tile(OFF_SDK);
+    float* sVec = vec(OFF_SVEC);
+    float* xch = vec(OFF_XS);
+    {   // the gradient state starts as dL/d(final state)
+      float w[16];
+      load_frag(p.gW_last + sid * 4096, w);
+      tok_st_tmem(tm, tmem + TM_G, w);
+      tmem_wait_st();
+    }
+    tc_fence_before_sync();
+    named_bar_sync(kBarS, kGroup);
+    tc_fence_after_sync();
+
+    // loads of one step, in parts, each issued when its tiles are free (loader)
+    auto issue_k = [&](int i, uint32_t cnt) {
+      const int s = cnt & 1;
+      expect(BAR_SK + s, TILE + 128);
+      tma_load_2d(tile(OFF_SK, s), &tmK, &bars[BAR_SK + s], 0, row_of(i));
+      bulk_load_1d(smem + OFF_SETA + s * 128, p.eta + (sid * NC + i) * 64, 128, &bars[BAR_SK + s]);
+    };
+    auto issue_qb = [&](int i, const uint8_t* sl) {
+      expect(BAR_SQB, 2 * TILE);
+      tma_load_2d(tQ, &tmQ, &bars[BAR_SQB], 0, row_of(i));
+      bulk_load_1d(tGZB, sl + SL_GZB, TILE, &bars[BAR_SQB]);
+    };
+    auto issue_gz = [&](const uint8_t* sl) {
+      expect(BAR_SGZ, 2 * TILE + 512);
+      bulk_load_1d(tGZ, sl + SL_GZ, TILE, &bars[BAR_SGZ]);
+      bulk_load_1d(tXF, sl + SL_XF, TILE, &bars[BAR_SGZ]);
+      bulk_load_1d(sVec, sl + SL_VEC, 512, &bars[BAR_SGZ]);
+    };
+    auto issue_v = [&](int i) {
+      expect(BAR_SV, TILE);
+      tma_load_2d(tV, &tmV, &bars[BAR_SV], 0, row_of(i));
+    };
+    auto issue_wp = [&](const uint8_t* sl) {
+      expect(BAR_SWP, TILE);
+      bulk_load_1d(tWP, sl + SL_W, TILE, &bars[BAR_SWP]);
+    };
+    f32x2 kpa[4], kpb[4];        // partial dK of the step before: gamma Bt - eta T1
+    // what the step of count c adds to the gradient state, and its dK product (MMA issuer)
+    auto issue_tail = [&](uint32_t c) {
+      wait_bar(BAR_SWP, c);
+      mma_seen();
+      mma_64_lead<true, false>(tmem + TM_SA, smem_u32(tZin), smem_u32(tWP), lead);
+      commit(BAR_DK);
+      mma_64_tn_lead(tmem + TM_G, smem_u32(tZin), smem_u32(tile(OFF_SK, c & 1)), lead);
+    };
+    auto finish_dk = [&](uint32_t c) {
+      wait_bar(BAR_DK, c);
+      mma_seen();
+      TokFrag x;
+      frag_ld(tm, tmem + TM_SA, x);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        x.a[q] = add2(x.a[q], kpa[q]);
+        x.b[q] = add2(x.b[q], kpb[q]);
+      }
+      frag_st_tile(tm, tDK, x);
+    };
+
+    uint32_t m = 0;
+    for (int g = 0; g < p.nck && !stop; ++g) {
+      const int i0 = first_of(g), gsz = size_of(g);
+      if (loader) {
+        wait_bar(BAR_GROUP, g);
+        const int j = gsz - 1;
+        const uint8_t* sl = slot_of(g, j);
+        issue_qb(i0 + j, sl);
+        issue_k(i0 + j, m);
+        issue_gz(sl);
+        tma_wait_group_read<0>();
+        issue_v(i0 + j);
+      }
+      __syncwarp();
+      for (int j = gsz - 1; j >= 0; --j, ++m) {
+        const uint32_t par = m & 1;
+        const bool first = j == gsz - 1;
+        uint8_t* tK = tile(OFF_SK, m & 1);
+        const __nv_bfloat16* eta = reinterpret_cast<const __nv_bfloat16*>(smem + OFF_SETA) + par * 64;
+
+        // ---- P1: the step before's dK product and state gradient; G^T += gZb^T Q
+        if (cta_warp == 8) {
+          tc_fence_after_sync();
+          if (!first) issue_tail(m - 1);
+          wait_bar(BAR_SQB, par);
+          mma_seen();
+          mma_64_tn_lead(tmem + TM_G, smem_u32(tGZB), smem_u32(tQ), lead);
+          commit(BAR_P1);
+        }
+        if (!first) finish_dk(m - 1);
+        wait_bar(BAR_P1, par);
+        mma_seen();
+        if (loader) {
+          if (!first) *freed = m;            // the step before's slot has been read (its last tile, W, just now)
+          issue_wp(slot_of(g, j));
+          if (j > 0) {
+            issue_k(i0 + j - 1, m + 1);
+            issue_qb(i0 + j - 1, slot_of(g, j - 1));
+          }
+        }
+        // ---- E2: bf16 copy of G^T
+        {
+          TokFrag w;
+          frag_ld(tm, tmem + TM_G, w);
+          frag_st_tile(tm, tG, w);
+        }
+        wait_bar(BAR_SGZ, par);
+        if (gtid < 64) sGb[gtid] += sVec[64 + gtid];
+        publish();
+
+        // ---- P2: K G, T1 = gZ G^T
+        if (cta_warp == 8) {
+          tc_fence_after_sync();
+          wait_bar(BAR_SK + par, m >> 1);
+          mma_seen();
+          mma_64_lead<false, false>(tmem + TM_SA, smem_u32(tK), smem_u32(tG), lead);
+          mma_64_lead<true, false>(tmem + TM_SB, smem_u32(tGZ), smem_u32(tG), lead);
+          commit(BAR_P2);
+        }
+        if (loader && !first) {
+          tma_store_2d(&tmDK, tDK, 0, row_of(i0 + j + 1));
+          tma_commit_group();
+        }
+        __syncwarp();
+        wait_bar(BAR_SK + par, m >> 1);
+        wait_bar(BAR_SV, par);
+        // ---- E4: second order through the fused LayerNorm + L2 gradient
+        {
+          TokFrag A, t1, go;
+          uint32_t gzw[8], xhw[8], kw[8];
+          frag_ld_raw(tm, tGZ, gzw);
+          frag_ld_raw(tm, tXF, xhw);
+          frag_ld_raw(tm, tK, kw);
+          {
+            uint32_t vw[8];
+            frag_ld_raw(tm, tV, vw);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {    // grad_output_fused = gamma x_hat_fused + beta - (V - K)
+              const f32x2 gam = frag_col(tm, sGamma, q), bet = frag_col(tm, sBeta, q), neg = pk1(-1.f);
+              go.a[q] = add2(fma2(bf16x2_to_f32x2(vw[2 * q]), neg, bf16x2_to_f32x2(kw[2 * q])),
+                             fma2(gam, bf16x2_to_f32x2(xhw[2 * q]), bet));
+              go.b[q] = add2(fma2(bf16x2_to_f32x2(vw[2 * q + 1]), neg, bf16x2_to_f32x2(kw[2 * q + 1])),
+                             fma2(gam, bf16x2_to_f32x2(xhw[2 * q + 1]), bet));
+            }
+          }
+          const float eta0 = __bfloat162float(eta[tm.r0]), eta1 = __bfloat162float(eta[tm.r1]);
+          const float rs0 = sVec[tm.r0], rs1 = sVec[tm.r1];      // 1 / std
+          wait_bar(BAR_P2, par);
+          mma_seen();
+          frag_ld(tm, tmem + TM_SA, A);
+          frag_ld(tm, tmem + TM_SB, t1);
+          float ra[4], rb[4];       // d_eta, sum A, sum A xh, sum g xh
+          {
+            f32x2 s0[4] = {0ull, 0ull, 0ull, 0ull}, s1[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const f32x2 gb = frag_col(tm, sGb, q), gam = frag_col(tm, sGamma, q);
+              const f32x2 x0 = bf16x2_to_f32x2(xhw[2 * q]), x1 = bf16x2_to_f32x2(xhw[2 * q + 1]);
+              s0[0] = fma2(t1.a[q], bf16x2_to_f32x2(kw[2 * q]), fma2(gb, bf16x2_to_f32x2(gzw[2 * q]), s0[0]));
+              s1[0] = fma2(t1.b[q], bf16x2_to_f32x2(kw[2 * q + 1]), fma2(gb, bf16x2_to_f32x2(gzw[2 * q + 1]), s1[0]));
+              kpa[q] = mul2(t1.a[q], pk1(-eta0));
+              kpb[q] = mul2(t1.b[q], pk1(-eta1));
+              A.a[q] = mul2(add2(A.a[q], gb), pk1(-eta0));
+              A.b[q] = mul2(add2(A.b[q], gb), pk1(-eta1));
+              s0[1] = add2(s0[1], A.a[q]);
+              s1[1] = add2(s1[1], A.b[q]);
+              s0[2] = fma2(A.a[q], x0, s0[2]);
+              s1[2] = fma2(A.b[q], x1, s1[2]);
+              s0[3] = fma2(mul2(go.a[q], gam), x0, s0[3]);
+              s1[3] = fma2(mul2(go.b[q], gam), x1, s1[3]);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { ra[i] = hsum(s0[i]); rb[i] = hsum(s1[i]); }
+          }
+          // all-reduce over the row's four lanes and two warps
+#pragma unroll
+          for (int sft = 1; sft <= 2; sft <<= 1)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              ra[i] += __shfl_xor_sync(0xffffffffu, ra[i], sft);
+              rb[i] += __shfl_xor_sync(0xffffffffu, rb[i], sft);
+            }
+          float4* x4 = reinterpret_cast<float4*>(xch);
+          if (tm.l3 == 0) {
+            x4[tm.colhalf * 64 + tm.r0] = make_float4(ra[0], ra[1], ra[2], ra[3]);
+            x4[tm.colhalf * 64 + tm.r1] = make_float4(rb[0], rb[1], rb[2], rb[3]);
+          }
+          named_bar_sync(kBarPairS + tm.quad, 64);
+          {
+            const float4 o0 = x4[(tm.colhalf ^ 1) * 64 + tm.r0], o1 = x4[(tm.colhalf ^ 1) * 64 + tm.r1];
+            ra[0] += o0.x; ra[1] += o0.y; ra[2] += o0.z; ra[3] += o0.w;
+            rb[0] += o1.x; rb[1] += o1.y; rb[2] += o1.z; rb[3] += o1.w;
+          }
+          f32x2 sa0 = 0ull, sa1 = 0ull, sb0 = 0ull, sb1 = 0ull;      // sum g_std, sum g_xhat of the two rows
+          f32x2 cs[4];
+          {
+            const f32x2 n64 = pk1(-1.f / 64.f);
+            const f32x2 mA = mul2(pk1(ra[1]), n64), xA = mul2(pk1(ra[2]), n64), mB = mul2(pk1(rb[1]), n64), xB = mul2(pk1(rb[2]), n64);
+            const f32x2 fA3 = pk1(-ra[2] * rs0 * (1.f / 64.f)), fA4 = pk1(-ra[3] * rs0 * (1.f / 64.f));
+            const f32x2 fB3 = pk1(-rb[2] * rs1 * (1.f / 64.f)), fB4 = pk1(-rb[3] * rs1 * (1.f / 64.f));
+            f32x2 cl[4];
+            TokFrag dv;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const f32x2 gm = frag_col(tm, sGamma, q), neg = pk1(-1.f);
+              const f32x2 x0 = bf16x2_to_f32x2(xhw[2 * q]), x1 = bf16x2_to_f32x2(xhw[2 * q + 1]);
+              const f32x2 bt0 = mul2(add2(A.a[q], fma2(x0, xA, mA)), pk1(rs0));
+              const f32x2 bt1 = mul2(add2(A.b[q], fma2(x1, xB, mB)), pk1(rs1));
+              const f32x2 gl0 = mul2(gm, bt0), gl1 = mul2(gm, bt1);
+              cs[q] = add2(fma2(go.a[q], bt0, mul2(gl0, x0)), fma2(go.b[q], bt1, mul2(gl1, x1)));
+              cl[q] = add2(gl0, gl1);
+              dv.a[q] = mul2(gl0, neg);
+              dv.b[q] = mul2(gl1, neg);
+              kpa[q] = add2(kpa[q], gl0);
+              kpb[q] = add2(kpb[q], gl1);
+              const f32x2 gx0 = fma2(gl0, gm, fma2(mul2(go.a[q], gm), fA3, mul2(A.a[q], fA4)));
+              const f32x2 gx1 = fma2(gl1, gm, fma2(mul2(go.b[q], gm), fB3, mul2(A.b[q], fB4)));
+              sa0 = fma2(gx0, x0, fma2(A.a[q], bf16x2_to_f32x2(gzw[2 * q]), sa0));
+              sb0 = fma2(gx1, x1, fma2(A.b[q], bf16x2_to_f32x2(gzw[2 * q + 1]), sb0));
+              sa1 = add2(sa1, gx0);
+              sb1 = add2(sb1, gx1);
+              A.a[q] = gx0;
+              A.b[q] = gx1;
+            }
+            frag_st_tile(tm, tV, dv);       // over V (every thread overwrites the elements it has read)
+            dgam += frag_colsum(cs, lane);
+            dbet += frag_colsum(cl, lane);
+          }
+          float sa[2] = {-hsum(sa0) * rs0, hsum(sa1)}, sb[2] = {-hsum(sb0) * rs1, hsum(sb1)};
+          frag_allreduce2<1>(tm, sa, sb, xch + 256, kBarPairS);       // (behind the 2 KB of the exchange above)
+          {
+            const f32x2 k0 = pk1(sa[0] * (1.f / 64.f)), l0 = pk1(-sa[1] * rs0 * (1.f / 64.f));
+            const f32x2 k1 = pk1(sb[0] * (1.f / 64.f)), l1 = pk1(-sb[1] * rs1 * (1.f / 64.f));
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              A.a[q] = fma2(A.a[q], pk1(rs0), fma2(bf16x2_to_f32x2(xhw[2 * q]), k0, l0));      // gZin
+              A.b[q] = fma2(A.b[q], pk1(rs1), fma2(bf16x2_to_f32x2(xhw[2 * q + 1]), k1, l1));
+              cs[q] = add2(A.a[q], A.b[q]);
+            }
+            frag_st_tile(tm, tZin, A);
+            vec(OFF_CSS)[quad * 64 + frag_colsum_col(tm, lane)] = frag_colsum(cs, lane);
+          }
+          if (row_writer) {
+            p.d_eta[(sid * NC + i0 + j) * 64 + tm.r0] = __float2bfloat16(-ra[0]);
+            p.d_eta[(sid * NC + i0 + j) * 64 + tm.r1] = __float2bfloat16(-rb[0]);
+          }
+        }
+        if (loader) tma_wait_group_read<0>();      // dK of the step before has left its tile
+        fence_proxy_async_smem();
+        tc_fence_before_sync();
+        stop = named_bar_or(kBarS, kGroup, *abort_flag != 0);
+        if (loader) {
+          tma_store_2d(&tmDV, tV, 0, row_of(i0 + j));
+          tma_commit_group();
+          if (j > 0 && !stop) {
+            issue_gz(slot_of(g, j - 1));
+            tma_wait_group_read<0>();              // dV has left its tile
+            issue_v(i0 + j - 1);
+          }
+        }
+        if (gtid < 64) sGb[gtid] += quad_sum(vec(OFF_CSS), gtid);
+        if (stop) break;
+      }
+      if (stop) break;
+      // ---- what the group's last step adds, and its dK
+      if (cta_warp == 8) {
+        tc_fence_after_sync();
+        issue_tail(m - 1);
+        commit(BAR_TAIL);
+      }
+      finish_dk(m - 1);
+      wait_bar(BAR_TAIL, g);
+      mma_seen();
+      if (loader) *freed = m;
+      publish();
+      if (loader) {
+        tma_store_2d(&tmDK, tDK, 0, row_of(i0));
         tma_commit_group();
-        if (j + kStages < gsz) issue_inputs(j + kStages, false);   // this stage's K, Q, V have been read by everybody
       }
-      if (aborted) break;
-    }
-    if (aborted) break;
-
-    // ================================================================== reverse sweep
-    // scratch was written partly with generic-proxy stores by all threads (the 1/std vectors), partly with bulk
-    // stores by one thread: order both before the bulk copies that read it back
-    asm volatile("fence.proxy.async;" ::: "memory");
-    if (tid == kProd) tma_wait_group<0>();
-    publish();
-    if (tid == kProd) {
-      issue_inputs(gsz - 1, true);
-      issue_scratch(gsz - 1);
-      issue_wp(gsz - 1);
-    }
-    for (int j = gsz - 1; j >= 0; --j) {
-      const int s = j & kSt;
-      const int row0 = static_cast<int>(tok_rows0 + (long)(i0 + j) * 64);
-      uint8_t* sDga = tGo(s);      // see Lay
-      // the state after this mini-batch's update: the next mini-batch's pre-update copy, loaded for the previous
-      // step, or the group's last state
-      const uint8_t* Wpost = (j == gsz - 1) ? sW : tWP((j & 1) ^ 1);
-      // two stages: the other stage is free (the previous step has ended), the next step's tiles are requested now
-      if (kStages == 2 && tid == kProd && j > 0) {
-        issue_inputs(j - 1, true);
-        issue_scratch(j - 1);
-      }
-      wait_bar(BAR_IN + s);
-      wait_bar(BAR_SC + s);
-      const float* sigf = sSig + s * 128;
-      const float* sigl = sigf + 64;
-      const __nv_bfloat16* eta = sEta + s * 64;
-
-      // ---- S4: backward of the output LayerNorm
-      {
-        float go[16], xl[16], gam[8];
-        tok_ld_tile(tm, tGo(s), go);
-        tok_ld_tile(tm, tXL(s), xl);
-        tok_ld_cols(tm, sGamma, gam);
-        float a[2] = {0.f, 0.f}, b[2] = {0.f, 0.f};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h;
-            go[x0] *= gam[2 * q + h];
-            go[x1] *= gam[2 * q + h];
-            a[0] += go[x0]; a[1] = fmaf(go[x0], xl[x0], a[1]);
-            b[0] += go[x1]; b[1] = fmaf(go[x1], xl[x1], b[1]);
-          }
-        }
-        tok_row_allreduce<2, 2>(tm, a, b, sXch);
-        const float q0 = sigl[tm.r0] * (1.f / 64.f), q1 = sigl[tm.r1] * (1.f / 64.f);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h;
-            go[x0] = (64.f * go[x0] - a[0] - xl[x0] * a[1]) * q0;
-            go[x1] = (64.f * go[x1] - b[0] - xl[x1] * b[1]) * q1;
-          }
-        }
-        tok_st_tile(tm, sA, go);
-      }
-      publish();
-      // ---- A: dQ part = gZb W+^T;  G^T += gZb^T Q
-      TTT_ISSUE1(mma_hid64<true>(tmem + TM_A, smem_u32(sA), smem_u32(Wpost), 0u);
-                 mma_mn_accumulate(tmem + TM_G, smem_u32(sA), smem_u32(tQ(s)));
-                 mma_colsum(tmem + TM_B, smem_u32(sA), sOnes);
-                 mma_colsum(tmem + TM_B + 8, smem_u32(tGo(s)), sOnes))
-      {
-        // column sums over the tokens: d_beta += sum go and G_b += sum gZb by the tensor pipe, d_gamma += sum
-        // go * x_ln (a product of two tiles) by the warps
-        float a = 0.f;
-#pragma unroll 8
-        for (int r = cs_q * 16; r < cs_q * 16 + 16; ++r) a = fmaf(ld_elem(tGo(s), r, cs_f), ld_elem(tXL(s), r, cs_f), a);
-        part[tid] = a;
-        __syncthreads();
-        if (tid < 64) sDG[tid] += part_sum(0);
-      }
-      wait_mma();
-      add_colsum(sGb, TM_B, 1.f);
-      add_colsum(sDB, TM_B + 8, 1.f);
-      if (kStages == 2 && tid == kProd && j > 0) issue_wp(j - 1);   // the post-update copy has been read: its tile takes the next step's
-      {
-        float dq[16], go[16], w[16];
-        tok_ld(tm, tmem + TM_A, dq);
-        tok_ld_tile(tm, tGo(s), go);
-#pragma unroll
-        for (int q = 0; q < 16; ++q) go[q] += dq[q];
-        tok_st_global(tm, p.dXQ + static_cast<long>(row0) * 64, go);
-        tok_ld(tm, tmem + TM_G, w);
-        tok_st_tile(tm, sG, w);
-      }
-      publish();     // also orders the update of G_b before its use below
-      // ---- B: A1raw = K G;  T1 = gZ G^T
-      TTT_ISSUE1(mma_hid64<false>(tmem + TM_A, smem_u32(tK(s)), smem_u32(sG), 0u);
-                 mma_hid64<true>(tmem + TM_B, smem_u32(tGZ(s)), smem_u32(sG), 0u))
-      wait_mma();
-      float kp[16];        // gamma Bt - eta T1, completed to dK after phase C
-      {
-        float A[16], t1[16], gz[16], xh[16], go[16], kk[16];
-        float gam[8], bet[8], gb[8];
-        tok_ld(tm, tmem + TM_A, A);
-        tok_ld(tm, tmem + TM_B, t1);
-        tok_ld_tile(tm, tGZ(s), gz);
-        tok_ld_tile(tm, tXF(s), xh);
-        tok_ld_tile(tm, tV(s), go);
-        tok_ld_tile(tm, tK(s), kk);
-        tok_ld_cols(tm, sGamma, gam);
-        tok_ld_cols(tm, sBeta, bet);
-        tok_ld_cols(tm, sGb, gb);
-        const float eta0 = __bfloat162float(eta[tm.r0]), eta1 = __bfloat162float(eta[tm.r1]);
-        const float rs0 = sigf[tm.r0], rs1 = sigf[tm.r1];      // 1 / std
-        float ra[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, rb[5] = {0.f, 0.f, 0.f, 0.f, 0.f};   // d_eta terms, (unused), sum A, sum A xh, sum g xh
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h, c = 2 * q + h;
-            ra[0] = fmaf(t1[x0], kk[x0], fmaf(gb[c], gz[x0], ra[0]));
-            rb[0] = fmaf(t1[x1], kk[x1], fmaf(gb[c], gz[x1], rb[0]));
-            kp[x0] = -eta0 * t1[x0];
-            kp[x1] = -eta1 * t1[x1];
-            A[x0] = -eta0 * (A[x0] + gb[c]);
-            A[x1] = -eta1 * (A[x1] + gb[c]);
-            // go[] arrives holding V: grad_output_fused = gamma x_hat_fused + beta - (V - K)
-            go[x0] = fmaf(gam[c], xh[x0], bet[c]) - (go[x0] - kk[x0]);
-            go[x1] = fmaf(gam[c], xh[x1], bet[c]) - (go[x1] - kk[x1]);
-            ra[2] += A[x0];
-            rb[2] += A[x1];
-            ra[3] = fmaf(A[x0], xh[x0], ra[3]);
-            rb[3] = fmaf(A[x1], xh[x1], rb[3]);
-            ra[4] = fmaf(go[x0] * gam[c], xh[x0], ra[4]);
-            rb[4] = fmaf(go[x1] * gam[c], xh[x1], rb[4]);
-          }
-        }
-        tok_row_allreduce<5, 0>(tm, ra, rb, sXch);
-        float sa[2] = {0.f, 0.f}, sb[2] = {0.f, 0.f};      // sum g_std, sum g_xhat
-        float dga[16], dv[16];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int c = 2 * q + h;
-            const float gm = gam[c];
-            {
-              const int x = 4 * q + h;
-              const float bt = (A[x] - (ra[2] + xh[x] * ra[3]) * (1.f / 64.f)) * rs0;
-              const float gly = gm * bt;
-              dga[x] = fmaf(go[x], bt, gly * xh[x]);
-              dv[x] = -gly;
-              kp[x] += gly;
-              const float gxh = fmaf(gly, gm, -(go[x] * gm * ra[3] + A[x] * ra[4]) * rs0 * (1.f / 64.f));
-              sa[0] += (-gxh * xh[x] - A[x] * gz[x]) * rs0;
-              sa[1] += gxh;
-              A[x] = gxh;
-            }
-            {
-              const int x = 4 * q + 2 + h;
-              const float bt = (A[x] - (rb[2] + xh[x] * rb[3]) * (1.f / 64.f)) * rs1;
-              const float gly = gm * bt;
-              dga[x] = fmaf(go[x], bt, gly * xh[x]);
-              dv[x] = -gly;
-              kp[x] += gly;
-              const float gxh = fmaf(gly, gm, -(go[x] * gm * rb[3] + A[x] * rb[4]) * rs1 * (1.f / 64.f));
-              sb[0] += (-gxh * xh[x] - A[x] * gz[x]) * rs1;
-              sb[1] += gxh;
-              A[x] = gxh;
-            }
-          }
-        }
-        tok_st_tile(tm, sDga, dga);                          // d_gamma addends
-        tok_st_tile(tm, tV(s), dv);                          // dV over V: column-summed for d_beta
-        tok_st_global(tm, p.dXV + static_cast<long>(row0) * 64, dv);
-        tok_row_allreduce<2, 5>(tm, sa, sb, sXch);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h;
-            A[x0] = fmaf(A[x0], rs0, (sa[0] * xh[x0] - sa[1] * rs0) * (1.f / 64.f));   // gZin
-            A[x1] = fmaf(A[x1], rs1, (sb[0] * xh[x1] - sb[1] * rs1) * (1.f / 64.f));
-          }
-        }
-        tok_st_tile(tm, sZin, A);
-        if (row_writer) {
-          p.d_eta[(sid * NC + i0 + j) * 64 + tm.r0] = __float2bfloat16(-ra[0]);
-          p.d_eta[(sid * NC + i0 + j) * 64 + tm.r1] = __float2bfloat16(-rb[0]);
-        }
-      }
-      publish();
-      // ---- C: dK part = gZin W^T;  G^T += gZin^T K
-      // (T1 in the second accumulator has been read: its columns take the three column sums of this phase)
-      TTT_ISSUE1(mma_hid64<true>(tmem + TM_A, smem_u32(sZin), smem_u32(tWP(j & 1)), 0u);
-                 mma_mn_accumulate(tmem + TM_G, smem_u32(sZin), smem_u32(tK(s)));
-                 mma_colsum(tmem + TM_B, smem_u32(sZin), sOnes);
-                 mma_colsum(tmem + TM_B + 8, smem_u32(sDga), sOnes);
-                 mma_colsum(tmem + TM_B + 16, smem_u32(tV(s)), sOnes))
-      wait_mma();
-      add_colsum(sGb, TM_B, 1.f);
-      add_colsum(sDG, TM_B + 8, 1.f);
-      add_colsum(sDB, TM_B + 16, -1.f);
-      {
-        float acc[16];
-        tok_ld(tm, tmem + TM_A, acc);
-#pragma unroll
-        for (int q = 0; q < 16; ++q) kp[q] += acc[q];
-        tok_st_global(tm, p.dXK + static_cast<long>(row0) * 64, kp);
-      }
-      aborted = publish_vote();
-      if (aborted) break;
-      // one stage: everything of this step has been read, the next step's tiles are requested now
-      if (kStages == 1 && tid == kProd && j > 0) {
-        issue_inputs(j - 1, true);
-        issue_scratch(j - 1);
-        issue_wp(j - 1);
-      }
-    }
-  }
-#undef TTT_ISSUE1
-
-  // ---- final outputs: dL/d(initial state), norm gradients of this stream
-  if (!aborted) {
-    float w[16];
-    tok_ld(tm, tmem + TM_G, w);
-    float* Wo = p.gW + sid * 4096;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = tm.col(j);
-      Wo[c * 64 + tm.r0] = w[4 * j];
-      Wo[(c + 1) * 64 + tm.r0] = w[4 * j + 1];
-      Wo[c * 64 + tm.r1] = w[4 * j + 2];
-      Wo[(c + 1) * 64 + tm.r1] = w[4 * j + 3];
-    }
-    if (tid < 64) {
-      p.gb[sid * 64 + tid] = sGb[tid];
-      p.d_gamma[sid * 64 + tid] = sDG[tid];
-      p.d_beta[sid * 64 + tid] = sDB[tid];
-    }
-  }
-  if (tid == kProd) tma_wait_group<0>();
-  if (aborted) {
-    // everything this CTA still has in flight is waited for (bounded, not cut short by the abort flag)
-    // before its shared and tensor memory go away: the issuer's tensor-core work ...
-    if (warp == 0) {
-      if (elect_one()) umma_commit(&bars[BAR_DRAIN]);
       __syncwarp();
     }
-    if (tid == kProd) {
+    // ---- dL/d(initial state)
+    if (!stop) {
+      float w[16];
+      tok_ld(tm, tmem + TM_G, w);
+      float* Wo = p.gW + sid * 4096;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int c = tm.col(j);
+        Wo[c * 64 + tm.r0] = w[4 * j];
+        Wo[(c + 1) * 64 + tm.r0] = w[4 * j + 1];
+        Wo[c * 64 + tm.r1] = w[4 * j + 2];
+        Wo[(c + 1) * 64 + tm.r1] = w[4 * j + 3];
+      }
+    }
+    if (loader) tma_wait_group<0>();
+  }
+
+  // ---- norm gradients of this stream; teardown
+  tc_fence_before_sync();
+  const bool aborted = __syncthreads_or(stop || *abort_flag != 0) != 0;
+  tc_fence_after_sync();
+  if (!aborted) {
+    float* sum = vec(OFF_RK);      // [2 groups][d_gamma, d_beta][4 quadrants][64]
+    const int at = (recompute ? 0 : 512) + quad * 64 + frag_colsum_col(tm, lane);
+    sum[at] = dgam;
+    sum[at + 256] = dbet;
+    __syncthreads();
+    if (tid < 64) {
+      p.gb[sid * 64 + tid] = sGb[tid];
+      p.d_gamma[sid * 64 + tid] = quad_sum(sum, tid) + quad_sum(sum + 512, tid);
+      p.d_beta[sid * 64 + tid] = quad_sum(sum + 256, tid) + quad_sum(sum + 768, tid);
+    }
+  } else {
+    // everything this CTA still has in flight is waited for (bounded, not cut short by the abort flag)
+    // before its shared and tensor memory go away: the tensor-core work of both issuers, and the loads
+    if (warp == 0 && lead) umma_commit(&bars[BAR_DRAIN]);
+    if (tid == 0) {
       mbar_wait_bounded(&bars[BAR_DRAIN], 0, never_flag, limit);
-      // ... and its own loads
-      for (int b = 0; b < BAR_MMA; ++b)
-        if (pending & (1u << b)) mbar_wait_bounded(&bars[b], (ph >> b) & 1u, never_flag, limit);
+      for (int b = 0; b < kLoadBars; ++b)
+        if (loads[1] >> b & 1u) mbar_wait_bounded(&bars[b], (loads[0] >> b & 1u) ^ 1u, never_flag, limit);
       atomicExch(p.status, static_cast<uint32_t>(TTT_B200_ERR_TIMEOUT));
     }
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, TM_COLS);
+  if (cta_warp == 0) tmem_dealloc(tmem, TM_COLS);
 }
 
 }  // namespace
@@ -721,11 +840,14 @@ uint64_t ttt_linear_backward_scratch_bytes(int B, int H, int cgs) {
 int ttt_launch_linear_backward(const ttt_b200_linear_bwd_args* a, cudaStream_t stream, uint32_t* status,
                                uint64_t limit_ns, int drop_load) {
   const uint64_t rows = static_cast<uint64_t>(a->B) * a->H * a->NC * 64;
-  CUtensorMap tmQ, tmK, tmV, tmGo;
+  CUtensorMap tmQ, tmK, tmV, tmGo, tmDQ, tmDK, tmDV;
   if (int rc = ttt_make_tile_map(&tmQ, a->XQ, rows)) return rc;
   if (int rc = ttt_make_tile_map(&tmK, a->XK, rows)) return rc;
   if (int rc = ttt_make_tile_map(&tmV, a->XV, rows)) return rc;
   if (int rc = ttt_make_tile_map(&tmGo, a->grad_L_XQW_mini_batch, rows)) return rc;
+  if (int rc = ttt_make_tile_map(&tmDQ, a->grad_L_XQ, rows)) return rc;
+  if (int rc = ttt_make_tile_map(&tmDK, a->grad_L_XK, rows)) return rc;
+  if (int rc = ttt_make_tile_map(&tmDV, a->grad_L_XV, rows)) return rc;
   LinBwdParams p;
   p.eta = static_cast<const __nv_bfloat16*>(a->last_eta);
   p.gamma = a->ttt_norm_weight;
@@ -736,41 +858,20 @@ int ttt_launch_linear_backward(const ttt_b200_linear_bwd_args* a, cudaStream_t s
   p.d_gamma = a->grad_L_ttt_norm_weight; p.d_beta = a->grad_L_ttt_norm_bias;
   p.gW = a->grad_L_W1_init; p.gb = a->grad_L_b1_init;
   p.d_eta = static_cast<__nv_bfloat16*>(a->grad_L_last_eta);
-  p.dXQ = static_cast<__nv_bfloat16*>(a->grad_L_XQ);
-  p.dXK = static_cast<__nv_bfloat16*>(a->grad_L_XK);
-  p.dXV = static_cast<__nv_bfloat16*>(a->grad_L_XV);
   p.H = a->H; p.NC = a->NC; p.cgs = a->checkpoint_group_size; p.nck = a->num_checkpoints;
   p.drop_load = drop_load;
   p.status = status;
   p.wait_limit_ns = limit_ns;
   static std::once_flag once[64];
   static cudaError_t attr_err[64];
-  static int sms[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return ttt_set_error(TTT_B200_ERR_LAUNCH, "device index out of range");
   std::call_once(once[dev], [&] {
-    attr_err[dev] = cudaFuncSetAttribute(ttt_linear_bwd_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Lay<1>::SMEM_BYTES);
-    if (attr_err[dev] == cudaSuccess)
-      attr_err[dev] = cudaFuncSetAttribute(ttt_linear_bwd_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           Lay<2>::SMEM_BYTES);
-    sms[dev] = 148;
-    cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
+    attr_err[dev] = cudaFuncSetAttribute(ttt_linear_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   });
   if (attr_err[dev] != cudaSuccess) return ttt_set_error(TTT_B200_ERR_LAUNCH, cudaGetErrorString(attr_err[dev]));
-  // more streams than SMs: the form of which two CTAs fit on an SM; else the one that prefetches a step ahead
-  // (TTT_B200_LINEAR_BWD_STAGES = 1 or 2 overrides, for measurements)
-  static const int forced = [] {
-    const char* e = std::getenv("TTT_B200_LINEAR_BWD_STAGES");
-    return e ? std::atoi(e) : 0;
-  }();
-  const int streams = a->B * a->H;
-  const bool two_per_sm = forced == 1 || (forced != 2 && streams > sms[dev]);
-  if (two_per_sm)
-    ttt_linear_bwd_kernel<1><<<dim3(streams), dim3(kThreads), Lay<1>::SMEM_BYTES, stream>>>(tmQ, tmK, tmV, tmGo, p);
-  else
-    ttt_linear_bwd_kernel<2><<<dim3(streams), dim3(kThreads), Lay<2>::SMEM_BYTES, stream>>>(tmQ, tmK, tmV, tmGo, p);
+  ttt_linear_bwd_kernel<<<dim3(a->B * a->H), dim3(kThreads), SMEM_BYTES, stream>>>(tmQ, tmK, tmV, tmGo, tmDQ, tmDK, tmDV, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return ttt_set_error(TTT_B200_ERR_LAUNCH, cudaGetErrorString(e));
   return TTT_B200_OK;
