@@ -376,16 +376,6 @@ __device__ __forceinline__ void mma_64_tn_lead(uint32_t tmem_d, uint32_t a_smem,
 #pragma unroll
   for (int j = 0; j < 4; ++j) mma_lead<true>(tmem_d, a0 + j * (2048u >> 4), b0 + j * (2048u >> 4), idesc, lead);
 }
-// column sums of a [64 tok][64] tile: D[64 feat x 8] = T^T * ones (8 rows of bf16 ones)
-__device__ __forceinline__ void mma_colsum_lead(uint32_t tmem_d, uint32_t tile_smem, uint32_t ones_smem, uint32_t lead) {
-  constexpr uint32_t idesc = umma_idesc_bf16(64, 8, true, false, false);
-  const uint32_t a0 = desc_lo(tile_smem, TILE);
-  const uint32_t b0 = desc_lo(ones_smem, 16);
-  mma_lead<false>(tmem_d, a0, b0, idesc, lead);
-#pragma unroll
-  for (int j = 1; j < 4; ++j) mma_lead<true>(tmem_d, a0 + j * (2048u >> 4), b0 + j * (32u >> 4), idesc, lead);
-}
-
 // A warp's 32 rows x 32 fp32 columns (lane = row) -> a row-major global matrix with 64 floats per row, as whole
 // 128-byte lines, turned through the warp's own 4 KB of a hidden-major tile (16-byte chunks XOR-swizzled by row:
 // both directions conflict-free).
@@ -554,6 +544,14 @@ __device__ __forceinline__ void frag_st_tile(const TokMap& m, uint8_t* tile, con
   for (int j = 0; j < 4; ++j) {
     *reinterpret_cast<uint32_t*>(tile + m.off(m.r0, j)) = f32x2_to_bf16x2(f.a[j]);
     *reinterpret_cast<uint32_t*>(tile + m.off(m.r1, j)) = f32x2_to_bf16x2(f.b[j]);
+  }
+}
+// ... straight to a row-major [64][64] bf16 tile in global memory
+__device__ __forceinline__ void frag_st_global(const TokMap& m, __nv_bfloat16* tile, const TokFrag& f) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    *reinterpret_cast<uint32_t*>(tile + m.r0 * 64 + m.col(j)) = f32x2_to_bf16x2(f.a[j]);
+    *reinterpret_cast<uint32_t*>(tile + m.r1 * 64 + m.col(j)) = f32x2_to_bf16x2(f.b[j]);
   }
 }
 // per-column vector (fp32[64] in shared memory): the thread's four column pairs

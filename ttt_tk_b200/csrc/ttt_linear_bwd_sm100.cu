@@ -60,32 +60,30 @@ constexpr uint32_t OFF_RV = OFF_RQ + 2 * TILE;          // V, then x_f on its wa
 constexpr uint32_t OFF_RGO = OFF_RV + 2 * TILE;         // dL/dOut, then dQ on its way out
 constexpr uint32_t OFF_RW = OFF_RGO + 2 * TILE;         // bf16 W^T before / after the update
 constexpr uint32_t OFF_RGZ = OFF_RW + 2 * TILE;
-constexpr uint32_t OFF_RU = OFF_RGZ + TILE;
-constexpr uint32_t OFF_RGZB = OFF_RU + TILE;
-constexpr uint32_t OFF_SK = OFF_RGZB + TILE;            // sweep: + stage
+constexpr uint32_t OFF_RU = OFF_RGZ + TILE;             // U, then gZb
+constexpr uint32_t OFF_SK = OFF_RU + TILE;              // sweep: + stage
 constexpr uint32_t OFF_SQ = OFF_SK + 2 * TILE;
-constexpr uint32_t OFF_SV = OFF_SQ + TILE;              // V, then dV on its way out
-constexpr uint32_t OFF_SXF = OFF_SV + TILE;
-constexpr uint32_t OFF_SGZ = OFF_SXF + TILE;
-constexpr uint32_t OFF_SGZB = OFF_SGZ + TILE;
+constexpr uint32_t OFF_SV = OFF_SQ + TILE;              // + stage: V, then dV on its way out
+constexpr uint32_t OFF_SXF = OFF_SV + 2 * TILE;         // + stage
+constexpr uint32_t OFF_SGZ = OFF_SXF + 2 * TILE;        // + stage
+constexpr uint32_t OFF_SGZB = OFF_SGZ + 2 * TILE;
 constexpr uint32_t OFF_SWP = OFF_SGZB + TILE;           // bf16 W^T before the update
 constexpr uint32_t OFF_SG = OFF_SWP + TILE;             // bf16 G^T
 constexpr uint32_t OFF_SZIN = OFF_SG + TILE;
 constexpr uint32_t OFF_SDK = OFF_SZIN + TILE;           // dK on its way out
-constexpr uint32_t OFF_ONES = OFF_SDK + TILE;           // bf16[8][64] ones: B operand of the column sums
-constexpr uint32_t OFF_RETA = OFF_ONES + 1024;          // bf16[2][64]
+constexpr uint32_t OFF_RETA = OFF_SDK + TILE;           // bf16[2][64]
 constexpr uint32_t OFF_SETA = OFF_RETA + 256;           // bf16[2][64]
 constexpr uint32_t OFF_RVEC = OFF_SETA + 256;           // fp32[2][128]: the slot's vectors on their way out
-constexpr uint32_t OFF_SVEC = OFF_RVEC + 1024;          // fp32[128]
-constexpr uint32_t OFF_B = OFF_SVEC + 512;
+constexpr uint32_t OFF_SVEC = OFF_RVEC + 1024;          // fp32[2][128]
+constexpr uint32_t OFF_B = OFF_SVEC + 1024;
 constexpr uint32_t OFF_GB = OFF_B + 256;
 constexpr uint32_t OFF_GAMMA = OFF_GB + 256;
 constexpr uint32_t OFF_BETA = OFF_GAMMA + 256;
 constexpr uint32_t OFF_CSR = OFF_BETA + 256;            // fp32[4][64] column sums, one row per quadrant
 constexpr uint32_t OFF_CSS = OFF_CSR + 1024;
 constexpr uint32_t OFF_XR = OFF_CSS + 1024;             // row-sum exchange of each group
-constexpr uint32_t OFF_XS = OFF_XR + 4096;
-constexpr uint32_t OFF_BAR = OFF_XS + 4096;
+constexpr uint32_t OFF_XS = OFF_XR + kXchBytes;
+constexpr uint32_t OFF_BAR = OFF_XS + 3072;
 constexpr uint32_t OFF_MISC = OFF_BAR + 192;
 constexpr uint32_t SMEM_USED = OFF_MISC + 64;
 constexpr uint32_t SMEM_BYTES = SMEM_USED + 1024;       // slack for the 1024-byte alignment
@@ -93,24 +91,21 @@ static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB per-CTA shared memory of
 
 // barriers: loads first (their completion is what an aborting CTA still waits for)
 constexpr int BAR_RIN = 0;                              // recompute, + stage: K, eta, Q, V, dL/dOut
-constexpr int BAR_SK = 2;                               // sweep, + stage: K, eta
-constexpr int BAR_SQB = 4;                              // Q, gZb, vectors
-constexpr int BAR_SGZ = 5;                              // gZ, x_f
-constexpr int BAR_SV = 6;
-constexpr int BAR_SWP = 7;
-constexpr int kLoadBars = 8;
-constexpr int BAR_RM = 8;                               // the recompute's products: four uses per mini-batch
-constexpr int BAR_DK = 9, BAR_P1 = 10, BAR_P2 = 11;     // the sweep's
-constexpr int BAR_GROUP = 12;                           // a group's slots are written
-constexpr int BAR_TAIL = 13;
-constexpr int BAR_DRAIN = 14;                           // abort path only
-constexpr int kBars = 15;
+constexpr int BAR_SIN = 2;                              // sweep, + stage: K, eta, V, gZ, x_f, vectors
+constexpr int BAR_SQB = 4;                              // Q, gZb
+constexpr int BAR_SWP = 5;
+constexpr int kLoadBars = 6;
+constexpr int BAR_RM = 6;                               // the recompute's products: four uses per mini-batch
+constexpr int BAR_DK = 7, BAR_P1 = 8, BAR_P2 = 9;       // the sweep's
+constexpr int BAR_GROUP = 10;                           // a group's slots are written
+constexpr int BAR_TAIL = 11;
+constexpr int BAR_DRAIN = 12;                           // abort path only
+constexpr int kBars = 13;
 
 // tensor-memory columns
 constexpr uint32_t TM_W = 0;
 constexpr uint32_t TM_G = 64;
 constexpr uint32_t TM_R = 128;        // recompute accumulator
-constexpr uint32_t TM_RC = 192;       // its column sums
 constexpr uint32_t TM_SA = 256;       // sweep accumulators
 constexpr uint32_t TM_SB = 320;
 constexpr uint32_t TM_COLS = 512;
@@ -195,8 +190,6 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     sBeta[tid] = p.beta[head * 64 + tid];
     sGb[tid] = p.gb_last[sid * 64 + tid];
   }
-  if (tid < 256) reinterpret_cast<uint32_t*>(smem + OFF_ONES)[tid] = 0x3F803F80u;     // 256 x two bf16 ones
-  fence_proxy_async_smem();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -303,7 +296,7 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         uint8_t* tWn = tile(OFF_RW, s ^ 1);
         uint8_t* tGZ = tile(OFF_RGZ);
         uint8_t* tU = tile(OFF_RU);
-        uint8_t* tGZB = tile(OFF_RGZB);
+        uint8_t* tGZB = tU;              // U is dead after MMA2
         float* sVec = vec(OFF_RVEC) + s * 128;
         float* xch = vec(OFF_XR);
         const __nv_bfloat16* eta = reinterpret_cast<const __nv_bfloat16*>(smem + OFF_RETA) + s * 64;
@@ -353,6 +346,7 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           frag_allreduce2<1>(tm, a, b, xch, kBarPairR);
           const f32x2 sc0 = pk1(rs0 * (1.f / 64.f)), sc1 = pk1(rs1 * (1.f / 64.f));
           const f32x2 ne0 = pk1(-__bfloat162float(eta[tm.r0])), ne1 = pk1(-__bfloat162float(eta[tm.r1]));
+          f32x2 su[4];
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const uint32_t w0 = f32x2_to_bf16x2(mul2(fma2(x.a[q], pk1(-a[1]), fma2(gr.a[q], pk1(64.f), pk1(-a[0]))), sc0));
@@ -361,8 +355,12 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             *reinterpret_cast<uint32_t*>(tGZ + tm.off(tm.r1, q)) = w1;
             gr.a[q] = mul2(bf16x2_to_f32x2(w0), ne0);
             gr.b[q] = mul2(bf16x2_to_f32x2(w1), ne1);
+            su[q] = add2(gr.a[q], gr.b[q]);
           }
           frag_st_tile(tm, tU, gr);
+          // (column sums in registers: seven shuffles, off the tensor pipe, where four N = 8 MMAs behind the update cost
+          // as much latency as a whole product)
+          vec(OFF_CSR)[quad * 64 + frag_colsum_col(tm, lane)] = frag_colsum(su, lane);
           if (row_writer) {
             sVec[tm.r0] = rs0;
             sVec[tm.r1] = rs1;
@@ -370,11 +368,10 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
         publish();
 
-        // ---- MMA2: W^T += U^T K;  b += column sums of U
+        // ---- MMA2: W^T += U^T K
         if (cta_warp == 0) {
           tc_fence_after_sync();
           mma_64_tn_lead(tmem + TM_W, smem_u32(tU), smem_u32(tK), lead);
-          mma_colsum_lead(tmem + TM_RC, smem_u32(tU), smem_u32(smem + OFF_ONES), lead);
           commit(BAR_RM);
         }
         if (loader) {
@@ -385,11 +382,8 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           tma_commit_group();
         }
         __syncwarp();
+        if (gtid < 64) sB[gtid] += quad_sum(vec(OFF_CSR), gtid);      // its next reader comes after the barrier below
         wait_mma();
-        if (warp < 4) {
-          const float cs = colsum_read(tmem + TM_RC, warp);
-          if (lane < 16) sB[16 * warp + lane] += cs;       // its next reader comes after the barrier below
-        }
         // ---- EPI: bf16 copy of the new W^T
         {
           TokFrag w;
@@ -453,6 +447,11 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           mma_64_lead<true, false>(tmem + TM_R, smem_u32(tGZB), smem_u32(tWn), lead);
           commit(BAR_RM);
         }
+        if (loader) {
+          bulk_store_1d(sl + SL_GZB, tGZB, TILE);
+          tma_commit_group();
+        }
+        __syncwarp();
         if (gtid < 64) sVec[64 + gtid] = quad_sum(vec(OFF_CSR), gtid);
         wait_mma();
         // ---- dQ = go + gZb W+^T, over the dL/dOut tile
@@ -468,13 +467,12 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           }
           frag_st_tile(tm, tGo, x);
         }
-        if (loader) tma_wait_group_read<0>();        // W, x_f and gZ have left their tiles
+        if (loader) tma_wait_group_read<0>();        // W, x_f, gZ and gZb have left their tiles
         fence_proxy_async_smem();
         tc_fence_before_sync();
         stop = named_bar_or(kBarR, kGroup, *abort_flag != 0);
         if (loader) {
           tma_store_2d(&tmDQ, tGo, 0, row_of(i0 + j));
-          bulk_store_1d(sl + SL_GZB, tGZB, TILE);
           bulk_store_1d(sl + SL_VEC, sVec, 512);
           tma_commit_group();
         }
@@ -494,15 +492,11 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       named_bar_sync(kBarS, kGroup);
     };
     uint8_t* tQ = tile(OFF_SQ);
-    uint8_t* tV = tile(OFF_SV);
-    uint8_t* tXF = tile(OFF_SXF);
-    uint8_t* tGZ = tile(OFF_SGZ);
     uint8_t* tGZB = tile(OFF_SGZB);
     uint8_t* tWP = tile(OFF_SWP);
     uint8_t* tG = tile(OFF_SG);
     uint8_t* tZin = tile(OFF_SZIN);
     uint8_t* tDK = tile(OFF_SDK);
-    float* sVec = vec(OFF_SVEC);
     float* xch = vec(OFF_XS);
     {   // the gradient state starts as dL/d(final state)
       float w[16];
@@ -515,26 +509,21 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     tc_fence_after_sync();
 
     // loads of one step, in parts, each issued when its tiles are free (loader)
-    auto issue_k = [&](int i, uint32_t cnt) {
+    auto issue_in = [&](int i, const uint8_t* sl, uint32_t cnt) {
       const int s = cnt & 1;
-      expect(BAR_SK + s, TILE + 128);
-      tma_load_2d(tile(OFF_SK, s), &tmK, &bars[BAR_SK + s], 0, row_of(i));
-      bulk_load_1d(smem + OFF_SETA + s * 128, p.eta + (sid * NC + i) * 64, 128, &bars[BAR_SK + s]);
+      uint64_t* b = &bars[BAR_SIN + s];
+      expect(BAR_SIN + s, 4 * TILE + 128 + 512);
+      tma_load_2d(tile(OFF_SK, s), &tmK, b, 0, row_of(i));
+      tma_load_2d(tile(OFF_SV, s), &tmV, b, 0, row_of(i));
+      bulk_load_1d(tile(OFF_SGZ, s), sl + SL_GZ, TILE, b);
+      bulk_load_1d(tile(OFF_SXF, s), sl + SL_XF, TILE, b);
+      bulk_load_1d(smem + OFF_SETA + s * 128, p.eta + (sid * NC + i) * 64, 128, b);
+      bulk_load_1d(vec(OFF_SVEC) + s * 128, sl + SL_VEC, 512, b);
     };
     auto issue_qb = [&](int i, const uint8_t* sl) {
       expect(BAR_SQB, 2 * TILE);
       tma_load_2d(tQ, &tmQ, &bars[BAR_SQB], 0, row_of(i));
       bulk_load_1d(tGZB, sl + SL_GZB, TILE, &bars[BAR_SQB]);
-    };
-    auto issue_gz = [&](const uint8_t* sl) {
-      expect(BAR_SGZ, 2 * TILE + 512);
-      bulk_load_1d(tGZ, sl + SL_GZ, TILE, &bars[BAR_SGZ]);
-      bulk_load_1d(tXF, sl + SL_XF, TILE, &bars[BAR_SGZ]);
-      bulk_load_1d(sVec, sl + SL_VEC, 512, &bars[BAR_SGZ]);
-    };
-    auto issue_v = [&](int i) {
-      expect(BAR_SV, TILE);
-      tma_load_2d(tV, &tmV, &bars[BAR_SV], 0, row_of(i));
     };
     auto issue_wp = [&](const uint8_t* sl) {
       expect(BAR_SWP, TILE);
@@ -570,16 +559,18 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const int j = gsz - 1;
         const uint8_t* sl = slot_of(g, j);
         issue_qb(i0 + j, sl);
-        issue_k(i0 + j, m);
-        issue_gz(sl);
         tma_wait_group_read<0>();
-        issue_v(i0 + j);
+        issue_in(i0 + j, sl, m);
       }
       __syncwarp();
       for (int j = gsz - 1; j >= 0; --j, ++m) {
         const uint32_t par = m & 1;
         const bool first = j == gsz - 1;
-        uint8_t* tK = tile(OFF_SK, m & 1);
+        uint8_t* tK = tile(OFF_SK, par);
+        uint8_t* tV = tile(OFF_SV, par);
+        uint8_t* tXF = tile(OFF_SXF, par);
+        uint8_t* tGZ = tile(OFF_SGZ, par);
+        const float* sVec = vec(OFF_SVEC) + par * 128;
         const __nv_bfloat16* eta = reinterpret_cast<const __nv_bfloat16*>(smem + OFF_SETA) + par * 64;
 
         // ---- P1: the step before's dK product and state gradient; G^T += gZb^T Q
@@ -598,8 +589,9 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           if (!first) *freed = m;            // the step before's slot has been read (its last tile, W, just now)
           issue_wp(slot_of(g, j));
           if (j > 0) {
-            issue_k(i0 + j - 1, m + 1);
             issue_qb(i0 + j - 1, slot_of(g, j - 1));
+            tma_wait_group_read<0>();        // dV of the step before has left the tile V comes into
+            issue_in(i0 + j - 1, slot_of(g, j - 1), m + 1);
           }
         }
         // ---- E2: bf16 copy of G^T
@@ -608,15 +600,13 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           frag_ld(tm, tmem + TM_G, w);
           frag_st_tile(tm, tG, w);
         }
-        wait_bar(BAR_SGZ, par);
+        wait_bar(BAR_SIN + par, m >> 1);
         if (gtid < 64) sGb[gtid] += sVec[64 + gtid];
         publish();
 
         // ---- P2: K G, T1 = gZ G^T
         if (cta_warp == 8) {
           tc_fence_after_sync();
-          wait_bar(BAR_SK + par, m >> 1);
-          mma_seen();
           mma_64_lead<false, false>(tmem + TM_SA, smem_u32(tK), smem_u32(tG), lead);
           mma_64_lead<true, false>(tmem + TM_SB, smem_u32(tGZ), smem_u32(tG), lead);
           commit(BAR_P2);
@@ -626,8 +616,6 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           tma_commit_group();
         }
         __syncwarp();
-        wait_bar(BAR_SK + par, m >> 1);
-        wait_bar(BAR_SV, par);
         // ---- E4: second order through the fused LayerNorm + L2 gradient
         {
           TokFrag A, t1, go;
@@ -756,11 +744,6 @@ ttt_linear_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (loader) {
           tma_store_2d(&tmDV, tV, 0, row_of(i0 + j));
           tma_commit_group();
-          if (j > 0 && !stop) {
-            issue_gz(slot_of(g, j - 1));
-            tma_wait_group_read<0>();              // dV has left its tile
-            issue_v(i0 + j - 1);
-          }
         }
         if (gtid < 64) sGb[gtid] += quad_sum(vec(OFF_CSS), gtid);
         if (stop) break;

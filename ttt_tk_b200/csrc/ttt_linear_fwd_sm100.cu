@@ -45,9 +45,9 @@ constexpr uint32_t OFF_GAMMA = OFF_B + 256;
 constexpr uint32_t OFF_BETA = OFF_GAMMA + 256;
 constexpr uint32_t OFF_BAR = OFF_BETA + 256;
 constexpr uint32_t OFF_MISC = OFF_BAR + 64;
-constexpr uint32_t OFF_XCH = OFF_MISC + 64;             // fp32[2][64][8] row-sum exchange between warp pairs
-constexpr uint32_t OFF_ONES = (OFF_XCH + 4096 + 1023) & ~1023u;   // bf16[8][64] ones: B operand of the column sums
-constexpr uint32_t SMEM_USED = OFF_ONES + 1024;
+constexpr uint32_t OFF_XCH = OFF_MISC + 64;             // row-sum exchange between warp pairs
+constexpr uint32_t OFF_CS = OFF_XCH + kXchBytes;        // fp32[4][64] column sums, one row per quadrant
+constexpr uint32_t SMEM_USED = OFF_CS + 1024;
 constexpr uint32_t SMEM_BYTES = SMEM_USED + 1024;       // slack for the 1024-byte alignment
 static_assert(3 * (SMEM_BYTES + 1024) <= 233472, "three CTAs per SM");
 
@@ -71,15 +71,6 @@ struct LinParams {
   uint32_t* status;
   uint64_t wait_limit_ns;
 };
-
-// D[64 x 64] += A^T B with both operands [64 k][64] tiles read MN-major (row = contraction index)
-__device__ __forceinline__ void mma_mn_accumulate(uint32_t tmem_d, uint32_t a_smem, uint32_t b_smem) {
-  constexpr uint32_t idesc = umma_idesc_bf16(64, 64, true, true, false);
-  const uint32_t a0 = desc_lo(a_smem, TILE);
-  const uint32_t b0 = desc_lo(b_smem, TILE);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) mma_issue_rt(tmem_d, a0 + j * (2048u >> 4), b0 + j * (2048u >> 4), idesc, 1u);
-}
 
 __global__ void __launch_bounds__(kThreads, 3)
 ttt_linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -129,7 +120,6 @@ ttt_linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     sBeta[tid] = p.beta[head * 64 + tid];
     sB[tid] = p.b[stream_id * 64 + tid];
   }
-  reinterpret_cast<uint32_t*>(smem + OFF_ONES)[tid] = 0x3F803F80u;     // 256 x two bf16 ones
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -197,15 +187,8 @@ ttt_linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     tc_fence_before_sync();
     __syncthreads();
   };
-#define TTT_ISSUE1(WORK)            \
-  if (warp == 0) {                  \
-    if (elect_one()) {              \
-      tc_fence_after_sync();        \
-      WORK;                         \
-      umma_commit(mma_bar);         \
-    }                               \
-    __syncwarp();                   \
-  }
+  const uint32_t lead = elect_one() ? 1u : 0u;      // the lane of warp 0 that issues the MMAs
+  float* sCS = reinterpret_cast<float*>(smem + OFF_CS);
 
   int it = 0;
   for (; it < NC; ++it) {
@@ -217,7 +200,11 @@ ttt_linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     mbar_wait_bounded(&full[s], (it / kStages) & 1, abort_flag, limit);
 
     // ---- MMA1: Z = K W
-    TTT_ISSUE1(mma_hid64<false>(tmem + TM_Z, smem_u32(sK), smem_u32(sW), 0u))
+    if (warp == 0) {
+      tc_fence_after_sync();
+      mma_64_lead<false, false>(tmem + TM_Z, smem_u32(sK), smem_u32(sW), lead);
+      if (lead) umma_commit(mma_bar);
+    }
     // a checkpoint (the state before this mini-batch) leaves while MMA1 runs: it only reads the state
     if (it % p.cgs == 0) {
       const long ckc = stream_id * p.nck + it / p.cgs;
@@ -225,98 +212,93 @@ ttt_linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       tc_fence_before_sync();      // the state columns are written by the second MMA group
     }
     wait_mma();
-    // ---- LN: fused LayerNorm + L2 gradient, U = -eta * dl/dZ
+    // ---- LN: fused LayerNorm + L2 gradient, U = -eta * dl/dZ; its column sums (in registers: four N = 8 MMAs behind the
+    // update would cost as much latency as a whole product)
     {
-      float xh[16], bc[8], gam[8], bet[8];
-      tok_ld(tm, tmem + TM_Z, xh);
-      tok_ld_cols(tm, sB, bc);
-      tok_ld_cols(tm, sGamma, gam);
-      tok_ld_cols(tm, sBeta, bet);
+      TokFrag x, g;
+      uint32_t kk[8], vv[8];
+      frag_ld(tm, tmem + TM_Z, x);
+      frag_ld_raw(tm, sK, kk);
+      frag_ld_raw(tm, sV, vv);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        xh[4 * j] += bc[2 * j]; xh[4 * j + 1] += bc[2 * j + 1];
-        xh[4 * j + 2] += bc[2 * j]; xh[4 * j + 3] += bc[2 * j + 1];
+        const f32x2 b = frag_col(tm, sB, j);
+        x.a[j] = add2(x.a[j], b);
+        x.b[j] = add2(x.b[j], b);
       }
       float rs0, rs1;
-      float kk[16], vv[16], g[16];
-      tok_ld_tile(tm, sK, kk);
-      tok_ld_tile(tm, sV, vv);
-      tok_layernorm(tm, xh, TTT_LN_EPS, sXch, rs0, rs1);
-      float a[2] = {0.f, 0.f}, b[2] = {0.f, 0.f};
+      frag_layernorm(tm, x, TTT_LN_EPS, sXch, 1, rs0, rs1);
+      f32x2 a0 = 0ull, a1 = 0ull, c0 = 0ull, c1 = 0ull;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i0 = 4 * j + e, i1 = 4 * j + 2 + e, c = 2 * j + e;
-          xh[i0] *= rs0;
-          xh[i1] *= rs1;
-          g[i0] = (fmaf(gam[c], xh[i0], bet[c]) - (vv[i0] - kk[i0])) * gam[c];
-          g[i1] = (fmaf(gam[c], xh[i1], bet[c]) - (vv[i1] - kk[i1])) * gam[c];
-          a[0] += g[i0]; a[1] = fmaf(g[i0], xh[i0], a[1]);
-          b[0] += g[i1]; b[1] = fmaf(g[i1], xh[i1], b[1]);
-        }
+        const f32x2 gam = frag_col(tm, sGamma, j), bet = frag_col(tm, sBeta, j), neg = pk1(-1.f);
+        const f32x2 t0 = fma2(bf16x2_to_f32x2(vv[2 * j]), neg, bf16x2_to_f32x2(kk[2 * j]));          // K - V
+        const f32x2 t1 = fma2(bf16x2_to_f32x2(vv[2 * j + 1]), neg, bf16x2_to_f32x2(kk[2 * j + 1]));
+        g.a[j] = mul2(fma2(gam, x.a[j], add2(t0, bet)), gam);
+        g.b[j] = mul2(fma2(gam, x.b[j], add2(t1, bet)), gam);
+        a0 = add2(a0, g.a[j]); a1 = fma2(g.a[j], x.a[j], a1);
+        c0 = add2(c0, g.b[j]); c1 = fma2(g.b[j], x.b[j], c1);
       }
-      tok_row_allreduce<2, 2>(tm, a, b, sXch);
-      const float sc0 = -__bfloat162float(sEta[tm.r0]) * rs0 * (1.f / 64.f);
-      const float sc1 = -__bfloat162float(sEta[tm.r1]) * rs1 * (1.f / 64.f);
+      float a[2] = {hsum(a0), hsum(a1)}, b[2] = {hsum(c0), hsum(c1)};
+      frag_allreduce2<1>(tm, a, b, sXch, 1);
+      const f32x2 sc0 = pk1(-__bfloat162float(sEta[tm.r0]) * rs0 * (1.f / 64.f));
+      const f32x2 sc1 = pk1(-__bfloat162float(sEta[tm.r1]) * rs1 * (1.f / 64.f));
+      f32x2 su[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i0 = 4 * j + e, i1 = 4 * j + 2 + e;
-          g[i0] = (64.f * g[i0] - a[0] - xh[i0] * a[1]) * sc0;
-          g[i1] = (64.f * g[i1] - b[0] - xh[i1] * b[1]) * sc1;
-        }
+        g.a[j] = mul2(fma2(x.a[j], pk1(-a[1]), fma2(g.a[j], pk1(64.f), pk1(-a[0]))), sc0);
+        g.b[j] = mul2(fma2(x.b[j], pk1(-b[1]), fma2(g.b[j], pk1(64.f), pk1(-b[0]))), sc1);
+        su[j] = add2(g.a[j], g.b[j]);
       }
-      tok_st_tile(tm, sU, g);
+      frag_st_tile(tm, sU, g);
+      sCS[tm.quad * 64 + frag_colsum_col(tm, lane)] = frag_colsum(su, lane);
     }
     publish();
 
-    // ---- MMA2: W^T += U^T K; the column sums of U (the bf16 operand the update sees) for b are taken by the
-    // tensor pipe in the same phase, into the accumulator columns that are free between Z and Zb
-    TTT_ISSUE1(mma_mn_accumulate(tmem + TM_W, smem_u32(sU), smem_u32(sK));
-               mma_colsum(tmem + TM_Z, smem_u32(sU), smem_u32(smem + OFF_ONES)))
-    wait_mma();
-    if (warp < 4) {
-      const float cs = colsum_read(tmem + TM_Z, warp);
-      if (lane < 16) sB[16 * warp + lane] += cs;       // its next reader comes after the barrier below
+    // ---- MMA2: W^T += U^T K;  b += column sums of U
+    if (warp == 0) {
+      tc_fence_after_sync();
+      mma_64_tn_lead(tmem + TM_W, smem_u32(sU), smem_u32(sK), lead);
+      if (lead) umma_commit(mma_bar);
     }
+    if (tid < 64) sB[tid] += (sCS[tid] + sCS[64 + tid]) + (sCS[128 + tid] + sCS[192 + tid]);     // read after the barrier below
+    wait_mma();
     // ---- EPI: refresh the bf16 operand copy of the state
     {
-      float w[16];
-      tok_ld(tm, tmem + TM_W, w);
-      tok_st_tile(tm, sW, w);
+      TokFrag w;
+      frag_ld(tm, tmem + TM_W, w);
+      frag_st_tile(tm, sW, w);
     }
     publish();
 
     // ---- MMA3: Zb = Q W
-    TTT_ISSUE1(mma_hid64<false>(tmem + TM_Z, smem_u32(sQ), smem_u32(sW), 0u))
+    if (warp == 0) {
+      tc_fence_after_sync();
+      mma_64_lead<false, false>(tmem + TM_Z, smem_u32(sQ), smem_u32(sW), lead);
+      if (lead) umma_commit(mma_bar);
+    }
     wait_mma();
     // ---- OUT: Q + gamma * LN(Zb + b) + beta, straight to global memory
     {
-      float z[16], bc[8], gam[8], bet[8], q[16];
-      tok_ld(tm, tmem + TM_Z, z);
-      tok_ld_cols(tm, sB, bc);
-      tok_ld_cols(tm, sGamma, gam);
-      tok_ld_cols(tm, sBeta, bet);
+      TokFrag x;
+      uint32_t q[8];
+      frag_ld(tm, tmem + TM_Z, x);
+      frag_ld_raw(tm, sQ, q);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        z[4 * j] += bc[2 * j]; z[4 * j + 1] += bc[2 * j + 1];
-        z[4 * j + 2] += bc[2 * j]; z[4 * j + 3] += bc[2 * j + 1];
+        const f32x2 b = frag_col(tm, sB, j);
+        x.a[j] = add2(x.a[j], b);
+        x.b[j] = add2(x.b[j], b);
       }
       float rs0, rs1;
-      tok_ld_tile(tm, sQ, q);
-      tok_layernorm(tm, z, TTT_LN_EPS, sXch, rs0, rs1);
+      frag_layernorm(tm, x, TTT_LN_EPS, sXch, 1, rs0, rs1);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i0 = 4 * j + e, i1 = 4 * j + 2 + e, c = 2 * j + e;
-          q[i0] += fmaf(gam[c], z[i0] * rs0, bet[c]);
-          q[i1] += fmaf(gam[c], z[i1] * rs1, bet[c]);
-        }
+        const f32x2 gam = frag_col(tm, sGamma, j), bet = frag_col(tm, sBeta, j);
+        x.a[j] = add2(bf16x2_to_f32x2(q[2 * j]), fma2(gam, x.a[j], bet));
+        x.b[j] = add2(bf16x2_to_f32x2(q[2 * j + 1]), fma2(gam, x.b[j], bet));
       }
-      tok_st_global(tm, p.out + (stream_id * NC + it) * 4096, q);
+      frag_st_global(tm, p.out + (stream_id * NC + it) * 4096, x);
     }
     // every warp has read this stage's tiles and the tensor-memory tile: the stage takes the loads of the
     // mini-batch kStages ahead, and all threads take the same decision on leaving the loop
@@ -328,7 +310,6 @@ ttt_linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       ++loads_issued;
     }
   }
-#undef TTT_ISSUE1
 
   // ---- epilogue: optional final state, then teardown
   const bool aborted = __syncthreads_or(*abort_flag != 0) != 0;
@@ -336,10 +317,7 @@ ttt_linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   if (aborted) {
     // everything this CTA still has in flight is waited for (bounded, not cut short by the abort flag)
     // before its shared and tensor memory go away: the issuer's tensor-core work ...
-    if (warp == 0) {
-      if (elect_one()) umma_commit(drain_bar);
-      __syncwarp();
-    }
+    if (warp == 0 && lead) umma_commit(drain_bar);
     if (tid == kProd) {
       mbar_wait_bounded(drain_bar, 0, never_flag, limit);
       // ... and its own loads
