@@ -79,9 +79,7 @@ constexpr uint32_t OFF_B2 = OFF_T + 7 * TILE;        // fp32[64]  b2 (recompute)
 constexpr uint32_t OFF_GB2 = OFF_B2 + 256;           // fp32[64]  dL/db2 state
 constexpr uint32_t OFF_GAMMA = OFF_GB2 + 256;
 constexpr uint32_t OFF_BETA = OFF_GAMMA + 256;
-constexpr uint32_t OFF_DG = OFF_BETA + 256;          // fp32[64]  d_gamma accumulator
-constexpr uint32_t OFF_DB = OFF_DG + 256;            // fp32[64]  d_beta accumulator
-constexpr uint32_t OFF_SIGLN = OFF_DB + 256;         // fp32[64]
+constexpr uint32_t OFF_SIGLN = OFF_BETA + 256;       // fp32[64]
 constexpr uint32_t OFF_SIGF = OFF_SIGLN + 256;       // fp32[64]
 constexpr uint32_t OFF_GB1 = OFF_SIGF + 256;         // fp32[256] copy of the per-thread dL/db1
 constexpr uint32_t OFF_PART = OFF_GB1 + 1024;        // fp32[8][64] partial sums for d_eta (one row per warp)
@@ -155,8 +153,6 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   float* sGb2 = reinterpret_cast<float*>(smem + OFF_GB2);
   float* sGamma = reinterpret_cast<float*>(smem + OFF_GAMMA);
   float* sBeta = reinterpret_cast<float*>(smem + OFF_BETA);
-  float* sDG = reinterpret_cast<float*>(smem + OFF_DG);
-  float* sDB = reinterpret_cast<float*>(smem + OFF_DB);
   float* sSigLn = reinterpret_cast<float*>(smem + OFF_SIGLN);
   float* sSigF = reinterpret_cast<float*>(smem + OFF_SIGF);
   float* sGb1 = reinterpret_cast<float*>(smem + OFF_GB1);
@@ -190,8 +186,6 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     sGamma[tid] = p.gamma[head * 64 + tid];
     sBeta[tid] = p.beta[head * 64 + tid];
     sGb2[tid] = p.gb2_last[sid * 64 + tid];
-    sDG[tid] = 0.f;
-    sDB[tid] = 0.f;
   }
   float Gb1 = p.gb1_last[sid * 256 + hrow];
   tc_fence_before_sync();
@@ -228,9 +222,13 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 
   const long tok_rows0 = sid * NC * 64;      // first row of this stream in the [rows][64] token tensors
 
-  // ---- column sums over the 64 tokens of token tiles, while the MMAs of a phase run: every thread
-  // sums 16 rows of one column (rows 16 cs_q .., column cs_f) into `part` (the exchange buffer of the
-  // token-major epilogues, idle in these windows); after a CTA barrier threads 0..63 add the four parts.
+  // ---- column sums over the 64 tokens of a token-major quantity are taken from the registers of the epilogue that
+  // produces it (frag_colsum: seven shuffles), one row of four per quadrant, added up by threads 0..63 after the next
+  // barrier.  (Passes over the bf16 tiles inside the MMA windows outlasted those windows by a thousand cycles.)
+  float* sCS = sXch + 512;      // fp32[4][64], behind the row-sum exchange
+  auto put_colsum = [&](const f32x2 (&v)[4]) { sCS[tm.quad * 64 + frag_colsum_col(tm, lane)] = frag_colsum(v, lane); };
+  auto quad_sum = [&](int f) { return (sCS[f] + sCS[64 + f]) + (sCS[128 + f] + sCS[192 + f]); };
+  float dgam = 0.f, dbet = 0.f;      // this lane's column (frag_colsum_col) of d_gamma / d_beta
   // All CTAs reach a group boundary together, and each then reads 132 KB of state: the lines are asked
   // into L2 one step ahead (two 64 KB matrices = 2 x 512 lines, two lines of each per thread).
   auto prefetch_state = [&](const float* m1, const float* m2) {
@@ -241,18 +239,6 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     prefetch_l2(b);
     prefetch_l2(b + 32768);
   };
-  const int cs_q = tid >> 6, cs_f = tid & 63;
-  float* part = sXch;      // [3][4][64]
-  auto colsum16 = [&](const uint8_t* t) {
-    float acc = 0.f;
-#pragma unroll 8
-    for (int r = cs_q * 16; r < cs_q * 16 + 16; ++r) acc += ld_elem(t, r, cs_f);
-    return acc;
-  };
-  auto part_sum = [&](int k) {
-    return (part[k * 256 + tid] + part[k * 256 + 64 + tid]) + (part[k * 256 + 128 + tid] + part[k * 256 + 192 + tid]);
-  };
-
   // =====================================================================================
   const float* Gsrc_W1 = p.gW1_last + sid * (64 * 256);
   const float* Gsrc_W2 = p.gW2_last + sid * (256 * 64);
@@ -370,16 +356,20 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           tmem_wait_ld();
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
-            float z[8], g[8], gp[8];
+            uint32_t z[4], g[4], gp[4];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              z[k] = __uint_as_float(v[c * 8 + k]) + b1v;
-              gelu_pair(z[k], g[k], gp[k]);
+            for (int k = 0; k < 4; ++k) {
+              const f32x2 x = add2(pk(v[c * 8 + 2 * k], v[c * 8 + 2 * k + 1]), pk1(b1v));
+              f32x2 y, yp;
+              gelu_pair2(x, y, yp);
+              z[k] = f32x2_to_f16x2(x);          // f16: the sweep evaluates gelu' and gelu'' of it in f16
+              g[k] = f32x2_to_bf16x2(y);
+              gp[k] = f32x2_to_bf16x2(yp);
             }
             const uint32_t off = sw128_off(hrow, half * 2 + c);
-            *reinterpret_cast<uint4*>(bX2 + off) = pack_chunk(g);
-            *reinterpret_cast<uint4*>(bGP + off) = pack_chunk(gp);
-            *reinterpret_cast<uint4*>(bZ1 + off) = pack_chunk(z);
+            *reinterpret_cast<uint4*>(bX2 + off) = make_uint4(g[0], g[1], g[2], g[3]);
+            *reinterpret_cast<uint4*>(bGP + off) = make_uint4(gp[0], gp[1], gp[2], gp[3]);
+            *reinterpret_cast<uint4*>(bZ1 + off) = make_uint4(z[0], z[1], z[2], z[3]);
           }
         }
       }
@@ -399,60 +389,50 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       wait_mma();
       wait_bar(BAR_V);
       {
-        float xh[16], b2c[8], gam[8], bet[8];
-        tok_ld(tm, tmem + TM_B, xh);
-        tok_ld_cols(tm, sB2, b2c);
-        tok_ld_cols(tm, sGamma, gam);
-        tok_ld_cols(tm, sBeta, bet);
+        TokFrag x, g;
+        uint32_t kk[8], vv[8];
+        frag_ld(tm, tmem + TM_B, x);
+        frag_ld_raw(tm, sK, kk);          // requested before the all-reduces of the LayerNorm, used after them
+        frag_ld_raw(tm, sV, vv);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          xh[4 * q] += b2c[2 * q]; xh[4 * q + 1] += b2c[2 * q + 1];
-          xh[4 * q + 2] += b2c[2 * q]; xh[4 * q + 3] += b2c[2 * q + 1];
+          const f32x2 b = frag_col(tm, sB2, q);
+          x.a[q] = add2(x.a[q], b);
+          x.b[q] = add2(x.b[q], b);
         }
         float rs0, rs1;
-        float kk[16], vv[16], g[16], e[16];
-        tok_ld_tile(tm, sK, kk);          // requested before the all-reduces of the LayerNorm, used after them
-        tok_ld_tile(tm, sV, vv);
-        tok_layernorm(tm, xh, TTT_LN_EPS, sXch, rs0, rs1);
-        float a[2] = {0.f, 0.f}, b[2] = {0.f, 0.f};
+        frag_layernorm(tm, x, TTT_LN_EPS, sXch, 1, rs0, rs1);
+        f32x2 a0 = 0ull, a1 = 0ull, c0 = 0ull, c1 = 0ull;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h, c = 2 * q + h;
-            xh[x0] *= rs0;
-            xh[x1] *= rs1;
-            e[x0] = fmaf(gam[c], xh[x0], bet[c]) - (vv[x0] - kk[x0]);
-            e[x1] = fmaf(gam[c], xh[x1], bet[c]) - (vv[x1] - kk[x1]);
-            g[x0] = e[x0] * gam[c];
-            g[x1] = e[x1] * gam[c];
-            a[0] += g[x0]; a[1] = fmaf(g[x0], xh[x0], a[1]);
-            b[0] += g[x1]; b[1] = fmaf(g[x1], xh[x1], b[1]);
-          }
+          const f32x2 gam = frag_col(tm, sGamma, q), bet = frag_col(tm, sBeta, q), neg = pk1(-1.f);
+          const f32x2 t0 = fma2(bf16x2_to_f32x2(vv[2 * q]), neg, bf16x2_to_f32x2(kk[2 * q]));          // K - V
+          const f32x2 t1 = fma2(bf16x2_to_f32x2(vv[2 * q + 1]), neg, bf16x2_to_f32x2(kk[2 * q + 1]));
+          g.a[q] = mul2(fma2(gam, x.a[q], add2(t0, bet)), gam);
+          g.b[q] = mul2(fma2(gam, x.b[q], add2(t1, bet)), gam);
+          a0 = add2(a0, g.a[q]); a1 = fma2(g.a[q], x.a[q], a1);
+          c0 = add2(c0, g.b[q]); c1 = fma2(g.b[q], x.b[q], c1);
         }
         // x_hat_fused leaves through the V tile (every thread overwrites exactly the elements it has just
         // read) as a bulk store; grad_output_fused is not kept: the sweep rebuilds it from x_hat_fused, K, V
-        tok_st_tile(tm, tV, xh);
-        tok_row_allreduce<2, 2>(tm, a, b, sXch);
-        const float sc0 = rs0 * (1.f / 64.f), sc1 = rs1 * (1.f / 64.f);
-        const float ne0 = -__bfloat162float(eta[tm.r0]), ne1 = -__bfloat162float(eta[tm.r1]);
+        frag_st_tile(tm, tV, x);
+        float a[2] = {hsum(a0), hsum(a1)}, b[2] = {hsum(c0), hsum(c1)};
+        frag_allreduce2<1>(tm, a, b, sXch, 1);
+        const f32x2 sc0 = pk1(rs0 * (1.f / 64.f)), sc1 = pk1(rs1 * (1.f / 64.f));
+        const f32x2 ne0 = pk1(-__bfloat162float(eta[tm.r0])), ne1 = pk1(-__bfloat162float(eta[tm.r1]));
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h;
-            // dl/dZ2, rounded to bf16 once: the update below uses -eta times the rounded value
-            g[x0] = __bfloat162float(__float2bfloat16((64.f * g[x0] - a[0] - xh[x0] * a[1]) * sc0));
-            g[x1] = __bfloat162float(__float2bfloat16((64.f * g[x1] - b[0] - xh[x1] * b[1]) * sc1));
-          }
+          // dl/dZ2, rounded to bf16 once: the update below uses -eta times the rounded value
+          const uint32_t w0 = f32x2_to_bf16x2(mul2(fma2(x.a[q], pk1(-a[1]), fma2(g.a[q], pk1(64.f), pk1(-a[0]))), sc0));
+          const uint32_t w1 = f32x2_to_bf16x2(mul2(fma2(x.b[q], pk1(-b[1]), fma2(g.b[q], pk1(64.f), pk1(-b[0]))), sc1));
+          *reinterpret_cast<uint32_t*>(tGZ2 + tm.off(tm.r0, q)) = w0;
+          *reinterpret_cast<uint32_t*>(tGZ2 + tm.off(tm.r1, q)) = w1;
+          g.a[q] = mul2(bf16x2_to_f32x2(w0), ne0);
+          g.b[q] = mul2(bf16x2_to_f32x2(w1), ne1);
+          x.a[q] = add2(g.a[q], g.b[q]);
         }
-        tok_st_tile(tm, tGZ2, g);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          g[4 * q] *= ne0; g[4 * q + 1] *= ne0;
-          g[4 * q + 2] *= ne1; g[4 * q + 3] *= ne1;
-        }
-        tok_st_tile(tm, tU2, g);
+        frag_st_tile(tm, tU2, g);
+        put_colsum(x.a);
         if (tm.colhalf == 0 && tm.l3 == 0) {
           p.sc_sigf[slot * 64 + tm.r0] = rs0;     // the slot keeps 1/std: the sweep only ever divides by std
           p.sc_sigf[slot * 64 + tm.r1] = rs1;
@@ -471,12 +451,10 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 mma_hidden_half(tmem + TM_A, smem_u32(bW2), smem_u32(tGZ2), false, false, 1),
                 ,
                 )
-      part[tid] = colsum16(tU2);
-      __syncthreads();
-      if (tid < 64) sB2[tid] += part_sum(0);
+      if (tid < 64) sB2[tid] += quad_sum(tid);
       wait_mma();
       {
-        float bsum = 0.f;
+        f32x2 bsum = 0ull;
 #pragma unroll 1
         for (int half = 0; half < 4; ++half) {   // 16 columns per pass
           uint32_t v[16];
@@ -485,25 +463,23 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           tmem_wait_ld();
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
-            float gp[8], u[8];
             const uint32_t off = sw128_off(hrow, half * 2 + c);
-            unpack_chunk(gr[c], gp);
+            const uint32_t gw[4] = {gr[c].x, gr[c].y, gr[c].z, gr[c].w};
+            const uint4 ew = *reinterpret_cast<const uint4*>(eta + half * 16 + c * 8);     // one broadcast load
+            const uint32_t et[4] = {ew.x, ew.y, ew.z, ew.w};
+            uint32_t w[4], u[4];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) gp[k] *= __uint_as_float(v[c * 8 + k]);     // dl/dZ1
-            const uint4 w = pack_chunk(gp);
-            *reinterpret_cast<uint4*>(bGP + off) = w;             // dl/dZ1 (bf16), in place over G'
-            float gb[8], et[8];
-            unpack_chunk(w, gb);
-            unpack_chunk(*reinterpret_cast<const uint4*>(eta + half * 16 + c * 8), et);   // one broadcast load
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              u[k] = -et[k] * gb[k];
-              bsum += u[k];
+            for (int k = 0; k < 4; ++k) {
+              w[k] = f32x2_to_bf16x2(mul2(bf16x2_to_f32x2(gw[k]), pk(v[c * 8 + 2 * k], v[c * 8 + 2 * k + 1])));   // dl/dZ1
+              const f32x2 t = mul2(bf16x2_to_f32x2(w[k]), bf16x2_to_f32x2(et[k] ^ 0x80008000u));   // -eta dl/dZ1
+              bsum = add2(bsum, t);
+              u[k] = f32x2_to_bf16x2(t);
             }
-            *reinterpret_cast<uint4*>(bZ1 + off) = pack_chunk(u);  // U1 = -eta dl/dZ1, over Z1
+            *reinterpret_cast<uint4*>(bGP + off) = make_uint4(w[0], w[1], w[2], w[3]);     // dl/dZ1 in place over G'
+            *reinterpret_cast<uint4*>(bZ1 + off) = make_uint4(u[0], u[1], u[2], u[3]);     // U1 over Z1
           }
         }
-        b1v += bsum;
+        b1v += hsum(bsum);
       }
       publish();
 
@@ -569,15 +545,18 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           tmem_wait_ld();
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
-            float z[8], g[8];
+            uint32_t z[4], g[4];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
+            for (int k = 0; k < 4; ++k) {
               // the sweep needs gelu'(Z1_bar) only: it is cheaper here, next to gelu, than there from a bf16 copy
-              gelu_pair(__uint_as_float(v[c * 8 + k]) + b1v, g[k], z[k]);
+              f32x2 y, yp;
+              gelu_pair2(add2(pk(v[c * 8 + 2 * k], v[c * 8 + 2 * k + 1]), pk1(b1v)), y, yp);
+              g[k] = f32x2_to_bf16x2(y);
+              z[k] = f32x2_to_bf16x2(yp);
             }
             const uint32_t off = sw128_off(hrow, half * 2 + c);
-            *reinterpret_cast<uint4*>(bX2 + off) = pack_chunk(g);
-            *reinterpret_cast<uint4*>(bZ1 + off) = pack_chunk(z);
+            *reinterpret_cast<uint4*>(bX2 + off) = make_uint4(g[0], g[1], g[2], g[3]);
+            *reinterpret_cast<uint4*>(bZ1 + off) = make_uint4(z[0], z[1], z[2], z[3]);
           }
         }
       }
@@ -595,22 +574,17 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 )
       wait_mma();
       {
-        float z[16], b2c[8];
-        tok_ld(tm, tmem + TM_B, z);
-        tok_ld_cols(tm, sB2, b2c);
+        TokFrag x;
+        frag_ld(tm, tmem + TM_B, x);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          z[4 * q] += b2c[2 * q]; z[4 * q + 1] += b2c[2 * q + 1];
-          z[4 * q + 2] += b2c[2 * q]; z[4 * q + 3] += b2c[2 * q + 1];
+          const f32x2 b = frag_col(tm, sB2, q);
+          x.a[q] = add2(x.a[q], b);
+          x.b[q] = add2(x.b[q], b);
         }
         float rs0, rs1;
-        tok_layernorm(tm, z, TTT_LN_EPS, sXch, rs0, rs1);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          z[4 * q] *= rs0; z[4 * q + 1] *= rs0;
-          z[4 * q + 2] *= rs1; z[4 * q + 3] *= rs1;
-        }
-        tok_st_tile(tm, tU2, z);      // the U2 tile is dead since MMA4; x_hat_ln leaves through it
+        frag_layernorm(tm, x, TTT_LN_EPS, sXch, 1, rs0, rs1);
+        frag_st_tile(tm, tU2, x);     // the U2 tile is dead since MMA4; x_hat_ln leaves through it
         if (tm.colhalf == 0 && tm.l3 == 0) {
           p.sc_sigln[slot * 64 + tm.r0] = rs0;
           p.sc_sigln[slot * 64 + tm.r1] = rs1;
@@ -709,7 +683,7 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     for (int j = gsz - 1; j >= 0; --j) {
       const long slot = slot0 + j;
       const int row0 = static_cast<int>(tok_rows0 + (long)(i0 + j) * 64);   // first token row of this mini-batch
-      float kp[16];                                                          // partial dK, completed in E6
+      f32x2 kpa[4], kpb[4];                                                  // partial dK, completed in E6
       if (j == 0 && ck > 0)                                                  // the next group's checkpoint
         prefetch_state(p.W1c + (sid * p.nck + ck - 1) * (64 * 256), p.W2c + (sid * p.nck + ck - 1) * (256 * 64));
 
@@ -717,34 +691,35 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       wait_bar(BAR_T + 0);
       wait_bar(BAR_T + 1);
       {
-        float go[16], xl[16], gam[8];
-        tok_ld_tile(tm, t_go, go);
-        tok_ld_tile(tm, t_a, xl);
-        tok_ld_cols(tm, sGamma, gam);
-        float a[2] = {0.f, 0.f}, b[2] = {0.f, 0.f};
+        uint32_t gw[8], xw[8];
+        frag_ld_raw(tm, t_go, gw);
+        frag_ld_raw(tm, t_a, xw);
+        TokFrag g;
+        f32x2 a0 = 0ull, a1 = 0ull, c0 = 0ull, c1 = 0ull, sb[4], sg[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h;
-            go[x0] *= gam[2 * q + h];
-            go[x1] *= gam[2 * q + h];
-            a[0] += go[x0]; a[1] = fmaf(go[x0], xl[x0], a[1]);
-            b[0] += go[x1]; b[1] = fmaf(go[x1], xl[x1], b[1]);
-          }
+          const f32x2 gam = frag_col(tm, sGamma, q);
+          g.a[q] = mul2(bf16x2_to_f32x2(gw[2 * q]), gam);
+          g.b[q] = mul2(bf16x2_to_f32x2(gw[2 * q + 1]), gam);
+          a0 = add2(a0, g.a[q]); a1 = fma2(g.a[q], bf16x2_to_f32x2(xw[2 * q]), a1);
+          c0 = add2(c0, g.b[q]); c1 = fma2(g.b[q], bf16x2_to_f32x2(xw[2 * q + 1]), c1);
+          sb[q] = add2(bf16x2_to_f32x2(gw[2 * q]), bf16x2_to_f32x2(gw[2 * q + 1]));
+          sg[q] = fma2(bf16x2_to_f32x2(gw[2 * q]), bf16x2_to_f32x2(xw[2 * q]),
+                       mul2(bf16x2_to_f32x2(gw[2 * q + 1]), bf16x2_to_f32x2(xw[2 * q + 1])));
         }
-        tok_row_allreduce<2, 2>(tm, a, b, sXch);
-        const float q0 = sSigLn[tm.r0] * (1.f / 64.f), q1 = sSigLn[tm.r1] * (1.f / 64.f);   // 1 / (64 std)
+        dbet += frag_colsum(sb, lane);
+        dgam += frag_colsum(sg, lane);
+        float a[2] = {hsum(a0), hsum(a1)}, b[2] = {hsum(c0), hsum(c1)};
+        frag_allreduce2<1>(tm, a, b, sXch, 1);
+        const f32x2 q0 = pk1(sSigLn[tm.r0] * (1.f / 64.f)), q1 = pk1(sSigLn[tm.r1] * (1.f / 64.f));   // 1 / (64 std)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h;
-            go[x0] = (64.f * go[x0] - a[0] - xl[x0] * a[1]) * q0;
-            go[x1] = (64.f * go[x1] - b[0] - xl[x1] * b[1]) * q1;
-          }
+          g.a[q] = mul2(fma2(bf16x2_to_f32x2(xw[2 * q]), pk1(-a[1]), fma2(g.a[q], pk1(64.f), pk1(-a[0]))), q0);
+          g.b[q] = mul2(fma2(bf16x2_to_f32x2(xw[2 * q + 1]), pk1(-b[1]), fma2(g.b[q], pk1(64.f), pk1(-b[0]))), q1);
+          sb[q] = add2(g.a[q], g.b[q]);
         }
-        tok_st_tile(tm, t_g, go);
+        frag_st_tile(tm, t_g, g);
+        put_colsum(sb);
       }
       publish();
       // G1: gX2b^T = W2+ gZ2b^T
@@ -752,32 +727,14 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 mma_hidden_half(tmem + TM_A, smem_u32(big(ib1)), smem_u32(t_g), false, false, 1),
                 ,
                 )
-      {
-        // column sums over the tokens: d_beta += sum go, d_gamma += sum go * x_hat_ln, G_b2 += sum gZ2b
-        float a = 0.f, b = 0.f;
-#pragma unroll 8
-        for (int r = cs_q * 16; r < cs_q * 16 + 16; ++r) {
-          const float go = ld_elem(t_go, r, cs_f);
-          b += go;
-          a = fmaf(go, ld_elem(t_a, r, cs_f), a);
-        }
-        part[tid] = b;
-        part[256 + tid] = a;
-        part[512 + tid] = colsum16(t_g);
-        __syncthreads();
-        if (tid < 64) {
-          sDB[tid] += part_sum(0);
-          sDG[tid] += part_sum(1);
-          sGb2[tid] += part_sum(2);
-        }
-      }
+      if (tid < 64) sGb2[tid] += quad_sum(tid);
       wait_mma();
       if (tid == kProd) load_big(ib1, p.sc_X2 + slot * BIG);   // W2+ is consumed (G1 was its only use): X2 for G5
       wait_bar(BAR_BIG + ib2);
       // ---- E1: gZ1b^T = gX2b^T * gelu'(Z1b^T), in place over Z1b^T
       {
         uint8_t* bz = big(ib2);
-        float bsum = 0.f;
+        f32x2 bsum = 0ull;
 #pragma unroll 1
         for (int half = 0; half < 4; ++half) {   // 16 columns per pass
           uint32_t v[16];
@@ -786,17 +743,18 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           tmem_wait_ld();
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
-            float z[8];
-            unpack_chunk(zr[c], z);
+            const uint32_t zw[4] = {zr[c].x, zr[c].y, zr[c].z, zr[c].w};      // gelu'(Z1_bar)
+            uint32_t w[4];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              z[k] *= __uint_as_float(v[c * 8 + k]);      // the tile holds gelu'(Z1_bar)
-              bsum += z[k];
+            for (int k = 0; k < 4; ++k) {
+              const f32x2 t = mul2(bf16x2_to_f32x2(zw[k]), pk(v[c * 8 + 2 * k], v[c * 8 + 2 * k + 1]));
+              bsum = add2(bsum, t);
+              w[k] = f32x2_to_bf16x2(t);
             }
-            st_chunk(bz, hrow, half * 2 + c, z);
+            *reinterpret_cast<uint4*>(bz + sw128_off(hrow, half * 2 + c)) = make_uint4(w[0], w[1], w[2], w[3]);
           }
         }
-        Gb1 += bsum;
+        Gb1 += hsum(bsum);
       }
       publish();
       if (tid == kProd) {   // x_hat_ln and its column sums are consumed: bring V into that tile (E4 rebuilds
@@ -840,12 +798,16 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         sGb1[hrow] = Gb1;
       }
       {   // dQ = go + gZ1b W1+^T, staged over the dL/dOut tile and stored by TMA
-        float acc[16], go[16];
-        tok_ld(tm, tmem + TM_B, acc);
-        tok_ld_tile(tm, t_go, go);
+        TokFrag x;
+        uint32_t gw[8];
+        frag_ld(tm, tmem + TM_B, x);
+        frag_ld_raw(tm, t_go, gw);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) go[q] += acc[q];
-        tok_st_tile(tm, t_go, go);
+        for (int q = 0; q < 4; ++q) {
+          x.a[q] = add2(x.a[q], bf16x2_to_f32x2(gw[2 * q]));
+          x.b[q] = add2(x.b[q], bf16x2_to_f32x2(gw[2 * q + 1]));
+        }
+        frag_st_tile(tm, t_go, x);
       }
       publish();
       if (tid == kProd) {
@@ -901,23 +863,24 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           tmem_wait_ld();
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
-            float z[8], pp[8], gp[8], et[8];
-            unpack_chunk(zr[c], z);
-            unpack_chunk(*reinterpret_cast<const uint4*>(sEta + half * 16 + c * 8), et);   // one broadcast load
+            const uint32_t zw[4] = {zr[c].x, zr[c].y, zr[c].z, zr[c].w};
+            const uint4 ew = *reinterpret_cast<const uint4*>(sEta + half * 16 + c * 8);     // one broadcast load
+            const uint32_t et[4] = {ew.x, ew.y, ew.z, ew.w};
+            uint32_t pw[4], sw[4], gw[4];
 #pragma unroll
-            for (int k = 0; k < 8; k += 2) {
-              const float a10 = -et[k] * (__uint_as_float(v[c * 8 + k]) + Gb1);
-              const float a11 = -et[k + 1] * (__uint_as_float(v[c * 8 + k + 1]) + Gb1);
-              float gpp0, gpp1;
-              gelu_grad_pair2(z[k], z[k + 1], gp[k], gp[k + 1], gpp0, gpp1);
-              pp[k] = a10 * gp[k];
-              pp[k + 1] = a11 * gp[k + 1];
-              z[k] = a10 * gpp0;
-              z[k + 1] = a11 * gpp1;
+            for (int k = 0; k < 4; ++k) {
+              const f32x2 a1 = mul2(bf16x2_to_f32x2(et[k] ^ 0x80008000u),
+                                    add2(pk(v[c * 8 + 2 * k], v[c * 8 + 2 * k + 1]), pk1(Gb1)));
+              uint32_t gp, gpp;
+              gelu_grad_h2(zw[k], gp, gpp);
+              gw[k] = gp;                                        // kept as f16
+              pw[k] = f32x2_to_bf16x2(mul2(a1, f16x2_to_f32x2(gp)));
+              sw[k] = f32x2_to_bf16x2(mul2(a1, f16x2_to_f32x2(gpp)));
             }
-            st_chunk(bp, hrow, half * 2 + c, pp);
-            st_chunk(bz, hrow, half * 2 + c, z);
-            st_chunk(bgp, hrow, half * 2 + c, gp);
+            const uint32_t off = sw128_off(hrow, half * 2 + c);
+            *reinterpret_cast<uint4*>(bp + off) = make_uint4(pw[0], pw[1], pw[2], pw[3]);
+            *reinterpret_cast<uint4*>(bz + off) = make_uint4(sw[0], sw[1], sw[2], sw[3]);
+            *reinterpret_cast<uint4*>(bgp + off) = make_uint4(gw[0], gw[1], gw[2], gw[3]);
           }
         }
       }
@@ -935,97 +898,118 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       wait_bar(BAR_T + 1);   // grad_output_fused
       // ---- E4: second order through the fused LayerNorm + L2 gradient (token-major, all 8 warps)
       {
-        float A2[16], t1[16], gz[16], xh[16], go[16];
-        float gam[8];
-        tok_ld_cols(tm, sGamma, gam);
+        TokFrag A2, t1, go;
+        uint32_t gzw[8], xhw[8], kw[8];
+        frag_ld_raw(tm, t_gz2, gzw);
+        frag_ld_raw(tm, t_xf, xhw);
+        frag_ld_raw(tm, t_k, kw);
         const float eta0 = __bfloat162float(sEta[tm.r0]), eta1 = __bfloat162float(sEta[tm.r1]);
         const float rs0 = sSigF[tm.r0], rs1 = sSigF[tm.r1];      // 1 / std
-        tok_ld_tile(tm, t_gz2, gz);
-        tok_ld_tile(tm, t_xf, xh);
-        tok_ld_tile(tm, t_a, go);
-        float ra[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, rb[5] = {0.f, 0.f, 0.f, 0.f, 0.f};   // d12, d3, sum A2, sum A2 xh, sum gxf xh
+        float ra[4], rb[4];       // d_eta's row terms, sum A2, sum A2 xh, sum gxf xh
         {
-          float acc1[16], acc2[16], kk[16], gb2[8], bet[8];
-          tok_ld_tile(tm, t_k, kk);
+          TokFrag acc1;
+          uint32_t vw[8];
+          frag_ld_raw(tm, t_a, vw);
           // X2 G_W2, P W2, gZ1 G_W1
-          tok_ld3(tm, tmem + TM_B + 64, acc1, tmem + TM_A, acc2, tmem + TM_B, t1);
-          tok_ld_cols(tm, sGb2, gb2);
-          tok_ld_cols(tm, sBeta, bet);
+          frag_ld(tm, tmem + TM_B + 64, acc1);
+          frag_ld(tm, tmem + TM_A, A2);
+          frag_ld(tm, tmem + TM_B, t1);
+          f32x2 s0[4] = {0ull, 0ull, 0ull, 0ull}, s1[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int x0 = 4 * q + h, x1 = 4 * q + 2 + h, c = 2 * q + h;
-              // go[] arrives holding V: grad_output_fused = gamma x_hat_fused + beta - (V - K)
-              go[x0] = fmaf(gam[c], xh[x0], bet[c]) - (go[x0] - kk[x0]);
-              go[x1] = fmaf(gam[c], xh[x1], bet[c]) - (go[x1] - kk[x1]);
-              const float u0 = acc1[x0] + gb2[c], u1 = acc1[x1] + gb2[c];
-              ra[0] = fmaf(gz[x0], u0, ra[0]);
-              rb[0] = fmaf(gz[x1], u1, rb[0]);
-              ra[1] = fmaf(t1[x0], kk[x0], ra[1]);
-              rb[1] = fmaf(t1[x1], kk[x1], rb[1]);
-              A2[x0] = fmaf(-eta0, u0, acc2[x0]);
-              A2[x1] = fmaf(-eta1, u1, acc2[x1]);
-              ra[2] += A2[x0];
-              rb[2] += A2[x1];
-              ra[3] = fmaf(A2[x0], xh[x0], ra[3]);
-              rb[3] = fmaf(A2[x1], xh[x1], rb[3]);
-              ra[4] = fmaf(go[x0] * gam[c], xh[x0], ra[4]);
-              rb[4] = fmaf(go[x1] * gam[c], xh[x1], rb[4]);
-            }
+            const f32x2 gam = frag_col(tm, sGamma, q), bet = frag_col(tm, sBeta, q), gb2 = frag_col(tm, sGb2, q), neg = pk1(-1.f);
+            const f32x2 x0 = bf16x2_to_f32x2(xhw[2 * q]), x1 = bf16x2_to_f32x2(xhw[2 * q + 1]);
+            const f32x2 k0 = bf16x2_to_f32x2(kw[2 * q]), k1 = bf16x2_to_f32x2(kw[2 * q + 1]);
+            // grad_output_fused = gamma x_hat_fused + beta - (V - K)
+            go.a[q] = add2(fma2(bf16x2_to_f32x2(vw[2 * q]), neg, k0), fma2(gam, x0, bet));
+            go.b[q] = add2(fma2(bf16x2_to_f32x2(vw[2 * q + 1]), neg, k1), fma2(gam, x1, bet));
+            const f32x2 u0 = add2(acc1.a[q], gb2), u1 = add2(acc1.b[q], gb2);
+            s0[0] = fma2(bf16x2_to_f32x2(gzw[2 * q]), u0, fma2(t1.a[q], k0, s0[0]));
+            s1[0] = fma2(bf16x2_to_f32x2(gzw[2 * q + 1]), u1, fma2(t1.b[q], k1, s1[0]));
+            A2.a[q] = fma2(u0, pk1(-eta0), A2.a[q]);
+            A2.b[q] = fma2(u1, pk1(-eta1), A2.b[q]);
+            s0[1] = add2(s0[1], A2.a[q]);
+            s1[1] = add2(s1[1], A2.b[q]);
+            s0[2] = fma2(A2.a[q], x0, s0[2]);
+            s1[2] = fma2(A2.b[q], x1, s1[2]);
+            s0[3] = fma2(mul2(go.a[q], gam), x0, s0[3]);
+            s1[3] = fma2(mul2(go.b[q], gam), x1, s1[3]);
           }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) { ra[i] = hsum(s0[i]); rb[i] = hsum(s1[i]); }
         }
-        tok_row_allreduce<5, 0>(tm, ra, rb, sXch);
-        float sa[2] = {0.f, 0.f}, sb[2] = {0.f, 0.f};      // sum g_std, sum g_xhat
-        float dga[16], dv[16];
+        // all-reduce over the row's four lanes and two warps
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int sft = 1; sft <= 2; sft <<= 1)
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int c = 2 * q + h;
-            const float gm = gam[c];
-            {
-              const int x = 4 * q + h;
-              const float bt = (A2[x] - (ra[2] + xh[x] * ra[3]) * (1.f / 64.f)) * rs0;
-              const float gly = gm * bt;
-              dga[x] = fmaf(go[x], bt, gly * xh[x]);
-              dv[x] = -gly;
-              kp[x] = fmaf(-eta0, t1[x], gly);
-              const float gxh = fmaf(gly, gm, -(go[x] * gm * ra[3] + A2[x] * ra[4]) * rs0 * (1.f / 64.f));
-              sa[0] += (-gxh * xh[x] - A2[x] * gz[x]) * rs0;
-              sa[1] += gxh;
-              A2[x] = gxh;
-            }
-            {
-              const int x = 4 * q + 2 + h;
-              const float bt = (A2[x] - (rb[2] + xh[x] * rb[3]) * (1.f / 64.f)) * rs1;
-              const float gly = gm * bt;
-              dga[x] = fmaf(go[x], bt, gly * xh[x]);
-              dv[x] = -gly;
-              kp[x] = fmaf(-eta1, t1[x], gly);
-              const float gxh = fmaf(gly, gm, -(go[x] * gm * rb[3] + A2[x] * rb[4]) * rs1 * (1.f / 64.f));
-              sb[0] += (-gxh * xh[x] - A2[x] * gz[x]) * rs1;
-              sb[1] += gxh;
-              A2[x] = gxh;
-            }
+          for (int i = 0; i < 4; ++i) {
+            ra[i] += __shfl_xor_sync(0xffffffffu, ra[i], sft);
+            rb[i] += __shfl_xor_sync(0xffffffffu, rb[i], sft);
           }
+        float4* x4 = reinterpret_cast<float4*>(sXch);      // 2 KB; the second exchange follows behind the column sums
+        if (tm.l3 == 0) {
+          x4[tm.colhalf * 64 + tm.r0] = make_float4(ra[0], ra[1], ra[2], ra[3]);
+          x4[tm.colhalf * 64 + tm.r1] = make_float4(rb[0], rb[1], rb[2], rb[3]);
         }
-        tok_st_tile(tm, t_a, dga);       // d_gamma addends, over grad_output_fused
-        tok_st_tile(tm, t_go, dv);       // dV: stored by TMA, and column-summed for d_beta
-        tok_row_allreduce<2, 5>(tm, sa, sb, sXch);
+        named_bar_sync(1 + tm.quad, 64);
+        {
+          const float4 o0 = x4[(tm.colhalf ^ 1) * 64 + tm.r0], o1 = x4[(tm.colhalf ^ 1) * 64 + tm.r1];
+          ra[0] += o0.x; ra[1] += o0.y; ra[2] += o0.z; ra[3] += o0.w;
+          rb[0] += o1.x; rb[1] += o1.y; rb[2] += o1.z; rb[3] += o1.w;
+        }
+        f32x2 sa0 = 0ull, sa1 = 0ull, sb0 = 0ull, sb1 = 0ull;      // sum g_std, sum g_xhat of the two rows
+        f32x2 cs[4];
+        {
+          const f32x2 n64 = pk1(-1.f / 64.f);
+          const f32x2 mA = mul2(pk1(ra[1]), n64), xA = mul2(pk1(ra[2]), n64), mB = mul2(pk1(rb[1]), n64), xB = mul2(pk1(rb[2]), n64);
+          const f32x2 fA3 = pk1(-ra[2] * rs0 * (1.f / 64.f)), fA4 = pk1(-ra[3] * rs0 * (1.f / 64.f));
+          const f32x2 fB3 = pk1(-rb[2] * rs1 * (1.f / 64.f)), fB4 = pk1(-rb[3] * rs1 * (1.f / 64.f));
+          f32x2 cl[4];
+          TokFrag dv;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h;
-            A2[x0] = fmaf(A2[x0], rs0, (sa[0] * xh[x0] - sa[1] * rs0) * (1.f / 64.f));   // gZ2in
-            A2[x1] = fmaf(A2[x1], rs1, (sb[0] * xh[x1] - sb[1] * rs1) * (1.f / 64.f));
-            gz[x0] *= -eta0;                                                            // U2 = -eta gZ2
-            gz[x1] *= -eta1;
+          for (int q = 0; q < 4; ++q) {
+            const f32x2 gm = frag_col(tm, sGamma, q), neg = pk1(-1.f);
+            const f32x2 x0 = bf16x2_to_f32x2(xhw[2 * q]), x1 = bf16x2_to_f32x2(xhw[2 * q + 1]);
+            const f32x2 bt0 = mul2(add2(A2.a[q], fma2(x0, xA, mA)), pk1(rs0));
+            const f32x2 bt1 = mul2(add2(A2.b[q], fma2(x1, xB, mB)), pk1(rs1));
+            const f32x2 gl0 = mul2(gm, bt0), gl1 = mul2(gm, bt1);
+            cs[q] = add2(fma2(go.a[q], bt0, mul2(gl0, x0)), fma2(go.b[q], bt1, mul2(gl1, x1)));
+            cl[q] = add2(gl0, gl1);
+            dv.a[q] = mul2(gl0, neg);
+            dv.b[q] = mul2(gl1, neg);
+            kpa[q] = fma2(t1.a[q], pk1(-eta0), gl0);
+            kpb[q] = fma2(t1.b[q], pk1(-eta1), gl1);
+            const f32x2 gx0 = fma2(gl0, gm, fma2(mul2(go.a[q], gm), fA3, mul2(A2.a[q], fA4)));
+            const f32x2 gx1 = fma2(gl1, gm, fma2(mul2(go.b[q], gm), fB3, mul2(A2.b[q], fB4)));
+            sa0 = fma2(gx0, x0, fma2(A2.a[q], bf16x2_to_f32x2(gzw[2 * q]), sa0));
+            sb0 = fma2(gx1, x1, fma2(A2.b[q], bf16x2_to_f32x2(gzw[2 * q + 1]), sb0));
+            sa1 = add2(sa1, gx0);
+            sb1 = add2(sb1, gx1);
+            A2.a[q] = gx0;
+            A2.b[q] = gx1;
           }
+          frag_st_tile(tm, t_go, dv);      // dV: stored by TMA
+          dgam += frag_colsum(cs, lane);
+          dbet += frag_colsum(cl, lane);
         }
-        tok_st_tile(tm, t_q, A2);
-        tok_st_tile(tm, t_g, gz);
+        float sa[2] = {-hsum(sa0) * rs0, hsum(sa1)}, sb[2] = {-hsum(sb0) * rs1, hsum(sb1)};
+        frag_allreduce2<0>(tm, sa, sb, sXch + 768, 1);
+        {
+          const f32x2 k0 = pk1(sa[0] * (1.f / 64.f)), l0 = pk1(-sa[1] * rs0 * (1.f / 64.f));
+          const f32x2 k1 = pk1(sb[0] * (1.f / 64.f)), l1 = pk1(-sb[1] * rs1 * (1.f / 64.f));
+          TokFrag u2;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            A2.a[q] = fma2(A2.a[q], pk1(rs0), fma2(bf16x2_to_f32x2(xhw[2 * q]), k0, l0));      // gZ2in
+            A2.b[q] = fma2(A2.b[q], pk1(rs1), fma2(bf16x2_to_f32x2(xhw[2 * q + 1]), k1, l1));
+            cs[q] = add2(A2.a[q], A2.b[q]);
+            u2.a[q] = mul2(bf16x2_to_f32x2(gzw[2 * q]), pk1(-eta0));                           // U2 = -eta gZ2
+            u2.b[q] = mul2(bf16x2_to_f32x2(gzw[2 * q + 1]), pk1(-eta1));
+          }
+          frag_st_tile(tm, t_q, A2);
+          frag_st_tile(tm, t_g, u2);
+          put_colsum(cs);
+        }
         if (tm.colhalf == 0 && tm.l3 == 0) {
           const int r0 = tm.r0, r1 = tm.r1;
           float p0 = 0.f, p1 = 0.f;
@@ -1034,10 +1018,8 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             p0 += sPart[w * 64 + r0];
             p1 += sPart[w * 64 + r1];
           }
-          const float de0 = -(ra[0] + ra[1] + p0);
-          const float de1 = -(rb[0] + rb[1] + p1);
-          p.d_eta[(sid * NC + i0 + j) * 64 + r0] = __float2bfloat16(de0);
-          p.d_eta[(sid * NC + i0 + j) * 64 + r1] = __float2bfloat16(de1);
+          p.d_eta[(sid * NC + i0 + j) * 64 + r0] = __float2bfloat16(-(ra[0] + p0));
+          p.d_eta[(sid * NC + i0 + j) * 64 + r1] = __float2bfloat16(-(rb[0] + p1));
         }
       }
       publish();
@@ -1052,17 +1034,7 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 mma_hidden_half(tmem + TM_B, smem_u32(big(ib1)), smem_u32(t_q), false, false, 1); mma_hidden_half(tmem + TM_B, smem_u32(big(ib3)), smem_u32(t_g), false, true, 1),
                 mma_hidden_half(tmem + TM_A, smem_u32(big(ib1)), smem_u32(t_gz2), false, false, 0),
                 mma_hidden_half(tmem + TM_A, smem_u32(big(ib1)), smem_u32(t_gz2), false, false, 1))
-      {
-        part[tid] = colsum16(t_q);
-        part[256 + tid] = colsum16(t_a);
-        part[512 + tid] = colsum16(t_go);
-        __syncthreads();
-        if (tid < 64) {
-          sGb2[tid] += part_sum(0);
-          sDG[tid] += part_sum(1);
-          sDB[tid] -= part_sum(2);
-        }
-      }
+      if (tid < 64) sGb2[tid] += quad_sum(tid);
       wait_mma();
       if (tid == kProd) {
         // the W2 state-gradient snapshot is consumed: X2 comes back into its buffer for G14 (it lands while
@@ -1076,7 +1048,7 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       {
         uint8_t* bs = big(ib2);
         const uint8_t* bgp = big(ib0);
-        float bsum = 0.f;
+        f32x2 bs2 = 0ull;
 #pragma unroll 1
         for (int half = 0; half < 4; ++half) {   // 16 columns per pass
           uint32_t v[16], w[16];
@@ -1087,18 +1059,20 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           tmem_wait_ld();
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
-            float gp[8], sv[8];
-            unpack_chunk(gr[c], gp);
-            unpack_chunk(sr[c], sv);
+            const uint32_t gw[4] = {gr[c].x, gr[c].y, gr[c].z, gr[c].w};      // gelu'(Z1), f16
+            const uint32_t sw[4] = {sr[c].x, sr[c].y, sr[c].z, sr[c].w};
+            uint32_t o[4];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              sv[k] = fmaf(__uint_as_float(v[c * 8 + k]), gp[k], __uint_as_float(w[c * 8 + k]) * sv[k]);
-              bsum += sv[k];
+            for (int k = 0; k < 4; ++k) {
+              const f32x2 t = fma2(pk(v[c * 8 + 2 * k], v[c * 8 + 2 * k + 1]), f16x2_to_f32x2(gw[k]),
+                                   mul2(pk(w[c * 8 + 2 * k], w[c * 8 + 2 * k + 1]), bf16x2_to_f32x2(sw[k])));
+              bs2 = add2(bs2, t);
+              o[k] = f32x2_to_bf16x2(t);
             }
-            st_chunk(bs, hrow, half * 2 + c, sv);
+            *reinterpret_cast<uint4*>(bs + sw128_off(hrow, half * 2 + c)) = make_uint4(o[0], o[1], o[2], o[3]);
           }
         }
-        Gb1 += bsum;
+        Gb1 += hsum(bs2);
       }
       publish();
       // gelu'(Z1) is consumed: the next step's gelu'(Z1_bar) comes into its buffer
@@ -1114,11 +1088,14 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       // ---- E6: dK = partial + gZ1in W1^T, staged over the dl/dZ2 tile (dead since G12) and stored by TMA;
       // nothing waits for the store here: the tile's next load is issue_gz2's
       {
-        float acc[16];
-        tok_ld(tm, tmem + TM_A, acc);
+        TokFrag x;
+        frag_ld(tm, tmem + TM_A, x);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) kp[q] += acc[q];
-        tok_st_tile(tm, t_gz2, kp);
+        for (int q = 0; q < 4; ++q) {
+          x.a[q] = add2(x.a[q], kpa[q]);
+          x.b[q] = add2(x.b[q], kpb[q]);
+        }
+        frag_st_tile(tm, t_gz2, x);
       }
       publish();
       if (tid == kProd) {
@@ -1161,10 +1138,13 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   // ---- final vector outputs
   if (!aborted) {
     p.gb1[sid * 256 + hrow] = Gb1;
+    sXch[tm.quad * 64 + frag_colsum_col(tm, lane)] = dgam;
+    sXch[256 + tm.quad * 64 + frag_colsum_col(tm, lane)] = dbet;
+    __syncthreads();
     if (tid < 64) {
       p.gb2[sid * 64 + tid] = sGb2[tid];
-      p.d_gamma[sid * 64 + tid] = sDG[tid];
-      p.d_beta[sid * 64 + tid] = sDB[tid];
+      p.d_gamma[sid * 64 + tid] = (sXch[tid] + sXch[64 + tid]) + (sXch[128 + tid] + sXch[192 + tid]);
+      p.d_beta[sid * 64 + tid] = (sXch[256 + tid] + sXch[320 + tid]) + (sXch[384 + tid] + sXch[448 + tid]);
     }
   }
   if (tid == kProd) tma_wait_group<0>();

@@ -114,6 +114,31 @@ __device__ __forceinline__ void gelu_grad_pair2(float x0, float x1, float& gp0, 
   gpp1 = gpp.y;
 }
 
+// the same from and to f16 pairs (a value beyond the f16 range has become infinite and is clamped like one beyond 20)
+__device__ __forceinline__ uint32_t f32x2_to_f16x2(f32x2 a) {
+  float lo, hi;
+  upk(a, lo, hi);
+  const __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ f32x2 f16x2_to_f32x2(uint32_t w) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+  return pk(f.x, f.y);
+}
+__device__ __forceinline__ void gelu_grad_h2(uint32_t z, uint32_t& gp, uint32_t& gpp) {
+  const __half2 x = __hmax2(__hmin2(*reinterpret_cast<const __half2*>(&z), h2c(20.f)), h2c(-20.f));
+  const __half2 x2 = __hmul2(x, x);
+  const __half2 t = tanh_h2(__hmul2(x, __hfma2(h2c(kG01), x2, h2c(kG0))));
+  const __half2 h = __hfma2(h2c(0.5f), t, h2c(0.5f));
+  const __half2 q = __hfma2(h2c(kG2), x2, h2c(kG0));
+  const __half2 g = __hmul2(x, h);
+  const __half2 a = __hfma2(__hfma2(__hneg2(g), t, g), q, h);
+  const __half2 c = __hfma2(h2c(2.f * kG2), x2, h2c(kG0));
+  const __half2 b = __hmul2(__hfma2(__hneg2(t), t, h2c(1.f)), __hfma2(__hneg2(__hmul2(__hmul2(x, t), q)), q, c));
+  gp = *reinterpret_cast<const uint32_t*>(&a);
+  gpp = *reinterpret_cast<const uint32_t*>(&b);
+}
+
 __device__ __forceinline__ uint4 pack_chunk(const float* v) {
   uint4 w;
   w.x = pack_bf16(v[0], v[1]);
@@ -323,6 +348,36 @@ __device__ __forceinline__ void mma_hidden_ta(uint32_t tmem_d, uint32_t tmem_a, 
   mma_lead_ta<kAccumulate>(tmem_d, tmem_a, b0, idesc, lead);
 #pragma unroll
   for (int j = 1; j < 4; ++j) mma_lead_ta<true>(tmem_d, tmem_a + j * 8, b0 + j * bstep, idesc, lead);
+}
+// The same products with rolled issue loops, for a kernel whose code is of the size of the instruction cache.
+__device__ __forceinline__ void mma_lead_rt(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc,
+                                            uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %4};\n\t"
+      "mov.b64 db, {%2, %4};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kDescHi), "r"(acc), "r"(lead)
+      : "memory");
+}
+template <bool kBMn, bool kAccumulate>
+__device__ __forceinline__ void mma_hidden_roll(uint32_t tmem_d, uint32_t a_smem, uint32_t b_smem, int blk, uint32_t lead) {
+  constexpr uint32_t idesc = umma_idesc_bf16(128, 64, false, kBMn, false);
+  const uint32_t a0 = desc_lo(a_smem, 16) + blk * (16384u >> 4);
+  const uint32_t b0 = desc_lo(b_smem, kBMn ? 8192 : 16);
+  constexpr uint32_t bstep = kBMn ? (2048u >> 4) : (32u >> 4);
+#pragma unroll 1
+  for (uint32_t j = 0; j < 4; ++j)
+    mma_lead_rt(tmem_d + blk * 64, a0 + j * 2, b0 + j * bstep, idesc, kAccumulate ? 1u : j, lead);
+}
+__device__ __forceinline__ void mma_token_roll(uint32_t tmem_d, uint32_t x_smem, uint32_t w_smem, uint32_t lead) {
+  constexpr uint32_t idesc = umma_idesc_bf16(64, 64, true, true, false);
+  const uint32_t a0 = desc_lo(x_smem, BIG);
+  const uint32_t b0 = desc_lo(w_smem, BIG);
+#pragma unroll 1
+  for (uint32_t j = 0; j < 16; ++j) mma_lead_rt(tmem_d, a0 + j * (2048u >> 4), b0 + j * (2048u >> 4), idesc, j, lead);
 }
 __device__ __forceinline__ void mma_token_lead(uint32_t tmem_d, uint32_t x_smem, uint32_t w_smem, uint32_t lead) {
   constexpr uint32_t idesc = umma_idesc_bf16(64, 64, true, true, false);
