@@ -228,6 +228,7 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   cluster_arrive();     // the peers' mbarriers and abort flags are initialised before anything is sent to them
   cluster_wait();
   const uint32_t tmem = *tmem_slot;
+  const uint32_t lead = elect_one() ? 1u : 0u;      // the lane of an issuing warp whose MMAs are enabled
 
   typename C::Sum csum;
   csum.bufp = smem + C::OFF_SUM;
@@ -282,24 +283,21 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   };
 #define TTT_ISSUE4(W0, W1_, W2_, W3)  \
   if (warp < 4) {                     \
-    if (elect_one()) {                \
-      tc_fence_after_sync();          \
-      if (warp == 0) { W0; }          \
-      else if (warp == 1) { W1_; }    \
-      else if (warp == 2) { W2_; }    \
-      else { W3; }                    \
-      umma_commit(&bars[BAR_MMA]);    \
-    }                                 \
-    __syncwarp();                     \
+    tc_fence_after_sync();            \
+    if (warp == 0) { W0; }            \
+    else if (warp == 1) { W1_; }      \
+    else if (warp == 2) { W2_; }      \
+    else { W3; }                      \
+    if (lead) umma_commit(&bars[BAR_MMA]);        \
   }
   // hidden-major block products over this CTA's NB blocks: D[b] (+)= A[b] * Bt
 #define HID_ALL(KBMN, D, A, BT, ACC)                                                          \
   do {                                                                                        \
     _Pragma("unroll") for (int b_ = 0; b_ < NB; ++b_)                                         \
-      mma_hid64<KBMN>(tmem + (D) + b_ * 64, smem_u32(A) + b_ * TILE, smem_u32(BT), (ACC));    \
+      mma_hid64<KBMN>(tmem + (D) + b_ * 64, smem_u32(A) + b_ * TILE, smem_u32(BT), (ACC), lead);    \
   } while (0)
 #define HID_ONE(KBMN, D, A, BT, ACC, B_)                                                      \
-  mma_hid64<KBMN>(tmem + (D) + (B_) * 64, smem_u32(A) + (B_) * TILE, smem_u32(BT), (ACC))
+  mma_hid64<KBMN>(tmem + (D) + (B_) * 64, smem_u32(A) + (B_) * TILE, smem_u32(BT), (ACC), lead)
 
   const long tok_rows0 = sid * NC * 64;
 
@@ -520,21 +518,18 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       wait_mma();
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
-        float z[16], g[16], gp[16];
-        tok_ld(tm, tmem + C::TM_A + b * 64, z);
+        TokFrag z, g, gp;
+        frag_ld(tm, tmem + C::TM_A + b * 64, z);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            z[4 * q + h] += b1v[b][0];
-            z[4 * q + 2 + h] += b1v[b][1];
-            gelu_pair(z[4 * q + h], g[4 * q + h], gp[4 * q + h]);
-            gelu_pair(z[4 * q + 2 + h], g[4 * q + 2 + h], gp[4 * q + 2 + h]);
-          }
+          z.a[q] = add2(z.a[q], pk1(b1v[b][0]));
+          z.b[q] = add2(z.b[q], pk1(b1v[b][1]));
+          gelu_pair2(z.a[q], g.a[q], gp.a[q]);
+          gelu_pair2(z.b[q], g.b[q], gp.b[q]);
         }
-        tok_st_tile(tm, bX2 + b * TILE, g);
-        tok_st_tile(tm, bGP + b * TILE, gp);
-        tok_st_tile(tm, bZ1 + b * TILE, z);
+        frag_st_tile(tm, bX2 + b * TILE, g);
+        frag_st_tile(tm, bGP + b * TILE, gp);
+        frag_st_tile(tm, bZ1 + b * TILE, z);
       }
       publish();
       if (tid == kProd) {
@@ -545,7 +540,7 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       }
 
       // MMA2: partial Z2 = X2 W2
-      TTT_ISSUE4(mma_tok_partial(tmem + C::TM_B, smem_u32(bX2), smem_u32(bW2), NB),
+      TTT_ISSUE4(mma_tok_partial(tmem + C::TM_B, smem_u32(bX2), smem_u32(bW2), NB, lead),
                  ,
                  ,
                  )
@@ -688,7 +683,7 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         // b2 += column sums of U2, taken by the tensor pipe in the same phase (the window of these small MMAs is
         // too short to hide a pass over the tile by the warps)
         TTT_ISSUE4(HID_ONE(false, C::TM_A, bW2, tGZ2, 0u, 0),
-                   mma_colsum(tmem + C::TM_CS, smem_u32(tU2), smem_u32(smem + C::OFF_ONES)),
+                   mma_colsum(tmem + C::TM_CS, smem_u32(tU2), smem_u32(smem + C::OFF_ONES), lead),
                    ,
                    )
         wait_mma();
@@ -779,19 +774,16 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       wait_mma();
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
-        float z[16], g[16];
-        tok_ld(tm, tmem + C::TM_A + b * 64, z);
+        TokFrag z, g;
+        frag_ld(tm, tmem + C::TM_A + b * 64, z);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            // the sweep needs gelu'(Z1_bar) only: it is cheaper here, next to gelu, than there from a bf16 copy
-            gelu_pair(z[4 * q + h] + b1v[b][0], g[4 * q + h], z[4 * q + h]);
-            gelu_pair(z[4 * q + 2 + h] + b1v[b][1], g[4 * q + 2 + h], z[4 * q + 2 + h]);
-          }
+          // the sweep needs gelu'(Z1_bar) only: it is cheaper here, next to gelu, than there from a bf16 copy
+          gelu_pair2(add2(z.a[q], pk1(b1v[b][0])), g.a[q], z.a[q]);
+          gelu_pair2(add2(z.b[q], pk1(b1v[b][1])), g.b[q], z.b[q]);
         }
-        tok_st_tile(tm, bX2 + b * TILE, g);
-        tok_st_tile(tm, bZ1 + b * TILE, z);
+        frag_st_tile(tm, bX2 + b * TILE, g);
+        frag_st_tile(tm, bZ1 + b * TILE, z);
       }
       publish();
 
@@ -801,7 +793,7 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         store_big(p.sc_Z1b + slot * BIG, bZ1);
         tma_commit_group();
       }
-      TTT_ISSUE4(mma_tok_partial(tmem + C::TM_B, smem_u32(bX2), smem_u32(bW2), NB),
+      TTT_ISSUE4(mma_tok_partial(tmem + C::TM_B, smem_u32(bX2), smem_u32(bW2), NB, lead),
                  ,
                  ,
                  )
@@ -1024,7 +1016,7 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       wait_bar(BAR_BIG + ib3);
       wait_bar(BAR_T + 2);
       // G7 (partial dQ) // G2 // G3
-      TTT_ISSUE4(mma_tok_partial(tmem + C::TM_B, smem_u32(big(ib2)), smem_u32(big(ib0)), NB),
+      TTT_ISSUE4(mma_tok_partial(tmem + C::TM_B, smem_u32(big(ib2)), smem_u32(big(ib0)), NB, lead),
                  HID_ALL(true, C::TM_S2, big(ib3), t_g, 1u),
                  HID_ONE(true, C::TM_S1, big(ib2), t_q, 1u, 0),
                  if (NB > 1) HID_ONE(true, C::TM_S1, big(ib2), t_q, 1u, NB - 1))
@@ -1061,8 +1053,8 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       wait_bar(BAR_T + 4);
       wait_bar(BAR_BIG + ib1);      // X2, requested two phases ago
       // G8 (partial T1) // G5 (partial acc1) // G4
-      TTT_ISSUE4(mma_tok_partial(tmem + C::TM_B, smem_u32(big(ib4)), smem_u32(big(ib0)), NB),
-                 mma_tok_partial(tmem + C::TM_B + 64, smem_u32(big(ib1)), smem_u32(big(ib3)), NB),
+      TTT_ISSUE4(mma_tok_partial(tmem + C::TM_B, smem_u32(big(ib4)), smem_u32(big(ib0)), NB, lead),
+                 mma_tok_partial(tmem + C::TM_B + 64, smem_u32(big(ib1)), smem_u32(big(ib3)), NB, lead),
                  HID_ONE(false, C::TM_A, big(ib0), t_k, 0u, 0),
                  if (NB > 1) HID_ONE(false, C::TM_A, big(ib0), t_k, 0u, NB - 1))
       // ---- while the MMAs run: partial sums over this CTA's hidden units of gZ1 * G_b1 (fourth term of d_eta)
@@ -1139,7 +1131,7 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       wait_bar(BAR_BIG + ib1);
       wait_bar(BAR_T + 5);
       // G6 (partial acc2) // G10
-      TTT_ISSUE4(mma_tok_partial(tmem + C::TM_A, smem_u32(big(ib4)), smem_u32(big(ib1)), NB),
+      TTT_ISSUE4(mma_tok_partial(tmem + C::TM_A, smem_u32(big(ib4)), smem_u32(big(ib1)), NB, lead),
                  HID_ONE(true, C::TM_S2, big(ib4), t_gz2, 1u, 0),
                  if (NB > 1) HID_ONE(true, C::TM_S2, big(ib4), t_gz2, 1u, NB - 1),
                  )
@@ -1385,7 +1377,7 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       }
       TTT_ISSUE4(HID_ONE(false, C::TM_B, big(ib1), t_q, 0u, 0); HID_ONE(false, C::TM_B, big(ib3), t_g, 1u, 0),
                  if (NB > 1) { HID_ONE(false, C::TM_B, big(ib1), t_q, 0u, NB - 1); HID_ONE(false, C::TM_B, big(ib3), t_g, 1u, NB - 1); }
-                 else if (C::kMmaColsum) mma_colsum(tmem + C::TM_CS + 8, smem_u32(t_q), smem_u32(smem + C::OFF_ONES)),
+                 else if (C::kMmaColsum) mma_colsum(tmem + C::TM_CS + 8, smem_u32(t_q), smem_u32(smem + C::OFF_ONES), lead),
                  HID_ONE(false, C::TM_A, big(ib1), t_gz2, 0u, 0),
                  if (NB > 1) HID_ONE(false, C::TM_A, big(ib1), t_gz2, 0u, NB - 1))
       if constexpr (C::kRowSplit && C::kMmaColsum) {
@@ -1488,7 +1480,7 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       wait_bar(BAR_BIG + ib4);
       wait_bar(BAR_BIG + ib3);
       // G13 (partial dK) // G15 // G14
-      TTT_ISSUE4(mma_tok_partial(tmem + C::TM_A, smem_u32(big(ib2)), smem_u32(big(ib4)), NB),
+      TTT_ISSUE4(mma_tok_partial(tmem + C::TM_A, smem_u32(big(ib2)), smem_u32(big(ib4)), NB, lead),
                  HID_ALL(true, C::TM_S1, big(ib2), t_k, 1u),
                  HID_ONE(true, C::TM_S2, big(ib3), t_q, 1u, 0),
                  if (NB > 1) HID_ONE(true, C::TM_S2, big(ib3), t_q, 1u, NB - 1))

@@ -103,39 +103,40 @@ __device__ __forceinline__ void tok_st_tmem(const TokMap& m, uint32_t tmem_acc, 
 // blocks of 64 rows: every accumulator is an M = 64 tile (row r in TMEM lane r % 16 + 32 (r / 16)) read
 // back with the 16x256b fragments of TokMap, whether its rows are hidden units or tokens.
 //
+// All are issued by a whole warp under a predicate (`lead`: see mma_lead).
 // "Hidden-major" block product: D[64 hid x 64] (+)= A * B with A one [64][64] bf16 block read K-major
 // (row = hidden unit) and B a [64][64] tile read K-major (row = N index) or MN-major (row = K index).
 template <bool kBMn>
-__device__ __forceinline__ void mma_hid64(uint32_t tmem_d, uint32_t a_smem, uint32_t b_smem, uint32_t accumulate) {
+__device__ __forceinline__ void mma_hid64(uint32_t tmem_d, uint32_t a_smem, uint32_t b_smem, uint32_t accumulate, uint32_t lead) {
   constexpr uint32_t idesc = umma_idesc_bf16(64, 64, false, kBMn, false);
   const uint32_t a0 = desc_lo(a_smem, 16);
   const uint32_t b0 = desc_lo(b_smem, kBMn ? 8192 : 16);
   constexpr uint32_t bstep = kBMn ? (2048u >> 4) : (32u >> 4);
-  mma_issue_rt(tmem_d, a0, b0, idesc, accumulate);
+  mma_lead_rt(tmem_d, a0, b0, idesc, accumulate, lead);
 #pragma unroll
-  for (int j = 1; j < 4; ++j) mma_issue_rt(tmem_d, a0 + j * 2, b0 + j * bstep, idesc, 1u);
+  for (int j = 1; j < 4; ++j) mma_lead_rt(tmem_d, a0 + j * 2, b0 + j * bstep, idesc, 1u, lead);
 }
 // Partial "token-major" product over this CTA's hidden units: D[64 tok x 64] = X[64 x R] * W[R x 64], both
 // operands [R][64] tiles read MN-major (row = hidden unit), R = 64 nblk.
-__device__ __forceinline__ void mma_tok_partial(uint32_t tmem_d, uint32_t x_smem, uint32_t w_smem, int nblk) {
+__device__ __forceinline__ void mma_tok_partial(uint32_t tmem_d, uint32_t x_smem, uint32_t w_smem, int nblk, uint32_t lead) {
   constexpr uint32_t idesc = umma_idesc_bf16(64, 64, true, true, false);
   const uint32_t a0 = desc_lo(x_smem, TILE);
   const uint32_t b0 = desc_lo(w_smem, TILE);
-  mma_issue_rt(tmem_d, a0, b0, idesc, 0u);
+  mma_lead_rt(tmem_d, a0, b0, idesc, 0u, lead);
 #pragma unroll 1
-  for (int j = 1; j < 4 * nblk; ++j) mma_issue_rt(tmem_d, a0 + j * (2048u >> 4), b0 + j * (2048u >> 4), idesc, 1u);
+  for (int j = 1; j < 4 * nblk; ++j) mma_lead_rt(tmem_d, a0 + j * (2048u >> 4), b0 + j * (2048u >> 4), idesc, 1u, lead);
 }
 
 // Column sums of a [64 tok][64] bf16 tile on the (otherwise idle) tensor pipe: D[64 feat x 8] = T^T * ones, the
 // tile read MN-major (row = token = contraction index) against 8 rows of bf16 ones (1 KB, 1024-byte aligned,
 // read K-major); every one of the 8 columns of D holds the sums.  Read back with colsum_read by warps 0..3.
-__device__ __forceinline__ void mma_colsum(uint32_t tmem_d, uint32_t tile_smem, uint32_t ones_smem) {
+__device__ __forceinline__ void mma_colsum(uint32_t tmem_d, uint32_t tile_smem, uint32_t ones_smem, uint32_t lead) {
   constexpr uint32_t idesc = umma_idesc_bf16(64, 8, true, false, false);
   const uint32_t a0 = desc_lo(tile_smem, TILE);
   const uint32_t b0 = desc_lo(ones_smem, 16);
-  mma_issue_rt(tmem_d, a0, b0, idesc, 0u);
+  mma_lead_rt(tmem_d, a0, b0, idesc, 0u, lead);
 #pragma unroll
-  for (int j = 1; j < 4; ++j) mma_issue_rt(tmem_d, a0 + j * (2048u >> 4), b0 + j * (32u >> 4), idesc, 1u);
+  for (int j = 1; j < 4; ++j) mma_lead_rt(tmem_d, a0 + j * (2048u >> 4), b0 + j * (32u >> 4), idesc, 1u, lead);
 }
 // Warp q of warps 0..3 (all 32 lanes call): lanes 0..15 return the sum of column 16 q + lane (row r of an M = 64
 // accumulator sits in tensor-memory lane r % 16 + 32 (r / 16)); the other lanes return garbage.

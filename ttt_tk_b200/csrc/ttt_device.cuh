@@ -315,6 +315,19 @@ __device__ __forceinline__ void mma_lead(uint32_t tmem_d, uint32_t a_lo, uint32_
       "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kDescHi), "n"(kAccumulate ? 1 : 0), "r"(lead)
       : "memory");
 }
+// ... with the accumulate flag in a register, for rolled issue loops
+__device__ __forceinline__ void mma_lead_rt(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+                                            uint32_t accumulate, uint32_t lead) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %4};\n\t"
+      "mov.b64 db, {%2, %4};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kDescHi), "r"(accumulate), "r"(lead)
+      : "memory");
+}
 // one 128-row block: D[128 x 64] (+)= A[128][64] B
 template <bool kBMn, bool kAccumulate>
 __device__ __forceinline__ void mma_hidden_lead(uint32_t tmem_d, uint32_t a_smem, uint32_t b_smem, int blk, uint32_t lead) {
@@ -348,36 +361,6 @@ __device__ __forceinline__ void mma_hidden_ta(uint32_t tmem_d, uint32_t tmem_a, 
   mma_lead_ta<kAccumulate>(tmem_d, tmem_a, b0, idesc, lead);
 #pragma unroll
   for (int j = 1; j < 4; ++j) mma_lead_ta<true>(tmem_d, tmem_a + j * 8, b0 + j * bstep, idesc, lead);
-}
-// The same products with rolled issue loops, for a kernel whose code is of the size of the instruction cache.
-__device__ __forceinline__ void mma_lead_rt(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc,
-                                            uint32_t lead) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
-      "mov.b64 da, {%1, %4};\n\t"
-      "mov.b64 db, {%2, %4};\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "setp.ne.b32 q, %6, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
-      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kDescHi), "r"(acc), "r"(lead)
-      : "memory");
-}
-template <bool kBMn, bool kAccumulate>
-__device__ __forceinline__ void mma_hidden_roll(uint32_t tmem_d, uint32_t a_smem, uint32_t b_smem, int blk, uint32_t lead) {
-  constexpr uint32_t idesc = umma_idesc_bf16(128, 64, false, kBMn, false);
-  const uint32_t a0 = desc_lo(a_smem, 16) + blk * (16384u >> 4);
-  const uint32_t b0 = desc_lo(b_smem, kBMn ? 8192 : 16);
-  constexpr uint32_t bstep = kBMn ? (2048u >> 4) : (32u >> 4);
-#pragma unroll 1
-  for (uint32_t j = 0; j < 4; ++j)
-    mma_lead_rt(tmem_d + blk * 64, a0 + j * 2, b0 + j * bstep, idesc, kAccumulate ? 1u : j, lead);
-}
-__device__ __forceinline__ void mma_token_roll(uint32_t tmem_d, uint32_t x_smem, uint32_t w_smem, uint32_t lead) {
-  constexpr uint32_t idesc = umma_idesc_bf16(64, 64, true, true, false);
-  const uint32_t a0 = desc_lo(x_smem, BIG);
-  const uint32_t b0 = desc_lo(w_smem, BIG);
-#pragma unroll 1
-  for (uint32_t j = 0; j < 16; ++j) mma_lead_rt(tmem_d, a0 + j * (2048u >> 4), b0 + j * (2048u >> 4), idesc, j, lead);
 }
 __device__ __forceinline__ void mma_token_lead(uint32_t tmem_d, uint32_t x_smem, uint32_t w_smem, uint32_t lead) {
   constexpr uint32_t idesc = umma_idesc_bf16(64, 64, true, true, false);

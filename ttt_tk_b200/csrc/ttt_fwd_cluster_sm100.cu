@@ -172,6 +172,7 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   cluster_arrive();
   cluster_wait();
   const uint32_t tmem = *tmem_slot;
+  const uint32_t lead = elect_one() ? 1u : 0u;      // the lane of an issuing warp whose MMAs are enabled
 
   typename C::RS rs;
   rs.bufp = smem + C::OFF_SUM;
@@ -293,15 +294,12 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   // without work too): the MMA barrier counts four arrivals per phase.
 #define TTT_ISSUE4(W0, W1_, W2_, W3)  \
   if (warp < 4) {                     \
-    if (elect_one()) {                \
-      tc_fence_after_sync();          \
-      if (warp == 0) { W0; }          \
-      else if (warp == 1) { W1_; }    \
-      else if (warp == 2) { W2_; }    \
-      else { W3; }                    \
-      umma_commit(mma_bar);           \
-    }                                 \
-    __syncwarp();                     \
+    tc_fence_after_sync();            \
+    if (warp == 0) { W0; }            \
+    else if (warp == 1) { W1_; }      \
+    else if (warp == 2) { W2_; }      \
+    else { W3; }                      \
+    if (lead) umma_commit(mma_bar);        \
   }
 
   // The output of a mini-batch: its partial Z2b tile is sent at the end of the mini-batch (reduce-scatter);
@@ -383,8 +381,8 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     mbar_wait_cl(&full[s], (it / kStages) & 1, abort_flag, limit, kC);
 
     // ---- MMA1: Z1^T = W1^T K^T (one block per issuer)
-    TTT_ISSUE4(mma_hid64<false>(tmem + C::TM_A, smem_u32(sW1), smem_u32(sK), 0u),
-               if (NB > 1) mma_hid64<false>(tmem + C::TM_A + 64, smem_u32(sW1 + TILE), smem_u32(sK), 0u),
+    TTT_ISSUE4(mma_hid64<false>(tmem + C::TM_A, smem_u32(sW1), smem_u32(sK), 0u, lead),
+               if (NB > 1) mma_hid64<false>(tmem + C::TM_A + 64, smem_u32(sW1 + TILE), smem_u32(sK), 0u, lead),
                ,
                )
     if (ckpt) {
@@ -400,23 +398,20 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // ---- EPI1: X2^T = gelu(Z1^T + b1), G' = gelu'(Z1^T + b1)
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
-      float z[16], g[16], gp[16];
-      tok_ld(tm, tmem + C::TM_A + b * 64, z);
+      TokFrag z, g, gp;
+      frag_ld(tm, tmem + C::TM_A + b * 64, z);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          gelu_pair(z[4 * j + e] + b1v[b][0], g[4 * j + e], gp[4 * j + e]);
-          gelu_pair(z[4 * j + 2 + e] + b1v[b][1], g[4 * j + 2 + e], gp[4 * j + 2 + e]);
-        }
+        gelu_pair2(add2(z.a[j], pk1(b1v[b][0])), g.a[j], gp.a[j]);
+        gelu_pair2(add2(z.b[j], pk1(b1v[b][1])), g.b[j], gp.b[j]);
       }
-      tok_st_tile(tm, sX2 + b * TILE, g);
-      tok_st_tile(tm, sGP + b * TILE, gp);
+      frag_st_tile(tm, sX2 + b * TILE, g);
+      frag_st_tile(tm, sGP + b * TILE, gp);
     }
     publish();
 
     // ---- MMA2: partial Z2 = X2 W2 over this CTA's hidden units
-    TTT_ISSUE4(mma_tok_partial(tmem + C::TM_Z, smem_u32(sX2), smem_u32(sW2), NB),
+    TTT_ISSUE4(mma_tok_partial(tmem + C::TM_Z, smem_u32(sX2), smem_u32(sW2), NB, lead),
                ,
                ,
                )
@@ -530,9 +525,9 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // ---- MMA3: R^T = W2 U2^T
     // the column sums of U2 (the bf16 operand the W2 update sees) for b2 are taken by the tensor pipe in the same
     // phase: the window of these small MMAs is too short to hide a pass over the tile by the warps
-    TTT_ISSUE4(mma_hid64<false>(tmem + C::TM_A, smem_u32(sW2), smem_u32(sU2), 0u),
-               if (NB > 1) mma_hid64<false>(tmem + C::TM_A + 64, smem_u32(sW2 + TILE), smem_u32(sU2), 0u),
-               mma_colsum(tmem + C::TM_S, smem_u32(sU2), smem_u32(smem + C::OFF_ONES)),
+    TTT_ISSUE4(mma_hid64<false>(tmem + C::TM_A, smem_u32(sW2), smem_u32(sU2), 0u, lead),
+               if (NB > 1) mma_hid64<false>(tmem + C::TM_A + 64, smem_u32(sW2 + TILE), smem_u32(sU2), 0u, lead),
+               mma_colsum(tmem + C::TM_S, smem_u32(sU2), smem_u32(smem + C::OFF_ONES), lead),
                )
     wait_mma();
     // b2 += column sums, the same in every CTA of the cluster (its next reader comes after the barrier below)
@@ -571,10 +566,10 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     publish();
 
     // ---- MMA4: W1^T += U1^T K ;  W2 += X2^T U2
-    TTT_ISSUE4(mma_hid64<true>(tmem + C::TM_W1, smem_u32(sGP), smem_u32(sK), 1u),
-               mma_hid64<true>(tmem + C::TM_W2, smem_u32(sX2), smem_u32(sU2), 1u),
-               if (NB > 1) mma_hid64<true>(tmem + C::TM_W1 + 64, smem_u32(sGP + TILE), smem_u32(sK), 1u),
-               if (NB > 1) mma_hid64<true>(tmem + C::TM_W2 + 64, smem_u32(sX2 + TILE), smem_u32(sU2), 1u))
+    TTT_ISSUE4(mma_hid64<true>(tmem + C::TM_W1, smem_u32(sGP), smem_u32(sK), 1u, lead),
+               mma_hid64<true>(tmem + C::TM_W2, smem_u32(sX2), smem_u32(sU2), 1u, lead),
+               if (NB > 1) mma_hid64<true>(tmem + C::TM_W1 + 64, smem_u32(sGP + TILE), smem_u32(sK), 1u, lead),
+               if (NB > 1) mma_hid64<true>(tmem + C::TM_W2 + 64, smem_u32(sX2 + TILE), smem_u32(sU2), 1u, lead))
     wait_mma();
     // ---- EPI4: refresh the bf16 operand copies of the state
 #pragma unroll
@@ -588,30 +583,28 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     publish();
 
     // ---- MMA5: Z1b^T = W1^T Q^T
-    TTT_ISSUE4(mma_hid64<false>(tmem + C::TM_A, smem_u32(sW1), smem_u32(sQ), 0u),
-               if (NB > 1) mma_hid64<false>(tmem + C::TM_A + 64, smem_u32(sW1 + TILE), smem_u32(sQ), 0u),
+    TTT_ISSUE4(mma_hid64<false>(tmem + C::TM_A, smem_u32(sW1), smem_u32(sQ), 0u, lead),
+               if (NB > 1) mma_hid64<false>(tmem + C::TM_A + 64, smem_u32(sW1 + TILE), smem_u32(sQ), 0u, lead),
                ,
                )
     wait_mma();
     // ---- EPI5: X2b^T = gelu(Z1b^T + b1)
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
-      float z[16];
-      tok_ld(tm, tmem + C::TM_A + b * 64, z);
+      TokFrag z;
+      frag_ld(tm, tmem + C::TM_A + b * 64, z);
+      const f32x2 h0 = pk1(0.5f * b1v[b][0]), h1 = pk1(0.5f * b1v[b][1]);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          z[4 * j + e] = gelu_only(z[4 * j + e] + b1v[b][0]);
-          z[4 * j + 2 + e] = gelu_only(z[4 * j + 2 + e] + b1v[b][1]);
-        }
+        z.a[j] = gelu_half2(fma2(z.a[j], pk1(0.5f), h0));
+        z.b[j] = gelu_half2(fma2(z.b[j], pk1(0.5f), h1));
       }
-      tok_st_tile(tm, sX2 + b * TILE, z);
+      frag_st_tile(tm, sX2 + b * TILE, z);
     }
     publish();
 
     // ---- MMA6: partial Z2b = X2b W2
-    TTT_ISSUE4(mma_tok_partial(tmem + C::TM_Z, smem_u32(sX2), smem_u32(sW2), NB),
+    TTT_ISSUE4(mma_tok_partial(tmem + C::TM_Z, smem_u32(sX2), smem_u32(sW2), NB, lead),
                ,
                ,
                )
