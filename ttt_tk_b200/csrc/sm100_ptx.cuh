@@ -18,6 +18,11 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// First 1024-byte boundary of the dynamic shared memory.  An offset is added to the array itself: after a round trip
+// through an integer the compiler no longer knows the address space, and every access through the result would be a
+// generic one with 64-bit addresses.
+__device__ __forceinline__ uint8_t* smem_align_1024(uint8_t* raw) { return raw + ((0u - smem_u32(raw)) & 1023u); }
+
 __device__ __forceinline__ uint64_t globaltimer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

@@ -154,7 +154,7 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmOut,
                const FwdParams p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = smem_align_1024(smem_raw);
 
   const int tid = threadIdx.x, lane = tid & 31;
   const int cta_warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // same value, known to be warp-uniform

@@ -25,7 +25,7 @@ struct ProbeParams {
 
 __global__ void __launch_bounds__(128, 1) umma_probe_kernel(ProbeParams p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = smem_align_1024(smem_raw);
   __shared__ uint64_t bar;
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t abort_flag;
