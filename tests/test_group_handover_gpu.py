@@ -1,0 +1,34 @@
+"""Edges of the kernels that split a stream between two groups of warps (MLP forward and TTT-Linear forward: chain and
+output; TTT-Linear backward: recompute of one checkpoint group beside the sweep of another), against the CPU oracles:
+the first mini-batches, where a group still waits for nothing, checkpoints after every one or a ragged last group, one or
+many checkpoint groups, and stream counts on both sides of the number of SMs."""
+import pytest
+
+import test_forward_gpu as mlp
+import test_linear_backward_gpu as lbwd
+import test_linear_forward_gpu as lfwd
+from oracle import ttt_mlp as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,H,NC,cgs", [(1, 1, 1, 1), (1, 2, 2, 1), (1, 1, 3, 2), (1, 3, 5, 2), (2, 74, 3, 2), (1, 149, 5, 1)])
+def test_two_group_kernels_match_oracle(B, H, NC, cgs):
+    d = orc.make_inputs(B, H, NC, seed=NC)
+    ref = orc.ttt_forward(d["XQ"], d["XK"], d["XV"], d["last_eta"], d["ttt_norm_weight"], d["ttt_norm_bias"],
+                          d["W1"], d["b1"], d["W2"], d["b2"], cgs)
+    mlp.check(mlp.run_forward(d, cgs, final=True), ref,
+              [("Out", mlp.TOL_OUT)] + [(k, mlp.TOL_STATE) for k in ("W1_checkpoints", "W2_checkpoints", "W1_final", "W2_final")])
+
+    d = lbwd.make(B, H, NC, seed=NC + 1)
+    ref_fwd, ref_bwd = lbwd.oracle(d, cgs)
+    lfwd.check(lfwd.run(d, cgs), ref_fwd)
+    lbwd.check(lbwd.run(d, cgs), ref_bwd)
+
+
+@pytest.mark.parametrize("NC,cgs", [(3, 4), (9, 1), (9, 2), (13, 4)])
+def test_linear_backward_group_edges(NC, cgs):
+    """One group only, groups of one mini-batch, and a ragged last group after odd and even numbers of whole ones."""
+    d = lbwd.make(1, 3, NC, seed=NC)
+    _, ref = lbwd.oracle(d, cgs)
+    lbwd.check(lbwd.run(d, cgs), ref)
