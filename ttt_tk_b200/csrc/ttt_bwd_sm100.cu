@@ -349,7 +349,9 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 )
       wait_mma();
       {
-#pragma unroll 1
+        // (this and the other passes over 64 columns are unrolled: one pass's stores run beside the next one's
+        // loads, 24.5 -> 24.0 us per mini-batch at 128 streams; all 64 columns loaded at once is slower, 24.2)
+#pragma unroll
         for (int half = 0; half < 4; ++half) {   // 16 columns per pass
           uint32_t v[16];
           tmem_ld16(tmem + lane_base + TM_A + wg * 64 + half * 16, v);
@@ -455,7 +457,7 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       wait_mma();
       {
         f32x2 bsum = 0ull;
-#pragma unroll 1
+#pragma unroll
         for (int half = 0; half < 4; ++half) {   // 16 columns per pass
           uint32_t v[16];
           tmem_ld16(tmem + lane_base + TM_A + wg * 64 + half * 16, v);
@@ -496,7 +498,7 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 mma_hidden_half(tmem + TM_S2, smem_u32(bX2), smem_u32(tU2), true, true, 1))
       wait_mma();
       {
-#pragma unroll 1
+#pragma unroll
         for (int half = 0; half < 4; ++half) {   // 16 columns per pass
           uint32_t v[16];
           float f[16];
@@ -538,7 +540,7 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 )
       wait_mma();
       {
-#pragma unroll 1
+#pragma unroll
         for (int half = 0; half < 4; ++half) {   // 16 columns per pass
           uint32_t v[16];
           tmem_ld16(tmem + lane_base + TM_A + wg * 64 + half * 16, v);
@@ -735,7 +737,7 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       {
         uint8_t* bz = big(ib2);
         f32x2 bsum = 0ull;
-#pragma unroll 1
+#pragma unroll
         for (int half = 0; half < 4; ++half) {   // 16 columns per pass
           uint32_t v[16];
           tmem_ld16(tmem + lane_base + TM_A + wg * 64 + half * 16, v);
@@ -778,7 +780,7 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       {
         uint8_t* s1b = big(ib0);
         uint8_t* s2b = big(ib3);
-#pragma unroll 1
+#pragma unroll
         for (int half = 0; half < 4; ++half) {   // 16 columns per pass
           uint32_t v[16];
           float f[16];
@@ -855,7 +857,7 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         uint8_t* bz = big(ib2);
         uint8_t* bp = big(ib4);
         uint8_t* bgp = big(ib0);
-#pragma unroll 1
+#pragma unroll
         for (int half = 0; half < 4; ++half) {   // 16 columns per pass
           uint32_t v[16];
           tmem_ld16(tmem + lane_base + TM_A + wg * 64 + half * 16, v);
@@ -1049,7 +1051,7 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         uint8_t* bs = big(ib2);
         const uint8_t* bgp = big(ib0);
         f32x2 bs2 = 0ull;
-#pragma unroll 1
+#pragma unroll
         for (int half = 0; half < 4; ++half) {   // 16 columns per pass
           uint32_t v[16], w[16];
           tmem_ld16(tmem + lane_base + TM_B + wg * 64 + half * 16, v);
