@@ -69,8 +69,9 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 // How many CTAs share one stream.  The mini-batches of a stream are strictly sequential, so with fewer
 // streams than SMs the idle SMs can only help by taking a share of every stream's hidden units.  The
 // thresholds are measured (B200, 148 SMs): four CTAs per stream win whenever they all fit on the GPU at
-// once (forward 18 %, backward 17-20 % per mini-batch over one CTA).  Two CTAs per stream win in the
-// forward whenever they fit (12-17 %).  In the backward they gain 6-11 % up to 32 streams, where four CTAs
+// once (forward 18 %, backward 17-20 % per mini-batch over one CTA).  Two CTAs per stream beat one
+// plain CTA in the forward (12-17 %), but not the two-group form that the forward launcher runs instead when nobody
+// asked for two (see there).  In the backward they gain 6-11 % up to 32 streams, where four CTAs
 // are the better choice anyway, and nothing beyond 37 streams (more than 74 CTAs: both SMs of a TPC are
 // then busy, and the backward, whose scratch traffic goes through the port the two share, slows down by
 // as much as the split gained), so the backward is never given two.

