@@ -472,20 +472,16 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const float2 b2c = *reinterpret_cast<const float2*>(sB2 + 2 * lane);
       float z[NR][2];
       rs.recv(z, warp, lane, zb_tag);
+      float rstd[NR];
+      RSx::row_layernorm(z, b2c, TTT_LN_EPS, rstd);
 #pragma unroll
       for (int i = 0; i < NR; ++i) {
         const int r = rs.row(i, warp);
-        z[i][0] += b2c.x;
-        z[i][1] += b2c.y;
-        const float mu = RSx::row_sum(z[i][0] + z[i][1]) * (1.f / 64.f);
-        z[i][0] -= mu;
-        z[i][1] -= mu;
-        const float rstd = rsqrtf(RSx::row_sum(fmaf(z[i][0], z[i][0], z[i][1] * z[i][1])) * (1.f / 64.f) + TTT_LN_EPS);
-        rs.all_gather_store(tXln, &bars[BAR_AG2], r, lane, z[i][0] * rstd, z[i][1] * rstd);
-        if (lane == 0) sSigAG[r] = rstd;
+        rs.all_gather_store(tXln, &bars[BAR_AG2], r, lane, z[i][0], z[i][1]);
+        if (lane == 0) sSigAG[r] = rstd[i];
         else if (lane < kC)
           st_async_f1(mapa(smem_u32(sSigAG + r), rank ^ static_cast<uint32_t>(lane)),
-                      mapa(smem_u32(&bars[BAR_AG2]), rank ^ static_cast<uint32_t>(lane)), rstd);
+                      mapa(smem_u32(&bars[BAR_AG2]), rank ^ static_cast<uint32_t>(lane)), rstd[i]);
       }
     };
     // after the barrier that follows the wait on BAR_AG2: the gathered tile and its 1/std leave for the slot
@@ -575,21 +571,21 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         }
         float z[NR][2];
         rs.recv(z, warp, lane, tag);
+        float rstd[NR], g[NR][2], a[2 * NR];
+        RSx::row_layernorm(z, b2c, TTT_LN_EPS, rstd);
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+          g[i][0] = (fmaf(gam.x, z[i][0], bet.x) - (vv[i].x - kk[i].x)) * gam.x;
+          g[i][1] = (fmaf(gam.y, z[i][1], bet.y) - (vv[i].y - kk[i].y)) * gam.y;
+          a[2 * i] = g[i][0] + g[i][1];
+          a[2 * i + 1] = fmaf(g[i][0], z[i][0], g[i][1] * z[i][1]);
+        }
+        RSx::row_sums(a);
 #pragma unroll
         for (int i = 0; i < NR; ++i) {
           const int r = rs.row(i, warp);
-          z[i][0] += b2c.x;
-          z[i][1] += b2c.y;
-          const float mu = RSx::row_sum(z[i][0] + z[i][1]) * (1.f / 64.f);
-          z[i][0] -= mu;
-          z[i][1] -= mu;
-          const float rstd = rsqrtf(RSx::row_sum(fmaf(z[i][0], z[i][0], z[i][1] * z[i][1])) * (1.f / 64.f) + TTT_LN_EPS);
-          const float x0 = z[i][0] * rstd, x1 = z[i][1] * rstd;
-          const float g0 = (fmaf(gam.x, x0, bet.x) - (vv[i].x - kk[i].x)) * gam.x;
-          const float g1 = (fmaf(gam.y, x1, bet.y) - (vv[i].y - kk[i].y)) * gam.y;
-          const float a0 = RSx::row_sum(g0 + g1);
-          const float a1 = RSx::row_sum(fmaf(g0, x0, g1 * x1));
-          const float sc = rstd * (1.f / 64.f);
+          const float x0 = z[i][0], x1 = z[i][1], g0 = g[i][0], g1 = g[i][1], a0 = a[2 * i], a1 = a[2 * i + 1];
+          const float sc = rstd[i] * (1.f / 64.f);
           // x_hat_fused leaves through this CTA's rows of the V tile; dl/dZ2 is rounded to bf16 once (the update
           // uses -eta times the rounded value)
           RSx::st_pair(tV, r, lane, x0, x1);
@@ -597,7 +593,7 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           const float d1 = __bfloat162float(__float2bfloat16((64.f * g1 - a0 - x1 * a1) * sc));
           rs.all_gather_store(tGZ2, &bars[BAR_AG], r, lane, d0, d1);
           rs.all_gather_store(tU2, &bars[BAR_AG], r, lane, neta[i] * d0, neta[i] * d1);
-          if (lane == 0) p.sc_sigf[slot * 64 + r] = rstd;
+          if (lane == 0) p.sc_sigf[slot * 64 + r] = rstd[i];
         }
         wait_bar(BAR_AG);
         if (xrow_slot >= 0) wait_bar(BAR_AG2);
@@ -1205,22 +1201,34 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             RSx::st_pair_global(p.dXQ + static_cast<long>(row0) * 64, rs.row(i, warp), lane, go[i].x + zq[i][0],
                                 go[i].y + zq[i][1]);
         }
+        // likewise: the row sums that need no A2.  grad_output_fused = gamma x_hat_fused + beta - (V - K)
+        float gof[NR][2], pre[2 * NR];
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+          gof[i][0] = fmaf(gam.x, xh[i].x, bet.x) - (vv[i].x - kr[i].x);
+          gof[i][1] = fmaf(gam.y, xh[i].y, bet.y) - (vv[i].y - kr[i].y);
+          pre[2 * i] = fmaf(gzr[i].x, gb2.x, gzr[i].y * gb2.y);
+          pre[2 * i + 1] = fmaf(gof[i][0] * gam.x, xh[i].x, gof[i][1] * gam.y * xh[i].y);
+        }
+        RSx::row_sums(pre);
         float z[NR][2], ex[NR];
         rs.recv_x(z, ex, warp, lane, a2_tag);
         float ca0 = 0.f, ca1 = 0.f, cv0 = 0.f, cv1 = 0.f;
+        float s23[2 * NR], gx[NR][2], sa[2 * NR];
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+          // the G_b2 parts of u = acc1 + G_b2
+          z[i][0] = fmaf(-etar[i], gb2.x, z[i][0]);
+          z[i][1] = fmaf(-etar[i], gb2.y, z[i][1]);
+          s23[2 * i] = z[i][0] + z[i][1];
+          s23[2 * i + 1] = fmaf(z[i][0], xh[i].x, z[i][1] * xh[i].y);
+        }
+        RSx::row_sums(s23);
 #pragma unroll
         for (int i = 0; i < NR; ++i) {
           const int r = rs.row(i, warp);
-          const float rstd = rsd[i];
-          // grad_output_fused = gamma x_hat_fused + beta - (V - K)
-          const float go0 = fmaf(gam.x, xh[i].x, bet.x) - (vv[i].x - kr[i].x);
-          const float go1 = fmaf(gam.y, xh[i].y, bet.y) - (vv[i].y - kr[i].y);
-          // the G_b2 parts of u = acc1 + G_b2
-          const float A0 = fmaf(-etar[i], gb2.x, z[i][0]), A1 = fmaf(-etar[i], gb2.y, z[i][1]);
-          const float de = ex[i] + RSx::row_sum(fmaf(gzr[i].x, gb2.x, gzr[i].y * gb2.y));
-          const float s2 = RSx::row_sum(A0 + A1);
-          const float s3 = RSx::row_sum(fmaf(A0, xh[i].x, A1 * xh[i].y));
-          const float s4 = RSx::row_sum(fmaf(go0 * gam.x, xh[i].x, go1 * gam.y * xh[i].y));
+          const float rstd = rsd[i], go0 = gof[i][0], go1 = gof[i][1], A0 = z[i][0], A1 = z[i][1];
+          const float s2 = s23[2 * i], s3 = s23[2 * i + 1], s4 = pre[2 * i + 1];
           const float bt0 = (A0 - (s2 + xh[i].x * s3) * (1.f / 64.f)) * rstd;
           const float bt1 = (A1 - (s2 + xh[i].y * s3) * (1.f / 64.f)) * rstd;
           const float gly0 = gam.x * bt0, gly1 = gam.y * bt1;
@@ -1233,12 +1241,20 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           RSx::st_pair_global(p.dXV + static_cast<long>(row0) * 64, r, lane, -gly0, -gly1);
           const float gx0 = fmaf(gly0, gam.x, -(go0 * gam.x * s3 + A0 * s4) * rstd * (1.f / 64.f));
           const float gx1 = fmaf(gly1, gam.y, -(go1 * gam.y * s3 + A1 * s4) * rstd * (1.f / 64.f));
-          const float sa0 = RSx::row_sum(((-gx0 * xh[i].x - A0 * gzr[i].x) + (-gx1 * xh[i].y - A1 * gzr[i].y)) * rstd);
-          const float sa1 = RSx::row_sum(gx0 + gx1);
+          sa[2 * i] = ((-gx0 * xh[i].x - A0 * gzr[i].x) + (-gx1 * xh[i].y - A1 * gzr[i].y)) * rstd;
+          sa[2 * i + 1] = gx0 + gx1;
+          gx[i][0] = gx0;
+          gx[i][1] = gx1;
+        }
+        RSx::row_sums(sa);
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+          const int r = rs.row(i, warp);
+          const float rstd = rsd[i], sa0 = sa[2 * i], sa1 = sa[2 * i + 1];
           rs.all_gather_store(t_q, &bars[BAR_AG], r, lane,
-                              fmaf(gx0, rstd, (sa0 * xh[i].x - sa1 * rstd) * (1.f / 64.f)),      // gZ2in
-                              fmaf(gx1, rstd, (sa0 * xh[i].y - sa1 * rstd) * (1.f / 64.f)));
-          if (lane == 0) p.d_eta[(sid * NC + i0 + j) * 64 + r] = __float2bfloat16(-de);
+                              fmaf(gx[i][0], rstd, (sa0 * xh[i].x - sa1 * rstd) * (1.f / 64.f)),      // gZ2in
+                              fmaf(gx[i][1], rstd, (sa0 * xh[i].y - sa1 * rstd) * (1.f / 64.f)));
+          if (lane == 0) p.d_eta[(sid * NC + i0 + j) * 64 + r] = __float2bfloat16(-(ex[i] + pre[2 * i]));
         }
         *reinterpret_cast<float2*>(sXch + warp * 64 + 2 * lane) = make_float2(ca0, ca1);
         *reinterpret_cast<float2*>(sXch + 512 + warp * 64 + 2 * lane) = make_float2(cv0, cv1);

@@ -502,10 +502,44 @@ struct RowSplit {
       e[2 * lq + 1] = acc.y;
     }
   }
-  static __device__ __forceinline__ float row_sum(float x) {
+  // N independent row sums, step by step: shuffles keep their program order, so that one value after the other would
+  // cost N times the latency of five dependent shuffles.  The row stages below are all latency, hence every reduction
+  // takes all rows (and all sums) of the thread at once (32 streams: backward 15.5 -> 14.9, forward 4.70 -> 4.46 us per
+  // mini-batch).
+  template <int N>
+  static __device__ __forceinline__ void row_sums(float (&x)[N]) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    return x;
+    for (int o = 16; o > 0; o >>= 1) {
+      float y[N];
+#pragma unroll
+      for (int i = 0; i < N; ++i) y[i] = __shfl_xor_sync(0xffffffffu, x[i], o);
+#pragma unroll
+      for (int i = 0; i < N; ++i) x[i] += y[i];
+    }
+  }
+  // LayerNorm of the thread's rows z + b in place, 1/std in rstd
+  static __device__ __forceinline__ void row_layernorm(float (&z)[NR][2], const float2 b, float eps, float (&rstd)[NR]) {
+    float m[NR], v[NR];
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      z[i][0] += b.x;
+      z[i][1] += b.y;
+      m[i] = z[i][0] + z[i][1];
+    }
+    row_sums(m);
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      z[i][0] = fmaf(m[i], -1.f / 64.f, z[i][0]);
+      z[i][1] = fmaf(m[i], -1.f / 64.f, z[i][1]);
+      v[i] = fmaf(z[i][0], z[i][0], z[i][1] * z[i][1]);
+    }
+    row_sums(v);
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      rstd[i] = rsqrtf(v[i] * (1.f / 64.f) + eps);
+      z[i][0] *= rstd[i];
+      z[i][1] *= rstd[i];
+    }
   }
   // the thread's column pair of row r of a swizzled bf16 tile
   static __device__ __forceinline__ float2 ld_pair(const uint8_t* tile, int r, int lane) {

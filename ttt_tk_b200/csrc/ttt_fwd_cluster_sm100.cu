@@ -349,17 +349,12 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     float z[NR][2];
     rs.recv(z, warp, lane, zo_tag);
     __nv_bfloat16* out_tile = p.out + (stream_id * NC + zo_it) * 4096;
+    float rstd[NR];
+    C::RS::row_layernorm(z, b2c, TTT_LN_EPS, rstd);
 #pragma unroll
-    for (int i = 0; i < NR; ++i) {
-      z[i][0] += b2c.x;
-      z[i][1] += b2c.y;
-      const float mu = C::RS::row_sum(z[i][0] + z[i][1]) * (1.f / 64.f);
-      z[i][0] -= mu;
-      z[i][1] -= mu;
-      const float rstd = rsqrtf(C::RS::row_sum(fmaf(z[i][0], z[i][0], z[i][1] * z[i][1])) * (1.f / 64.f) + TTT_LN_EPS);
-      C::RS::st_pair_global(out_tile, rs.row(i, warp), lane, q[i].x + fmaf(gam.x, z[i][0] * rstd, bet.x),
-                            q[i].y + fmaf(gam.y, z[i][1] * rstd, bet.y));
-    }
+    for (int i = 0; i < NR; ++i)
+      C::RS::st_pair_global(out_tile, rs.row(i, warp), lane, q[i].x + fmaf(gam.x, z[i][0], bet.x),
+                            q[i].y + fmaf(gam.y, z[i][1], bet.y));
     zo_it = -1;
   };
 
@@ -447,22 +442,21 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       if (zo_it >= 0) finish_out();
       float z[NR][2];
       rs.recv(z, warp, lane, tag);
+      float rstd[NR], g[NR][2], a[2 * NR];
+      C::RS::row_layernorm(z, b2c, TTT_LN_EPS, rstd);
 #pragma unroll
       for (int i = 0; i < NR; ++i) {
-        z[i][0] += b2c.x;
-        z[i][1] += b2c.y;
-        const float mu = C::RS::row_sum(z[i][0] + z[i][1]) * (1.f / 64.f);
-        z[i][0] -= mu;
-        z[i][1] -= mu;
-        const float rstd = rsqrtf(C::RS::row_sum(fmaf(z[i][0], z[i][0], z[i][1] * z[i][1])) * (1.f / 64.f) + TTT_LN_EPS);
-        const float x0 = z[i][0] * rstd, x1 = z[i][1] * rstd;
-        const float g0 = (fmaf(gam.x, x0, bet.x) - (vv[i].x - kk[i].x)) * gam.x;
-        const float g1 = (fmaf(gam.y, x1, bet.y) - (vv[i].y - kk[i].y)) * gam.y;
-        const float a0 = C::RS::row_sum(g0 + g1);
-        const float a1 = C::RS::row_sum(fmaf(g0, x0, g1 * x1));
-        const float sc = neta[i] * rstd * (1.f / 64.f);
-        rs.all_gather_store(sU2, ag_bar, rs.row(i, warp), lane, (64.f * g0 - a0 - x0 * a1) * sc,
-                            (64.f * g1 - a0 - x1 * a1) * sc);
+        g[i][0] = (fmaf(gam.x, z[i][0], bet.x) - (vv[i].x - kk[i].x)) * gam.x;
+        g[i][1] = (fmaf(gam.y, z[i][1], bet.y) - (vv[i].y - kk[i].y)) * gam.y;
+        a[2 * i] = g[i][0] + g[i][1];
+        a[2 * i + 1] = fmaf(g[i][0], z[i][0], g[i][1] * z[i][1]);
+      }
+      C::RS::row_sums(a);
+#pragma unroll
+      for (int i = 0; i < NR; ++i) {
+        const float sc = neta[i] * rstd[i] * (1.f / 64.f), a0 = a[2 * i], a1 = a[2 * i + 1];
+        rs.all_gather_store(sU2, ag_bar, rs.row(i, warp), lane, (64.f * g[i][0] - a0 - z[i][0] * a1) * sc,
+                            (64.f * g[i][1] - a0 - z[i][1] * a1) * sc);
       }
     }
     mbar_wait_cl(ag_bar, ag_phase, abort_flag, limit, kC);
