@@ -35,6 +35,11 @@
 //   (column sums of gathered tiles); the d_gamma / d_beta addends of the second-order stage are summed per
 //   CTA over its own rows and added up by rank 0, in rank order, at the end.
 //
+// Bound by the chain: at four CTAs per stream the work of a phase is a few hundred cycles beside the latencies of MMA,
+// exchange, row sums and barriers.  Hence the epilogues work on packed fp32 pairs, take column sums from registers, and
+// leave the row sums that only the bias gradients need to the next MMA window.  Measured per mini-batch, 32 streams in
+// groups of 4: 15.5 -> 14.9 us (all rows' sums at once), -> 14.2 us (the rest); two CTAs per stream 22.1 -> 20.5 us.
+//
 // Every wait is bounded; a wait that runs out raises the abort flag of the whole cluster, the vote on
 // leaving a loop is taken CTA-wide at a barrier, and no CTA exits before its peers have reached the
 // exit barrier.
@@ -311,14 +316,9 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   auto part_sum = [&](int k) {
     return (part[k * 256 + tid] + part[k * 256 + 64 + tid]) + (part[k * 256 + 128 + tid] + part[k * 256 + 192 + tid]);
   };
-  // the thread's eight token columns of the bf16 eta vector
-  auto ld_eta_cols = [&](const __nv_bfloat16* e, float (&c)[8]) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const __nv_bfloat162 w = *reinterpret_cast<const __nv_bfloat162*>(e + tm.col(j));
-      c[2 * j] = __bfloat162float(w.x);
-      c[2 * j + 1] = __bfloat162float(w.y);
-    }
+  // -eta of the thread's token column pair q
+  auto neg_eta_col = [&](const __nv_bfloat16* e, int q) {
+    return bf16x2_to_f32x2(*reinterpret_cast<const uint32_t*>(e + tm.col(q)) ^ 0x80008000u);
   };
 
   // ---- state <-> global memory (this CTA's rows): W1-shaped matrices are [64 feat][256 hid], W2-shaped
@@ -525,7 +525,7 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         }
         frag_st_tile(tm, bX2 + b * TILE, g);
         frag_st_tile(tm, bGP + b * TILE, gp);
-        frag_st_tile(tm, bZ1 + b * TILE, z);
+        frag_st_tile_h(tm, bZ1 + b * TILE, z);      // f16: the sweep evaluates gelu' and gelu'' of it in f16
       }
       publish();
       if (tid == kProd) {
@@ -697,39 +697,29 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         if (tid < 64) sB2[tid] += part_sum(0);
         wait_mma();
       }
-      {
-        float et[8];
-        ld_eta_cols(eta, et);
-        float ra[NB], rb[NB];
+      float ra[NB], rb[NB];      // row sums of U1 (for b1): this thread's part, reduced in the next MMA window
 #pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          float r[16], gp[16], u[16];
-          tok_ld(tm, tmem + C::TM_A + b * 64, r);
-          tok_ld_tile(tm, bGP + b * TILE, gp);
-          ra[b] = 0.f; rb[b] = 0.f;
+      for (int b = 0; b < NB; ++b) {
+        TokFrag r;
+        uint32_t gw[8];
+        frag_ld(tm, tmem + C::TM_A + b * 64, r);
+        frag_ld_raw(tm, bGP + b * TILE, gw);
+        f32x2 s0 = 0ull, s1 = 0ull;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int x0 = 4 * q + h, x1 = 4 * q + 2 + h, c = 2 * q + h;
-              // dl/dZ1 rounded to bf16 (the value the scratch slot and the sweep see); U1 = -eta dl/dZ1
-              gp[x0] = __bfloat162float(__float2bfloat16(gp[x0] * r[x0]));
-              gp[x1] = __bfloat162float(__float2bfloat16(gp[x1] * r[x1]));
-              u[x0] = -et[c] * gp[x0];
-              u[x1] = -et[c] * gp[x1];
-              ra[b] += u[x0];
-              rb[b] += u[x1];
-            }
-          }
-          tok_st_tile(tm, bGP + b * TILE, gp);     // dl/dZ1, in place over G'
-          tok_st_tile(tm, bZ1 + b * TILE, u);      // U1, over Z1
+        for (int q = 0; q < 4; ++q) {
+          const f32x2 ne = neg_eta_col(eta, q);
+          // dl/dZ1 rounded to bf16 (the value the scratch slot and the sweep see), in place over G'; U1 = -eta dl/dZ1
+          gw[2 * q] = f32x2_to_bf16x2(mul2(bf16x2_to_f32x2(gw[2 * q]), r.a[q]));
+          gw[2 * q + 1] = f32x2_to_bf16x2(mul2(bf16x2_to_f32x2(gw[2 * q + 1]), r.b[q]));
+          r.a[q] = mul2(bf16x2_to_f32x2(gw[2 * q]), ne);
+          r.b[q] = mul2(bf16x2_to_f32x2(gw[2 * q + 1]), ne);
+          s0 = add2(s0, r.a[q]);
+          s1 = add2(s1, r.b[q]);
         }
-        tok_row_allreduce<NB, 4>(tm, ra, rb, sXch);
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          b1v[b][0] += ra[b];
-          b1v[b][1] += rb[b];
-        }
+        frag_st_raw(tm, bGP + b * TILE, gw);
+        frag_st_tile(tm, bZ1 + b * TILE, r);     // U1, over Z1
+        ra[b] = hsum(s0);
+        rb[b] = hsum(s1);
       }
       publish();
 
@@ -744,6 +734,12 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                  HID_ONE(true, C::TM_S2, bX2, tU2, 1u, 0),
                  if (NB > 1) HID_ONE(true, C::TM_S1, bZ1, sK, 1u, NB - 1),
                  if (NB > 1) HID_ONE(true, C::TM_S2, bX2, tU2, 1u, NB - 1))
+      tok_row_allreduce<NB, 4>(tm, ra, rb, sXch);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        b1v[b][0] += ra[b];
+        b1v[b][1] += rb[b];
+      }
       wait_mma();
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
@@ -907,34 +903,39 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       wait_bar(BAR_T + 0);
       wait_bar(BAR_T + 1);
       {
-        float go[16], xl[16], gam[8];
-        tok_ld_tile(tm, t_go, go);
-        tok_ld_tile(tm, t_a, xl);
-        tok_ld_cols(tm, sGamma, gam);
-        float a[2] = {0.f, 0.f}, bb[2] = {0.f, 0.f};
+        uint32_t gw[8], xw[8];
+        frag_ld_raw(tm, t_go, gw);
+        frag_ld_raw(tm, t_a, xw);
+        TokFrag g;
+        f32x2 a0 = 0ull, a1 = 0ull, c0 = 0ull, c1 = 0ull, sb[4], sg[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h;
-            go[x0] *= gam[2 * q + h];
-            go[x1] *= gam[2 * q + h];
-            a[0] += go[x0]; a[1] = fmaf(go[x0], xl[x0], a[1]);
-            bb[0] += go[x1]; bb[1] = fmaf(go[x1], xl[x1], bb[1]);
-          }
+          const f32x2 gam = frag_col(tm, sGamma, q);
+          const f32x2 go0 = bf16x2_to_f32x2(gw[2 * q]), go1 = bf16x2_to_f32x2(gw[2 * q + 1]);
+          const f32x2 x0 = bf16x2_to_f32x2(xw[2 * q]), x1 = bf16x2_to_f32x2(xw[2 * q + 1]);
+          g.a[q] = mul2(go0, gam);
+          g.b[q] = mul2(go1, gam);
+          a0 = add2(a0, g.a[q]); a1 = fma2(g.a[q], x0, a1);
+          c0 = add2(c0, g.b[q]); c1 = fma2(g.b[q], x1, c1);
+          sb[q] = add2(go0, go1);
+          sg[q] = fma2(go0, x0, mul2(go1, x1));
         }
-        tok_row_allreduce<2, 2>(tm, a, bb, sXch);
-        const float q0 = sSigLn[tm.r0] * (1.f / 64.f), q1 = sSigLn[tm.r1] * (1.f / 64.f);   // 1 / (64 std)
+        // column sums over the tokens (d_beta, d_gamma, G_b2) from the registers: a pass over the tiles beside G1 was
+        // longer than G1
+        const int fc = tm.quad * 64 + frag_colsum_col(tm, lane);
+        part[fc] = frag_colsum(sb, lane);
+        part[256 + fc] = frag_colsum(sg, lane);
+        float a[2] = {hsum(a0), hsum(a1)}, b[2] = {hsum(c0), hsum(c1)};
+        frag_allreduce2<1>(tm, a, b, sXch, 1);
+        const f32x2 q0 = pk1(sSigLn[tm.r0] * (1.f / 64.f)), q1 = pk1(sSigLn[tm.r1] * (1.f / 64.f));   // 1 / (64 std)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h;
-            go[x0] = (64.f * go[x0] - a[0] - xl[x0] * a[1]) * q0;
-            go[x1] = (64.f * go[x1] - bb[0] - xl[x1] * bb[1]) * q1;
-          }
+          g.a[q] = mul2(fma2(bf16x2_to_f32x2(xw[2 * q]), pk1(-a[1]), fma2(g.a[q], pk1(64.f), pk1(-a[0]))), q0);
+          g.b[q] = mul2(fma2(bf16x2_to_f32x2(xw[2 * q + 1]), pk1(-b[1]), fma2(g.b[q], pk1(64.f), pk1(-b[0]))), q1);
+          sb[q] = add2(g.a[q], g.b[q]);
         }
-        tok_st_tile(tm, t_g, go);
+        frag_st_tile(tm, t_g, g);
+        part[512 + fc] = frag_colsum(sb, lane);
       }
       publish();
       // G1: gX2b^T = W2+ gZ2b^T
@@ -942,24 +943,10 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                  if (NB > 1) HID_ONE(false, C::TM_A, big(ib1), t_g, 0u, NB - 1),
                  ,
                  )
-      {
-        // column sums over the tokens: d_beta += sum go, d_gamma += sum go * x_hat_ln, G_b2 += sum gZ2b
-        float a = 0.f, bsum = 0.f;
-#pragma unroll 8
-        for (int r = cs_q * 16; r < cs_q * 16 + 16; ++r) {
-          const float go = ld_elem(t_go, r, cs_f);
-          bsum += go;
-          a = fmaf(go, ld_elem(t_a, r, cs_f), a);
-        }
-        part[tid] = bsum;
-        part[256 + tid] = a;
-        part[512 + tid] = colsum16(t_g);
-        __syncthreads();
-        if (tid < 64) {
-          sDB[tid] += part_sum(0);
-          sDG[tid] += part_sum(1);
-          sGb2[tid] += part_sum(2);
-        }
+      if (tid < 64) {
+        sDB[tid] += part_sum(0);
+        sDG[tid] += part_sum(1);
+        sGb2[tid] += part_sum(2);
       }
       if (dk_row0 >= 0) {     // the previous step's dK
         if constexpr (C::kRowSplit) {
@@ -973,33 +960,24 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       if (tid == kProd) load_big(ib1, p.sc_X2 + slot * BIG);   // W2+ is consumed (G1 was its only use): X2 for G5
       wait_bar(BAR_BIG + ib2);
       // ---- E1: gZ1b^T = gX2b^T * gelu'(Z1b^T), in place over the gelu'(Z1_bar) tile
-      {
-        uint8_t* bz = big(ib2);
-        float ra[NB], rb[NB];
+      float ga[NB], gb[NB];      // row sums (for G_b1): this thread's part, reduced in the next MMA window
 #pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          float v[16], z[16];
-          tok_ld(tm, tmem + C::TM_A + b * 64, v);
-          tok_ld_tile(tm, bz + b * TILE, z);
-          ra[b] = 0.f; rb[b] = 0.f;
+      for (int b = 0; b < NB; ++b) {
+        TokFrag v;
+        uint32_t zw[8];
+        frag_ld(tm, tmem + C::TM_A + b * 64, v);
+        frag_ld_raw(tm, big(ib2) + b * TILE, zw);
+        f32x2 s0 = 0ull, s1 = 0ull;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              z[4 * q + h] *= v[4 * q + h];
-              z[4 * q + 2 + h] *= v[4 * q + 2 + h];
-              ra[b] += z[4 * q + h];
-              rb[b] += z[4 * q + 2 + h];
-            }
-          }
-          tok_st_tile(tm, bz + b * TILE, z);
+        for (int q = 0; q < 4; ++q) {
+          v.a[q] = mul2(bf16x2_to_f32x2(zw[2 * q]), v.a[q]);
+          v.b[q] = mul2(bf16x2_to_f32x2(zw[2 * q + 1]), v.b[q]);
+          s0 = add2(s0, v.a[q]);
+          s1 = add2(s1, v.b[q]);
         }
-        tok_row_allreduce<NB, 4>(tm, ra, rb, sXch);
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          Gb1[b][0] += ra[b];
-          Gb1[b][1] += rb[b];
-        }
+        frag_st_tile(tm, big(ib2) + b * TILE, v);
+        ga[b] = hsum(s0);
+        gb[b] = hsum(s1);
       }
       publish();
       if (tid == kProd) {   // x_hat_ln and its column sums are consumed: bring V into that tile (E4 rebuilds
@@ -1016,6 +994,12 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                  HID_ALL(true, C::TM_S2, big(ib3), t_g, 1u),
                  HID_ONE(true, C::TM_S1, big(ib2), t_q, 1u, 0),
                  if (NB > 1) HID_ONE(true, C::TM_S1, big(ib2), t_q, 1u, NB - 1))
+      tok_row_allreduce<NB, 4>(tm, ga, gb, sXch);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        Gb1[b][0] += ga[b];
+        Gb1[b][1] += gb[b];
+      }
       wait_mma();
       // gZ1b is consumed: Z1 of this step comes in while E2 runs (X2_bar's buffer takes the W2 snapshot)
       if (tid == kProd) load_big(ib2, p.sc_Z1 + slot * BIG);
@@ -1090,38 +1074,29 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         tma_wait_group_read<0>();     // dQ has left the dL/dOut tile (E4 reuses it for dV)
       }
       wait_bar(BAR_BIG + ib2);
-      // ---- E3: A1, P = A1 gelu'(Z1), S = A1 gelu''(Z1), gelu'(Z1)
-      {
-        uint8_t* bz = big(ib2);
-        uint8_t* bp = big(ib4);
-        uint8_t* bgp = big(ib0);
-        float et[8];
-        ld_eta_cols(sEta, et);
+      // ---- E3: A1, P = A1 gelu'(Z1), S = A1 gelu''(Z1), gelu'(Z1) (kept as f16)
 #pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          float v[16], z[16], pp[16], gp[16];
-          tok_ld(tm, tmem + C::TM_A + b * 64, v);
-          tok_ld_tile(tm, bz + b * TILE, z);
+      for (int b = 0; b < NB; ++b) {
+        TokFrag v, sv;
+        uint32_t zw[8], gp[8];
+        frag_ld(tm, tmem + C::TM_A + b * 64, v);
+        frag_ld_raw(tm, big(ib2) + b * TILE, zw);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {       // h = 0: the pair of row r0, h = 1: the pair of row r1
-              const int x = 4 * q + 2 * h;
-              const float gb = Gb1[b][h];
-              const float a10 = -et[2 * q] * (v[x] + gb);
-              const float a11 = -et[2 * q + 1] * (v[x + 1] + gb);
-              float gpp0, gpp1;
-              gelu_grad_pair2(z[x], z[x + 1], gp[x], gp[x + 1], gpp0, gpp1);
-              pp[x] = a10 * gp[x];
-              pp[x + 1] = a11 * gp[x + 1];
-              z[x] = a10 * gpp0;
-              z[x + 1] = a11 * gpp1;
-            }
-          }
-          tok_st_tile(tm, bp + b * TILE, pp);
-          tok_st_tile(tm, bz + b * TILE, z);
-          tok_st_tile(tm, bgp + b * TILE, gp);
+        for (int q = 0; q < 4; ++q) {
+          const f32x2 ne = neg_eta_col(sEta, q);
+          uint32_t gpp;
+          v.a[q] = mul2(ne, add2(v.a[q], pk1(Gb1[b][0])));
+          gelu_grad_h2(zw[2 * q], gp[2 * q], gpp);
+          sv.a[q] = mul2(v.a[q], f16x2_to_f32x2(gpp));
+          v.a[q] = mul2(v.a[q], f16x2_to_f32x2(gp[2 * q]));
+          v.b[q] = mul2(ne, add2(v.b[q], pk1(Gb1[b][1])));
+          gelu_grad_h2(zw[2 * q + 1], gp[2 * q + 1], gpp);
+          sv.b[q] = mul2(v.b[q], f16x2_to_f32x2(gpp));
+          v.b[q] = mul2(v.b[q], f16x2_to_f32x2(gp[2 * q + 1]));
         }
+        frag_st_tile(tm, big(ib4) + b * TILE, v);
+        frag_st_tile(tm, big(ib2) + b * TILE, sv);
+        frag_st_raw(tm, big(ib0) + b * TILE, gp);
       }
       publish();
       wait_bar(BAR_BIG + ib1);
@@ -1398,9 +1373,8 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                  if (NB > 1) HID_ONE(false, C::TM_A, big(ib1), t_gz2, 0u, NB - 1))
       if constexpr (C::kRowSplit && C::kMmaColsum) {
         // the second-order stage's d_gamma / d_beta partials (this CTA's rows only: summed over the cluster at
-        // the end) are read out of the row-sum exchange area before the barrier below; the next epilogue, which
-        // uses that area again, comes after it.  The column sums of the gathered gZ2in tile (G_b2 stays
-        // replicated) come from the tensor pipe after the phase.
+        // the end) are read out of the row-sum exchange area, which is used again after the next epilogue's barrier.  The
+        // column sums of the gathered gZ2in tile (G_b2 stays replicated) come from the tensor pipe after the phase.
         if (tid < 64) {
           float a = 0.f, v = 0.f;
 #pragma unroll
@@ -1411,7 +1385,6 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           sDGp[tid] += a;
           sDGp[64 + tid] += v;
         }
-        __syncthreads();
       } else if constexpr (C::kRowSplit) {
         // the second-order stage's d_gamma / d_beta partials (this CTA's rows only: summed over the cluster at
         // the end) are read out of the row-sum exchange area before the barrier below; the next epilogue, which
@@ -1458,37 +1431,25 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         if (j > 0) issue_tiles_a(j - 1);
       }
       // ---- E5: gZ1in^T = gX2^T gelu'(Z1^T) + R^T S^T, in place over S^T
-      {
-        uint8_t* bs = big(ib2);
-        const uint8_t* bgp = big(ib0);
-        float ra[NB], rb[NB];
 #pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          float v[16], w[16], gp[16], sv[16];
-          tok_ld(tm, tmem + C::TM_B + b * 64, v);
-          tok_ld(tm, tmem + C::TM_A + b * 64, w);
-          tok_ld_tile(tm, bgp + b * TILE, gp);
-          tok_ld_tile(tm, bs + b * TILE, sv);
-          ra[b] = 0.f; rb[b] = 0.f;
+      for (int b = 0; b < NB; ++b) {
+        TokFrag v, w;
+        uint32_t gp[8], sw[8];
+        frag_ld(tm, tmem + C::TM_B + b * 64, v);
+        frag_ld(tm, tmem + C::TM_A + b * 64, w);
+        frag_ld_raw(tm, big(ib0) + b * TILE, gp);
+        frag_ld_raw(tm, big(ib2) + b * TILE, sw);
+        f32x2 s0 = 0ull, s1 = 0ull;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int x0 = 4 * q + h, x1 = 4 * q + 2 + h;
-              sv[x0] = fmaf(v[x0], gp[x0], w[x0] * sv[x0]);
-              sv[x1] = fmaf(v[x1], gp[x1], w[x1] * sv[x1]);
-              ra[b] += sv[x0];
-              rb[b] += sv[x1];
-            }
-          }
-          tok_st_tile(tm, bs + b * TILE, sv);
+        for (int q = 0; q < 4; ++q) {
+          v.a[q] = fma2(v.a[q], f16x2_to_f32x2(gp[2 * q]), mul2(w.a[q], bf16x2_to_f32x2(sw[2 * q])));
+          v.b[q] = fma2(v.b[q], f16x2_to_f32x2(gp[2 * q + 1]), mul2(w.b[q], bf16x2_to_f32x2(sw[2 * q + 1])));
+          s0 = add2(s0, v.a[q]);
+          s1 = add2(s1, v.b[q]);
         }
-        tok_row_allreduce<NB, 0>(tm, ra, rb, sXch);
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          Gb1[b][0] += ra[b];
-          Gb1[b][1] += rb[b];
-        }
+        frag_st_tile(tm, big(ib2) + b * TILE, v);
+        ga[b] = hsum(s0);
+        gb[b] = hsum(s1);
       }
       publish();
       // gelu'(Z1) is consumed: the next step's gelu'(Z1_bar) comes into its buffer
@@ -1500,6 +1461,12 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                  HID_ALL(true, C::TM_S1, big(ib2), t_k, 1u),
                  HID_ONE(true, C::TM_S2, big(ib3), t_q, 1u, 0),
                  if (NB > 1) HID_ONE(true, C::TM_S2, big(ib3), t_q, 1u, NB - 1))
+      tok_row_allreduce<NB, 0>(tm, ga, gb, sXch);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        Gb1[b][0] += ga[b];
+        Gb1[b][1] += gb[b];
+      }
       wait_mma();
       // ---- E6: dK = sum over the cluster of (share of dK + gZ1in W1^T): an output only, summed by
       // reduce-scatter; every CTA stores the token rows it owns.  Sent now, received inside the first MMA

@@ -53,47 +53,14 @@ __device__ __forceinline__ f32x2 gelu_half2(f32x2 y) {
 // operand; one instruction then serves two elements.  The argument is clamped to +-20, beyond which
 // gelu' is 0 or 1 and gelu'' is 0 to fp16 precision (and x^3 would leave the fp16 range); gelu
 // itself stays in fp32: on fp32 arguments the conversions cost what the packed arithmetic saves, so
-// only the derivatives of arguments read from bf16 tiles use this path.
-struct GeluH2 {
-  __half2 x, x2, t, hh;   // clamped argument, its square, tanh(u), 0.5 (1 + tanh(u))
-};
+// only the derivatives of Z1, which the recompute keeps as f16 tiles, use this path.
 __device__ __forceinline__ __half2 h2c(float v) { return __float2half2_rn(v); }
 __device__ __forceinline__ __half2 tanh_h2(__half2 u) {
   uint32_t r;
   asm("tanh.approx.f16x2 %0, %1;" : "=r"(r) : "r"(*reinterpret_cast<const uint32_t*>(&u)));
   return *reinterpret_cast<__half2*>(&r);
 }
-__device__ __forceinline__ GeluH2 gelu_h2_core(float x0, float x1) {
-  GeluH2 c;
-  c.x = __hmax2(__hmin2(__floats2half2_rn(x0, x1), h2c(20.f)), h2c(-20.f));
-  c.x2 = __hmul2(c.x, c.x);
-  const __half2 u = __hmul2(c.x, __hfma2(h2c(kG01), c.x2, h2c(kG0)));
-  c.t = tanh_h2(u);
-  c.hh = __hfma2(h2c(0.5f), c.t, h2c(0.5f));
-  return c;
-}
-// gelu'(x) from the core values: h + (g - g t) q
-__device__ __forceinline__ __half2 gelu_h2_grad(const GeluH2& c, __half2& q) {
-  const __half2 g = __hmul2(c.x, c.hh);
-  q = __hfma2(h2c(kG2), c.x2, h2c(kG0));
-  return __hfma2(__hfma2(__hneg2(g), c.t, g), q, c.hh);
-}
-__device__ __forceinline__ void gelu_grad_pair2(float x0, float x1, float& gp0, float& gp1, float& gpp0,
-                                                float& gpp1) {
-  const GeluH2 c = gelu_h2_core(x0, x1);
-  __half2 q;
-  const float2 gp = __half22float2(gelu_h2_grad(c, q));
-  const __half2 s = __hfma2(__hneg2(c.t), c.t, h2c(1.f));
-  const __half2 cc = __hfma2(h2c(2.f * kG2), c.x2, h2c(kG0));
-  const __half2 xtq = __hmul2(__hmul2(c.x, c.t), q);
-  const float2 gpp = __half22float2(__hmul2(s, __hfma2(__hneg2(xtq), q, cc)));
-  gp0 = gp.x;
-  gp1 = gp.y;
-  gpp0 = gpp.x;
-  gpp1 = gpp.y;
-}
 
-// the same from and to f16 pairs (a value beyond the f16 range has become infinite and is clamped like one beyond 20)
 __device__ __forceinline__ uint32_t f32x2_to_f16x2(f32x2 a) {
   float lo, hi;
   upk(a, lo, hi);
@@ -104,6 +71,7 @@ __device__ __forceinline__ f32x2 f16x2_to_f32x2(uint32_t w) {
   const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
   return pk(f.x, f.y);
 }
+// gelu'(z) and gelu''(z); a value beyond the f16 range has become infinite and is clamped like one beyond 20
 __device__ __forceinline__ void gelu_grad_h2(uint32_t z, uint32_t& gp, uint32_t& gpp) {
   const __half2 x = __hmax2(__hmin2(*reinterpret_cast<const __half2*>(&z), h2c(20.f)), h2c(-20.f));
   const __half2 x2 = __hmul2(x, x);
@@ -125,12 +93,6 @@ __device__ __forceinline__ uint4 pack_chunk(const float* v) {
   w.z = pack_bf16(v[4], v[5]);
   w.w = pack_bf16(v[6], v[7]);
   return w;
-}
-__device__ __forceinline__ void unpack_chunk(const uint4 w, float* v) {
-  v[0] = bf16_lo(w.x); v[1] = bf16_hi(w.x);
-  v[2] = bf16_lo(w.y); v[3] = bf16_hi(w.y);
-  v[4] = bf16_lo(w.z); v[5] = bf16_hi(w.z);
-  v[6] = bf16_lo(w.w); v[7] = bf16_hi(w.w);
 }
 // 8 consecutive elements (16-byte chunk `chunk`) of row `row` of a swizzled tile
 __device__ __forceinline__ void st_chunk(uint8_t* tile, uint32_t row, uint32_t chunk, const float* v) {
@@ -558,6 +520,21 @@ __device__ __forceinline__ void frag_st_tile(const TokMap& m, uint8_t* tile, con
   for (int j = 0; j < 4; ++j) {
     *reinterpret_cast<uint32_t*>(tile + m.off(m.r0, j)) = f32x2_to_bf16x2(f.a[j]);
     *reinterpret_cast<uint32_t*>(tile + m.off(m.r1, j)) = f32x2_to_bf16x2(f.b[j]);
+  }
+}
+// ... as f16, and raw words as frag_ld_raw gives them
+__device__ __forceinline__ void frag_st_tile_h(const TokMap& m, uint8_t* tile, const TokFrag& f) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    *reinterpret_cast<uint32_t*>(tile + m.off(m.r0, j)) = f32x2_to_f16x2(f.a[j]);
+    *reinterpret_cast<uint32_t*>(tile + m.off(m.r1, j)) = f32x2_to_f16x2(f.b[j]);
+  }
+}
+__device__ __forceinline__ void frag_st_raw(const TokMap& m, uint8_t* tile, const uint32_t (&w)[8]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    *reinterpret_cast<uint32_t*>(tile + m.off(m.r0, j)) = w[2 * j];
+    *reinterpret_cast<uint32_t*>(tile + m.off(m.r1, j)) = w[2 * j + 1];
   }
 }
 // ... straight to a row-major [64][64] bf16 tile in global memory
