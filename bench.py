@@ -258,7 +258,7 @@ def run_ours(args, rank, world, local_rank):
     cl_used = cluster or lib.ttt_b200_pick_cluster(Bl * Hl, 1)
     cl_fwd = cluster or lib.ttt_b200_pick_cluster(Bl * Hl, 0)
     if not cluster and "TTT_B200_CLUSTER" not in os.environ and cl_fwd == 2:
-        cl_fwd = 1      # the forward's two-group form of one CTA runs there
+        cl_fwd, cl_used = 1, 2      # the launchers' choice where two CTAs per stream fit and four do not
 
     sampler = ClockSampler(local_rank)
     # warm-up happens inside timed_steps; the sampler is started just before so that most of its samples

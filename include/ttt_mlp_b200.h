@@ -285,8 +285,8 @@ int ttt_b200_version(void);
  * (batch, head) stream of a problem with `streams` = B*H streams on the current device when the flags leave
  * the choice to it: four when the device runs that many clusters of four at once
  * (ttt_b200_cluster_capacity), else (forward only) two when those fit, else one (measured thresholds).
- * Where it answers two, ttt_b200_forward runs one CTA per stream all the same, with its output pass on a second group
- * of warps, which is faster; two CTAs run when the flags or the environment ask for them.
+ * Between the two capacities the operators refine that answer when neither the flags nor the environment name a size:
+ * the forward runs one CTA per stream with its output pass on a second group of warps, the backward two CTAs.
  * TTT_B200_CLUSTER overrides.  The reference fixes the split at compile time
  * (kernels/ttt/ttt.cu:11-12, kernels/ttt_backward/ttt.cu:12-16).  Returns -1 on error. */
 int ttt_b200_pick_cluster(int streams, int backward);

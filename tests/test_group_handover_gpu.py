@@ -4,6 +4,7 @@ the first mini-batches, where a group still waits for nothing, checkpoints after
 many checkpoint groups, and stream counts on both sides of the number of SMs."""
 import pytest
 
+import test_backward_gpu as bwd
 import test_forward_gpu as mlp
 import test_linear_backward_gpu as lbwd
 import test_linear_forward_gpu as lfwd
@@ -32,3 +33,12 @@ def test_linear_backward_group_edges(NC, cgs):
     d = lbwd.make(1, 3, NC, seed=NC)
     _, ref = lbwd.oracle(d, cgs)
     lbwd.check(lbwd.run(d, cgs), ref)
+
+
+@pytest.mark.parametrize("H,NC,cgs", [(34, 3, 2), (74, 1, 1), (75, 3, 2)])
+def test_mlp_backward_between_the_cluster_sizes(H, NC, cgs):
+    """The stream counts at which the backward turns from four CTAs per stream to two and from two to one."""
+    d = orc.make_inputs(1, H, NC, seed=H, backward=True)
+    ck = orc.ttt_forward(d["XQ"], d["XK"], d["XV"], d["last_eta"], d["ttt_norm_weight"], d["ttt_norm_bias"],
+                         d["W1"], d["b1"], d["W2"], d["b2"], cgs)
+    bwd.check(bwd.run_backward(d, ck, cgs), bwd.oracle_backward(d, ck, cgs))

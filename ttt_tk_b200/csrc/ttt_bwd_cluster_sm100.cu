@@ -38,7 +38,7 @@
 // Bound by the chain: at four CTAs per stream the work of a phase is a few hundred cycles beside the latencies of MMA,
 // exchange, row sums and barriers.  Hence the epilogues work on packed fp32 pairs, take column sums from registers, and
 // leave the row sums that only the bias gradients need to the next MMA window.  Measured per mini-batch, 32 streams in
-// groups of 4: 15.5 -> 14.9 us (all rows' sums at once), -> 14.2 us (the rest); two CTAs per stream 22.1 -> 20.5 us.
+// groups of 4: 15.5 -> 14.9 us (all rows' sums at once), -> 14.2 us (the rest); two CTAs per stream 22.1 -> 19.9 us.
 //
 // Every wait is bounded; a wait that runs out raises the abort flag of the whole cluster, the vote on
 // leaving a loop is taken CTA-wide at a barrier, and no CTA exits before its peers have reached the
@@ -306,13 +306,6 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 
   const long tok_rows0 = sid * NC * 64;
 
-  const int cs_q = tid >> 6, cs_f = tid & 63;
-  auto colsum16 = [&](const uint8_t* t) {
-    float acc = 0.f;
-#pragma unroll 8
-    for (int r = cs_q * 16; r < cs_q * 16 + 16; ++r) acc += ld_elem(t, r, cs_f);
-    return acc;
-  };
   auto part_sum = [&](int k) {
     return (part[k * 256 + tid] + part[k * 256 + 64 + tid]) + (part[k * 256 + 128 + tid] + part[k * 256 + 192 + tid]);
   };
@@ -445,21 +438,16 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     uint8_t* tXln = tile(7);  // x_hat_ln on its way to the scratch slot
     auto finish_xhln = [&]() {
       csum.allreduce_recv(zb, tid, zb_tag);
-      float b2c[8];
-      tok_ld_cols(tm, sB2, b2c);
+      TokFrag x;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        zb[4 * q] += b2c[2 * q]; zb[4 * q + 1] += b2c[2 * q + 1];
-        zb[4 * q + 2] += b2c[2 * q]; zb[4 * q + 3] += b2c[2 * q + 1];
+        const f32x2 b = frag_col(tm, sB2, q);
+        x.a[q] = add2(pk(zb[4 * q], zb[4 * q + 1]), b);
+        x.b[q] = add2(pk(zb[4 * q + 2], zb[4 * q + 3]), b);
       }
       float rs0, rs1;
-      tok_layernorm(tm, zb, TTT_LN_EPS, sXch, rs0, rs1);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        zb[4 * q] *= rs0; zb[4 * q + 1] *= rs0;
-        zb[4 * q + 2] *= rs1; zb[4 * q + 3] *= rs1;
-      }
-      tok_st_tile(tm, tXln, zb);
+      frag_layernorm(tm, x, TTT_LN_EPS, sXch, 1, rs0, rs1);
+      frag_st_tile(tm, tXln, x);
       if (row_writer) {
         p.sc_sigln[zb_slot * 64 + tm.r0] = rs0;
         p.sc_sigln[zb_slot * 64 + tm.r1] = rs1;
@@ -598,61 +586,51 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         wait_bar(BAR_AG);
         if (xrow_slot >= 0) wait_bar(BAR_AG2);
       } else {
-        float xh[16], b2c[8], gam[8], bet[8];
-        tok_ld(tm, tmem + C::TM_B, xh);
-        cluster_sum(xh);
-        tok_ld_cols(tm, sB2, b2c);
-        tok_ld_cols(tm, sGamma, gam);
-        tok_ld_cols(tm, sBeta, bet);
+        float zs[16];
+        uint32_t kk[8], vv[8];
+        tok_ld(tm, tmem + C::TM_B, zs);
+        frag_ld_raw(tm, sK, kk);
+        frag_ld_raw(tm, sV, vv);
+        cluster_sum(zs);
+        TokFrag x, g;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          xh[4 * q] += b2c[2 * q]; xh[4 * q + 1] += b2c[2 * q + 1];
-          xh[4 * q + 2] += b2c[2 * q]; xh[4 * q + 3] += b2c[2 * q + 1];
+          const f32x2 b = frag_col(tm, sB2, q);
+          x.a[q] = add2(pk(zs[4 * q], zs[4 * q + 1]), b);
+          x.b[q] = add2(pk(zs[4 * q + 2], zs[4 * q + 3]), b);
         }
         float rs0, rs1;
-        float kk[16], vv[16], g[16], e[16];
-        tok_ld_tile(tm, sK, kk);
-        tok_ld_tile(tm, sV, vv);
-        tok_layernorm(tm, xh, TTT_LN_EPS, sXch, rs0, rs1);
-        float a[2] = {0.f, 0.f}, bb[2] = {0.f, 0.f};
+        frag_layernorm(tm, x, TTT_LN_EPS, sXch, 1, rs0, rs1);
+        f32x2 a0 = 0ull, a1 = 0ull, c0 = 0ull, c1 = 0ull;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h, c = 2 * q + h;
-            xh[x0] *= rs0;
-            xh[x1] *= rs1;
-            e[x0] = fmaf(gam[c], xh[x0], bet[c]) - (vv[x0] - kk[x0]);
-            e[x1] = fmaf(gam[c], xh[x1], bet[c]) - (vv[x1] - kk[x1]);
-            g[x0] = e[x0] * gam[c];
-            g[x1] = e[x1] * gam[c];
-            a[0] += g[x0]; a[1] = fmaf(g[x0], xh[x0], a[1]);
-            bb[0] += g[x1]; bb[1] = fmaf(g[x1], xh[x1], bb[1]);
-          }
+          const f32x2 gam = frag_col(tm, sGamma, q), bet = frag_col(tm, sBeta, q), neg = pk1(-1.f);
+          const f32x2 t0 = fma2(bf16x2_to_f32x2(vv[2 * q]), neg, bf16x2_to_f32x2(kk[2 * q]));          // K - V
+          const f32x2 t1 = fma2(bf16x2_to_f32x2(vv[2 * q + 1]), neg, bf16x2_to_f32x2(kk[2 * q + 1]));
+          g.a[q] = mul2(fma2(gam, x.a[q], add2(t0, bet)), gam);
+          g.b[q] = mul2(fma2(gam, x.b[q], add2(t1, bet)), gam);
+          a0 = add2(a0, g.a[q]); a1 = fma2(g.a[q], x.a[q], a1);
+          c0 = add2(c0, g.b[q]); c1 = fma2(g.b[q], x.b[q], c1);
         }
         // x_hat_fused leaves through the V tile (every thread overwrites exactly the elements it has just
         // read) as a bulk store; grad_output_fused is rebuilt in the sweep from x_hat_fused, K, V
-        tok_st_tile(tm, tV, xh);
-        tok_row_allreduce<2, 2>(tm, a, bb, sXch);
-        const float sc0 = rs0 * (1.f / 64.f), sc1 = rs1 * (1.f / 64.f);
-        const float ne0 = -__bfloat162float(eta[tm.r0]), ne1 = -__bfloat162float(eta[tm.r1]);
+        frag_st_tile(tm, tV, x);
+        float a[2] = {hsum(a0), hsum(a1)}, bb[2] = {hsum(c0), hsum(c1)};
+        frag_allreduce2<1>(tm, a, bb, sXch, 1);
+        const f32x2 sc0 = pk1(rs0 * (1.f / 64.f)), sc1 = pk1(rs1 * (1.f / 64.f));
+        const f32x2 ne0 = pk1(-__bfloat162float(eta[tm.r0])), ne1 = pk1(-__bfloat162float(eta[tm.r1]));
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h;
-            // dl/dZ2, rounded to bf16 once: the update below uses -eta times the rounded value
-            g[x0] = __bfloat162float(__float2bfloat16((64.f * g[x0] - a[0] - xh[x0] * a[1]) * sc0));
-            g[x1] = __bfloat162float(__float2bfloat16((64.f * g[x1] - bb[0] - xh[x1] * bb[1]) * sc1));
-          }
+          // dl/dZ2, rounded to bf16 once: the update below uses -eta times the rounded value
+          kk[2 * q] = f32x2_to_bf16x2(mul2(fma2(x.a[q], pk1(-a[1]), fma2(g.a[q], pk1(64.f), pk1(-a[0]))), sc0));
+          kk[2 * q + 1] = f32x2_to_bf16x2(mul2(fma2(x.b[q], pk1(-bb[1]), fma2(g.b[q], pk1(64.f), pk1(-bb[0]))), sc1));
+          g.a[q] = mul2(bf16x2_to_f32x2(kk[2 * q]), ne0);
+          g.b[q] = mul2(bf16x2_to_f32x2(kk[2 * q + 1]), ne1);
+          x.a[q] = add2(g.a[q], g.b[q]);
         }
-        tok_st_tile(tm, tGZ2, g);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          g[4 * q] *= ne0; g[4 * q + 1] *= ne0;
-          g[4 * q + 2] *= ne1; g[4 * q + 3] *= ne1;
-        }
-        tok_st_tile(tm, tU2, g);
+        frag_st_raw(tm, tGZ2, kk);
+        frag_st_tile(tm, tU2, g);
+        part[tm.quad * 64 + frag_colsum_col(tm, lane)] = frag_colsum(x.a, lane);
         if (row_writer) {
           p.sc_sigf[slot * 64 + tm.r0] = rs0;     // the slot keeps 1/std: the sweep only ever divides by std
           p.sc_sigf[slot * 64 + tm.r1] = rs1;
@@ -692,8 +670,6 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                    if (NB > 1) HID_ONE(false, C::TM_A, bW2, tGZ2, 0u, NB - 1),
                    ,
                    )
-        part[tid] = colsum16(tU2);
-        __syncthreads();
         if (tid < 64) sB2[tid] += part_sum(0);
         wait_mma();
       }
@@ -1235,124 +1211,149 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         *reinterpret_cast<float2*>(sXch + 512 + warp * 64 + 2 * lane) = make_float2(cv0, cv1);
         wait_bar(BAR_AG);
       } else {
-        float A2[16], gz[16], xh[16], go[16];
-        float gam[8];
-        tok_ld_cols(tm, sGamma, gam);
+        TokFrag A2, t1, go;
+        uint32_t gzw[8], xhw[8], kw[8], vw[8];
+        frag_ld_raw(tm, t_gz2, gzw);
+        frag_ld_raw(tm, t_xf, xhw);
+        frag_ld_raw(tm, t_k, kw);
+        frag_ld_raw(tm, t_a, vw);
         const float eta0 = __bfloat162float(sEta[tm.r0]), eta1 = __bfloat162float(sEta[tm.r1]);
         const float rs0 = sSigF[tm.r0], rs1 = sSigF[tm.r1];      // 1 / std
-        tok_ld_tile(tm, t_gz2, gz);
-        tok_ld_tile(tm, t_xf, xh);
-        tok_ld_tile(tm, t_a, go);
-        float ra[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, rb[5] = {0.f, 0.f, 0.f, 0.f, 0.f};   // d_eta terms, (unused), sum A2, sum A2 xh, sum gxf xh
+        float de0, de1;
         {
-          float kk[16], gb2[8], bet[8];
-          tok_ld_tile(tm, t_k, kk);
-          {
-            // this CTA's shares: X2 G_W2 (acc1), P W2 (acc2), gZ1 G_W1 (t1).  Everything the step needs
-            // from them is linear: A2 = -eta acc1 + acc2, the d_eta row sums of gz acc1 and of t1 K, and
-            // -eta t1 inside dK; one cluster sum carries the first three, the dK sum the last.
-            float acc1[16], acc2[16], t1[16];
-            tok_ld3(tm, tmem + C::TM_B + 64, acc1, tmem + C::TM_A, acc2, tmem + C::TM_B, t1);
-            float de0 = 0.f, de1 = 0.f;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const int x0 = 4 * q + h, x1 = 4 * q + 2 + h;
-                A2[x0] = fmaf(-eta0, acc1[x0], acc2[x0]);
-                A2[x1] = fmaf(-eta1, acc1[x1], acc2[x1]);
-                de0 = fmaf(gz[x0], acc1[x0], fmaf(t1[x0], kk[x0], de0));
-                de1 = fmaf(gz[x1], acc1[x1], fmaf(t1[x1], kk[x1], de1));
-                kp[x0] = -eta0 * t1[x0];
-                kp[x1] = -eta1 * t1[x1];
-              }
-            }
-            if (row_writer) {     // the partial sums over this CTA's hidden units of gZ1 * G_b1, once per row
-#pragma unroll
-              for (int w = 0; w < 8; ++w) {
-                de0 += sPart[w * 64 + tm.r0];
-                de1 += sPart[w * 64 + tm.r1];
-              }
-            }
-            csum.run_with_extras(A2, de0, de1, tid, lane);
-            ra[0] = de0;
-            rb[0] = de1;
-          }
-          tok_ld_cols(tm, sGb2, gb2);
-          tok_ld_cols(tm, sBeta, bet);
+          // this CTA's shares: X2 G_W2 (acc1), P W2 (acc2), gZ1 G_W1 (t1).  Everything the step needs
+          // from them is linear: A2 = -eta acc1 + acc2, the d_eta row sums of gz acc1 and of t1 K, and
+          // -eta t1 inside dK; one cluster sum carries the first three, the dK sum the last.
+          TokFrag acc1;
+          frag_ld(tm, tmem + C::TM_B + 64, acc1);
+          frag_ld(tm, tmem + C::TM_A, A2);
+          frag_ld(tm, tmem + C::TM_B, t1);
+          f32x2 s0 = 0ull, s1 = 0ull;
+          float sum[16];
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
+            s0 = fma2(bf16x2_to_f32x2(gzw[2 * q]), acc1.a[q], fma2(t1.a[q], bf16x2_to_f32x2(kw[2 * q]), s0));
+            s1 = fma2(bf16x2_to_f32x2(gzw[2 * q + 1]), acc1.b[q], fma2(t1.b[q], bf16x2_to_f32x2(kw[2 * q + 1]), s1));
+            upk(fma2(acc1.a[q], pk1(-eta0), A2.a[q]), sum[4 * q], sum[4 * q + 1]);
+            upk(fma2(acc1.b[q], pk1(-eta1), A2.b[q]), sum[4 * q + 2], sum[4 * q + 3]);
+          }
+          de0 = hsum(s0);
+          de1 = hsum(s1);
+          if (row_writer) {     // the partial sums over this CTA's hidden units of gZ1 * G_b1, once per row
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int x0 = 4 * q + h, x1 = 4 * q + 2 + h, c = 2 * q + h;
-              // go[] arrives holding V: grad_output_fused = gamma x_hat_fused + beta - (V - K)
-              go[x0] = fmaf(gam[c], xh[x0], bet[c]) - (go[x0] - kk[x0]);
-              go[x1] = fmaf(gam[c], xh[x1], bet[c]) - (go[x1] - kk[x1]);
-              // the G_b2 parts of u = acc1 + G_b2
-              ra[0] = fmaf(gz[x0], gb2[c], ra[0]);
-              rb[0] = fmaf(gz[x1], gb2[c], rb[0]);
-              A2[x0] = fmaf(-eta0, gb2[c], A2[x0]);
-              A2[x1] = fmaf(-eta1, gb2[c], A2[x1]);
-              ra[2] += A2[x0];
-              rb[2] += A2[x1];
-              ra[3] = fmaf(A2[x0], xh[x0], ra[3]);
-              rb[3] = fmaf(A2[x1], xh[x1], rb[3]);
-              ra[4] = fmaf(go[x0] * gam[c], xh[x0], ra[4]);
-              rb[4] = fmaf(go[x1] * gam[c], xh[x1], rb[4]);
+            for (int w = 0; w < 8; ++w) {
+              de0 += sPart[w * 64 + tm.r0];
+              de1 += sPart[w * 64 + tm.r1];
             }
           }
-        }
-        tok_row_allreduce<5, 0>(tm, ra, rb, sXch);
-        float sa[2] = {0.f, 0.f}, sb[2] = {0.f, 0.f};      // sum g_std, sum g_xhat
-        float dga[16], dv[16];
+          csum.run_with_extras(sum, de0, de1, tid, lane);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int c = 2 * q + h;
-            const float gm = gam[c];
-            {
-              const int x = 4 * q + h;
-              const float bt = (A2[x] - (ra[2] + xh[x] * ra[3]) * (1.f / 64.f)) * rs0;
-              const float gly = gm * bt;
-              dga[x] = fmaf(go[x], bt, gly * xh[x]);
-              dv[x] = -gly;
-              if (kp_owner) kp[x] += gly;         // added once across the cluster: by the CTA that owns the row
-              const float gxh = fmaf(gly, gm, -(go[x] * gm * ra[3] + A2[x] * ra[4]) * rs0 * (1.f / 64.f));
-              sa[0] += (-gxh * xh[x] - A2[x] * gz[x]) * rs0;
-              sa[1] += gxh;
-              A2[x] = gxh;
-            }
-            {
-              const int x = 4 * q + 2 + h;
-              const float bt = (A2[x] - (rb[2] + xh[x] * rb[3]) * (1.f / 64.f)) * rs1;
-              const float gly = gm * bt;
-              dga[x] = fmaf(go[x], bt, gly * xh[x]);
-              dv[x] = -gly;
-              if (kp_owner) kp[x] += gly;
-              const float gxh = fmaf(gly, gm, -(go[x] * gm * rb[3] + A2[x] * rb[4]) * rs1 * (1.f / 64.f));
-              sb[0] += (-gxh * xh[x] - A2[x] * gz[x]) * rs1;
-              sb[1] += gxh;
-              A2[x] = gxh;
-            }
+          for (int q = 0; q < 4; ++q) {
+            A2.a[q] = pk(sum[4 * q], sum[4 * q + 1]);
+            A2.b[q] = pk(sum[4 * q + 2], sum[4 * q + 3]);
           }
         }
-        tok_st_tile(tm, t_a, dga);       // d_gamma addends, over V
-        tok_st_tile(tm, t_go, dv);       // dV: stored by TMA, and column-summed for d_beta
-        tok_row_allreduce<2, 5>(tm, sa, sb, sXch);
+        float ra[4], rb[4];       // d_eta's row terms, sum A2, sum A2 xh, sum gxf xh
+        {
+          f32x2 s0[4] = {0ull, 0ull, 0ull, 0ull}, s1[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int x0 = 4 * q + h, x1 = 4 * q + 2 + h;
-            A2[x0] = fmaf(A2[x0], rs0, (sa[0] * xh[x0] - sa[1] * rs0) * (1.f / 64.f));   // gZ2in
-            A2[x1] = fmaf(A2[x1], rs1, (sb[0] * xh[x1] - sb[1] * rs1) * (1.f / 64.f));
-            gz[x0] *= -eta0;                                                            // U2 = -eta gZ2
-            gz[x1] *= -eta1;
+          for (int q = 0; q < 4; ++q) {
+            const f32x2 gam = frag_col(tm, sGamma, q), bet = frag_col(tm, sBeta, q), gb2 = frag_col(tm, sGb2, q), neg = pk1(-1.f);
+            const f32x2 x0 = bf16x2_to_f32x2(xhw[2 * q]), x1 = bf16x2_to_f32x2(xhw[2 * q + 1]);
+            // grad_output_fused = gamma x_hat_fused + beta - (V - K)
+            go.a[q] = add2(fma2(bf16x2_to_f32x2(vw[2 * q]), neg, bf16x2_to_f32x2(kw[2 * q])), fma2(gam, x0, bet));
+            go.b[q] = add2(fma2(bf16x2_to_f32x2(vw[2 * q + 1]), neg, bf16x2_to_f32x2(kw[2 * q + 1])), fma2(gam, x1, bet));
+            // the G_b2 parts of u = acc1 + G_b2
+            s0[0] = fma2(bf16x2_to_f32x2(gzw[2 * q]), gb2, s0[0]);
+            s1[0] = fma2(bf16x2_to_f32x2(gzw[2 * q + 1]), gb2, s1[0]);
+            A2.a[q] = fma2(gb2, pk1(-eta0), A2.a[q]);
+            A2.b[q] = fma2(gb2, pk1(-eta1), A2.b[q]);
+            s0[1] = add2(s0[1], A2.a[q]);
+            s1[1] = add2(s1[1], A2.b[q]);
+            s0[2] = fma2(A2.a[q], x0, s0[2]);
+            s1[2] = fma2(A2.b[q], x1, s1[2]);
+            s0[3] = fma2(mul2(go.a[q], gam), x0, s0[3]);
+            s1[3] = fma2(mul2(go.b[q], gam), x1, s1[3]);
           }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) { ra[i] = hsum(s0[i]); rb[i] = hsum(s1[i]); }
+          ra[0] += de0;
+          rb[0] += de1;
         }
-        tok_st_tile(tm, t_q, A2);
-        tok_st_tile(tm, t_g, gz);
+        // all-reduce over the row's four lanes and two warps
+#pragma unroll
+        for (int sft = 1; sft <= 2; sft <<= 1)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            ra[i] += __shfl_xor_sync(0xffffffffu, ra[i], sft);
+            rb[i] += __shfl_xor_sync(0xffffffffu, rb[i], sft);
+          }
+        float4* x4 = reinterpret_cast<float4*>(sXch);      // 2 KB; the second exchange follows behind
+        if (tm.l3 == 0) {
+          x4[tm.colhalf * 64 + tm.r0] = make_float4(ra[0], ra[1], ra[2], ra[3]);
+          x4[tm.colhalf * 64 + tm.r1] = make_float4(rb[0], rb[1], rb[2], rb[3]);
+        }
+        named_bar_sync(1 + tm.quad, 64);
+        {
+          const float4 o0 = x4[(tm.colhalf ^ 1) * 64 + tm.r0], o1 = x4[(tm.colhalf ^ 1) * 64 + tm.r1];
+          ra[0] += o0.x; ra[1] += o0.y; ra[2] += o0.z; ra[3] += o0.w;
+          rb[0] += o1.x; rb[1] += o1.y; rb[2] += o1.z; rb[3] += o1.w;
+        }
+        const int fc = tm.quad * 64 + frag_colsum_col(tm, lane);
+        f32x2 sa0 = 0ull, sa1 = 0ull, sb0 = 0ull, sb1 = 0ull;      // sum g_std, sum g_xhat of the two rows
+        f32x2 cs[4];
+        {
+          const f32x2 n64 = pk1(-1.f / 64.f);
+          const f32x2 mA = mul2(pk1(ra[1]), n64), xA = mul2(pk1(ra[2]), n64), mB = mul2(pk1(rb[1]), n64), xB = mul2(pk1(rb[2]), n64);
+          const f32x2 fA3 = pk1(-ra[2] * rs0 * (1.f / 64.f)), fA4 = pk1(-ra[3] * rs0 * (1.f / 64.f));
+          const f32x2 fB3 = pk1(-rb[2] * rs1 * (1.f / 64.f)), fB4 = pk1(-rb[3] * rs1 * (1.f / 64.f));
+          const f32x2 own = pk1(kp_owner ? 1.f : 0.f);     // gly enters dK once across the cluster: by the row's owner
+          f32x2 cl[4];
+          TokFrag dv;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const f32x2 gm = frag_col(tm, sGamma, q), neg = pk1(-1.f);
+            const f32x2 x0 = bf16x2_to_f32x2(xhw[2 * q]), x1 = bf16x2_to_f32x2(xhw[2 * q + 1]);
+            const f32x2 bt0 = mul2(add2(A2.a[q], fma2(x0, xA, mA)), pk1(rs0));
+            const f32x2 bt1 = mul2(add2(A2.b[q], fma2(x1, xB, mB)), pk1(rs1));
+            const f32x2 gl0 = mul2(gm, bt0), gl1 = mul2(gm, bt1);
+            cs[q] = add2(fma2(go.a[q], bt0, mul2(gl0, x0)), fma2(go.b[q], bt1, mul2(gl1, x1)));
+            cl[q] = add2(gl0, gl1);
+            dv.a[q] = mul2(gl0, neg);
+            dv.b[q] = mul2(gl1, neg);
+            upk(fma2(t1.a[q], pk1(-eta0), mul2(gl0, own)), kp[4 * q], kp[4 * q + 1]);
+            upk(fma2(t1.b[q], pk1(-eta1), mul2(gl1, own)), kp[4 * q + 2], kp[4 * q + 3]);
+            const f32x2 gx0 = fma2(gl0, gm, fma2(mul2(go.a[q], gm), fA3, mul2(A2.a[q], fA4)));
+            const f32x2 gx1 = fma2(gl1, gm, fma2(mul2(go.b[q], gm), fB3, mul2(A2.b[q], fB4)));
+            sa0 = fma2(gx0, x0, fma2(A2.a[q], bf16x2_to_f32x2(gzw[2 * q]), sa0));
+            sb0 = fma2(gx1, x1, fma2(A2.b[q], bf16x2_to_f32x2(gzw[2 * q + 1]), sb0));
+            sa1 = add2(sa1, gx0);
+            sb1 = add2(sb1, gx1);
+            A2.a[q] = gx0;
+            A2.b[q] = gx1;
+          }
+          frag_st_tile(tm, t_go, dv);      // dV: stored by TMA
+          part[256 + fc] = frag_colsum(cs, lane);
+          part[512 + fc] = frag_colsum(cl, lane);
+        }
+        float sa[2] = {-hsum(sa0) * rs0, hsum(sa1)}, sb[2] = {-hsum(sb0) * rs1, hsum(sb1)};
+        frag_allreduce2<0>(tm, sa, sb, sXch + 512, 1);
+        {
+          const f32x2 k0 = pk1(sa[0] * (1.f / 64.f)), l0 = pk1(-sa[1] * rs0 * (1.f / 64.f));
+          const f32x2 k1 = pk1(sb[0] * (1.f / 64.f)), l1 = pk1(-sb[1] * rs1 * (1.f / 64.f));
+          TokFrag u2;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            A2.a[q] = fma2(A2.a[q], pk1(rs0), fma2(bf16x2_to_f32x2(xhw[2 * q]), k0, l0));      // gZ2in
+            A2.b[q] = fma2(A2.b[q], pk1(rs1), fma2(bf16x2_to_f32x2(xhw[2 * q + 1]), k1, l1));
+            cs[q] = add2(A2.a[q], A2.b[q]);
+            u2.a[q] = mul2(bf16x2_to_f32x2(gzw[2 * q]), pk1(-eta0));                           // U2 = -eta gZ2
+            u2.b[q] = mul2(bf16x2_to_f32x2(gzw[2 * q + 1]), pk1(-eta1));
+          }
+          frag_st_tile(tm, t_q, A2);
+          frag_st_tile(tm, t_g, u2);
+          part[fc] = frag_colsum(cs, lane);
+        }
         if (row_writer && rank == 0) {
           p.d_eta[(sid * NC + i0 + j) * 64 + tm.r0] = __float2bfloat16(-ra[0]);
           p.d_eta[(sid * NC + i0 + j) * 64 + tm.r1] = __float2bfloat16(-rb[0]);
@@ -1371,7 +1372,7 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                  else if (C::kMmaColsum) mma_colsum(tmem + C::TM_CS + 8, smem_u32(t_q), smem_u32(smem + C::OFF_ONES), lead),
                  HID_ONE(false, C::TM_A, big(ib1), t_gz2, 0u, 0),
                  if (NB > 1) HID_ONE(false, C::TM_A, big(ib1), t_gz2, 0u, NB - 1))
-      if constexpr (C::kRowSplit && C::kMmaColsum) {
+      if constexpr (C::kRowSplit) {
         // the second-order stage's d_gamma / d_beta partials (this CTA's rows only: summed over the cluster at
         // the end) are read out of the row-sum exchange area, which is used again after the next epilogue's barrier.  The
         // column sums of the gathered gZ2in tile (G_b2 stays replicated) come from the tensor pipe after the phase.
@@ -1385,38 +1386,15 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           sDGp[tid] += a;
           sDGp[64 + tid] += v;
         }
-      } else if constexpr (C::kRowSplit) {
-        // the second-order stage's d_gamma / d_beta partials (this CTA's rows only: summed over the cluster at
-        // the end) are read out of the row-sum exchange area before the barrier below; the next epilogue, which
-        // uses that area again, comes after it
-        float a = 0.f, v = 0.f;
-        if (tid < 64) {
-#pragma unroll
-          for (int w = 0; w < 8; ++w) {
-            a += sXch[w * 64 + tid];
-            v += sXch[512 + w * 64 + tid];
-          }
-        }
-        part[tid] = colsum16(t_q);      // the gathered gZ2in tile: G_b2 stays replicated
-        __syncthreads();
-        if (tid < 64) {
-          sGb2[tid] += part_sum(0);
-          sDGp[tid] += a;
-          sDGp[64 + tid] += v;
-        }
       } else {
-        part[tid] = colsum16(t_q);
-        part[256 + tid] = colsum16(t_a);
-        part[512 + tid] = colsum16(t_go);
-        __syncthreads();
         if (tid < 64) {
           sGb2[tid] += part_sum(0);
           sDG[tid] += part_sum(1);
-          sDB[tid] -= part_sum(2);
+          sDB[tid] += part_sum(2);
         }
       }
       wait_mma();
-      if constexpr (C::kRowSplit && C::kMmaColsum) {
+      if constexpr (C::kRowSplit) {
         if (warp < 4) {
           const float cs = colsum_read(tmem + C::TM_CS + 8, warp);
           if (lane < 16) sGb2[16 * warp + lane] += cs;

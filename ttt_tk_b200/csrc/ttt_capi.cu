@@ -67,14 +67,10 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 }  // namespace
 
 // How many CTAs share one stream.  The mini-batches of a stream are strictly sequential, so with fewer
-// streams than SMs the idle SMs can only help by taking a share of every stream's hidden units.  The
-// thresholds are measured (B200, 148 SMs): four CTAs per stream win whenever they all fit on the GPU at
-// once (forward 18 %, backward 17-20 % per mini-batch over one CTA).  Two CTAs per stream beat one
-// plain CTA in the forward (12-17 %), but not the two-group form that the forward launcher runs instead when nobody
-// asked for two (see there).  In the backward they gain 6-11 % up to 32 streams, where four CTAs
-// are the better choice anyway, and nothing beyond 37 streams (more than 74 CTAs: both SMs of a TPC are
-// then busy, and the backward, whose scratch traffic goes through the port the two share, slows down by
-// as much as the split gained), so the backward is never given two.
+// streams than SMs the idle SMs can only help by taking a share of every stream's hidden units.  Four
+// CTAs per stream win whenever they all fit on the GPU at once (32 streams on a B200: forward 4.4 against 4.9 us per
+// mini-batch with one CTA, backward 14.2 against 23.2).  Between that and the streams of which two CTAs each fit, this
+// names the plain choice and the launchers refine it: ttt_launch_cluster below.
 int ttt_pick_cluster(int streams, uint32_t flags, bool backward, int* cluster) {
   int forced = static_cast<int>((flags & TTT_B200_FLAG_CLUSTER_MASK) >> TTT_B200_FLAG_CLUSTER_SHIFT);
   if (forced == 0) {
@@ -91,12 +87,24 @@ int ttt_pick_cluster(int streams, uint32_t flags, bool backward, int* cluster) {
     return TTT_B200_OK;
   }
   // all streams must be resident at once for the sharding to pay: the widest cluster size whose capacity
-  // (clusters the device runs at the same time) covers them.  The backward gains nothing from two CTAs per
-  // stream beyond the stream counts four CTAs cover (measured), so it never picks two.
+  // (clusters the device runs at the same time) covers them
   auto capacity = [&](int c) { return backward ? ttt_backward_cluster_capacity(c) : ttt_forward_cluster_capacity(c); };
   if (streams <= capacity(4)) *cluster = 4;
   else if (!backward && streams <= capacity(2)) *cluster = 2;
   else *cluster = 1;
+  return TTT_B200_OK;
+}
+
+// What a launch runs.  Where two CTAs per stream fit but four do not (34 to 74 streams on a B200) and nobody asked for a
+// size: one CTA in the forward, whose output pass runs beside the chain in two groups of warps (5.0 us per mini-batch
+// against 6.1 with two CTAs), and two in the backward (48 / 60 / 74 streams in groups of 4: 19.9 / 20.8 / 21.5 us per
+// mini-batch against 23.2 / 23.2 / 23.3 with one).
+static int ttt_launch_cluster(int streams, uint32_t flags, bool backward, int* cluster) {
+  if (int rc = ttt_pick_cluster(streams, flags, backward, cluster)) return rc;
+  static const bool env = std::getenv("TTT_B200_CLUSTER") != nullptr;
+  if ((flags & TTT_B200_FLAG_CLUSTER_MASK) || env) return TTT_B200_OK;
+  if (!backward && *cluster == 2) *cluster = 1;
+  else if (backward && *cluster == 1 && streams <= ttt_backward_cluster_capacity(2)) *cluster = 2;
   return TTT_B200_OK;
 }
 
@@ -225,10 +233,7 @@ extern "C" int ttt_b200_forward(const ttt_b200_fwd_args* a, void* stream_) {
   uint32_t* status = nullptr;
   if (int rc = pre_launch(&status)) return rc;
   int cluster = 1;
-  if (int rc = ttt_pick_cluster(a->B * a->H, a->flags, false, &cluster)) return rc;
-  // Where two CTAs per stream would fit but four do not (34 to 74 streams on a B200), the one-CTA kernel is the
-  // faster one since its output pass runs beside the chain: 341 against 420 us for 48 streams of 64 mini-batches.
-  if (cluster == 2 && !(a->flags & TTT_B200_FLAG_CLUSTER_MASK) && !std::getenv("TTT_B200_CLUSTER")) cluster = 1;
+  if (int rc = ttt_launch_cluster(a->B * a->H, a->flags, false, &cluster)) return rc;
   const int drop = (a->flags & TTT_B200_FLAG_TEST_LOST_LOAD) ? (a->NC > 1 ? 1 : 0) : -1;
   if (int rc = cluster == 1 ? ttt_launch_forward(a, stream, status, wait_limit_ns(), drop)
                             : ttt_launch_forward_cluster(a, cluster, stream, status, wait_limit_ns(), drop))
@@ -308,7 +313,7 @@ extern "C" int ttt_b200_backward(const ttt_b200_bwd_args* a, void* stream_) {
   uint32_t* status = nullptr;
   if (int rc = pre_launch(&status)) return rc;
   int cluster = 1;
-  if (int rc = ttt_pick_cluster(a->B * a->H, a->flags, true, &cluster)) return rc;
+  if (int rc = ttt_launch_cluster(a->B * a->H, a->flags, true, &cluster)) return rc;
   // the hook drops the recompute inputs of the last group's second mini-batch (its only one if it has one)
   const int last0 = (a->num_checkpoints - 1) * a->checkpoint_group_size;
   const int drop = (a->flags & TTT_B200_FLAG_TEST_LOST_LOAD) ? (last0 + 1 < a->NC ? last0 + 1 : last0) : -1;
