@@ -100,6 +100,13 @@ static __device__ TTT_WAIT_FN bool mbar_wait_slow(uint64_t* bar, uint32_t parity
   }
 }
 
+// ------------------------------------------------------------------ programmatic dependent launch
+// A forward kernel lets its successor in the stream start as soon as all its own CTAs have (griddep_launch), and waits
+// for its predecessor to have completed before it touches global memory (griddep_wait): its set-up (barriers, tensor
+// memory, descriptors) then runs under the predecessor's tail.  Both do nothing in an ordinary launch.
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ------------------------------------------------------------------ proxies / fences
 // Generic-proxy writes to shared memory -> visible to the async proxy (TMA, tcgen05.mma).
 __device__ __forceinline__ void fence_proxy_async_smem() {

@@ -159,6 +159,52 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     tmem_alloc(tmem_slot, C::TM_COLS);
     tmem_relinquish();
   }
+  cluster_arrive();      // (this thread's part of the set-up is done; waited for below)
+  griddep_launch();
+  griddep_wait();
+  // all of the first mini-batch's loads go out before the barriers below: the inputs, and the state into registers
+  auto issue_loads = [&](int i) {   // thread 0 only
+    if (i == p.drop_load && stream_id == 0) return;
+    const int s = i % kStages;
+    const int row0 = static_cast<int>((stream_id * NC + i) * 64);
+    mbar_expect_tx(&full[s], 3 * TILE + 128);
+    tma_load_2d(smem + C::OFF_K + s * TILE, &tmK, &full[s], 0, row0);
+    tma_load_2d(smem + C::OFF_V + s * TILE, &tmV, &full[s], 0, row0);
+    tma_load_2d(smem + C::OFF_Q + s * TILE, &tmQ, &full[s], 0, row0);
+    bulk_load_1d(smem + C::OFF_ETA + s * 128, p.eta + (stream_id * NC + i) * 64, 128, &full[s]);
+  };
+  int loads_issued = 0;
+  if (tid == kProd) {
+    for (; loads_issued < kStages && loads_issued < NC; ++loads_issued) issue_loads(loads_issued);
+  }
+  // ---- state <-> global memory.  In the fragment of block b a thread holds hidden units
+  // hid0 + 64 b + r0 / r1 (rows) and, for j = 0..3, the feature pair col(j), col(j) + 1.
+  // W1 is [64 feat][256 hid] in global memory, W2 [256 hid][64 feat].
+  auto w1_index = [&](int b, int r, int c) { return c * 256 + hid0 + 64 * b + r; };
+  auto w2_index = [&](int b, int r, int c) { return (hid0 + 64 * b + r) * 64 + c; };
+  float b1v[NB][2];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    b1v[b][0] = p.b1[stream_id * 256 + hid0 + 64 * b + tm.r0];
+    b1v[b][1] = p.b1[stream_id * 256 + hid0 + 64 * b + tm.r1];
+  }
+  float w1i[NB][16], w2i[NB][16];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    const float* W1g = p.W1 + stream_id * (64 * 256);
+    const float* W2g = p.W2 + stream_id * (256 * 64);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = tm.col(j);
+      w1i[b][4 * j] = W1g[w1_index(b, tm.r0, c)];
+      w1i[b][4 * j + 1] = W1g[w1_index(b, tm.r0, c + 1)];
+      w1i[b][4 * j + 2] = W1g[w1_index(b, tm.r1, c)];
+      w1i[b][4 * j + 3] = W1g[w1_index(b, tm.r1, c + 1)];
+      const float2 a = *reinterpret_cast<const float2*>(W2g + w2_index(b, tm.r0, c));
+      const float2 d = *reinterpret_cast<const float2*>(W2g + w2_index(b, tm.r1, c));
+      w2i[b][4 * j] = a.x; w2i[b][4 * j + 1] = a.y; w2i[b][4 * j + 2] = d.x; w2i[b][4 * j + 3] = d.y;
+    }
+  }
   if (tid < 64) {
     sGamma[tid] = p.gamma[head * 64 + tid];
     sBeta[tid] = p.beta[head * 64 + tid];
@@ -169,7 +215,6 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   __syncthreads();
   tc_fence_after_sync();
   // the peers' mbarriers and abort flags are initialised before anything is sent to them
-  cluster_arrive();
   cluster_wait();
   const uint32_t tmem = *tmem_slot;
   const uint32_t lead = elect_one() ? 1u : 0u;      // the lane of an issuing warp whose MMAs are enabled
@@ -191,44 +236,6 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   csum.abort_flag = abort_flag;
   csum.limit = limit;
 
-  auto issue_loads = [&](int i) {   // thread 0 only
-    if (i == p.drop_load && stream_id == 0) return;
-    const int s = i % kStages;
-    const int row0 = static_cast<int>((stream_id * NC + i) * 64);
-    mbar_expect_tx(&full[s], 3 * TILE + 128);
-    tma_load_2d(smem + C::OFF_K + s * TILE, &tmK, &full[s], 0, row0);
-    tma_load_2d(smem + C::OFF_V + s * TILE, &tmV, &full[s], 0, row0);
-    tma_load_2d(smem + C::OFF_Q + s * TILE, &tmQ, &full[s], 0, row0);
-    bulk_load_1d(smem + C::OFF_ETA + s * 128, p.eta + (stream_id * NC + i) * 64, 128, &full[s]);
-  };
-  int loads_issued = 0;
-  if (tid == kProd) {
-    for (; loads_issued < kStages && loads_issued < NC; ++loads_issued) issue_loads(loads_issued);
-  }
-
-  // ---- state <-> global memory.  In the fragment of block b a thread holds hidden units
-  // hid0 + 64 b + r0 / r1 (rows) and, for j = 0..3, the feature pair col(j), col(j) + 1.
-  // W1 is [64 feat][256 hid] in global memory, W2 [256 hid][64 feat].
-  auto w1_index = [&](int b, int r, int c) { return c * 256 + hid0 + 64 * b + r; };
-  auto w2_index = [&](int b, int r, int c) { return (hid0 + 64 * b + r) * 64 + c; };
-  auto load_state_block = [&](const float* W1g, const float* W2g, int b) {
-    float w1[16], w2[16];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = tm.col(j);
-      w1[4 * j] = W1g[w1_index(b, tm.r0, c)];
-      w1[4 * j + 1] = W1g[w1_index(b, tm.r0, c + 1)];
-      w1[4 * j + 2] = W1g[w1_index(b, tm.r1, c)];
-      w1[4 * j + 3] = W1g[w1_index(b, tm.r1, c + 1)];
-      const float2 a = *reinterpret_cast<const float2*>(W2g + w2_index(b, tm.r0, c));
-      const float2 d = *reinterpret_cast<const float2*>(W2g + w2_index(b, tm.r1, c));
-      w2[4 * j] = a.x; w2[4 * j + 1] = a.y; w2[4 * j + 2] = d.x; w2[4 * j + 3] = d.y;
-    }
-    tok_st_tmem(tm, tmem + C::TM_W1 + b * 64, w1);
-    tok_st_tmem(tm, tmem + C::TM_W2 + b * 64, w2);
-    tok_st_tile(tm, sW1 + b * TILE, w1);
-    tok_st_tile(tm, sW2 + b * TILE, w2);
-  };
   auto store_w1_block = [&](float* W1o, int b) {
     float w1[16];
     tok_ld(tm, tmem + C::TM_W1 + b * 64, w1);
@@ -252,12 +259,6 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     }
   };
 
-  float b1v[NB][2];
-#pragma unroll
-  for (int b = 0; b < NB; ++b) {
-    b1v[b][0] = p.b1[stream_id * 256 + hid0 + 64 * b + tm.r0];
-    b1v[b][1] = p.b1[stream_id * 256 + hid0 + 64 * b + tm.r1];
-  }
   // of the 8 threads that hold a row's bias, this one writes it out
   const bool b1_writer = tm.colhalf == 0 && tm.l3 == 0;
   auto store_b1 = [&](float* b1o) {
@@ -270,8 +271,12 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     }
   };
 #pragma unroll
-  for (int b = 0; b < NB; ++b)
-    load_state_block(p.W1 + stream_id * (64 * 256), p.W2 + stream_id * (256 * 64), b);
+  for (int b = 0; b < NB; ++b) {
+    tok_st_tmem(tm, tmem + C::TM_W1 + b * 64, w1i[b]);
+    tok_st_tmem(tm, tmem + C::TM_W2 + b * 64, w2i[b]);
+    tok_st_tile(tm, sW1 + b * TILE, w1i[b]);
+    tok_st_tile(tm, sW2 + b * TILE, w2i[b]);
+  }
   tmem_wait_st();
   fence_proxy_async_smem();
   tc_fence_before_sync();
@@ -721,13 +726,15 @@ int launch_cluster(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtenso
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = C::SMEM_BYTES;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = kC;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   cudaError_t e = cudaLaunchKernelEx(&cfg, ttt_fwd_cluster_kernel<kC>, tmQ, tmK, tmV, tmOut, p);
   if (e != cudaSuccess) return ttt_set_error(TTT_B200_ERR_LAUNCH, cudaGetErrorString(e));
   return TTT_B200_OK;

@@ -198,6 +198,8 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     tmem_alloc(tmem_slot, TM_COLS);
     tmem_relinquish();
   }
+  griddep_launch();
+  griddep_wait();
   if (tid < 64) {
     sGamma[tid] = p.gamma[head * 64 + tid];
     sBeta[tid] = p.beta[head * 64 + tid];
@@ -708,8 +710,7 @@ int ttt_launch_forward(const ttt_b200_fwd_args* a, cudaStream_t stream, uint32_t
     attr_err[dev] = cudaFuncSetAttribute(ttt_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   });
   if (attr_err[dev] != cudaSuccess) return ttt_set_error(TTT_B200_ERR_LAUNCH, cudaGetErrorString(attr_err[dev]));
-  ttt_fwd_kernel<<<dim3(a->B * a->H), dim3(kThreads), SMEM_BYTES, stream>>>(tmQ, tmK, tmV, tmOut, p);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = ttt_launch_overlapped(ttt_fwd_kernel, a->B * a->H, kThreads, SMEM_BYTES, stream, tmQ, tmK, tmV, tmOut, p);
   if (e != cudaSuccess) return ttt_set_error(TTT_B200_ERR_LAUNCH, cudaGetErrorString(e));
   return TTT_B200_OK;
 }

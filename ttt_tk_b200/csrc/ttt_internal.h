@@ -36,3 +36,23 @@ uint64_t ttt_wait_limit_ns();
 
 // Read and clear the device status word of ttt_b200_backward_noalloc (0 = nothing reported).
 uint32_t ttt_noalloc_take_status();
+
+// Launch a forward kernel so that its set-up may run under the tail of its predecessor in the stream (programmatic
+// dependent launch; the kernel itself waits before it touches global memory).  A run of one-mini-batch calls on 12 streams:
+// 12.3 -> 8.9 us per call.
+#ifdef __CUDACC__
+template <typename... P, typename... A>
+cudaError_t ttt_launch_overlapped(void (*kernel)(P...), int grid, int block, uint32_t smem, cudaStream_t stream, const A&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+#endif

@@ -184,6 +184,8 @@ ttt_linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     tmem_alloc(tmem_slot, TM_COLS);
     tmem_relinquish();
   }
+  griddep_launch();
+  griddep_wait();
   if (tid < 64) {
     sGamma[tid] = p.gamma[head * 64 + tid];
     sBeta[tid] = p.beta[head * 64 + tid];
@@ -422,6 +424,8 @@ ttt_linear_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
     tmem_alloc(tmem_slot, TM_COLS);
     tmem_relinquish();
   }
+  griddep_launch();
+  griddep_wait();
   if (tid < 64) {
     sGamma[tid] = p.gamma[head * 64 + tid];
     sBeta[tid] = p.beta[head * 64 + tid];
@@ -660,15 +664,15 @@ int ttt_launch_linear_forward(const ttt_b200_linear_fwd_args* a, cudaStream_t st
   if (attr_err[dev] != cudaSuccess) return ttt_set_error(TTT_B200_ERR_LAUNCH, cudaGetErrorString(attr_err[dev]));
   // no more streams than SMs: one CTA of two groups per stream.  Beyond that two or three plain CTAs share an SM and fill
   // each other's waits (296 streams: 3.5 us per mini-batch of all, against 2 x 1.9 in two turns of the form above).
+  cudaError_t e;
   if (a->B * a->H <= sms[dev]) {
     CUtensorMap tmOut;
     if (int rc = ttt_make_tile_map(&tmOut, a->Out, rows)) return rc;
-    pair::ttt_linear_fwd_pair_kernel<<<dim3(a->B * a->H), dim3(2 * pair::kGroup), pair::SMEM_BYTES, stream>>>(tmQ, tmK, tmV,
-                                                                                                              tmOut, p);
+    e = ttt_launch_overlapped(pair::ttt_linear_fwd_pair_kernel, a->B * a->H, 2 * pair::kGroup, pair::SMEM_BYTES, stream, tmQ,
+                              tmK, tmV, tmOut, p);
   } else {
-    ttt_linear_fwd_kernel<<<dim3(a->B * a->H), dim3(kThreads), SMEM_BYTES, stream>>>(tmQ, tmK, tmV, p);
+    e = ttt_launch_overlapped(ttt_linear_fwd_kernel, a->B * a->H, kThreads, SMEM_BYTES, stream, tmQ, tmK, tmV, p);
   }
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return ttt_set_error(TTT_B200_ERR_LAUNCH, cudaGetErrorString(e));
   return TTT_B200_OK;
 }
