@@ -184,8 +184,6 @@ ttt_linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     tmem_alloc(tmem_slot, TM_COLS);
     tmem_relinquish();
   }
-  griddep_launch();
-  griddep_wait();
   if (tid < 64) {
     sGamma[tid] = p.gamma[head * 64 + tid];
     sBeta[tid] = p.beta[head * 64 + tid];
@@ -671,7 +669,9 @@ int ttt_launch_linear_forward(const ttt_b200_linear_fwd_args* a, cudaStream_t st
     e = ttt_launch_overlapped(pair::ttt_linear_fwd_pair_kernel, a->B * a->H, 2 * pair::kGroup, pair::SMEM_BYTES, stream, tmQ,
                               tmK, tmV, tmOut, p);
   } else {
-    e = ttt_launch_overlapped(ttt_linear_fwd_kernel, a->B * a->H, kThreads, SMEM_BYTES, stream, tmQ, tmK, tmV, p);
+    // not overlapped: CTAs placed while the predecessor's still fill most slots would crowd on the SMs that are free first
+    ttt_linear_fwd_kernel<<<dim3(a->B * a->H), dim3(kThreads), SMEM_BYTES, stream>>>(tmQ, tmK, tmV, p);
+    e = cudaGetLastError();
   }
   if (e != cudaSuccess) return ttt_set_error(TTT_B200_ERR_LAUNCH, cudaGetErrorString(e));
   return TTT_B200_OK;
