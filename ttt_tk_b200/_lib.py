@@ -5,6 +5,8 @@ There is no fallback: if the library is missing the import fails.
 import ctypes
 import os
 
+import torch
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "lib", "libttt_mlp_b200.so")
 
@@ -128,3 +130,18 @@ def lib():
     if _LIB is None:
         _LIB = load()
     return _LIB
+
+
+def call_on(device, name, *args):
+    """Call a C entry point whose last argument is the stream: the current one of `device`, with that device current.
+    Asks torch for the raw handle, and changes the device only if it is another one: the layer's seven such calls spent
+    more time in the stream and device objects of torch.cuda than in the calls."""
+    fn = getattr(lib(), name)
+    stream = ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(device.index))
+    if device.index == torch._C._cuda_getDevice():
+        rc = fn(*args, stream)
+    else:
+        with torch.cuda.device(device):
+            rc = fn(*args, stream)
+    if rc != 0:
+        raise RuntimeError(f"{name} failed ({rc}): {lib().ttt_b200_last_error().decode()}")

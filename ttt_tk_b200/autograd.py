@@ -17,7 +17,7 @@ _scratch_cache = {}
 
 
 def _scratch(B, H, NC, cgs, device):
-    key = (B, H, cgs, str(device), torch.cuda.current_stream(device).cuda_stream)
+    key = (B, H, cgs, device.index, torch._C._cuda_getCurrentRawStream(device.index))
     if key not in _scratch_cache:
         _scratch_cache[key] = alloc_backward_buffers(B, H, 1, cgs, device)[0]
     return _scratch_cache[key]
@@ -92,7 +92,7 @@ _linear_scratch_cache = {}
 
 def _linear_scratch(B, H, cgs, device):
     from .ops import linear_backward_scratch_bytes
-    key = (B, H, cgs, str(device), torch.cuda.current_stream(device).cuda_stream)
+    key = (B, H, cgs, device.index, torch._C._cuda_getCurrentRawStream(device.index))
     if key not in _linear_scratch_cache:
         _linear_scratch_cache[key] = torch.empty(linear_backward_scratch_bytes(B, H, cgs), dtype=torch.uint8,
                                                  device=device)

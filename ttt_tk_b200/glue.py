@@ -15,21 +15,9 @@ import torch
 from . import _lib
 
 
-def _stream(dev):
-    return ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-
-
 def _need(cond, msg):
     if not cond:
         raise ValueError(msg)
-
-
-def _call(name, dev, *args):
-    lib = _lib.lib()
-    with torch.cuda.device(dev):
-        rc = getattr(lib, name)(*args, _stream(dev))
-    if rc != 0:
-        raise RuntimeError(f"{name} failed ({rc}): {lib.ttt_b200_last_error().decode()}")
 
 
 def eta_gate(logits, scale):
@@ -41,7 +29,7 @@ def eta_gate(logits, scale):
     B, T, H = logits.shape
     _need(T % 64 == 0, "T must be a multiple of 64")
     out = torch.empty(B, H, T // 64, 64, dtype=torch.bfloat16, device=logits.device)
-    _call("ttt_b200_eta_gate", logits.device, logits.data_ptr(), out.data_ptr(), ctypes.c_float(scale), B, T, H)
+    _lib.call_on(logits.device, "ttt_b200_eta_gate", logits.data_ptr(), out.data_ptr(), ctypes.c_float(scale), B, T, H)
     return out
 
 
@@ -53,8 +41,8 @@ def eta_gate_backward(logits, grad_last_eta, scale):
           and grad_last_eta.numel() == B * T * H and grad_last_eta.shape[:2] == (B, H),
           "grad_last_eta must be a contiguous bf16 CUDA tensor [B, H, T // 64, 64(, 1)]")
     out = torch.empty_like(logits)
-    _call("ttt_b200_eta_gate_backward", logits.device, logits.data_ptr(), grad_last_eta.data_ptr(), out.data_ptr(),
-          ctypes.c_float(scale), B, T, H)
+    _lib.call_on(logits.device, "ttt_b200_eta_gate_backward", logits.data_ptr(), grad_last_eta.data_ptr(), out.data_ptr(),
+                 ctypes.c_float(scale), B, T, H)
     return out
 
 
@@ -71,8 +59,8 @@ def unpack_layernorm(out, gamma, beta, eps=1e-6, return_stats=False):
               f"{n} must be a contiguous fp32 CUDA tensor with H * 64 elements")
     y = torch.empty(B, NC * 64, H * 64, dtype=torch.bfloat16, device=out.device)
     stats = torch.empty(B, NC * 64, 2, dtype=torch.float32, device=out.device) if return_stats else None
-    _call("ttt_b200_unpack_layernorm", out.device, out.data_ptr(), gamma.data_ptr(), beta.data_ptr(), y.data_ptr(),
-          stats.data_ptr() if return_stats else None, ctypes.c_float(eps), B, NC * 64, H)
+    _lib.call_on(out.device, "ttt_b200_unpack_layernorm", out.data_ptr(), gamma.data_ptr(), beta.data_ptr(), y.data_ptr(),
+                 stats.data_ptr() if return_stats else None, ctypes.c_float(eps), B, NC * 64, H)
     return (y, stats) if return_stats else y
 
 
@@ -91,6 +79,6 @@ def pack_layernorm_backward(grad_y, out, gamma, stats):
     grad_out = torch.empty_like(out)
     g_gamma = torch.zeros(H * 64, dtype=torch.float32, device=out.device)
     g_beta = torch.zeros(H * 64, dtype=torch.float32, device=out.device)
-    _call("ttt_b200_pack_layernorm_backward", out.device, grad_y.data_ptr(), out.data_ptr(), gamma.data_ptr(),
-          stats.data_ptr(), grad_out.data_ptr(), g_gamma.data_ptr(), g_beta.data_ptr(), B, T, H)
+    _lib.call_on(out.device, "ttt_b200_pack_layernorm_backward", grad_y.data_ptr(), out.data_ptr(), gamma.data_ptr(),
+                 stats.data_ptr(), grad_out.data_ptr(), g_gamma.data_ptr(), g_beta.data_ptr(), B, T, H)
     return grad_out, g_gamma, g_beta

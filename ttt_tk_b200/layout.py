@@ -34,11 +34,7 @@ def _run(name, srcs, dsts, B, T, H):
     n = len(srcs)
     a_src = (ctypes.c_void_p * n)(*[t.data_ptr() for t in srcs])
     a_dst = (ctypes.c_void_p * n)(*[t.data_ptr() for t in dsts])
-    with torch.cuda.device(srcs[0].device):
-        stream = torch.cuda.current_stream().cuda_stream
-        rc = getattr(_lib.lib(), name)(a_src, a_dst, n, B, T, H, ctypes.c_void_p(stream))
-    if rc != 0:
-        raise RuntimeError(f"{name} failed ({rc}): {_lib.lib().ttt_b200_last_error().decode()}")
+    _lib.call_on(srcs[0].device, name, a_src, a_dst, n, B, T, H)
     return dsts
 
 
