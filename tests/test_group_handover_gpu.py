@@ -3,12 +3,15 @@ output; TTT-Linear backward: recompute of one checkpoint group beside the sweep 
 the first mini-batches, where a group still waits for nothing, checkpoints after every one or a ragged last group, one or
 many checkpoint groups, and stream counts on both sides of the number of SMs."""
 import pytest
+import torch
 
 import test_backward_gpu as bwd
 import test_forward_gpu as mlp
 import test_linear_backward_gpu as lbwd
 import test_linear_forward_gpu as lfwd
 from oracle import ttt_mlp as orc
+from ttt_tk_b200 import take_status, ttt_forward
+from ttt_tk_b200.buffers import alloc_checkpoints
 
 pytestmark = pytest.mark.gpu
 
@@ -42,3 +45,24 @@ def test_mlp_backward_between_the_cluster_sizes(H, NC, cgs):
     ck = orc.ttt_forward(d["XQ"], d["XK"], d["XV"], d["last_eta"], d["ttt_norm_weight"], d["ttt_norm_bias"],
                          d["W1"], d["b1"], d["W2"], d["b2"], cgs)
     bwd.check(bwd.run_backward(d, ck, cgs), bwd.oracle_backward(d, ck, cgs))
+
+
+@pytest.mark.parametrize("NC,cgs", [(96, 1), (97, 2)])
+def test_mlp_forward_with_every_sm_storing_checkpoints(NC, cgs):
+    """One stream on every SM, a checkpoint after every one or two mini-batches: the output groups fall behind their chains
+    on the stores.  Every stream must come out bit for bit as from a call of its own, where nothing competes."""
+    B = torch.cuda.get_device_properties(0).multi_processor_count
+    t = {k: v.cuda() for k, v in orc.make_inputs(B, 1, NC, seed=NC).items()}
+
+    def call(lo, hi):
+        x = {k: v if k.startswith("ttt_norm") else v[lo:hi] for k, v in t.items()}
+        ck, out = alloc_checkpoints(hi - lo, 1, NC, cgs), torch.empty_like(x["XQ"])
+        ttt_forward(x["XQ"], x["XK"], x["XV"], x["last_eta"], x["ttt_norm_weight"], x["ttt_norm_bias"],
+                    x["W1"], x["b1"], x["W2"], x["b2"], *ck, out, cgs, cluster=1)
+        return [out, *ck]
+
+    together = call(0, B)
+    for b in range(B):
+        for a, s in zip(together, call(b, b + 1)):
+            assert torch.equal(a[b:b + 1], s), b
+    assert take_status() == 0

@@ -43,7 +43,11 @@
 //   sread   the output group has read the state columns and
 //           taken note of w1rdy                                output group -> chain (MMA4)
 //   w1rdy   bf16 W1 and the shared copy of b1 are refreshed    chain -> output group (MMA5)
-//   accb[1] MMA5 has completed: the bf16 W1 may be rewritten   output's tensor work -> chain (EPI4)
+//   w1read  MMA5 has completed: the bf16 W1 may be rewritten   output's tensor work -> chain (EPI4)
+// A waiter tells only odd from even completions, so a barrier that the other group waits for must complete once per
+// mini-batch and be waited for in every one.  (w1read is apart from accb, the accumulator's own barrier, which completes
+// once per 128-row block: with its second use in the place of w1read, the use of the mini-batch before satisfied EPI4
+// while an output group held up by its checkpoint stores had not issued MMA5 yet, and Out took a state one step too new.)
 //
 // All waits are bounded (see sm100_ptx.cuh); on expiry the CTA reports through the status
 // word, drains its own copies, frees its tensor memory and returns.
@@ -92,7 +96,8 @@ static_assert(kXchBytes >= 8 * 64 * 4, "the partial column sums fit the exchange
 constexpr int BAR_K = 0, BAR_V = 2, BAR_Q = 4;          // + stage
 constexpr int BAR_ACCA = 6;                             // + block (the two 128-row halves of the accumulator)
 constexpr int BAR_Z = 8;
-constexpr int BAR_ACCB = 9;                             // two uses per mini-batch
+constexpr int BAR_ACCB = 9;                             // two uses per mini-batch, within the output group
+constexpr int BAR_W1READ = 10;
 constexpr int BAR_ZB = 11;
 constexpr int BAR_W2UPD = 12, BAR_W2RDY = 13, BAR_SREAD = 14, BAR_W1RDY = 15;
 constexpr int BAR_DRAIN = 16;                           // abort path only
@@ -431,7 +436,7 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         mma_hidden_lead<true, true>(tmem + TM_W2, smem_u32(sX2), smem_u32(sU2), 1, lead);
         if (lead) umma_commit(&bars[BAR_W2UPD]);
       }
-      if (it > 0) wait_bar(BAR_ACCB, 1);              // the last mini-batch's MMA5 has read the bf16 W1 (second use)
+      if (it > 0) wait_bar(BAR_W1READ, prev);         // the last mini-batch's MMA5 has read the bf16 W1
       wait_acca();
       // ---- EPI4: bf16 operand copy of the new W1
 #pragma unroll
@@ -562,6 +567,7 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         tc_fence_after_sync();
         mma_hidden_ta<false, false>(tmem + TM_B, tmem + TM_W1B + blk * 32, smem_u32(sQ), lead);
         if (lead) umma_commit(&bars[BAR_ACCB]);
+        if (lead && blk == 1) umma_commit(&bars[BAR_W1READ]);
       };
       __syncwarp();
       if (warp == 0) issue_mma5(0);
