@@ -255,10 +255,7 @@ def run_ours(args, rank, world, local_rank):
         step = DeviceStep(host, cgs, dev, cluster)
     Bl, Hl = b1 - b0, h1 - h0
     lib = _lib.lib()
-    cl_used = cluster or lib.ttt_b200_pick_cluster(Bl * Hl, 1)
-    cl_fwd = cluster or lib.ttt_b200_pick_cluster(Bl * Hl, 0)
-    if not cluster and "TTT_B200_CLUSTER" not in os.environ and cl_fwd == 2:
-        cl_fwd, cl_used = 1, 2      # the launchers' choice where two CTAs per stream fit and four do not
+    cl_fwd, cl_used = (lib.ttt_b200_launch_cluster(Bl * Hl, (cluster or 0) << 8, backward) for backward in (0, 1))
 
     sampler = ClockSampler(local_rank)
     # warm-up happens inside timed_steps; the sampler is started just before so that most of its samples

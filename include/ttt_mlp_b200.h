@@ -281,14 +281,17 @@ int ttt_b200_take_status(void);
 /* Library / ABI version (major * 1000 + minor). */
 int ttt_b200_version(void);
 
-/* How many CTAs (1, 2 or 4) the forward (backward = 0) or backward (backward != 0) launcher gives each
- * (batch, head) stream of a problem with `streams` = B*H streams on the current device when the flags leave
- * the choice to it: four when the device runs that many clusters of four at once
- * (ttt_b200_cluster_capacity), else (forward only) two when those fit, else one (measured thresholds).
- * Between the two capacities the operators refine that answer when neither the flags nor the environment name a size:
- * the forward runs one CTA per stream with its output pass on a second group of warps, the backward two CTAs.
- * TTT_B200_CLUSTER overrides.  The reference fixes the split at compile time
- * (kernels/ttt/ttt.cu:11-12, kernels/ttt_backward/ttt.cu:12-16).  Returns -1 on error. */
+/* How many CTAs (1, 2 or 4) a call of ttt_b200_forward (backward = 0) or ttt_b200_backward (backward != 0) with these
+ * `flags` gives each (batch, head) stream of a problem with `streams` = B*H streams on the current device.  The size that
+ * the flags name; else the one that TTT_B200_CLUSTER names (0 or empty: none); else four when the device runs that many
+ * clusters of four at once (ttt_b200_cluster_capacity), else two in the backward when those fit, else one (measured
+ * thresholds).  The reference fixes the split at compile time (kernels/ttt/ttt.cu:11-12,
+ * kernels/ttt_backward/ttt.cu:12-16).  Returns -1 on error. */
+int ttt_b200_launch_cluster(int streams, uint32_t flags, int backward);
+
+/* The widest cluster size whose capacity on the current device covers `streams`: four, else (forward only) two, else one.
+ * TTT_B200_CLUSTER overrides.  Not what a launch runs between the two capacities: ttt_b200_launch_cluster is.  Returns
+ * -1 on error. */
 int ttt_b200_pick_cluster(int streams, int backward);
 
 /* How many clusters of `cluster` (2 or 4) CTAs of the forward (backward = 0) or backward kernel the current

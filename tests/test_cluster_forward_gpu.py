@@ -86,8 +86,8 @@ def test_cluster_forward_long_sequence_heads_only():
 
 def test_launcher_choice_follows_the_cluster_capacity():
     """The launcher gives a stream four CTAs only while the device runs that many clusters of four at
-    the same time (the occupancy query, not SMs / 4), the forward two while those fit, else one; the
-    backward never picks two."""
+    the same time (the occupancy query, not SMs / 4).  Between the capacities for four and two this entry names the widest
+    size that fits, in the forward only; what a call runs there is the next test's."""
     from ttt_tk_b200 import _lib
     lib = _lib.lib()
     sms = torch.cuda.get_device_properties(0).multi_processor_count
@@ -101,6 +101,26 @@ def test_launcher_choice_follows_the_cluster_capacity():
         assert lib.ttt_b200_pick_cluster(c2, backward) == (1 if backward else 2)
         assert lib.ttt_b200_pick_cluster(c2 + 1, backward) == 1
         assert lib.ttt_b200_pick_cluster(0, backward) == -1
+
+
+def test_launched_cluster_size():
+    from ttt_tk_b200 import _lib
+    lib = _lib.lib()
+    for backward in (0, 1):
+        c2, c4 = lib.ttt_b200_cluster_capacity(2, backward), lib.ttt_b200_cluster_capacity(4, backward)
+        launch = lambda n, forced=0: lib.ttt_b200_launch_cluster(n, forced << 8, backward)
+        assert [launch(n) for n in (1, c4, c4 + 1, c2, c2 + 1)] == [4, 4, 1 + backward, 1 + backward, 1]
+        assert [launch(c2, c) for c in (1, 2, 4, 3)] == [1, 2, 4, -1] and launch(0) == -1
+
+
+@pytest.mark.parametrize("H", [33, 34, 74, 75])
+def test_a_call_runs_the_cluster_size_that_the_library_names(H):
+    """Bit for bit the call that is forced to that size, and no other size's (their sums over the hidden units differ)."""
+    from ttt_tk_b200 import _lib
+    d = nonzero_bias_inputs(1, H, 3, seed=H, eta_scale=1.0)
+    named = _lib.lib().ttt_b200_launch_cluster(H, 0, 0)
+    out = {c: run_forward(d, 2, c)["W1_final"] for c in (None, 1, 2, 4)}
+    assert [c for c in (1, 2, 4) if torch.equal(out[c], out[None])] == [named]
 
 
 def test_a_problem_at_the_capacity_of_four_cta_clusters_runs_in_one_wave():

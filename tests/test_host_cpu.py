@@ -4,6 +4,8 @@ anything is launched (no compute calls here: there is no GPU)."""
 import ctypes
 import os
 import re
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -98,3 +100,14 @@ def test_package_input_recipe_equals_the_oracles():
     assert a.keys() == b.keys()
     for k in a:
         assert torch.equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("env,want", [(None, "1 2 4 -1"), ("0", "1 2 4 -1"), ("", "1 2 4 -1"), ("2", "2 2 4 -1"), ("3", "-1 2 4 -1")])
+def test_launch_cluster_takes_the_flags_then_the_environment(env, want):
+    """The flags' size, else the variable's (0 or empty names none), else the choice by capacity (none without a device)."""
+    code = ("from ttt_tk_b200 import _lib; f = _lib.lib().ttt_b200_launch_cluster; "
+            "assert f(0, 0, 0) == f(0, 0, 1) == -1; "
+            "print(f(60, 0, 0), f(60, 2 << 8, 0), f(60, 4 << 8, 1), f(60, 3 << 8, 0))")
+    e = {k: v for k, v in os.environ.items() if k != "TTT_B200_CLUSTER"}
+    e.update({} if env is None else {"TTT_B200_CLUSTER": env}, CUDA_VISIBLE_DEVICES="")
+    assert subprocess.check_output([sys.executable, "-c", code], env=e, cwd=ROOT, text=True).split("\n")[-2] == want

@@ -66,45 +66,42 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 
 }  // namespace
 
-// How many CTAs share one stream.  The mini-batches of a stream are strictly sequential, so with fewer
-// streams than SMs the idle SMs can only help by taking a share of every stream's hidden units.  Four
-// CTAs per stream win whenever they all fit on the GPU at once (32 streams on a B200: forward 4.4 against 4.9 us per
-// mini-batch with one CTA, backward 14.2 against 23.2).  Between that and the streams of which two CTAs each fit, this
-// names the plain choice and the launchers refine it: ttt_launch_cluster below.
-int ttt_pick_cluster(int streams, uint32_t flags, bool backward, int* cluster) {
-  int forced = static_cast<int>((flags & TTT_B200_FLAG_CLUSTER_MASK) >> TTT_B200_FLAG_CLUSTER_SHIFT);
-  if (forced == 0) {
+namespace {
+
+// The cluster size that the flags or, failing them, TTT_B200_CLUSTER ask for; 0: neither names one.
+int asked_cluster(uint32_t flags, int* cluster) {
+  *cluster = static_cast<int>((flags & TTT_B200_FLAG_CLUSTER_MASK) >> TTT_B200_FLAG_CLUSTER_SHIFT);
+  if (*cluster == 0) {
     static const int env = [] {
       const char* e = std::getenv("TTT_B200_CLUSTER");
       return e ? std::atoi(e) : 0;
     }();
-    forced = env;
+    *cluster = env;
   }
-  if (forced != 0) {
-    if (forced != 1 && forced != 2 && forced != 4)
-      return ttt_set_error(TTT_B200_ERR_BAD_ARGS, "cluster size must be 1, 2 or 4");
-    *cluster = forced;
-    return TTT_B200_OK;
-  }
-  // all streams must be resident at once for the sharding to pay: the widest cluster size whose capacity
-  // (clusters the device runs at the same time) covers them
-  auto capacity = [&](int c) { return backward ? ttt_backward_cluster_capacity(c) : ttt_forward_cluster_capacity(c); };
-  if (streams <= capacity(4)) *cluster = 4;
-  else if (!backward && streams <= capacity(2)) *cluster = 2;
-  else *cluster = 1;
+  if (*cluster != 0 && *cluster != 1 && *cluster != 2 && *cluster != 4)
+    return ttt_set_error(TTT_B200_ERR_BAD_ARGS, "cluster size must be 1, 2 or 4");
   return TTT_B200_OK;
 }
 
-// What a launch runs.  Where two CTAs per stream fit but four do not (34 to 74 streams on a B200) and nobody asked for a
-// size: one CTA in the forward, whose output pass runs beside the chain in two groups of warps (5.0 us per mini-batch
-// against 6.1 with two CTAs), and two in the backward (48 / 60 / 74 streams in groups of 4: 19.9 / 20.8 / 21.5 us per
-// mini-batch against 23.2 / 23.2 / 23.3 with one).
+int capacity(int cluster, bool backward) {
+  return backward ? ttt_backward_cluster_capacity(cluster) : ttt_forward_cluster_capacity(cluster);
+}
+
+}  // namespace
+
+// How many CTAs share one stream.  The mini-batches of a stream are strictly sequential, so with fewer
+// streams than SMs the idle SMs can only help by taking a share of every stream's hidden units, and only while all
+// streams are resident at once.  Four CTAs per stream win whenever the device runs that many clusters of four (32 streams
+// on a B200: forward 4.4 against 4.9 us per mini-batch with one CTA, backward 14.2 against 23.2).  Where only clusters of
+// two fit (34 to 74 streams), the forward runs one CTA, whose output pass runs beside the chain in two groups of warps
+// (5.0 us per mini-batch against 6.1 with two CTAs), and the backward two (48 / 60 / 74 streams in groups of 4: 19.9 /
+// 20.8 / 21.5 us per mini-batch against 23.2 / 23.2 / 23.3 with one).  Beyond, one.
 static int ttt_launch_cluster(int streams, uint32_t flags, bool backward, int* cluster) {
-  if (int rc = ttt_pick_cluster(streams, flags, backward, cluster)) return rc;
-  static const bool env = std::getenv("TTT_B200_CLUSTER") != nullptr;
-  if ((flags & TTT_B200_FLAG_CLUSTER_MASK) || env) return TTT_B200_OK;
-  if (!backward && *cluster == 2) *cluster = 1;
-  else if (backward && *cluster == 1 && streams <= ttt_backward_cluster_capacity(2)) *cluster = 2;
+  if (int rc = asked_cluster(flags, cluster)) return rc;
+  if (*cluster != 0) return TTT_B200_OK;
+  if (streams <= capacity(4, backward)) *cluster = 4;
+  else if (backward && streams <= capacity(2, backward)) *cluster = 2;
+  else *cluster = 1;
   return TTT_B200_OK;
 }
 
@@ -338,8 +335,18 @@ extern "C" int ttt_b200_cluster_capacity(int cluster, int backward) {
   return backward ? ttt_backward_cluster_capacity(cluster) : ttt_forward_cluster_capacity(cluster);
 }
 
+// The widest size whose capacity covers the streams (two in the forward only): a property of the device, kept for its
+// callers.  What a launch runs is ttt_b200_launch_cluster's answer.
 extern "C" int ttt_b200_pick_cluster(int streams, int backward) {
-  int c = 1;
-  if (streams < 1 || ttt_pick_cluster(streams, 0u, backward != 0, &c) != TTT_B200_OK) return -1;
+  int c = 0;
+  if (streams < 1 || asked_cluster(0u, &c) != TTT_B200_OK) return -1;
+  if (c != 0) return c;
+  if (streams <= capacity(4, backward != 0)) return 4;
+  return !backward && streams <= capacity(2, false) ? 2 : 1;
+}
+
+extern "C" int ttt_b200_launch_cluster(int streams, uint32_t flags, int backward) {
+  int c = 0;
+  if (streams < 1 || ttt_launch_cluster(streams, flags, backward != 0, &c) != TTT_B200_OK) return -1;
   return c;
 }
