@@ -111,3 +111,19 @@ def test_launch_cluster_takes_the_flags_then_the_environment(env, want):
     e = {k: v for k, v in os.environ.items() if k != "TTT_B200_CLUSTER"}
     e.update({} if env is None else {"TTT_B200_CLUSTER": env}, CUDA_VISIBLE_DEVICES="")
     assert subprocess.check_output([sys.executable, "-c", code], env=e, cwd=ROOT, text=True).split("\n")[-2] == want
+
+
+def test_load_host_rebuilds_a_module_older_than_the_abi_header(monkeypatch, tmp_path):
+    """A module compiled against an older header fills argument structs of another layout."""
+    from ttt_tk_b200 import build
+    built = []
+    module = tmp_path / build.HOST_NAME
+    module.write_bytes(b"")
+    monkeypatch.setattr(build, "_module_path", lambda name: str(tmp_path / name))
+    monkeypatch.setattr(build, "_build_torch_module", lambda name, source, out, *rest: built.append(out))
+    monkeypatch.setattr(build, "_load", lambda name, path: path)
+    newest = max(os.path.getmtime(p) for p in (build.HOST_SOURCE, os.path.join(ROOT, "include", "ttt_mlp_b200.h")))
+    for age, want in ((1, []), (-1, [str(module)])):
+        os.utime(module, (newest + age, newest + age))
+        assert build.load_host() == str(module)
+        assert built == want

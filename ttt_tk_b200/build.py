@@ -72,11 +72,16 @@ def extension_path():
     return _module_path(EXT_NAME)
 
 
+def _module_needs_build(source, out):
+    """Missing, or older than its source or the C ABI's header, whose argument structs it fills."""
+    deps = [source, os.path.join(CSRC, "..", "..", "include", "ttt_mlp_b200.h")]
+    return not os.path.exists(out) or any(os.path.getmtime(d) > os.path.getmtime(out) for d in deps)
+
+
 def _build_torch_module(name, source, out, force, verbose):
     """Compile one C++ module against the installed torch and the C-ABI library, with g++, in-tree."""
     build(force=False, verbose=verbose)
-    deps = [source, os.path.join(CSRC, "..", "..", "include", "ttt_mlp_b200.h")]
-    if not force and os.path.exists(out) and all(os.path.getmtime(d) <= os.path.getmtime(out) for d in deps):
+    if not force and not _module_needs_build(source, out):
         return out
     import sysconfig
     import torch
@@ -125,9 +130,9 @@ def load_extension():
 
 
 def load_host():
-    """Import and return the operators' native host side (building it if it is missing)."""
+    """Import and return the operators' native host side (building it, and the library, if it is out of date)."""
     path = _module_path(HOST_NAME)
-    if not os.path.exists(path):
+    if _module_needs_build(HOST_SOURCE, path):
         _build_torch_module(HOST_NAME, HOST_SOURCE, path, False, False)
     return _load(HOST_NAME, path)
 

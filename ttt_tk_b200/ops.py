@@ -29,8 +29,9 @@ _HOST = None
 def _host():
     global _HOST
     if _HOST is None:
+        host = load_host()      # may build: before the library is loaded
         _lib.lib()
-        _HOST = load_host()
+        _HOST = host
     return _HOST
 
 
