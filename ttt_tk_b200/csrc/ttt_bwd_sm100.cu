@@ -48,9 +48,6 @@
 // not accumulated; `Out` is never touched.  Every wait is bounded.
 #include <mutex>
 
-#ifndef TTT_MMA_ROLLED
-#define TTT_MMA_ROLLED 1
-#endif
 #include "ttt_device.cuh"
 #include "ttt_internal.h"
 

@@ -102,55 +102,20 @@ __device__ __forceinline__ void st_chunk(uint8_t* tile, uint32_t row, uint32_t c
 __device__ __forceinline__ uint4 ld_chunk_raw(const uint8_t* tile, uint32_t row, uint32_t chunk) {
   return *reinterpret_cast<const uint4*>(tile + sw128_off(row, chunk));
 }
-__device__ __forceinline__ float ld_elem(const uint8_t* tile, uint32_t row, uint32_t col) {
-  return __bfloat162float(
-      *reinterpret_cast<const __nv_bfloat16*>(tile + sw128_off(row, col >> 3) + (col & 7) * 2));
-}
 
-// A kernel whose instruction footprint exceeds the instruction cache defines TTT_MMA_ROLLED 1 before
-// including this header (rolled issue loops); a small kernel keeps them unrolled (lower issue latency).
-#ifndef TTT_MMA_ROLLED
-#define TTT_MMA_ROLLED 0
-#endif
-#ifndef TTT_MMA_SHARED_LOOP
-#define TTT_MMA_SHARED_LOOP (TTT_MMA_ROLLED == 1)
-#endif
-#if TTT_MMA_ROLLED == 1
-#define TTT_MMA_LOOP _Pragma("unroll 1")
-#define TTT_MMA_OUTER _Pragma("unroll 1")
-#elif TTT_MMA_ROLLED == 2
-#define TTT_MMA_LOOP _Pragma("unroll 4")
-#define TTT_MMA_OUTER _Pragma("unroll 1")
-#else
-#define TTT_MMA_LOOP _Pragma("unroll")
-#define TTT_MMA_OUTER _Pragma("unroll")
-#endif
-
-// ---- MMA issue.  Four threads (lane 0 of warps 0..3) issue the MMAs of a phase; the instruction
-// stream around each tcgen05.mma is kept to two integer adds: the descriptors' high words are the
-// same constant for every operand (stride byte offset 1024, version 1, 128-byte swizzle) and
+// ---- MMA issue.  The instruction stream around each tcgen05.mma is kept to two integer adds: the descriptors' high
+// words are the same constant for every operand (stride byte offset 1024, version 1, 128-byte swizzle) and
 // the low words (start address | leading byte offset) advance by a constant per K step.
 constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
   return ((smem_addr & 0x3FFFFu) >> 4) | ((lbo_bytes >> 4) << 16);
 }
-template <bool kAccumulate>
-__device__ __forceinline__ void mma_issue(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-      "mov.b64 da, {%1, %4};\n\t"
-      "mov.b64 db, {%2, %4};\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
-      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kDescHi), "n"(kAccumulate ? 1 : 0)
-      : "memory");
-}
 
-// Issue with the accumulate flag in a register, and the one shared copy of the issue loop that a
-// kernel with rolled loops (TTT_MMA_ROLLED 1) calls for every product: n MMAs whose operand
-// descriptors advance by a constant per K step; the first one overwrites D unless `acc` is set.
-// A tcgen05.mma costs about ten instructions of set-up, so one out-of-line loop instead of one per
-// product shrinks such a kernel by roughly a tenth; only the issuing threads ever run it.
+// ---- Products issued by single threads (lane 0 of warps 0..3, one product or half each), through one out-of-line loop
+// that every product of the kernel shares: n MMAs whose operand descriptors advance by a constant per K step; the first
+// one overwrites D unless `acc` is set.  For the one-CTA backward, whose instruction footprint exceeds the instruction
+// cache: a tcgen05.mma costs about ten instructions of set-up, so one loop instead of one per product shrinks it by
+// roughly a tenth.
 __device__ __forceinline__ void mma_issue_rt(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
                                              uint32_t accumulate) {
   asm volatile(
@@ -180,61 +145,22 @@ static __device__ __noinline__ void mma_run(uint32_t tmem_d, uint32_t a_lo, uint
 // tmem_d + 64) (+)= A * B with A a [256][64] bf16 tile read K-major (row = hidden unit) and B a
 // [64][64] tile read K-major (row = N index) or MN-major (row = K index).
 // One M = 128 block (`blk` = 0 or 1: hidden units 128 blk .. 128 blk + 127) of the product.  The two
-// blocks are independent, so two threads may issue one each.
-template <bool kBMn, bool kAccumulate>
-__device__ __forceinline__ void mma_hidden_half_t(uint32_t tmem_d, uint32_t a_smem, uint32_t b_smem, int blk) {
-  constexpr uint32_t idesc = umma_idesc_bf16(128, 64, false, kBMn, false);
-  const uint32_t a0 = desc_lo(a_smem, 16) + blk * (16384u >> 4);
-  const uint32_t b0 = desc_lo(b_smem, kBMn ? 8192 : 16);
-  constexpr uint32_t bstep = kBMn ? (2048u >> 4) : (32u >> 4);
-  const uint32_t d = tmem_d + blk * 64;
-#if TTT_MMA_SHARED_LOOP
-  mma_run(d, a0, b0, idesc, 4, 2, bstep, kAccumulate ? 1u : 0u);
-#else
-  if (kAccumulate) mma_issue<true>(d, a0, b0, idesc);
-  else             mma_issue<false>(d, a0, b0, idesc);
-TTT_MMA_LOOP
-  for (int j = 1; j < 4; ++j) mma_issue<true>(d, a0 + j * 2, b0 + j * bstep, idesc);
-#endif
-}
-template <bool kBMn, bool kAccumulate>
-__device__ __forceinline__ void mma_hidden_major_t(uint32_t tmem_d, uint32_t a_smem, uint32_t b_smem) {
-TTT_MMA_OUTER
-  for (int blk = 0; blk < 2; ++blk) mma_hidden_half_t<kBMn, kAccumulate>(tmem_d, a_smem, b_smem, blk);
-}
+// blocks are independent, so two threads may issue one each.  The flags are constants at every call.
 __device__ __forceinline__ void mma_hidden_half(uint32_t tmem_d, uint32_t a_smem, uint32_t b_smem, bool b_mn,
                                                 bool accumulate, int blk) {
-  if (b_mn) {
-    if (accumulate) mma_hidden_half_t<true, true>(tmem_d, a_smem, b_smem, blk);
-    else            mma_hidden_half_t<true, false>(tmem_d, a_smem, b_smem, blk);
-  } else {
-    if (accumulate) mma_hidden_half_t<false, true>(tmem_d, a_smem, b_smem, blk);
-    else            mma_hidden_half_t<false, false>(tmem_d, a_smem, b_smem, blk);
-  }
+  mma_run(tmem_d + blk * 64, desc_lo(a_smem, 16) + blk * (16384u >> 4), desc_lo(b_smem, b_mn ? 8192 : 16),
+          umma_idesc_bf16(128, 64, false, b_mn, false), 4, 2, b_mn ? (2048u >> 4) : (32u >> 4), accumulate ? 1u : 0u);
 }
 __device__ __forceinline__ void mma_hidden_major(uint32_t tmem_d, uint32_t a_smem, uint32_t b_smem, bool b_mn,
                                                  bool accumulate) {
-  if (b_mn) {
-    if (accumulate) mma_hidden_major_t<true, true>(tmem_d, a_smem, b_smem);
-    else            mma_hidden_major_t<true, false>(tmem_d, a_smem, b_smem);
-  } else {
-    if (accumulate) mma_hidden_major_t<false, true>(tmem_d, a_smem, b_smem);
-    else            mma_hidden_major_t<false, false>(tmem_d, a_smem, b_smem);
-  }
+#pragma unroll 1
+  for (int blk = 0; blk < 2; ++blk) mma_hidden_half(tmem_d, a_smem, b_smem, b_mn, accumulate, blk);
 }
 // "Token-major" product: D[64 tok x 64] (M = 64: row r in TMEM lane (r % 16) + 32 * (r / 16))
 // = X[64 x 256] * W[256 x 64], both operands [256][64] tiles read MN-major (row = hidden unit).
 __device__ __forceinline__ void mma_token_major(uint32_t tmem_d, uint32_t x_smem, uint32_t w_smem) {
-  constexpr uint32_t idesc = umma_idesc_bf16(64, 64, true, true, false);
-  const uint32_t a0 = desc_lo(x_smem, BIG);
-  const uint32_t b0 = desc_lo(w_smem, BIG);
-#if TTT_MMA_SHARED_LOOP
-  mma_run(tmem_d, a0, b0, idesc, 16, 2048u >> 4, 2048u >> 4, 0u);
-#else
-  mma_issue<false>(tmem_d, a0, b0, idesc);
-TTT_MMA_LOOP
-  for (int j = 1; j < 16; ++j) mma_issue<true>(tmem_d, a0 + j * (2048u >> 4), b0 + j * (2048u >> 4), idesc);
-#endif
+  mma_run(tmem_d, desc_lo(x_smem, BIG), desc_lo(w_smem, BIG), umma_idesc_bf16(64, 64, true, true, false), 16,
+          2048u >> 4, 2048u >> 4, 0u);
 }
 
 // ---- The same products issued by a whole warp under a predicate: the warp runs the code uniformly, so that the
