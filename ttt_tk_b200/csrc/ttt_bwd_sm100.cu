@@ -428,7 +428,10 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         const f32x2 ne0 = pk1(-__bfloat162float(eta[tm.r0])), ne1 = pk1(-__bfloat162float(eta[tm.r1]));
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          // dl/dZ2, rounded to bf16 once: the update below uses -eta times the rounded value
+          // dl/dZ2, rounded to bf16 once: the update below uses -eta times the rounded value.  The forward rounds the
+          // product instead, and adds up b2 from the rounded products (the recompute with four CTAs per stream does so
+          // too, this one and that with two take the fp32 ones): the state rebuilt inside a group differs from the
+          // forward's by about that rounding, 2e-3 of b2's change since the checkpoint.
           const uint32_t w0 = f32x2_to_bf16x2(mul2(fma2(x.a[q], pk1(-a[1]), fma2(g.a[q], pk1(64.f), pk1(-a[0]))), sc0));
           const uint32_t w1 = f32x2_to_bf16x2(mul2(fma2(x.b[q], pk1(-b[1]), fma2(g.b[q], pk1(64.f), pk1(-b[0]))), sc1));
           *reinterpret_cast<uint32_t*>(tGZ2 + tm.off(tm.r0, q)) = w0;

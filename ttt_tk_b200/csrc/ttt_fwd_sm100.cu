@@ -503,6 +503,7 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       tc_fence_after_sync();
       // ---- b2 += column sums of U2 (bf16 values, the operand the W2 update sees), fp32 accumulate: a thread
       // sums 8 rows of a column pair, threads 0..63 add the eight parts.  bf16 operand copy of the new W2.
+      // (The backward's recompute rebuilds the state from another rounding of the same update: see its LN stage.)
       float* part = reinterpret_cast<float*>(smem + OFF_XCHO);
       {
         const int pr = gtid & 31;
