@@ -38,11 +38,13 @@
 //   E5   gZ1in^T = gX2^T gelu'(Z1^T) + R^T S^T;  G_b1 += row sums
 //   G13  dK += gZ1in W1^T       G14 G_W2 += X2^T gZ2in     G15 G_W1^T += gZ1in^T K
 //
-// What bounds it: one chain of 14 MMA phases and as many epilogues, of which the tensor pipe is busy for a quarter; the
-// epilogues issue on two warps per scheduler.  They run on packed fp32 pairs and take column sums from registers.
-// Measured per mini-batch, 128 streams: 25.1 -> 23.5 us (packed pairs; 64 mini-batches in groups of 8) and 25.5 -> 24.0 us
-// (shared-space addresses, unrolled column passes; 32 mini-batches in groups of 4).  Sixteen warps with the recompute's output pass beside its chain were
-// no faster (24.4-26 us: 128 registers a thread and more code than the instruction cache holds).
+// What bounds it: one chain of 14 MMA phases and as many epilogues on two warps per scheduler (128 streams: tensor pipe
+// 15 %, issue slots 30 %, DRAM 38 %; the warps wait for tensor memory, the MMAs and, half a warp per issue, for
+// instructions).  The epilogues run on packed fp32 pairs and take column sums from registers.  Measured per mini-batch, 128
+// streams of 128: 25.2 -> 21.6 us in groups of 8, 23.6 in groups of 4 (64 mini-batches in groups of 8: 25.1 -> 23.5 by the
+// packed pairs; 32 in groups of 4: 25.5 -> 24.0 by shared-space addresses and unrolled column passes).  Sixteen warps
+// with the recompute's output pass beside its chain were no faster (24.4-26 us: 128 registers a thread and more code
+// than the instruction cache holds).
 //
 // Deviations from the reference kernel (see include/ttt_mlp_b200.h): outputs are overwritten,
 // not accumulated; `Out` is never touched.  Every wait is bounded.

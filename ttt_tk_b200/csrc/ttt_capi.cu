@@ -91,10 +91,10 @@ int capacity(int cluster, bool backward) {
 // How many CTAs share one stream.  The mini-batches of a stream are strictly sequential, so with fewer
 // streams than SMs the idle SMs can only help by taking a share of every stream's hidden units, and only while all
 // streams are resident at once.  Four CTAs per stream win whenever the device runs that many clusters of four (32 streams
-// on a B200: forward 4.4 against 4.9 us per mini-batch with one CTA, backward 14.2 against 23.2).  Where only clusters of
-// two fit (34 to 74 streams), the forward runs one CTA, whose output pass runs beside the chain in two groups of warps
-// (5.0 us per mini-batch against 6.1 with two CTAs), and the backward two (48 / 60 / 74 streams in groups of 4: 19.9 /
-// 20.8 / 21.5 us per mini-batch against 23.2 / 23.2 / 23.3 with one).  Beyond, one.
+// of 128 mini-batches in groups of 4 on a B200: forward 4.3 against 4.6 us per mini-batch with one CTA, backward 14.0
+// against 22.7).  Where only clusters of two fit (34 to 74 streams), the forward runs one CTA, whose output pass runs
+// beside the chain in two groups of warps (4.6 us per mini-batch against 5.8 with two CTAs), and the backward two (48 / 60
+// / 74 streams: 19.0 / 20.1 / 21.0 us per mini-batch against 22.8 / 22.9 / 23.1 with one).  Beyond, one.
 static int ttt_launch_cluster(int streams, uint32_t flags, bool backward, int* cluster) {
   if (int rc = asked_cluster(flags, cluster)) return rc;
   if (*cluster != 0) return TTT_B200_OK;

@@ -29,13 +29,14 @@
 // trips per mini-batch instead of six, and each group's MMA latencies are filled with the other's epilogues (four
 // warps per scheduler).
 //
-// What bounds it: instruction issue and the fp32 / MUFU pipes (EPI1 alone is 1300 cycles of fp32 pipe per mini-batch
-// at 9 packed operations and 2 conversions per pair of elements) and shared-memory bandwidth.  So the arithmetic
-// runs on packed fp32 pairs; what only one thread needs stays out of shared memory (G' in registers from EPI1 to
-// EPI3, U1 and the bf16 W1 in tensor memory as A operands of their MMAs, which then read 2 KB of shared memory
-// instead of 6); and the MMAs are issued from warp-uniform code.  Measured (B200, 128 streams, one checkpoint in 8
-// mini-batches): 8.0 us per mini-batch before, one group of 8 warps, 6.0 with the two groups, 5.3 now; 1536 streams of
-// 64 mini-batches 5.43 -> 3.68 ms.
+// What bounds it: the chain's four round trips.  No pipe is full over a mini-batch (128 streams: issue slots 44 %, fp32
+// pipe 35 %, tensor pipe 20 %, DRAM 11 %), but within its epilogues the fp32 and MUFU pipes set the pace (EPI1 alone is
+// 1300 cycles of fp32 pipe at 9 packed operations and 2 conversions per pair of elements) and within its products the
+// shared-memory operands.  So the arithmetic runs on packed fp32 pairs; what only one thread needs stays out of shared
+// memory (G' in registers from EPI1 to EPI3, U1 and the bf16 W1 in tensor memory as A operands of their MMAs, which then
+// read 2 KB of shared memory instead of 6); and the MMAs are issued from warp-uniform code.  Measured (B200, 128 streams
+// of 128 mini-batches, one checkpoint in 8): 8.0 us per mini-batch as one group of 8 warps, 6.0 with the two groups, 4.6
+// with the rest; 1536 streams of 64 mini-batches 5.43 -> 3.23 ms.
 //
 // Hand-over between the groups (mbarriers, each completed once per mini-batch):
 //   w2upd   MMA4's W2 update has completed                     chain's tensor work -> output group

@@ -1,7 +1,7 @@
 // Host side of the Python operators (`ttt_tk_b200.ops`): argument validation, the C ABI's argument structs and the
 // launch, in native code.  For short sequences a call is bound by its host time, and checking 15 to 42 tensors one
-// attribute at a time from Python took most of it.  Measured: the forward's enqueue 50 -> 7 us; forwards of one
-// mini-batch in a row 57 -> 12.3 us each (the kernel's own time), of four TTT-Linear mini-batches 44 -> 16.4.
+// attribute at a time from Python took most of it.  Measured: the forward's enqueue 50 -> 4.2 us; forwards of one
+// mini-batch in a row 57 -> 8.9 us each (the kernel's own time), of four TTT-Linear mini-batches 44 -> 10.6.
 //
 // Plain CPython functions (METH_FASTCALL, positional arguments in the operators' order); every failed check raises
 // RuntimeError like the reference's TORCH_CHECKs (kernels/ttt/ttt.cu:621-630, kernels/ttt_backward/ttt.cu:1507-1760).

@@ -29,9 +29,10 @@
 //   slot <- bf16 W^T before the update, x_f, gZ, gZb (raw images of the swizzled shared-memory tiles, stored and read
 //   back with bulk copies), 1/std of the fused LayerNorm, the column sums of gZb.
 //
-// What bounds it: instruction issue (15 k warp-instructions per mini-batch in token-major epilogues) and the latency
-// of the two chains.  Measured at 128 streams: 8.4 us per mini-batch as one chain of eight warps, 5.3 with the recompute
-// beside the sweep, less with packed epilogues and shared-space addresses.  All waits are bounded; on expiry the CTA
+// What bounds it: the latency of the two chains and their shared issue slots (16.2 k warp-instructions per mini-batch,
+// most in token-major epilogues; 128 streams: issue slots 50 %, fp32 pipe 34 %, DRAM 33 %, tensor pipe 12 %).  Measured
+// at 128 streams: 8.4 us per mini-batch as one chain of eight warps, 5.3 with the recompute beside the sweep, 4.5 with
+// packed epilogues and shared-space addresses.  All waits are bounded; on expiry the CTA
 // reports through the status word, drains its own copies, frees its tensor memory and returns.
 #include <mutex>
 

@@ -22,8 +22,9 @@
 // when there are more streams than SMs (72 KB of shared memory with a two-stage input ring, 128
 // tensor-memory columns, 80 registers per thread each), which hides the latency of the three dependent MMA
 // phases (measured at
-// 1536 streams: 1.43 ms with two CTAs per SM and a three-stage ring, 1.34 ms with three).  All waits are bounded; on expiry the CTA reports through
-// the status word, drains its own copies, frees its tensor memory and returns.
+// 1536 streams of 64 mini-batches: 1.43 ms with two CTAs per SM and a three-stage ring, 1.34 ms with three, 1.04-1.10 with
+// packed epilogues; issue slots 56 %, fp32 pipe 40 %, DRAM 36 %).  All waits are bounded; on expiry the CTA reports
+// through the status word, drains its own copies, frees its tensor memory and returns.
 #include <mutex>
 
 #include "ttt_cluster.cuh"
@@ -348,9 +349,10 @@ ttt_linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
 // ---- The form for launches with no more streams than SMs: nothing but the stream itself could fill its SM, so the
 // output pass runs on eight warps of its own beside the chain of the other eight (Z -> U -> state -> bf16 copy), one step
-// behind, as in the MLP forward (148 streams of 64 mini-batches: 2.8 -> 2.25 us per mini-batch; bound by the latency of
-// the chain, two products and the LayerNorm with its two exchanges).  Two copies of the bf16 state alternate, so that the chain does not wait for the output
-// product; the output group also stores the checkpoints.
+// behind, as in the MLP forward (148 streams of 64 mini-batches: 2.8 -> 1.95 us per mini-batch; bound by the latency of
+// the chain, two products and the LayerNorm with its two exchanges: issue slots 45 %, tensor pipe 10 %).  Two copies of the
+// bf16 state alternate, so that the chain does not wait for the output product; the output group also stores the
+// checkpoints.
 namespace pair {
 
 constexpr int kGroup = 256;
@@ -661,7 +663,7 @@ int ttt_launch_linear_forward(const ttt_b200_linear_fwd_args* a, cudaStream_t st
   });
   if (attr_err[dev] != cudaSuccess) return ttt_set_error(TTT_B200_ERR_LAUNCH, cudaGetErrorString(attr_err[dev]));
   // no more streams than SMs: one CTA of two groups per stream.  Beyond that two or three plain CTAs share an SM and fill
-  // each other's waits (296 streams: 3.5 us per mini-batch of all, against 2 x 1.9 in two turns of the form above).
+  // each other's waits (296 streams: 3.5 us per mini-batch of all, against 2 x 1.95 in two turns of the form above).
   cudaError_t e;
   if (a->B * a->H <= sms[dev]) {
     CUtensorMap tmOut;
