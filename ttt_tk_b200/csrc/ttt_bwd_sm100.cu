@@ -21,7 +21,7 @@
 //   X2_group, grad_l_wrt_Z1_group, Z1_bar_group (holds gelu'(Z1_bar)), X2_bar_group : [256][64 tok] bf16
 //   Z1_group : [256][64 tok] f16 (the sweep evaluates gelu' and gelu'' of it in packed f16)
 //   W1_init_group / W2_init_group (first 32 KB of each slot): bf16 W1^T / W2 before the update
-//   x_hat_fused, grad_output_fused, grad_l_wrt_Z2, x_hat_ln_group : [64 tok][64] bf16
+//   x_hat_fused, grad_l_wrt_Z2, x_hat_ln_group : [64 tok][64] bf16
 //   std_fused_group, std_ln_group : fp32 [64]
 //
 // Reverse step for mini-batch i (G* = gradient w.r.t. the state after the update, go = dL/dOut):
@@ -38,7 +38,7 @@
 //   E5   gZ1in^T = gX2^T gelu'(Z1^T) + R^T S^T;  G_b1 += row sums
 //   G13  dK += gZ1in W1^T       G14 G_W2 += X2^T gZ2in     G15 G_W1^T += gZ1in^T K
 //
-// What bounds it: one chain of 14 MMA phases and as many epilogues on two warps per scheduler (128 streams: tensor pipe
+// What bounds it: one chain of 12 MMA phases and as many epilogues on two warps per scheduler (128 streams: tensor pipe
 // 15 %, issue slots 30 %, DRAM 38 %; the warps wait for tensor memory, the MMAs and, half a warp per issue, for
 // instructions).  The epilogues run on packed fp32 pairs and take column sums from registers.  Measured per mini-batch, 128
 // streams of 128: 25.2 -> 21.6 us in groups of 8, 23.6 in groups of 4 (64 mini-batches in groups of 8: 25.1 -> 23.5 by the
