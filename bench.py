@@ -55,8 +55,8 @@ FWD_U, BWD_U = 7, 22                  # algorithmic GEMM units: forward; backwar
 STATE_BYTES = 132352                  # fp32 W1 + b1 + W2 + b2 of one (b,h)
 # DRAM bytes per (stream, mini-batch) of the one-CTA backward from an ncu capture of the `prof` workload
 # (dram__bytes_read.sum + dram__bytes_write.sum over 128 streams x 16 mini-batches); the traffic grows in
-# proportion to the number of (stream, mini-batch) pairs, so a full-size launch is scaled from it.  Not for the cluster
-# kernels: their small captures stay in L2.
+# proportion to the number of (stream, mini-batch) pairs, so a full-size launch is scaled from it.  The cluster kernels
+# ask for the same scratch bytes, but have no capture of their own that does not stay in L2.
 NCU_BWD_DRAM_BYTES_PER_MB = (583522304 + 587919104) / 2048
 # Scratch bytes the backward asks for per (stream, mini-batch): the recompute writes seven [256][64] bf16 images
 # (X2, Z1, dl/dZ1, gelu'(Z1_bar), X2_bar, W1^T, W2), three [64][64] bf16 tiles and two fp32[64] vectors; the sweep
@@ -414,7 +414,7 @@ def run_ours(args, rank, world, local_rank):
     both_tf = (fwd_flop + bwd_flop) / ((fwd_ms + bwd_ms) * 1e-3) / 1e12
     n = -(-NC // cgs)
     remat_bytes = Bl * Hl * (2 * n * STATE_BYTES + NC * (SCRATCH_WRITE_PER_MB + SCRATCH_READ_PER_MB))
-    dram_bwd = NCU_BWD_DRAM_BYTES_PER_MB * Bl * Hl * NC if cl_used == 1 else None
+    dram_bwd = NCU_BWD_DRAM_BYTES_PER_MB * Bl * Hl * NC
     bwd_kernel = "ttt_bwd_kernel" if cl_used == 1 else f"ttt_bwd_cluster_kernel<{cl_used}>"
     res = {
         "metric": "ttt_mlp_fwd_bwd_tokens_per_s", "value": tokens_per_step / (ms_per_step * 1e-3),
@@ -441,13 +441,13 @@ def run_ours(args, rank, world, local_rank):
                           "hbm_gbs_achieved": remat_bytes / ((fwd_ms + bwd_ms) * 1e-3) / 1e9,
                           "frac_of_hbm_peak": remat_bytes / ((fwd_ms + bwd_ms) * 1e-3) / 1e9 / pk["hbm_gbs"],
                           "dram_bytes_measured_bwd": dram_bwd,
-                          "dram_gbs_measured_bwd": dram_bwd and dram_bwd / (bwd_ms * 1e-3) / 1e9},
+                          "dram_gbs_measured_bwd": dram_bwd / (bwd_ms * 1e-3) / 1e9},
         "roofline": {"kernel": bwd_kernel, "bound": "tensor", "achieved": bwd_tf, "peak": peak_tf,
                      "unit": "TFLOP/s", "frac": bwd_tf / peak_tf,
                      "frac_of_burst": bwd_tf / burst, "frac_of_sustained": bwd_tf / sustained,
                      "traffic": dram_bwd,
-                     "traffic_note": "bytes per launch of the one-CTA kernel, scaled from an ncu capture of a smaller "
-                                     "launch by (streams x mini-batches); null for the cluster kernels",
+                     "traffic_note": "bytes per launch, scaled from an ncu capture of a smaller launch of the one-CTA "
+                                     "kernel by (streams x mini-batches); an estimate where a cluster kernel runs",
                      "peak_source": f"{pk_src}, " + ("burst cuBLAS bf16 (timed region under 1 s at full clock)" if use_burst
                                                      else "sustained cuBLAS bf16 (clock below maximum or a long region)")},
         "e2e": {"value": tokens_per_step / (e2e_ms * 1e-3), "unit": "tokens/s", "ms_per_step": e2e_ms,
