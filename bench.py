@@ -255,7 +255,8 @@ def run_ours(args, rank, world, local_rank):
         step = DeviceStep(host, cgs, dev, cluster)
     Bl, Hl = b1 - b0, h1 - h0
     lib = _lib.lib()
-    cl_fwd, cl_used = (lib.ttt_b200_launch_cluster(Bl * Hl, (cluster or 0) << 8, backward) for backward in (0, 1))
+    cl_fwd = lib.ttt_b200_launch_cluster(Bl * Hl, (cluster or 0) << 8, 0)
+    cl_used = lib.ttt_b200_backward_ctas(Bl * Hl, NC, cgs, (cluster or 0) << 8)
 
     sampler = ClockSampler(local_rank)
     # warm-up happens inside timed_steps; the sampler is started just before so that most of its samples
@@ -415,7 +416,8 @@ def run_ours(args, rank, world, local_rank):
     n = -(-NC // cgs)
     remat_bytes = Bl * Hl * (2 * n * STATE_BYTES + NC * (SCRATCH_WRITE_PER_MB + SCRATCH_READ_PER_MB))
     dram_bwd = NCU_BWD_DRAM_BYTES_PER_MB * Bl * Hl * NC
-    bwd_kernel = "ttt_bwd_kernel" if cl_used == 1 else f"ttt_bwd_cluster_kernel<{cl_used}>"
+    bwd_kernel = "ttt_bwd_kernel" if cl_used == 1 else \
+        "ttt_bwd_pair_kernel" if cl_used == 2 and 1 < cgs < NC else f"ttt_bwd_cluster_kernel<{cl_used}>"
     res = {
         "metric": "ttt_mlp_fwd_bwd_tokens_per_s", "value": tokens_per_step / (ms_per_step * 1e-3),
         "unit": "tokens/s", "n_gpus": world, "steps": K, "warmup": W, "ms_per_step": ms_per_step,

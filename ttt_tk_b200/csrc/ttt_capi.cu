@@ -19,6 +19,8 @@ int ttt_launch_forward(const ttt_b200_fwd_args* a, cudaStream_t stream, uint32_t
                        int drop_load);
 int ttt_launch_backward(const ttt_b200_bwd_args* a, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
                         int drop_load);
+int ttt_launch_backward_pair(const ttt_b200_bwd_args* a, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
+                             int drop_load);
 int ttt_launch_backward_cluster(const ttt_b200_bwd_args* a, int cluster, cudaStream_t stream, uint32_t* status,
                                 uint64_t limit_ns, int drop_load);
 int ttt_launch_linear_forward(const ttt_b200_linear_fwd_args* a, cudaStream_t stream, uint32_t* status,
@@ -92,15 +94,32 @@ int capacity(int cluster, bool backward) {
 // streams than SMs the idle SMs can only help by taking a share of every stream's hidden units, and only while all
 // streams are resident at once.  Four CTAs per stream win whenever the device runs that many clusters of four (32 streams
 // of 128 mini-batches in groups of 4 on a B200: forward 4.3 against 4.6 us per mini-batch with one CTA, backward 14.0
-// against 22.7).  Where only clusters of two fit (34 to 74 streams), the forward runs one CTA, whose output pass runs
-// beside the chain in two groups of warps (4.6 us per mini-batch against 5.8 with two CTAs), and the backward two (48 / 60
-// / 74 streams: 19.0 / 20.1 / 21.0 us per mini-batch against 22.8 / 22.9 / 23.1 with one).  Beyond, one.
+// against 22.7; of the backward's longer calls: backward_ctas).  Where only clusters of two fit (34 to 74 streams), the
+// forward runs one CTA, whose output pass runs beside the chain in two groups of warps (4.6 us per mini-batch against 5.8
+// with two CTAs), and the backward two (60 streams in groups of 4: 14.3 us per mini-batch against 22.9 with one).  Beyond, one.
 static int ttt_launch_cluster(int streams, uint32_t flags, bool backward, int* cluster) {
   if (int rc = asked_cluster(flags, cluster)) return rc;
   if (*cluster != 0) return TTT_B200_OK;
   if (streams <= capacity(4, backward)) *cluster = 4;
   else if (backward && streams <= capacity(2, backward)) *cluster = 2;
   else *cluster = 1;
+  return TTT_B200_OK;
+}
+
+// A backward with two CTAs per stream gives them the recompute and the sweep (ttt_bwd_pair_sm100.cu) where there is
+// something to do side by side: groups of several mini-batches, and more than one of them.  Else each takes half of the
+// hidden units: a single group is within 4 % either way, groups of one mini-batch (one scratch slot, so that the two CTAs
+// take turns) 26 us per mini-batch against 28.
+static bool runs_pair(int ctas, int NC, int cgs) { return ctas == 2 && cgs > 1 && NC > cgs; }
+
+// CTAs per stream of a backward.  Where four would fit, two are faster once a call has four groups of four mini-batches to
+// pipeline: the first group's recompute runs alone, and a group that has few slots to spare ends with a wait for the last of
+// the next (32 streams, pair against four CTAs per mini-batch: 128 mini-batches in groups of 16 10.5 against 13.2 us, 32 in
+// groups of 8 12.2 / 13.7, 16 in groups of 4 14.2 / 14.4, 12 in groups of 4 14.8 / 14.6, 12 in groups of 3 16.6 / 14.9).
+static int backward_ctas(int streams, int NC, int cgs, uint32_t flags, int* ctas) {
+  if (int rc = ttt_launch_cluster(streams, flags, true, ctas)) return rc;
+  int asked = 0;
+  if (asked_cluster(flags, &asked) == TTT_B200_OK && asked == 0 && *ctas == 4 && cgs >= 4 && NC >= 4 * cgs) *ctas = 2;
   return TTT_B200_OK;
 }
 
@@ -297,12 +316,14 @@ extern "C" int ttt_b200_backward(const ttt_b200_bwd_args* a, void* stream_) {
   uint32_t* status = nullptr;
   if (int rc = pre_launch(&status)) return rc;
   int cluster = 1;
-  if (int rc = ttt_launch_cluster(a->B * a->H, a->flags, true, &cluster)) return rc;
+  if (int rc = backward_ctas(a->B * a->H, a->NC, a->checkpoint_group_size, a->flags, &cluster)) return rc;
   // the hook drops the recompute inputs of the last group's second mini-batch (its only one if it has one)
   const int last0 = (a->num_checkpoints - 1) * a->checkpoint_group_size;
   const int drop = (a->flags & TTT_B200_FLAG_TEST_LOST_LOAD) ? (last0 + 1 < a->NC ? last0 + 1 : last0) : -1;
   if (int rc = cluster == 1 ? ttt_launch_backward(a, stream, status, wait_limit_ns(), drop)
-                            : ttt_launch_backward_cluster(a, cluster, stream, status, wait_limit_ns(), drop))
+               : runs_pair(cluster, a->NC, a->checkpoint_group_size)
+                   ? ttt_launch_backward_pair(a, stream, status, wait_limit_ns(), drop)
+                   : ttt_launch_backward_cluster(a, cluster, stream, status, wait_limit_ns(), drop))
     return rc;
   if (a->flags & TTT_B200_FLAG_SYNC) return ttt_check_status(stream);
   return TTT_B200_OK;
@@ -330,6 +351,12 @@ extern "C" int ttt_b200_pick_cluster(int streams, int backward) {
   if (c != 0) return c;
   if (streams <= capacity(4, backward != 0)) return 4;
   return !backward && streams <= capacity(2, false) ? 2 : 1;
+}
+
+extern "C" int ttt_b200_backward_ctas(int streams, int NC, int checkpoint_group_size, uint32_t flags) {
+  int c = 0;
+  if (streams < 1 || NC < 1 || checkpoint_group_size < 1) return -1;
+  return backward_ctas(streams, NC, checkpoint_group_size, flags, &c) == TTT_B200_OK ? c : -1;
 }
 
 extern "C" int ttt_b200_launch_cluster(int streams, uint32_t flags, int backward) {

@@ -98,6 +98,19 @@ __device__ __forceinline__ uint4 pack_chunk(const float* v) {
 __device__ __forceinline__ void st_chunk(uint8_t* tile, uint32_t row, uint32_t chunk, const float* v) {
   *reinterpret_cast<uint4*>(tile + sw128_off(row, chunk)) = pack_chunk(v);
 }
+// the four 16-byte chunks of 32 fp32 accumulator columns as bf16, to row `row` of a swizzled tile
+__device__ __forceinline__ void st_cols32(uint8_t* tile, int row, int half, const uint32_t (&v)[32]) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint4 w;
+    w.x = pack_bf16(__uint_as_float(v[c * 8 + 0]), __uint_as_float(v[c * 8 + 1]));
+    w.y = pack_bf16(__uint_as_float(v[c * 8 + 2]), __uint_as_float(v[c * 8 + 3]));
+    w.z = pack_bf16(__uint_as_float(v[c * 8 + 4]), __uint_as_float(v[c * 8 + 5]));
+    w.w = pack_bf16(__uint_as_float(v[c * 8 + 6]), __uint_as_float(v[c * 8 + 7]));
+    *reinterpret_cast<uint4*>(tile + sw128_off(row, half * 4 + c)) = w;
+  }
+}
+
 // the raw 16 bytes of a chunk: requested between a tensor-memory load and its wait, unpacked after
 __device__ __forceinline__ uint4 ld_chunk_raw(const uint8_t* tile, uint32_t row, uint32_t chunk) {
   return *reinterpret_cast<const uint4*>(tile + sw128_off(row, chunk));

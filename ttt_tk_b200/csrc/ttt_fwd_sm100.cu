@@ -134,19 +134,6 @@ struct FwdParams {
   uint64_t wait_limit_ns;
 };
 
-// the four 16-byte chunks of 32 fp32 accumulator columns as bf16, to row `row` of a swizzled tile
-__device__ __forceinline__ void st_cols32(uint8_t* tile, int row, int half, const uint32_t (&v)[32]) {
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    uint4 w;
-    w.x = pack_bf16(__uint_as_float(v[c * 8 + 0]), __uint_as_float(v[c * 8 + 1]));
-    w.y = pack_bf16(__uint_as_float(v[c * 8 + 2]), __uint_as_float(v[c * 8 + 3]));
-    w.z = pack_bf16(__uint_as_float(v[c * 8 + 4]), __uint_as_float(v[c * 8 + 5]));
-    w.w = pack_bf16(__uint_as_float(v[c * 8 + 6]), __uint_as_float(v[c * 8 + 7]));
-    *reinterpret_cast<uint4*>(tile + sw128_off(row, half * 4 + c)) = w;
-  }
-}
-
 // 32 fp32 accumulator columns as bf16 pairs to 16 columns of tensor memory (an A operand of the MMAs)
 __device__ __forceinline__ void st_cols32_tmem(uint32_t taddr, const uint32_t (&v)[32]) {
   uint32_t w[16];
