@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("B,H,NC,cgs", [(1, 1, 4, 2), (1, 3, 5, 2), (1, 1, 10, 3), (2, 1, 13, 4), (1, 2, 16, 4), (3, 1, 23, 9),
-                                        (1, 1, 36, 16), (1, 2, 72, 24)])
+                                        (1, 1, 36, 16), (1, 2, 72, 24), (1, 32, 64, 16)])
 @pytest.mark.parametrize("eta_scale", [0.1, 1.0])
 def test_pair_backward_matches_oracle(B, H, NC, cgs, eta_scale):
     d = inputs(B, H, NC, seed=NC, eta_scale=eta_scale)

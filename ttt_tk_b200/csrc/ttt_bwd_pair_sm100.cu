@@ -24,9 +24,10 @@
 //   MMA2  Z2 = X2 W2                          EPI5   X2b = gelu, gelu'
 //   LN    x_hat_fused, gZ2, U2 = -eta gZ2     MMA6   Z2b = X2b W2
 //   MMA3  R^T = W2 gZ2^T                      S4     gZ2b = LNbwd(go gamma; LN(Z2b + b2));  d_gamma, d_beta
-//   EPI3  gZ1 = R G', U1 = -eta gZ1, b1       G1     gX2b^T = W2 gZ2b^T
-//   MMA4  W1^T += U1^T K; W2 += X2^T U2       E1     gZ1b^T = gX2b^T gelu'(Z1b^T)
-//   EPI4  bf16 copy of the new W1^T           G7     dQ = go + gZ1b W1^T
+//   EPI3  gZ1 = R G'                          G1     gX2b^T = W2 gZ2b^T
+//   MMA4  W1^T += gZ1^T (-eta K), b1;         E1     gZ1b^T = gX2b^T gelu'(Z1b^T)
+//         W2 += X2^T U2                       G7     dQ = go + gZ1b W1^T
+//   EPI4  bf16 copy of the new W1^T
 // Tensor memory: W1^T | W2 (fp32) | chain accumulator | output accumulator, 128 columns each.
 //
 // Scratch.  Per mini-batch the recompute leaves, in the caller's `*_group` tensors, raw images of swizzled shared-memory
@@ -53,10 +54,11 @@
 // What bounds it: issue and the fp32 pipe in the epilogues of either role, then instruction fetch: both programs together
 // exceed the 128 KB instruction cache that the SMs of a TPC share, which is why the helper warps run tables in loops and
 // why two streams share a cluster of four.  Registers come next (104 a thread: E4 runs with E5's 32 in place).  Measured
-// per mini-batch: 60 streams in groups of 5 20.2 us with the hidden units split over two CTAs -> 13.6; 32 streams in
-// groups of 16 13.2 with four -> 10.0; 4 streams in groups of 4 14.0 with four -> 12.6, most of it the turn from group to
+// per mini-batch: 60 streams in groups of 5 20.2 us with the hidden units split over two CTAs -> 12.7; 32 streams in
+// groups of 16 13.2 with four -> 9.4; 4 streams in groups of 4 14.0 with four -> 12.0, most of it the turn from group to
 // group (one slot to spare).  Steps on the way, at 60 streams: 21.6 with helpers written out and 860 bytes of spills, 19.3
-// with rolled MMA issue, 16.2 with tables, 14.4 with two streams to a cluster, 13.6 with a branch per role.
+// with rolled MMA issue, 16.2 with tables, 14.4 with two streams to a cluster, 13.6 with a branch per role, 13.0 with X2
+// loaded where Z1 was and products prepared before their waits, 12.7 with -eta in K (no U1) and checkpoints loaded ahead.
 //
 // Deviations from the reference kernel (see include/ttt_mlp_b200.h): outputs are overwritten,
 // not accumulated; `Out` is never touched.  Every wait is bounded.
@@ -85,7 +87,8 @@ constexpr uint32_t kBarQuad = 1;                                             // 
 // ---- shared memory: five hidden-major buffers and seven token tiles in either role, then vectors
 constexpr uint32_t OFF_BIG = 0;
 constexpr uint32_t OFF_T = 5 * BIG;
-constexpr uint32_t OFF_GAMMA = OFF_T + 7 * TILE;
+constexpr uint32_t OFF_NETA = OFF_T + 7 * TILE;        // recompute: bf16[64] -eta, a row of a swizzled tile (1024-byte aligned)
+constexpr uint32_t OFF_GAMMA = OFF_NETA + 128;
 constexpr uint32_t OFF_BETA = OFF_GAMMA + 256;
 constexpr uint32_t OFF_BAR = OFF_BETA + 256;
 constexpr uint32_t OFF_MISC = OFF_BAR + 512;
@@ -136,17 +139,17 @@ enum : int {
   RK, RK1, RV, RQ, RGO,
   // products: MMA1, MMA3, MMA4's W1 (one per 128-row block), MMA2, MMA4's W2, MMA5, MMA6, G1, G7
   RA, RA1, RZ, RW2UPD, RB, RBZ, RG1, RG7,
-  // epilogues done: a checkpoint's W1 and W2 in place, EPI1, LN, EPI3, EPI4, W2 copy, EPI5, S4, E1, dQ
-  E_LD1, E_LD2, E_1, E_2, E_3, E_W1, E_W2, E_O5, E_OS4, E_OE1, E_ODQ,
+  // epilogues done: a checkpoint in tensor memory, its bf16 W1 and W2 in place, EPI1, LN, EPI3, EPI4, W2 copy, EPI5, S4, E1, dQ
+  E_LDT, E_LD1, E_LD2, E_1, E_2, E_3, E_W1, E_W2, E_O5, E_OS4, E_OE1, E_ODQ,
   // images have left shared memory: Z1 and W1^T; X2, gZ1, gZ2; X2b and W2 (and a checkpoint's W2); gZ1b
   F_ZG, F_X, F_XB, F_XB2,
   kRecBars,
   // sweep: loads
   SW2 = kRecBars, SW1, SGZ1, SX2, SZ1, SGZ1B, SX2B, SK, SGZ2, SV, SXF, SQ,
-  // products: G4, G8, G10, G5, G11b and G2, G11a, G3, G15, G13
-  C1, C2, C10, C4, CB, C5, C3, C6, C7,
-  // epilogues done: E2 (G_W1), E2 (G_W2, dK), E3, E4's accumulators read and U2, gZ2in, dV, d_eta's addends, E5; gZ1 G_b1 summed
-  E_S1, E_S2, E_P, E_T, E_Z, E_V, E_DE, E_5, E_PART,
+  // products: G4 and G8, G10, G5 and G6, G11b and G2, G11a, G3, G15, G13
+  C2, C10, C4, CB, C5, C3, C6, C7,
+  // epilogues done: Z1 read, E2 (G_W1), E2 (G_W2, dK), E3, E4's accumulators read and U2, gZ2in, dV, d_eta's addends, E5; gZ1 G_b1 summed
+  E_D, E_S1, E_S2, E_P, E_T, E_Z, E_V, E_DE, E_5, E_PART,
   BGROUP,      // the scratch slots of a group are written (two CTAs per stream)
   BDRAIN,      // abort path only
   kBars
@@ -273,6 +276,15 @@ __device__ __forceinline__ int f16_colsum_col(const TokMap16& m, int lane) {
   return m.cq * 16 + ((lane >> 4) & 1) * 8 + m.l3 * 2 + ((lane >> 3) & 1);
 }
 
+// D[128 x 16] = A B^T with A in tensor memory (as in mma_hidden_ta) and B 16 rows of 64 bf16 from `b_smem` on (K-major)
+__device__ __forceinline__ void mma_rowsum_ta(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_smem, uint32_t lead) {
+  constexpr uint32_t idesc = umma_idesc_bf16(128, 16, false, false, false);
+  const uint32_t b0 = desc_lo(b_smem, 16);
+  mma_lead_ta<false>(tmem_d, tmem_a, b0, idesc, lead);
+#pragma unroll
+  for (int j = 1; j < 4; ++j) mma_lead_ta<true>(tmem_d, tmem_a + j * 8, b0 + j * (32u >> 4), idesc, lead);
+}
+
 // ---- across the two CTAs of a stream
 __device__ __forceinline__ void mbar_arrive_remote(uint64_t* bar, uint32_t rank) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa(smem_u32(bar), rank)) : "memory");
@@ -292,23 +304,23 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
 }
 __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
-enum : uint8_t { V_S2, V_C2, V_PART, V_C10, V_CB, V_C5, V_V, V_C3, V_C6, V_C7, V_COUNT };      // the sweep copies' events
-__constant__ const uint8_t kSweepEvent[V_COUNT] = {E_S2, C2, E_PART, C10, CB, C5, E_V, C3, C6, C7};
+enum : uint8_t { V_D, V_S2, V_C2, V_PART, V_C10, V_CB, V_C5, V_V, V_C3, V_C6, V_C7, V_COUNT };      // the sweep copies' events
+__constant__ const uint8_t kSweepEvent[V_COUNT] = {E_D, E_S2, C2, E_PART, C10, CB, C5, E_V, C3, C6, C7};
 constexpr int kSweepCopies = 19;
 __constant__ const CopyOp kSweepCopy[kSweepCopies] = {
-    {V_PART, K_LOAD, A_X2, SX2, R_GZ, 0, 0, 0, 0, 0, BIG, BIG},
-    {V_PART, K_LOAD, A_X2B, SX2B, R_S1, 1, 1, 0, 0, 0, BIG, BIG + TILE + 1280},
+    {V_D, K_LOAD, A_X2, SX2, R_Z, 0, 0, 0, 0, 0, BIG, BIG},
+    {V_PART, K_LOAD, A_X2B, SX2B, R_GZ, 1, 1, 0, 0, 0, BIG, BIG + TILE + 1280},
     {V_PART, K_LOAD, A_GZ2B, SX2B, R_NONE, 1, 1, 0, S_GZB, 0, TILE, 0},
     {V_PART, K_LOAD, A_RS, SX2B, R_NONE, 1, 1, 0, S_VEC, 0, 1024, 0},
     {V_PART, K_LOAD, A_CS, SX2B, R_NONE, 1, 1, 0, S_VEC + 1024, 0, 256, 0},
-    {V_C10, K_LOAD, A_GZ1B, SGZ1B, R_Z, 1, 1, 0, 0, 0, BIG, BIG},
+    {V_C10, K_LOAD, A_GZ1B, SGZ1B, R_S1, 1, 1, 0, 0, 0, BIG, BIG},
     {V_CB, K_TMA, M_Q, SQ, R_NONE, 1, 1, 0, S_Q, 0, TILE, TILE},
     {V_C5, K_LOAD, A_W1, SW1, R_A, 0, 0, 0, 0, 0, BIG, BIG},
     {V_CB, K_LOAD, A_Z1, SZ1, R_S2, 1, 1, 0, 0, 0, BIG, BIG},
     {V_C5, K_LOAD, A_GZ2, SGZ2, R_NONE, 1, 1, 0, S_GZ2, 0, TILE, TILE},
     {V_V, K_TMA, M_K, SK, R_NONE, 1, 1, 0, S_K, TILE, TILE, TILE + 128},
     {V_V, K_LOAD, A_ETA, SK, R_NONE, 1, 1, 0, S_ETA, 128, 128, 0},
-    {V_C3, K_LOAD, A_GZ1, SGZ1, R_Z, 1, 1, 0, 0, 0, BIG, BIG},
+    {V_C3, K_LOAD, A_GZ1, SGZ1, R_S1, 1, 1, 0, 0, 0, BIG, BIG},
     {V_C3, K_LOAD, A_XHF, SXF, R_NONE, 1, 1, 0, S_XF, 0, TILE, TILE + 512},
     {V_C3, K_LOAD, A_SIG, SXF, R_NONE, 1, 1, 0, S_SIG, 0, 256, 0},
     {V_C3, K_LOAD, A_S3, SXF, R_NONE, 1, 1, 0, S_SIG + 256, 0, 256, 0},
@@ -317,19 +329,19 @@ __constant__ const CopyOp kSweepCopy[kSweepCopies] = {
     {V_COUNT, K_NONE, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0}};
 constexpr int kSweepMmas = 13;
 __constant__ const MmaOp kSweepMma[kSweepMmas] = {
-    {E_S1, SK, C1, P_HID, R_S1, R_NONE, 0, 0, 0, S_K, TM_A},                  // G4
+    {E_S1, SK, kNo, P_HID, R_S1, R_NONE, 0, 0, 0, S_K, TM_A},                  // G4
     {SGZ1, kNo, C2, P_TOK, R_GZ, R_S1, 0, 0, 0, 0, TM_B},                     // G8
-    {E_P, SW2, kNo, P_TOK, R_Z, R_A, 0, 0, 0, 0, TM_A},                       // G6
-    {E_S2, SX2, C4, P_TOK, R_GZ, R_S2, 0, 0, 0, 0, TM_B + 64},                // G5
-    {SGZ2, kNo, C10, P_HID_MN, R_Z, R_NONE, 0, 0, 0, S_GZ2, TM_S2},           // G10
+    {E_S2, SX2, kNo, P_TOK, R_Z, R_S2, 0, 0, 0, 0, TM_B + 64},                // G5
+    {E_P, SW2, C4, P_TOK, R_S1, R_A, 0, 0, 0, 0, TM_A},                       // G6
+    {SGZ2, kNo, C10, P_HID_MN, R_S1, R_NONE, 0, 0, 0, S_GZ2, TM_S2},          // G10
     {E_T, kNo, kNo, P_HID, R_A, R_NONE, 0, 0, 0, S_GZ2, TM_A},                // G12
     {kNo, kNo, kNo, P_HID, R_S2, R_NONE, 0, 0, 0, S_Q, TM_B},                 // G11b
-    {SX2B, kNo, CB, P_HID_MN, R_S1, R_NONE, 1, 0, 0, S_GZB, TM_S2},           // G2 of the next step
+    {SX2B, kNo, CB, P_HID_MN, R_GZ, R_NONE, 1, 0, 0, S_GZB, TM_S2},           // G2 of the next step
     {E_Z, kNo, C5, P_HID_ACC, R_A, R_NONE, 0, 0, 0, S_XF, TM_B},              // G11a
-    {kNo, kNo, kNo, P_HID_MN, R_GZ, R_NONE, 0, 0, 0, S_XF, TM_S2},            // G14
-    {SGZ1B, SQ, C3, P_HID_MN, R_Z, R_NONE, 1, 0, 0, S_Q, TM_S1},              // G3 of the next step
-    {E_5, kNo, C6, P_HID_MN, R_S1, R_NONE, 0, 0, 0, S_K, TM_S1},              // G15
-    {SW1, kNo, C7, P_TOK, R_S1, R_A, 0, 0, 0, 0, TM_B + 64}};                 // G13
+    {kNo, kNo, kNo, P_HID_MN, R_Z, R_NONE, 0, 0, 0, S_XF, TM_S2},             // G14
+    {SGZ1B, SQ, C3, P_HID_MN, R_S1, R_NONE, 1, 0, 0, S_Q, TM_S1},             // G3 of the next step
+    {E_5, kNo, C6, P_HID_MN, R_GZ, R_NONE, 0, 0, 0, S_K, TM_S1},              // G15
+    {SW1, kNo, C7, P_TOK, R_GZ, R_A, 0, 0, 0, 0, TM_B + 64}};                 // G13
 
 // copies of the recompute: chain (loads of K, eta, V; images out) and output group (loads of Q, dL/dOut; images out)
 enum : uint8_t { Y_LD, Y_1, Y_2, Y_3, Y_W, Y_LOADS };      // events: checkpoint in place, then the group's epilogues in order
@@ -395,7 +407,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   if (tid == kEpi) {
     for (int i = 0; i < kBars; ++i)
-      mbar_init(&bars[i], i >= E_LD1 && i <= E_ODQ ? 8 : i >= E_S1 && i <= E_5 ? 16 : i == E_PART || i == BGROUP || i == BDRAIN ? 2 : 1);
+      mbar_init(&bars[i], i >= E_LDT && i <= E_ODQ ? 8 : i >= E_D && i <= E_5 ? 16 : i == E_PART || i == BGROUP || i == BDRAIN ? 2 : 1);
     fence_mbar_init();
     *abort_flag = 0;
     *never_flag = 0;
@@ -577,26 +589,57 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   // A group's warps meet at named barriers, so they leave the loop by a vote (true: left).  The sweep's never do: once the
   // abort flag is up their waits fail at once, and they run through what is left.
+  // A checkpoint into tensor memory, by the chain group: the first one, later ones while the output group is at its last
+  // products of the group before (which use the bf16 copies)
+  auto load_checkpoint = [&](int g) {
+    const long ck = long{sid} * nck + nck - 1 - g;
+    const float* W1g = p.W1c + ck * (64 * 256) + hrow8;
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+      uint32_t v[32];
+#pragma unroll
+      for (int q = 0; q < 32; ++q) v[q] = __float_as_uint(W1g[(half * 32 + q) * 256]);
+      tmem_st32(tmem + lane_base + TM_S1 + wg * 64 + half * 32, v);
+    }
+    if (g > 0) {      // MMA6 has waited for the last W2 copy
+      bounded(RBZ, (nrec - 1) & 1);
+      __syncwarp();
+      tc_fence_after_sync();
+    }
+    const float4* W2g = reinterpret_cast<const float4*>(p.W2c + ck * (256 * 64) + hrow8 * 64);
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+      uint32_t v[32];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float4 f = W2g[half * 8 + q];
+        v[4 * q] = __float_as_uint(f.x); v[4 * q + 1] = __float_as_uint(f.y);
+        v[4 * q + 2] = __float_as_uint(f.z); v[4 * q + 3] = __float_as_uint(f.w);
+      }
+      tmem_st32(tmem + lane_base + TM_S2 + wg * 64 + half * 32, v);
+    }
+    tmem_wait_st();
+    done(E_LDT);
+  };
+  auto copy_state = [&](uint32_t col, uint8_t* dst) {      // this thread's row as bf16
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+      uint32_t v[32];
+      tmem_ld32(tmem + lane_base + col + wg * 64 + half * 32, v);
+      tmem_wait_ld();
+      st_cols32(dst, hrow8, half, v);
+    }
+  };
   auto rec_chain = [&](int g) -> bool {
     const int gsz = size_of(g);
-    const long ck = long{sid} * nck + nck - 1 - g;
-    float b1v = p.b1c[ck * 256 + hrow8];
-    {   // checkpoint -> tensor memory (fp32) and shared memory (bf16)
-      const float* W1g = p.W1c + ck * (64 * 256) + hrow8;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t v[32];
-#pragma unroll
-        for (int q = 0; q < 32; ++q) v[q] = __float_as_uint(W1g[(half * 32 + q) * 256]);
-        tmem_st32(tmem + lane_base + TM_S1 + wg * 64 + half * 32, v);
-        st_cols32(rW1, hrow8, half, v);
-      }
-      tmem_wait_st();
-    }
+    float b1v = p.b1c[(long{sid} * nck + nck - 1 - g) * 256 + hrow8];
+    if (g == 0) load_checkpoint(0);
+    __syncwarp();
+    copy_state(TM_S1, rW1);
     done(E_LD1);
     for (int j = 0; j < gsz; ++j, ++nrec) {
       const int s = j & 1;
-      const uint8_t* sK = smem + R_K + s * TILE;
+      uint8_t* sK = smem + R_K + s * TILE;
       uint8_t* sV = smem + R_V;
       const __nv_bfloat16* eta = reinterpret_cast<const __nv_bfloat16*>(smem + R_ETA) + s * 64;
       wait(RK + s);
@@ -684,7 +727,6 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           x.a[q] = add2(gr.a[q], gr.b[q]);
         }
         frag_st_tile(tm8, smem + R_U2, gr);
-        reinterpret_cast<float*>(smem + R_CSC)[tm8.quad * 64 + frag_colsum_col(tm8, lane)] = frag_colsum(x.a, lane);
         if (tm8.colhalf == 0 && tm8.l3 == 0) {
           float* sig = reinterpret_cast<float*>(smem + R_SIG);      // 1/std, and sum(grad_x_hat_fused x_hat_fused)
           sig[tm8.r0] = rs0;
@@ -692,39 +734,36 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           sig[64 + tm8.r0] = a[1];
           sig[64 + tm8.r1] = b[1];
         }
+        done(E_2);
+        // under the product: column sums of U2, and -eta K over K, MMA4's operand (dl/dZ1 then is its other as it stands)
+        reinterpret_cast<float*>(smem + R_CSC)[tm8.quad * 64 + frag_colsum_col(tm8, lane)] = frag_colsum(x.a, lane);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          gr.a[q] = mul2(bf16x2_to_f32x2(kk[2 * q]), ne0);
+          gr.b[q] = mul2(bf16x2_to_f32x2(kk[2 * q + 1]), ne1);
+        }
+        frag_st_tile(tm8, sK, gr);
+        if (gtid < 32) reinterpret_cast<uint32_t*>(smem + OFF_NETA)[gtid] = reinterpret_cast<const uint32_t*>(eta)[gtid] ^ 0x80008000u;
       }
-      done(E_2);
 
-      // ---- EPI3: dl/dZ1 over Z1, U1 = -eta dl/dZ1 over R in tensor memory (the A operand of its MMA)
+      // ---- EPI3: dl/dZ1 over Z1 (its image) and over R in tensor memory (the A operand of its MMAs)
       wait(F_ZG);
       wait_mma(RA + wg);
       {
-        f32x2 bsum = 0ull;
         const uint32_t acc = tmem + lane_base + TM_A + wg * 64;
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-          uint32_t v[32], u[16];
+          uint32_t v[32], w[16];
           tmem_ld32(acc + half * 32, v);
           tmem_wait_ld();
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const uint4 ew = *reinterpret_cast<const uint4*>(eta + half * 32 + c * 8);     // one broadcast load
-            const uint32_t et[4] = {ew.x, ew.y, ew.z, ew.w};
-            uint32_t w[4];
+          for (int k = 0; k < 16; ++k)
+            w[k] = f32x2_to_bf16x2(mul2(bf16x2_to_f32x2(gp[half * 16 + k]), pk(v[2 * k], v[2 * k + 1])));
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              w[k] = f32x2_to_bf16x2(mul2(bf16x2_to_f32x2(gp[c * 4 + k]), pk(v[c * 8 + 2 * k], v[c * 8 + 2 * k + 1])));
-              const f32x2 t = mul2(bf16x2_to_f32x2(w[k]), bf16x2_to_f32x2(et[k] ^ 0x80008000u));
-              bsum = add2(bsum, t);
-              u[c * 4 + k] = f32x2_to_bf16x2(t);
-            }
-            *reinterpret_cast<uint4*>(rZG + sw128_off(hrow8, half * 4 + c)) = make_uint4(w[0], w[1], w[2], w[3]);
-          }
-          tmem_st16(acc + half * 16, u);
-#pragma unroll
-          for (int k = 0; k < 16; ++k) gp[k] = gp[16 + k];
+          for (int c = 0; c < 4; ++c)
+            *reinterpret_cast<uint4*>(rZG + sw128_off(hrow8, half * 4 + c)) = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+          tmem_st16(acc + half * 16, w);
         }
-        b1v += hsum(bsum);
         tmem_wait_st();
       }
       done(E_3);
@@ -732,41 +771,27 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // ---- EPI4: bf16 copy of the new W1, and b1, once the output group has used the last ones
       if (j > 0) wait(RG7);
       wait_mma(RA + wg);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t v[32];
-        tmem_ld32(tmem + lane_base + TM_S1 + wg * 64 + half * 32, v);
+      {
+        uint32_t v[8];
+        tmem_ld8(tmem + lane_base + TM_A + wg * 64 + 32, v);
         tmem_wait_ld();
-        st_cols32(rW1, hrow8, half, v);
+        b1v += __uint_as_float(v[0]);
       }
+      copy_state(TM_S1, rW1);
       rB1[hrow8] = b1v;
       done(E_W1);
       if (named_bar_or(kBarC, kGroup, *abort_flag != 0)) return true;
     }
+    if (g + 1 < nck) load_checkpoint(g + 1);
     wait(RG7);
     return false;
   };
 
   auto rec_out = [&](int g) -> bool {
     const int gsz = size_of(g);
-    const long ck = long{sid} * nck + nck - 1 - g;
-    {   // checkpoint -> tensor memory (fp32) and shared memory (bf16)
-      const float4* W2g = reinterpret_cast<const float4*>(p.W2c + ck * (256 * 64) + hrow8 * 64);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t v[32];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const float4 f = W2g[half * 8 + q];
-          v[4 * q] = __float_as_uint(f.x); v[4 * q + 1] = __float_as_uint(f.y);
-          v[4 * q + 2] = __float_as_uint(f.z); v[4 * q + 3] = __float_as_uint(f.w);
-        }
-        tmem_st32(tmem + lane_base + TM_S2 + wg * 64 + half * 32, v);
-        st_cols32(rW2, hrow8, half, v);
-      }
-      if (gtid < 64) rB2[gtid] = p.b2c[ck * 64 + gtid];
-      tmem_wait_st();
-    }
+    wait_mma(E_LDT);
+    copy_state(TM_S2, rW2);
+    if (gtid < 64) rB2[gtid] = p.b2c[(long{sid} * nck + nck - 1 - g) * 64 + gtid];
     done(E_LD2);
     auto finish_dq = [&]() {      // dQ = go + gZ1b W1^T, over the dL/dOut tile
       wait_mma(RG7);
@@ -786,13 +811,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // ---- bf16 copy of the new W2; b2
       if (j == 0) wait(F_XB);                   // the checkpoint's image has left
       wait_mma(RW2UPD);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t v[32];
-        tmem_ld32(tmem + lane_base + TM_S2 + wg * 64 + half * 32, v);
-        tmem_wait_ld();
-        st_cols32(rW2, hrow8, half, v);
-      }
+      copy_state(TM_S2, rW2);
       if (gtid < 64) rB2[gtid] += quad_sum(reinterpret_cast<const float*>(smem + R_CSC), gtid);
       done(E_W2);
       if (j > 0) finish_dq();
@@ -958,7 +977,10 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (!seen(E_3)) return;
 #pragma unroll 1
       for (int blk = 0; blk < 2; ++blk) {
+        // W1^T += gZ1^T (-eta K); b1's sums gZ1^T (-eta) to 16 columns behind gZ1, of which the first is used (the others
+        // multiply what lies behind -eta)
         mma_hidden_ta<true, true>(tmem + TM_S1 + blk * 64, tmem + TM_A + blk * 64, smem_u32(sK), lead);
+        mma_rowsum_ta(tmem + TM_A + blk * 64 + 32, tmem + TM_A + blk * 64, smem_u32(smem + OFF_NETA), lead);
         commit(RA + blk);
       }
       hidden(T{}, T{}, tmem + TM_S2, rX2, smem + R_U2);
@@ -1092,14 +1114,14 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   float* sVec = reinterpret_cast<float*>(smem + S_VEC);
   float* sCS = reinterpret_cast<float*>(smem + S_CS);
   // hidden-major buffers: buffer 0 holds W2 then W1; the other four, as offsets, by what they hold first in a step:
-  //   gz  gZ1, X2             -> the next step's G_W1 snapshot
-  //   z   Z1, P, gZ1b(i - 1)  -> gZ1
-  //   s1  G_W1 snapshot, X2b(i - 1), gZ1in -> G_W2 snapshot
-  //   s2  G_W2 snapshot       -> Z1
+  //   gz  gZ1, X2b(i - 1), gZ1in                 -> the next step's G_W2 snapshot
+  //   z   Z1, X2                                 -> G_W1 snapshot
+  //   s1  G_W1 snapshot, P, gZ1b(i - 1)          -> gZ1
+  //   s2  G_W2 snapshot                          -> Z1
   uint32_t o_gz = BIG, o_z = 2 * BIG, o_s1 = 3 * BIG, o_s2 = 4 * BIG;
   auto turn = [&]() {
     const uint32_t g = o_gz, z = o_z, s1 = o_s1, s2 = o_s2;
-    o_gz = z; o_z = s2; o_s1 = g; o_s2 = s1;
+    o_z = s2; o_gz = s1; o_s1 = z; o_s2 = g;
   };
 
   auto sweep_epi = [&](int g) {
@@ -1155,51 +1177,64 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     };
     for (int j = gsz - 1; j >= 0; --j) {
+      const bool first = j == gsz - 1;
       const int par = nsw & 1;
       const __nv_bfloat16* eta = reinterpret_cast<const __nv_bfloat16*>(smem + S_ETA) + par * 64;
-      // ---- gelu'(Z1) and gelu''(Z1) in f16, under the last products of the step before
+      // ---- gelu'(Z1) and gelu''(Z1) in f16: half of them under the last products of the step before, half under G4 and G8
       uint32_t sS[16], sG[16];
+      uint4 zr[4];
       wait(SZ1);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint4 zr = ld_chunk_raw(smem + o_z, hrow, ch * 4 + q);
-        const uint32_t zw[4] = {zr.x, zr.y, zr.z, zr.w};
+      for (int q = 0; q < 4; ++q) zr[q] = ld_chunk_raw(smem + o_z, hrow, ch * 4 + q);
+      __syncwarp();
+      if (lane == 0) arrive(E_D);
+      auto derivatives = [&](int q0) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) gelu_grad_h2(zw[k], sG[q * 4 + k], sS[q * 4 + k]);
-      }
+        for (int q = q0; q < q0 + 2; ++q) {
+          const uint32_t zw[4] = {zr[q].x, zr[q].y, zr[q].z, zr[q].w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) gelu_grad_h2(zw[k], sG[q * 4 + k], sS[q * 4 + k]);
+        }
+      };
+      derivatives(0);
       // ---- E2: bf16 snapshots of the gradient state
-      if (j == gsz - 1) wait(SX2B);
+      if (first) wait(SX2B);
       wait_mma(C6);
       {
         if (ch == 0) sGb1[hrow] += sVec[hrow];
-        if (tid < 64) sGb2[tid] += (j < gsz - 1 ? quad_sum(sCS, tid) : 0.f) + sVec[256 + tid];
+        if (tid < 64) sGb2[tid] += (first ? 0.f : quad_sum(sCS, tid)) + sVec[256 + tid];
         snapshot(tmem + TM_S1 + hl, smem + o_s1);
       }
       done(E_S1);
       wait_mma(C7);
       snapshot(tmem + TM_S2 + hl, smem + o_s2);
-      if (j < gsz - 1) finish_dk();
+      if (!first) finish_dk();
       done(E_S2);
+      derivatives(2);
 
-      // ---- E3: A1, P = A1 gelu'(Z1) over Z1; S = A1 gelu''(Z1) in the place of gelu''(Z1)
+      // ---- E3: A1, P = A1 gelu'(Z1) over the G_W1 snapshot, which G4 and G8 have read; S = A1 gelu''(Z1) in the place of
+      // gelu''(Z1)
       wait(SK);
-      wait_mma(C1);
+      wait_mma(C2);
       {
         const f32x2 gb = pk1(sGb1[hrow]);
+        uint32_t v[2][16];
+        tmem_ld16(tmem + TM_A + hl, v[0]);
+        tmem_ld16(tmem + TM_A + hl + 16, v[1]);
+        tmem_wait_ld();
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {   // 8 columns per pass
-          uint32_t v[8], pw[4];
-          tmem_ld8(tmem + TM_A + hl + q * 8, v);
+        for (int q = 0; q < 4; ++q) {
+          uint32_t pw[4];
           const uint4 ew = *reinterpret_cast<const uint4*>(eta + ch * 32 + q * 8);     // one broadcast load
-          tmem_wait_ld();
           const uint32_t et[4] = {ew.x, ew.y, ew.z, ew.w};
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            const f32x2 a1 = mul2(bf16x2_to_f32x2(et[k] ^ 0x80008000u), add2(pk(v[2 * k], v[2 * k + 1]), gb));
+            const uint32_t* w = v[q >> 1] + (q & 1) * 8 + 2 * k;
+            const f32x2 a1 = mul2(bf16x2_to_f32x2(et[k] ^ 0x80008000u), add2(pk(w[0], w[1]), gb));
             pw[k] = f32x2_to_bf16x2(mul2(a1, f16x2_to_f32x2(sG[q * 4 + k])));
             sS[q * 4 + k] = f32x2_to_bf16x2(mul2(a1, f16x2_to_f32x2(sS[q * 4 + k])));
           }
-          *reinterpret_cast<uint4*>(smem + o_z + sw128_off(hrow, ch * 4 + q)) = make_uint4(pw[0], pw[1], pw[2], pw[3]);
+          *reinterpret_cast<uint4*>(smem + o_s1 + sw128_off(hrow, ch * 4 + q)) = make_uint4(pw[0], pw[1], pw[2], pw[3]);
         }
       }
       done(E_P);
@@ -1387,7 +1422,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             bs = add2(bs, t);
             o[k] = f32x2_to_bf16x2(t);
           }
-          *reinterpret_cast<uint4*>(smem + o_s1 + sw128_off(hrow, ch * 4 + q)) = make_uint4(o[0], o[1], o[2], o[3]);
+          *reinterpret_cast<uint4*>(smem + o_gz + sw128_off(hrow, ch * 4 + q)) = make_uint4(o[0], o[1], o[2], o[3]);
         }
         if (j > 0) wait(SX2B);      // the next step's row sums of gZ1b, which this adds to
         if (ch == 0) sGb1[hrow] += hsum(bs);
@@ -1415,7 +1450,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       tmem_wait_ld();
       // whole lines through a staging area in the two buffers that hold nothing an MMA or a copy still reads
       store_rows_own(p.gW2 + long{sid} * (256 * 64) + (hrow - lane) * 64 + ch * 32, v,
-                     smem + (warp < 8 ? o_gz + warp * 4096 : o_z + (warp - 8) * 4096), lane);
+                     smem + (warp < 8 ? o_s1 + warp * 4096 : o_z + (warp - 8) * 4096), lane);
       if (ch == 0) p.gb1[long{sid} * 256 + hrow] = sGb1[hrow];
       if (tid < 64) p.gb2[long{sid} * 64 + tid] = sGb2[tid];
     }
@@ -1423,23 +1458,40 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   auto role = [&](uint32_t r) { return r == R_GZ ? o_gz : r == R_Z ? o_z : r == R_S1 ? o_s1 : r == R_S2 ? o_s2 : 0u; };
   // One product.  All its MMAs are groups of four: a hidden-major product two (one per 128-row block), a token-major one four.
-  auto product = [&](uint32_t kind, uint32_t d, uint32_t a_off, uint32_t b_off) {
+  // What the loop needs is prepared before the product's barriers are waited for; it is the same in all lanes, and known to
+  // be through the shuffle, so that the issue runs on uniform registers.
+  struct Product {
+    uint32_t a, b, d, idesc, as, bs, da, db, dd, acc, n, tok;
+  };
+  auto uniform = [&](uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); };
+  auto prepare = [&](uint32_t kind, uint32_t d, uint32_t a_off, uint32_t b_off) {
+    Product q;
     const bool tok = kind == P_TOK, mn = kind >= P_HID_MN;
     const uint32_t base = smem_u32(smem);
-    const uint32_t idesc = tok ? umma_idesc_bf16(64, 64, true, true, false)
-                               : mn ? umma_idesc_bf16(128, 64, false, true, false) : umma_idesc_bf16(128, 64, false, false, false);
-    uint32_t a = desc_lo(base + a_off, tok ? BIG : 16), b = desc_lo(base + b_off, tok ? BIG : mn ? 8192 : 16);
-    const uint32_t as = tok ? 2048u >> 4 : 2u, bs = mn ? 2048u >> 4 : 2u;
-    const uint32_t da = tok ? 4 * as : 16384u >> 4, db = tok ? 4 * bs : 0u, dd = tok ? 0u : 64u;
-    uint32_t acc = kind == P_HID_ACC || kind == P_HID_MN ? 1u : 0u;
+    q.idesc = uniform(tok ? umma_idesc_bf16(64, 64, true, true, false)
+                          : mn ? umma_idesc_bf16(128, 64, false, true, false) : umma_idesc_bf16(128, 64, false, false, false));
+    q.a = uniform(desc_lo(base + a_off, tok ? BIG : 16));
+    q.b = uniform(desc_lo(base + b_off, tok ? BIG : mn ? 8192 : 16));
+    q.d = uniform(tmem + d);
+    q.as = uniform(tok ? 2048u >> 4 : 2u);
+    q.bs = uniform(mn ? 2048u >> 4 : 2u);
+    q.da = uniform(tok ? 4 * (2048u >> 4) : 16384u >> 4);
+    q.db = uniform(tok ? 4 * (2048u >> 4) : 0u);
+    q.dd = uniform(tok ? 0u : 64u);
+    q.acc = uniform(kind == P_HID_ACC || kind == P_HID_MN ? 1u : 0u);
+    q.n = uniform(tok ? 4u : 2u);
+    q.tok = uniform(tok ? 1u : 0u);
+    return q;
+  };
+  auto issue = [&](Product q) {
 #pragma unroll 1
-    for (int k = tok ? 4 : 2; k > 0; --k) {
-      mma_lead_rt(tmem + d, a, b, idesc, acc, lead);
-      mma_lead_rt(tmem + d, a + as, b + bs, idesc, 1u, lead);
-      mma_lead_rt(tmem + d, a + 2 * as, b + 2 * bs, idesc, 1u, lead);
-      mma_lead_rt(tmem + d, a + 3 * as, b + 3 * bs, idesc, 1u, lead);
-      a += da; b += db; d += dd;
-      acc |= tok ? 1u : 0u;
+    for (uint32_t k = q.n; k > 0; --k) {
+      mma_lead_rt(q.d, q.a, q.b, q.idesc, q.acc, lead);
+      mma_lead_rt(q.d, q.a + q.as, q.b + q.bs, q.idesc, 1u, lead);
+      mma_lead_rt(q.d, q.a + 2 * q.as, q.b + 2 * q.bs, q.idesc, 1u, lead);
+      mma_lead_rt(q.d, q.a + 3 * q.as, q.b + 3 * q.bs, q.idesc, 1u, lead);
+      q.a += q.da; q.b += q.db; q.d += q.dd;
+      q.acc |= q.tok;
     }
   };
   auto sweep_issue = [&](int g) {
@@ -1447,18 +1499,18 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (!seen(E_5) || !seen(SX2B) || !seen(SGZ1B) || !seen(SQ)) return;
 #pragma unroll 1
     for (int k = 0; k < 2; ++k)       // G2, G3 of the group's first step
-      product(P_HID_MN, k ? TM_S1 : TM_S2, k ? o_s2 : o_s1, k ? S_Q : S_GZB);
+      issue(prepare(P_HID_MN, k ? TM_S1 : TM_S2, k ? o_s2 : o_s1, k ? S_Q : S_GZB));
     commit(C6);
     commit(C7);
     for (int j = gsz - 1; j >= 0; --j) {
 #pragma unroll 1
       for (int o = 0; o < kSweepMmas; ++o) {
         const MmaOp op = kSweepMma[o];
-        const uint32_t a = role(op.ra) + op.a, b = role(op.rb) + op.b + (op.b == S_K ? (nsw & 1) * TILE : 0u);
+        const Product q = prepare(op.kind, op.d, role(op.ra) + op.a, role(op.rb) + op.b + (op.b == S_K ? (nsw & 1) * TILE : 0u));
         if (!op.only_next || j > 0) {
           if (op.w0 != kNo && !seen(op.w0)) return;
           if (op.w1 != kNo && !seen(op.w1)) return;
-          product(op.kind, op.d, a, b);
+          issue(q);
         }
         if (op.commit != kNo) commit(op.commit);
       }
@@ -1510,8 +1562,6 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       turn();
       ++nsw;
-      // everything of this slot has been read (W1, the last, by G13)
-      if (lane == 0) st_release_cluster(mapa(smem_u32(freed), peer), static_cast<uint32_t>(nsw));
     }
     if (!seen_all(E_S2)) return;
     if (lane == 0) {
@@ -1525,6 +1575,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // d_eta; its fourth term, gZ1 G_b1, is summed over half of the hidden units by each of two warps: lane l takes the token pair (2 l, 2 l + 1)
   auto sweep_part = [&](int g, int half) {
     const int gsz = size_of(g);
+    if (half == 0 && !seen(C7)) return;      // the one that goes with the group's first products
     for (int j = gsz - 1; j >= 0; --j) {
       if (!seen(E_S1) || !seen(SGZ1)) return;
       const uint8_t* bg = smem + o_gz + half * 16384 + (lane & 3) * 4;      // (128 rows: the swizzle's phase is the same)
@@ -1557,6 +1608,10 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           __float2bfloat16(-(quad_sum(reinterpret_cast<const float*>(smem + S_X1), t) + (part[t] + part[64 + t])));
       turn();
       ++nsw;
+      if (half == 0) {      // everything of this step's slot has been read (W1, the last, by G13): the recompute may have it
+        if (!seen(C7)) return;
+        if (lane == 0) st_release_cluster(mapa(smem_u32(freed), peer), static_cast<uint32_t>(nsw));
+      }
     }
   };
 
