@@ -36,5 +36,5 @@ def test_every_stream_count_matches_the_one_cta_kernel(H):
 def test_calls_that_pipeline_groups_take_two_ctas():
     f = _lib.lib().ttt_b200_backward_ctas
     c4, c2 = (_lib.lib().ttt_b200_cluster_capacity(c, 1) for c in (4, 2))
-    assert [f(c4, 16, 4, 0), f(c4, 15, 4, 0), f(c4, 64, 3, 0), f(c4 + 1, 1, 1, 0), f(c2 + 1, 64, 8, 0)] == [2, 4, 4, 2, 1]
+    assert [f(c4, 12, 4, 0), f(c4, 11, 4, 0), f(c4, 64, 3, 0), f(c4 + 1, 1, 1, 0), f(c2 + 1, 64, 8, 0)] == [2, 4, 4, 2, 1]
     assert [f(c4, 64, 8, c << 8) for c in (1, 2, 4, 3)] == [1, 2, 4, -1]

@@ -112,14 +112,15 @@ static int ttt_launch_cluster(int streams, uint32_t flags, bool backward, int* c
 // take turns) 26 us per mini-batch against 28.
 static bool runs_pair(int ctas, int NC, int cgs) { return ctas == 2 && cgs > 1 && NC > cgs; }
 
-// CTAs per stream of a backward.  Where four would fit, two are faster once a call has four groups of four mini-batches to
+// CTAs per stream of a backward.  Where four would fit, two are faster once a call has three groups of four mini-batches to
 // pipeline: the first group's recompute runs alone, and a group that has few slots to spare ends with a wait for the last of
-// the next (32 streams, pair against four CTAs per mini-batch: 128 mini-batches in groups of 16 10.5 against 13.2 us, 32 in
-// groups of 8 12.2 / 13.7, 16 in groups of 4 14.2 / 14.4, 12 in groups of 4 14.8 / 14.6, 12 in groups of 3 16.6 / 14.9).
+// the next (32 streams, pair against four CTAs, us per mini-batch: 256 mini-batches in groups of 16 9.3 / 13.2, 48 in groups
+// of 16 11.7 / 13.3, 24 in groups of 8 12.5 / 13.9, 12 in groups of 4 13.9 / 14.6; two groups: 16 in groups of 8 14.3 / 14.0,
+// 8 in groups of 4 15.5 / 14.7; small groups: 32 in groups of 3 14.8 / 14.7, in groups of 2 17.2 / 15.4).
 static int backward_ctas(int streams, int NC, int cgs, uint32_t flags, int* ctas) {
   if (int rc = ttt_launch_cluster(streams, flags, true, ctas)) return rc;
   int asked = 0;
-  if (asked_cluster(flags, &asked) == TTT_B200_OK && asked == 0 && *ctas == 4 && cgs >= 4 && NC >= 4 * cgs) *ctas = 2;
+  if (asked_cluster(flags, &asked) == TTT_B200_OK && asked == 0 && *ctas == 4 && cgs >= 4 && NC >= 3 * cgs) *ctas = 2;
   return TTT_B200_OK;
 }
 
