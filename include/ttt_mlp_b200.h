@@ -291,8 +291,12 @@ int ttt_b200_version(void);
 int ttt_b200_launch_cluster(int streams, uint32_t flags, int backward);
 
 /* The same for a backward of NC mini-batches in groups of checkpoint_group_size: without a size in the flags or the
- * environment it is two instead of four from four groups of four mini-batches on. */
+ * environment it is two instead of four from three groups of four mini-batches on. */
 int ttt_b200_backward_ctas(int streams, int NC, int checkpoint_group_size, uint32_t flags);
+
+/* Of a backward whose answer there is one: how many of its last streams (those beyond a multiple of the SMs) a second launch
+ * gives two CTAs each.  0 if there is only one launch, -1 on error. */
+int ttt_b200_backward_tail(int streams, int NC, int checkpoint_group_size, uint32_t flags);
 
 /* The widest cluster size whose capacity on the current device covers `streams`: four, else (forward only) two, else one.
  * TTT_B200_CLUSTER overrides.  Not what a launch runs between the two capacities: ttt_b200_launch_cluster is.  Returns

@@ -204,7 +204,8 @@ struct BwdParams {
   float* d_gamma; float* d_beta;
   float* gW1; float* gb1; float* gW2; float* gb2;
   __nv_bfloat16* d_eta;
-  int H, NC, cgs, nck, streams;
+  int H, NC, cgs, nck;
+  int first, streams;       // this launch's first stream, and the call's number of them
   int drop_load;            // test only: mini-batch whose recompute inputs stream 0 never loads (-1: none)
   uint32_t* status;
   uint64_t wait_limit_ns;
@@ -392,7 +393,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t crank = cluster_ctarank();
   const bool sweeper = crank < kStreams;
   const uint32_t peer = sweeper ? crank + kStreams : crank - kStreams;
-  const int sid = (blockIdx.x / (2 * kStreams)) * kStreams + (crank % kStreams);
+  const int sid = p.first + (blockIdx.x / (2 * kStreams)) * kStreams + (crank % kStreams);
   const bool idle = sid >= p.streams;      // the last cluster's second stream, if there is none: it only keeps step
   const int head = sid % p.H;
   const int NC = p.NC, cgs = p.cgs, nck = p.nck;
@@ -1749,7 +1750,8 @@ int clusters_at_once() {
 // How many streams the device runs at once with two CTAs each.
 int ttt_backward_pair_capacity() { return clusters_at_once<1>(); }
 
-int ttt_launch_backward_pair(const ttt_b200_bwd_args* a, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
+// The streams from `first` on, to the last.
+int ttt_launch_backward_pair(const ttt_b200_bwd_args* a, int first, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
                              int drop_load) {
   const uint64_t rows = static_cast<uint64_t>(a->B) * a->H * a->NC * 64;
   CUtensorMap tmQ, tmK, tmV, tmGo, tmDQ, tmDK, tmDV;
@@ -1785,11 +1787,11 @@ int ttt_launch_backward_pair(const ttt_b200_bwd_args* a, cudaStream_t stream, ui
   p.d_gamma = a->grad_L_ttt_norm_weight; p.d_beta = a->grad_L_ttt_norm_bias;
   p.gW1 = a->grad_L_W1_init; p.gb1 = a->grad_L_b1_init; p.gW2 = a->grad_L_W2_init; p.gb2 = a->grad_L_b2_init;
   p.d_eta = static_cast<__nv_bfloat16*>(a->grad_L_last_eta);
-  p.streams = a->B * a->H; p.H = a->H; p.NC = a->NC; p.cgs = a->checkpoint_group_size; p.nck = a->num_checkpoints;
+  p.first = first; p.streams = a->B * a->H; p.H = a->H; p.NC = a->NC; p.cgs = a->checkpoint_group_size; p.nck = a->num_checkpoints;
   p.drop_load = drop_load;
   p.status = status;
   p.wait_limit_ns = limit_ns;
-  const int streams = a->B * a->H;
+  const int streams = a->B * a->H - first;
   // streams to a cluster: one only where clusters of one stream hold all streams at once and clusters of two do not
   const int per = streams > 2 * clusters_at_once<2>() && streams <= clusters_at_once<1>() ? 1 : 2;
   if (int rc = per == 1 ? prepare_kernel<1>() : prepare_kernel<2>()) return rc;

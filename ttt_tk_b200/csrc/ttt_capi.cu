@@ -17,9 +17,9 @@
 
 int ttt_launch_forward(const ttt_b200_fwd_args* a, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
                        int drop_load);
-int ttt_launch_backward(const ttt_b200_bwd_args* a, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
+int ttt_launch_backward(const ttt_b200_bwd_args* a, int streams, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
                         int drop_load);
-int ttt_launch_backward_pair(const ttt_b200_bwd_args* a, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
+int ttt_launch_backward_pair(const ttt_b200_bwd_args* a, int first, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
                              int drop_load);
 int ttt_launch_backward_cluster(const ttt_b200_bwd_args* a, int cluster, cudaStream_t stream, uint32_t* status,
                                 uint64_t limit_ns, int drop_load);
@@ -30,6 +30,7 @@ int ttt_launch_linear_backward(const ttt_b200_linear_bwd_args* a, cudaStream_t s
 uint64_t ttt_linear_backward_scratch_bytes(int B, int H, int cgs);
 int ttt_forward_cluster_capacity(int cluster);
 int ttt_backward_cluster_capacity(int cluster);
+int ttt_backward_pair_capacity();
 int ttt_launch_forward_cluster(const ttt_b200_fwd_args* a, int cluster, cudaStream_t stream, uint32_t* status,
                                uint64_t limit_ns, int drop_load);
 
@@ -122,6 +123,22 @@ static int backward_ctas(int streams, int NC, int cgs, uint32_t flags, int* ctas
   int asked = 0;
   if (asked_cluster(flags, &asked) == TTT_B200_OK && asked == 0 && *ctas == 4 && cgs >= 4 && NC >= 3 * cgs) *ctas = 2;
   return TTT_B200_OK;
+}
+
+// Streams of a backward with one CTA per stream that two CTAs per stream take, in a launch of their own after the others': those
+// beyond a multiple of the SMs, when the device runs them as pairs at once.  A turn over the SMs with one CTA per stream lasts
+// 21.7 us per mini-batch however few streams are in it, one of pairs 12.6 and some us of launch.  Backward, us, without and
+// with it: 176 streams x 64 in groups of 8 2798 / 2087, 192 x 37 in groups of 6 1700 / 1321, 312 x 52 in groups of 7 3480 /
+// 2918, 1536 x 16 in groups of 4 4312 / 4173; where pairs are most and have least to pipeline, 222 streams x 8 in groups of 2
+// 471 / 434, x 3 213 / 203, 370 x 3 313 / 307.
+static int backward_tail(int streams, int NC, int cgs, uint32_t flags, int ctas) {
+  int asked = 0, dev = 0, sms = 0;
+  if (ctas != 1 || !runs_pair(2, NC, cgs) || asked_cluster(flags, &asked) != TTT_B200_OK || asked != 0) return 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+    return 0;
+  const int rest = streams % sms;      // SMs hold one CTA each
+  return streams > sms && rest <= ttt_backward_pair_capacity() ? rest : 0;
 }
 
 int ttt_set_error(int code, const char* msg) {
@@ -321,11 +338,16 @@ extern "C" int ttt_b200_backward(const ttt_b200_bwd_args* a, void* stream_) {
   // the hook drops the recompute inputs of the last group's second mini-batch (its only one if it has one)
   const int last0 = (a->num_checkpoints - 1) * a->checkpoint_group_size;
   const int drop = (a->flags & TTT_B200_FLAG_TEST_LOST_LOAD) ? (last0 + 1 < a->NC ? last0 + 1 : last0) : -1;
-  if (int rc = cluster == 1 ? ttt_launch_backward(a, stream, status, wait_limit_ns(), drop)
-               : runs_pair(cluster, a->NC, a->checkpoint_group_size)
-                   ? ttt_launch_backward_pair(a, stream, status, wait_limit_ns(), drop)
-                   : ttt_launch_backward_cluster(a, cluster, stream, status, wait_limit_ns(), drop))
+  const int streams = a->B * a->H, tail = backward_tail(streams, a->NC, a->checkpoint_group_size, a->flags, cluster);
+  if (cluster == 1) {
+    if (int rc = ttt_launch_backward(a, streams - tail, stream, status, wait_limit_ns(), drop)) return rc;
+    if (tail > 0)
+      if (int rc = ttt_launch_backward_pair(a, streams - tail, stream, status, wait_limit_ns(), drop)) return rc;
+  } else if (runs_pair(cluster, a->NC, a->checkpoint_group_size)) {
+    if (int rc = ttt_launch_backward_pair(a, 0, stream, status, wait_limit_ns(), drop)) return rc;
+  } else if (int rc = ttt_launch_backward_cluster(a, cluster, stream, status, wait_limit_ns(), drop)) {
     return rc;
+  }
   if (a->flags & TTT_B200_FLAG_SYNC) return ttt_check_status(stream);
   return TTT_B200_OK;
 }
@@ -358,6 +380,11 @@ extern "C" int ttt_b200_backward_ctas(int streams, int NC, int checkpoint_group_
   int c = 0;
   if (streams < 1 || NC < 1 || checkpoint_group_size < 1) return -1;
   return backward_ctas(streams, NC, checkpoint_group_size, flags, &c) == TTT_B200_OK ? c : -1;
+}
+
+extern "C" int ttt_b200_backward_tail(int streams, int NC, int checkpoint_group_size, uint32_t flags) {
+  const int c = ttt_b200_backward_ctas(streams, NC, checkpoint_group_size, flags);
+  return c < 0 ? -1 : backward_tail(streams, NC, checkpoint_group_size, flags, c);
 }
 
 extern "C" int ttt_b200_launch_cluster(int streams, uint32_t flags, int backward) {
