@@ -295,7 +295,7 @@ int ttt_b200_launch_cluster(int streams, uint32_t flags, int backward);
 int ttt_b200_backward_ctas(int streams, int NC, int checkpoint_group_size, uint32_t flags);
 
 /* Of a backward whose answer there is one: how many of its last streams (those beyond a multiple of the SMs) a second launch
- * gives two CTAs each (four where there are no groups of several mini-batches to pipeline).  0 if there is only one launch, -1 on error. */
+ * gives two CTAs each.  0 if there is only one launch, -1 on error. */
 int ttt_b200_backward_tail(int streams, int NC, int checkpoint_group_size, uint32_t flags);
 
 /* The widest cluster size whose capacity on the current device covers `streams`: four, else (forward only) two, else one.

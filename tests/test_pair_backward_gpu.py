@@ -40,21 +40,20 @@ def test_calls_that_pipeline_groups_take_two_ctas():
     assert [f(c4, 64, 8, c << 8) for c in (1, 2, 4, 3)] == [1, 2, 4, -1]
 
 
-@pytest.mark.parametrize("rest", [1, 2, 33, 67, 74])
-@pytest.mark.parametrize("NC,cgs", [(3, 2), (9, 4), (1, 1), (3, 1), (4, 4)])
-def test_last_small_turn_gets_more_ctas(rest, NC, cgs):
+@pytest.mark.parametrize("rest", [1, 2, 67, 74])
+@pytest.mark.parametrize("NC,cgs", [(3, 2), (9, 4)])
+def test_last_small_turn_runs_as_pairs(rest, NC, cgs):
     """Streams beyond a multiple of the SMs: a second launch, whose streams start where the first's end (heads differ)."""
     lib, sms = _lib.lib(), torch.cuda.get_device_properties(0).multi_processor_count
     H = sms + rest
-    ctas = 2 if 1 < cgs < NC else 4
-    tail = rest if rest <= lib.ttt_b200_cluster_capacity(ctas, 1) else 0
-    assert [lib.ttt_b200_backward_tail(s, NC, cgs, 0) for s in (sms, H, 2 * sms, 2 * sms + rest)] == [0, tail, 0, tail]
+    if rest > lib.ttt_b200_cluster_capacity(2, 1):
+        pytest.skip("more streams than the device runs as pairs at once")
+    assert [lib.ttt_b200_backward_tail(s, NC, cgs, 0) for s in (sms, H, 2 * sms, 2 * sms + rest)] == [0, rest, 0, rest]
+    assert lib.ttt_b200_backward_tail(H, cgs, cgs, 0) == lib.ttt_b200_backward_tail(H, NC, 1, 0) == 0
     assert lib.ttt_b200_backward_tail(H, NC, cgs, 1 << 8) == 0
-    if tail == 0:
-        return
     d = inputs(1, H, NC, seed=rest)
     ck = oracle_forward(d, cgs)
-    now, one, several = (run_backward(d, ck, cgs, c) for c in (None, 1, ctas))
+    now, one, two = (run_backward(d, ck, cgs, c) for c in (None, 1, 2))
     for k in GRAD_NAMES:
         assert torch.equal(now[k][:, :sms], one[k][:, :sms]), f"{k} of the first launch"
-        assert torch.equal(now[k][:, sms:], several[k][:, sms:]), f"{k} of the second"
+        assert torch.equal(now[k][:, sms:], two[k][:, sms:]), f"{k} of the second"

@@ -138,7 +138,6 @@ struct BwdClParams {
   __nv_bfloat16* d_eta;
   __nv_bfloat16* dXQ; __nv_bfloat16* dXK; __nv_bfloat16* dXV;   // bf16 [rows][64], row-major
   int H, NC, cgs, nck;
-  int first;                // this launch's first stream
   int drop_load;            // test only: mini-batch whose recompute inputs stream 0 never loads (-1: none)
   uint32_t* status;
   uint64_t wait_limit_ns;
@@ -160,7 +159,7 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const TokMap tm(warp, lane);
   const uint32_t rank = cluster_ctarank();
-  const long sid = p.first + static_cast<int>(blockIdx.x) / kC;
+  const long sid = blockIdx.x / kC;
   const int head = static_cast<int>(sid % p.H);
   const int NC = p.NC, cgs = p.cgs;
   const int hid0 = static_cast<int>(rank) * C::R;
@@ -1630,8 +1629,7 @@ int launch_cluster(const CUtensorMap* tm, const BwdClParams& p, int streams, cud
 
 }  // namespace
 
-// The streams from `first` on, to the last.
-int ttt_launch_backward_cluster(const ttt_b200_bwd_args* a, int cluster, int first, cudaStream_t stream, uint32_t* status,
+int ttt_launch_backward_cluster(const ttt_b200_bwd_args* a, int cluster, cudaStream_t stream, uint32_t* status,
                                 uint64_t limit_ns, int drop_load) {
   const uint64_t rows = static_cast<uint64_t>(a->B) * a->H * a->NC * 64;
   CUtensorMap tm[7];
@@ -1663,11 +1661,11 @@ int ttt_launch_backward_cluster(const ttt_b200_bwd_args* a, int cluster, int fir
   p.dXQ = static_cast<__nv_bfloat16*>(a->grad_L_XQ);
   p.dXK = static_cast<__nv_bfloat16*>(a->grad_L_XK);
   p.dXV = static_cast<__nv_bfloat16*>(a->grad_L_XV);
-  p.first = first; p.H = a->H; p.NC = a->NC; p.cgs = a->checkpoint_group_size; p.nck = a->num_checkpoints;
+  p.H = a->H; p.NC = a->NC; p.cgs = a->checkpoint_group_size; p.nck = a->num_checkpoints;
   p.drop_load = drop_load;
   p.status = status;
   p.wait_limit_ns = limit_ns;
-  const int streams = a->B * a->H - first;
+  const int streams = a->B * a->H;
   if (cluster == 2) return launch_cluster<2>(tm, p, streams, stream);
   if (cluster == 4) return launch_cluster<4>(tm, p, streams, stream);
   return ttt_set_error(TTT_B200_ERR_BAD_ARGS, "cluster size must be 2 or 4");

@@ -21,7 +21,7 @@ int ttt_launch_backward(const ttt_b200_bwd_args* a, int streams, cudaStream_t st
                         int drop_load);
 int ttt_launch_backward_pair(const ttt_b200_bwd_args* a, int first, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
                              int drop_load);
-int ttt_launch_backward_cluster(const ttt_b200_bwd_args* a, int cluster, int first, cudaStream_t stream, uint32_t* status,
+int ttt_launch_backward_cluster(const ttt_b200_bwd_args* a, int cluster, cudaStream_t stream, uint32_t* status,
                                 uint64_t limit_ns, int drop_load);
 int ttt_launch_linear_forward(const ttt_b200_linear_fwd_args* a, cudaStream_t stream, uint32_t* status,
                               uint64_t limit_ns, int drop_load);
@@ -125,25 +125,20 @@ static int backward_ctas(int streams, int NC, int cgs, uint32_t flags, int* ctas
   return TTT_B200_OK;
 }
 
-// Streams of a backward with one CTA per stream that get several, in a launch of their own after the others': those
-// beyond a multiple of the SMs, when the device runs them all at once.  A turn over the SMs with one CTA per stream lasts
+// Streams of a backward with one CTA per stream that two CTAs per stream take, in a launch of their own after the others': those
+// beyond a multiple of the SMs, when the device runs them as pairs at once.  A turn over the SMs with one CTA per stream lasts
 // 21.7 us per mini-batch however few streams are in it, one of pairs 12.6 and some us of launch.  Backward, us, without and
 // with it: 176 streams x 64 in groups of 8 2798 / 2087, 192 x 37 in groups of 6 1700 / 1321, 312 x 52 in groups of 7 3480 /
 // 2918, 1536 x 16 in groups of 4 4312 / 4173; where pairs are most and have least to pipeline, 222 streams x 8 in groups of 2
 // 471 / 434, x 3 213 / 203, 370 x 3 313 / 307.
-// Where pairs have no groups to pipeline, four CTAs with a quarter of the hidden units each take a rest that the device runs
-// in such clusters at once: 181 streams x 32 in one group 1335 / 1120, x 4 220 / 194, 176 x 2 138 / 126, 160 x 16 in groups of
-// 1 1062 / 853, 320 x 2 202 / 188; one mini-batch 96 / 93 with 176 streams, 96.7 / 96.4 with 149.
-static int backward_tail(int streams, int NC, int cgs, uint32_t flags, int ctas, int* tail_ctas) {
+static int backward_tail(int streams, int NC, int cgs, uint32_t flags, int ctas) {
   int asked = 0, dev = 0, sms = 0;
-  if (ctas != 1 || asked_cluster(flags, &asked) != TTT_B200_OK || asked != 0) return 0;
+  if (ctas != 1 || !runs_pair(2, NC, cgs) || asked_cluster(flags, &asked) != TTT_B200_OK || asked != 0) return 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
     return 0;
-  const bool pairs = runs_pair(2, NC, cgs);
-  *tail_ctas = pairs ? 2 : 4;
   const int rest = streams % sms;      // SMs hold one CTA each
-  return streams > sms && rest <= (pairs ? ttt_backward_pair_capacity() : capacity(4, true)) ? rest : 0;
+  return streams > sms && rest <= ttt_backward_pair_capacity() ? rest : 0;
 }
 
 int ttt_set_error(int code, const char* msg) {
@@ -343,17 +338,16 @@ extern "C" int ttt_b200_backward(const ttt_b200_bwd_args* a, void* stream_) {
   // the hook drops the recompute inputs of the last group's second mini-batch (its only one if it has one)
   const int last0 = (a->num_checkpoints - 1) * a->checkpoint_group_size;
   const int drop = (a->flags & TTT_B200_FLAG_TEST_LOST_LOAD) ? (last0 + 1 < a->NC ? last0 + 1 : last0) : -1;
-  const int streams = a->B * a->H, cgs = a->checkpoint_group_size;
-  const uint64_t limit = wait_limit_ns();
-  int first = 0;      // of the streams that more than one CTA each take
+  const int streams = a->B * a->H, tail = backward_tail(streams, a->NC, a->checkpoint_group_size, a->flags, cluster);
   if (cluster == 1) {
-    first = streams - backward_tail(streams, a->NC, cgs, a->flags, cluster, &cluster);
-    if (int rc = ttt_launch_backward(a, first, stream, status, limit, drop)) return rc;
+    if (int rc = ttt_launch_backward(a, streams - tail, stream, status, wait_limit_ns(), drop)) return rc;
+    if (tail > 0)
+      if (int rc = ttt_launch_backward_pair(a, streams - tail, stream, status, wait_limit_ns(), drop)) return rc;
+  } else if (runs_pair(cluster, a->NC, a->checkpoint_group_size)) {
+    if (int rc = ttt_launch_backward_pair(a, 0, stream, status, wait_limit_ns(), drop)) return rc;
+  } else if (int rc = ttt_launch_backward_cluster(a, cluster, stream, status, wait_limit_ns(), drop)) {
+    return rc;
   }
-  if (first < streams)
-    if (int rc = runs_pair(cluster, a->NC, cgs) ? ttt_launch_backward_pair(a, first, stream, status, limit, drop)
-                                                : ttt_launch_backward_cluster(a, cluster, first, stream, status, limit, drop))
-      return rc;
   if (a->flags & TTT_B200_FLAG_SYNC) return ttt_check_status(stream);
   return TTT_B200_OK;
 }
@@ -390,8 +384,7 @@ extern "C" int ttt_b200_backward_ctas(int streams, int NC, int checkpoint_group_
 
 extern "C" int ttt_b200_backward_tail(int streams, int NC, int checkpoint_group_size, uint32_t flags) {
   const int c = ttt_b200_backward_ctas(streams, NC, checkpoint_group_size, flags);
-  int tail_ctas = 0;
-  return c < 0 ? -1 : backward_tail(streams, NC, checkpoint_group_size, flags, c, &tail_ctas);
+  return c < 0 ? -1 : backward_tail(streams, NC, checkpoint_group_size, flags, c);
 }
 
 extern "C" int ttt_b200_launch_cluster(int streams, uint32_t flags, int backward) {
