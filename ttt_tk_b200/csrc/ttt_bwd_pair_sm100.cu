@@ -1601,8 +1601,8 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       *reinterpret_cast<float2*>(part + half * 64 + 2 * lane) = make_float2(a0 + c0, a1 + c1);
       __syncwarp();
       if (lane == 0) arrive(E_PART);
-      // d_eta of 32 tokens, when E4 has left its addends
-      if (!seen(E_DE)) return;
+      // d_eta of 32 tokens, when the other half of the sums is there and E4 has left its addends
+      if (!seen(E_PART) || !seen(E_DE)) return;
       const int t = half * 32 + lane;
       p.d_eta[(sid * NC + first_of(g) + j) * 64 + t] =
           __float2bfloat16(-(quad_sum(reinterpret_cast<const float*>(smem + S_X1), t) + (part[t] + part[64 + t])));
