@@ -59,7 +59,8 @@ def test_every_wait_ends_and_the_scratch_holds_what_was_stored(case):
     assert r.problems == [] and r.provenance() == []
 
 
-AREAS = ["S_PART"]
+# (OFF_BIG: the hidden-major buffers)
+AREAS = ["S_PART", "OFF_BIG", "S_GB1"]
 
 
 @pytest.mark.parametrize("area", AREAS)

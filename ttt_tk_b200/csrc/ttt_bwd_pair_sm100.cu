@@ -339,7 +339,7 @@ __constant__ const MmaOp kSweepMma[kSweepMmas] = {
     {E_T, kNo, kNo, P_HID, R_A, R_NONE, 0, 0, 0, S_GZ2, TM_A},                // G12
     {kNo, kNo, kNo, P_HID, R_S2, R_NONE, 0, 0, 0, S_Q, TM_B},                 // G11b
     {SX2B, kNo, CB, P_HID_MN, R_GZ, R_NONE, 1, 0, 0, S_GZB, TM_S2},           // G2 of the next step
-    {E_Z, kNo, C5, P_HID_ACC, R_A, R_NONE, 0, 0, 0, S_XF, TM_B},              // G11a
+    {E_Z, E_PART, C5, P_HID_ACC, R_A, R_NONE, 0, 0, 0, S_XF, TM_B},           // G11a (E5 overwrites gZ1 and adds to G_b1)
     {kNo, kNo, kNo, P_HID_MN, R_Z, R_NONE, 0, 0, 0, S_XF, TM_S2},             // G14
     {SGZ1B, SQ, C3, P_HID_MN, R_S1, R_NONE, 1, 0, 0, S_Q, TM_S1},             // G3 of the next step
     {E_5, kNo, C6, P_HID_MN, R_GZ, R_NONE, 0, 0, 0, S_K, TM_S1},              // G15
