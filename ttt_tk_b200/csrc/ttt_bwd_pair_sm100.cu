@@ -149,8 +149,9 @@ enum : int {
   SW2 = kRecBars, SW1, SGZ1, SX2, SZ1, SGZ1B, SX2B, SK, SGZ2, SV, SXF, SQ,
   // products: G4 and G8, G10, G5 and G6, G11b and G2, G11a, G3, G15, G13
   C2, C10, C4, CB, C5, C3, C6, C7,
-  // epilogues done: Z1 read, E2 (G_W1), E2 (G_W2, dK), E3, E4's accumulators read and U2, gZ2in, dV, d_eta's addends, E5; gZ1 G_b1 summed
-  E_D, E_S1, E_S2, E_P, E_T, E_Z, E_V, E_DE, E_5, E_PART,
+  // epilogues done: Z1 read, E2 (G_W1), E2 (G_W2, dK), E3, E4's accumulators read and U2, gZ2in, dV, E5 and d_eta's addends;
+  // gZ1 G_b1 summed, d_eta's addends read
+  E_D, E_S1, E_S2, E_P, E_T, E_Z, E_V, E_5, E_PART, E_X,
   BGROUP,      // the scratch slots of a group are written (two CTAs per stream)
   BDRAIN,      // abort path only
   kBars
@@ -306,8 +307,8 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
 }
 __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
-enum : uint8_t { V_D, V_S2, V_C2, V_PART, V_C10, V_CB, V_C5, V_V, V_C3, V_C6, V_C7, V_COUNT };      // the sweep copies' events
-__constant__ const uint8_t kSweepEvent[V_COUNT] = {E_D, E_S2, C2, E_PART, C10, CB, C5, E_V, C3, C6, C7};
+enum : uint8_t { V_D, V_S2, V_C2, V_PART, V_C10, V_CB, V_C5, V_V, V_C3, V_C6, V_X, V_C7, V_COUNT };      // the sweep copies' events
+__constant__ const uint8_t kSweepEvent[V_COUNT] = {E_D, E_S2, C2, E_PART, C10, CB, C5, E_V, C3, C6, E_X, C7};
 constexpr int kSweepCopies = 19;
 __constant__ const CopyOp kSweepCopy[kSweepCopies] = {
     {V_D, K_LOAD, A_X2, SX2, R_Z, 0, 0, 0, 0, 0, BIG, BIG},
@@ -409,7 +410,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   if (tid == kEpi) {
     for (int i = 0; i < kBars; ++i)
-      mbar_init(&bars[i], i >= E_LDT && i <= E_ODQ ? 8 : i >= E_D && i <= E_5 ? 16 : i == E_PART || i == BGROUP || i == BDRAIN ? 2 : 1);
+      mbar_init(&bars[i], i >= E_LDT && i <= E_ODQ ? 8 : i >= E_D && i <= E_5 ? 16 : i >= E_PART ? 2 : 1);
     fence_mbar_init();
     *abort_flag = 0;
     *never_flag = 0;
@@ -1146,8 +1147,8 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (ch == 0) sGb1[hrow] = p.gb1_last[long{sid} * 256 + hrow];
       if (tid < 64) sGb2[tid] = p.gb2_last[long{sid} * 64 + tid];
       tmem_wait_st();
+      done(E_5);
     }
-    done(E_5);
     Frag16 kp;                // partial dK of the last step
     auto finish_dk = [&]() {  // after C7
       uint32_t u[8];
@@ -1258,6 +1259,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       wait(SXF);
       wait(SV);
       wait_mma(C4);
+      float de0, de1;                      // d_eta's row terms
       {
         uint32_t gzw[4], xw[4], kw[4], vw[4];
         f16_ld_raw(tm, smem + S_GZ2, gzw);
@@ -1268,7 +1270,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const float rs0 = sig[tm.r0], rs1 = sig[tm.r1];      // 1 / std
         Frag16 A2, go;
         f32x2 cl[2];                       // dV's addends to d_beta
-        float de0, de1, ra[2], rb[2];      // d_eta's row terms; sum A2, sum A2 x_hat
+        float ra[2], rb[2];                // sum A2, sum A2 x_hat
         {
           uint32_t u0[8], u1[8];
           tmem_ld_16x256b_x2(tmem + TM_B + 64 + tm.taddr, u0);
@@ -1388,7 +1390,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
         done(E_Z);
         if (lane == 0) arrive(E_V);
-        // ---- what nothing on the chain waits for: column sums, d_eta
+        // ---- what nothing on the chain waits for: column sums, d_eta's rows
         sCS[quad * 64 + f16_colsum_col(tm, lane)] = f16_colsum(add2(A2.a[0], A2.b[0]), add2(A2.a[1], A2.b[1]), lane);
         dgam_s += f16_colsum(cs[0], cs[1], lane);
         dbet_s += f16_colsum(cl[0], cl[1], lane);
@@ -1397,18 +1399,17 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           de0 += __shfl_xor_sync(0xffffffffu, de0, sft);
           de1 += __shfl_xor_sync(0xffffffffu, de1, sft);
         }
-        // (the first exchange's area: all four warps have passed the second one's barrier)
-        float* xe = reinterpret_cast<float*>(smem + S_X1);
-        if (tm.l3 == 0) {
-          xe[cq * 64 + tm.r0] = de0;
-          xe[cq * 64 + tm.r1] = de1;
-        }
-        __syncwarp();
-        if (lane == 0) arrive(E_DE);
       }
 
       // ---- E5: gZ1in^T = gX2^T gelu'(Z1^T) + R^T S^T
       wait_mma(C5);
+      // (over the first exchange: its last reader is behind E_Z, and E4 of the next step, which writes there again, needs the
+      // W2 that is loaded after E_X)
+      if (tm.l3 == 0) {
+        float* xe = reinterpret_cast<float*>(smem + S_X1);
+        xe[cq * 64 + tm.r0] = de0;
+        xe[cq * 64 + tm.r1] = de1;
+      }
       {
         f32x2 bs = 0ull;
 #pragma unroll
@@ -1498,7 +1499,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   };
   auto sweep_issue = [&](int g) {
     const int gsz = size_of(g);
-    if (!seen(E_5) || !seen(SX2B) || !seen(SGZ1B) || !seen(SQ)) return;
+    if ((g == 0 && !seen(E_5)) || !seen(SX2B) || !seen(SGZ1B) || !seen(SQ)) return;
 #pragma unroll 1
     for (int k = 0; k < 2; ++k)       // G2, G3 of the group's first step
       issue(prepare(P_HID_MN, k ? TM_S1 : TM_S2, k ? o_s2 : o_s1, k ? S_Q : S_GZB));
@@ -1576,6 +1577,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // d_eta; its fourth term, gZ1 G_b1, is summed over half of the hidden units by each of two warps: lane l takes the token pair (2 l, 2 l + 1)
   auto sweep_part = [&](int g, int half) {
     const int gsz = size_of(g);
+    if (g == 0 && !seen(E_5)) return;     // (the gradient state)
     for (int j = gsz - 1; j >= 0; --j) {
       if (!seen(E_S1) || !seen(SGZ1)) return;
       const uint8_t* bg = smem + o_gz + half * 16384 + (lane & 3) * 4;      // (128 rows: the swizzle's phase is the same)
@@ -1601,17 +1603,19 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       *reinterpret_cast<float2*>(part + half * 64 + 2 * lane) = make_float2(a0 + c0, a1 + c1);
       __syncwarp();
       if (lane == 0) arrive(E_PART);
-      // d_eta of 32 tokens, when the other half of the sums is there and E4 has left its addends
-      if (!seen(E_PART) || !seen(E_DE)) return;
+      if (half == 0) {      // all of this step's slot is in shared memory (W1 came last): the recompute may have it
+        if (!seen(SW1)) return;
+        if (lane == 0) st_release_cluster(mapa(smem_u32(freed), peer), static_cast<uint32_t>(nsw + 1));
+      }
+      // d_eta of 32 tokens, when the other half of the sums is there and E5 has left the addends
+      if (!seen(E_PART) || !seen(E_5)) return;
       const int t = half * 32 + lane;
       p.d_eta[(sid * NC + first_of(g) + j) * 64 + t] =
           __float2bfloat16(-(quad_sum(reinterpret_cast<const float*>(smem + S_X1), t) + (part[t] + part[64 + t])));
+      __syncwarp();
+      if (lane == 0) arrive(E_X);
       turn();
       ++nsw;
-      if (half == 0) {      // all of this step's slot is in shared memory (W1 came last): the recompute may have it
-        if (!seen(SW1)) return;
-        if (lane == 0) st_release_cluster(mapa(smem_u32(freed), peer), static_cast<uint32_t>(nsw));
-      }
     }
   };
 
