@@ -805,11 +805,11 @@ class Agent:
         m[2].append(self)
         self.at.pred.append(m[1])
 
-    def f_st_release_cluster(self, w, p, value): self.r.released.append((int(value), self.sync("frees")))
+    def f_st_release_cluster(self, w, p, value): self.r.released.append((p.cta, int(value), self.sync("frees")))
 
     def acquire(self, w, need):
         if need > 0:
-            self.r.acquired.append((int(need), self.sync(f"sees {need} freed")))
+            self.r.acquired.append((self.cta, int(need), self.sync(f"sees {need} freed")))
 
     # -- bulk copies (of the active lanes)
     def f_mbar_expect_tx(self, w, p, nbytes):
@@ -976,9 +976,8 @@ class Run:
             if arrived.get(b, {}).get(phase) != self.count[b]:
                 self.problems.append(f"{n.what}: never completes")
             n.pred += by
-        rel = sorted(self.released, key=lambda x: x[0])
-        for need, n in self.acquired:
-            first = next((r for v, r in rel if v >= need), None)
+        for cta, need, n in self.acquired:               # (released in rising order by one warp)
+            first = next((r for c, v, r in self.released if c == cta and v >= need), None)
             if first is None:
                 self.problems.append(f"{n.what}: never freed")
             else:

@@ -152,11 +152,13 @@ enum : int {
   // epilogues done: Z1 read, E2 (G_W1), E2 (G_W2, dK), E3, E4's accumulators read and U2, gZ2in, dV, E5 and d_eta's addends;
   // gZ1 G_b1 summed, d_eta's addends read
   E_D, E_S1, E_S2, E_P, E_T, E_Z, E_V, E_5, E_PART, E_X,
-  BGROUP,      // the scratch slots of a group are written (two CTAs per stream)
+  // the scratch slots of a group are written, by parity of the group: where a short first group and the next fit in beside
+  // each other, both can be before the sweep has looked
+  BGROUP, BGROUP1,
   BDRAIN,      // abort path only
   kBars
 };
-static_assert(kBars * 8 <= 512 && kRecBars <= 32 && kBars - kRecBars <= 32, "barrier storage, parity masks");
+static_assert(kBars * 8 <= 512 && kRecBars <= 32 && BDRAIN - kRecBars <= 32, "barrier storage, parity masks");
 
 // tensor-memory columns: see the head of the file
 constexpr uint32_t TM_S1 = 0;
@@ -444,7 +446,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // (one small loop: there are some eighty of these, and the instruction cache is short)
   auto bounded = [&](int b, uint32_t parity) -> bool {
     uint64_t t0 = 0;
-    while (!(b == BGROUP ? mbar_try_wait_cluster(&bars[b], parity) : mbar_try_wait(&bars[b], parity))) {
+    while (!(b >= BGROUP ? mbar_try_wait_cluster(&bars[b], parity) : mbar_try_wait(&bars[b], parity))) {
       if (*abort_flag) return false;
       const uint64_t t = globaltimer_ns();
       if (t0 == 0) t0 = t;
@@ -518,12 +520,12 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     return __all_sync(0xffffffffu, ok);
   };
   // a group's slots are complete: the bulk stores of this warp are, and the sweep may read them
-  auto group_written = [&]() {
+  auto group_written = [&](int g) {
     tma_wait_group<0>();
     fence_proxy_async_all();
     __threadfence();
     __syncwarp();
-    if (lane == 0) mbar_arrive_remote(&bars[BGROUP], peer);
+    if (lane == 0) mbar_arrive_remote(&bars[BGROUP + (g & 1)], peer);
   };
   // A copying warp's lane: its copy, and where that is in global memory.
   struct Lane {
@@ -1051,7 +1053,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     }
     if (g + 1 < nck) first(g + 1);
-    group_written();
+    group_written(g);
   };
   auto rec_out_copy = [&](int g) {
     const Lane c = lane_of(kOutCopy, kRecCopies);
@@ -1100,7 +1102,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tma_wait_group_read<0>();
     __syncwarp();
     if (g + 1 < nck) copy(c, lane == kLaneQ || lane == kLaneGo, first_of(g + 1), 0, op.off, 0, dropped(first_of(g + 1)));
-    group_written();
+    group_written(g);
   };
 
   // =====================================================================================================
@@ -1536,7 +1538,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll 1
       for (int k = 0; k < 2; ++k) {
         if (k == 1) {
-          if (!seen_all(BGROUP)) return;
+          if (!seen_all(BGROUP + (g & 1))) return;
           fence_proxy_async_all();      // the slots were written by the other CTA
         }
         copy(c, any && outside == (k == 0), i, slot, off, nsw & 1, false);
@@ -1681,7 +1683,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (warp >= 16) {
       for (int b = 0; b < kRecBars; ++b)
         if ((ldaR >> b) & 1u) mbar_wait_bounded(&bars[b], ((ldpR >> b) & 1u) ^ 1u, never_flag, limit);
-      for (int b = 0; b < kBars - kRecBars; ++b)
+      for (int b = 0; b < BDRAIN - kRecBars; ++b)
         if ((ldaS >> b) & 1u) mbar_wait_bounded(&bars[kRecBars + b], ((ldpS >> b) & 1u) ^ 1u, never_flag, limit);
     }
     if (tid == 0) {
