@@ -15,7 +15,7 @@ SCRATCH = {"X2_group": 32768, "Z1_group": 32768, "grad_l_wrt_Z1_group": 32768, "
            "x_hat_ln_group": 8192, "b1_init_group": 1024, "std_ln_group": 256, "std_fused_group": 256, "b2_init_group": 256}
 # mini-batches, group size, streams, streams to a cluster: no, one and two slots beyond the group's; a last group of one
 # mini-batch, incomplete and whole; a cluster of two streams, and one whose second is missing
-CASES = [(5, 2, 1, 1), (9, 4, 1, 1), (16, 4, 1, 1), (10, 3, 1, 1), (17, 8, 1, 1), (5, 2, 2, 2), (3, 2, 1, 2)]
+CASES = [(5, 2, 1, 1), (9, 4, 1, 1), (12, 4, 1, 1), (8, 3, 1, 1), (10, 8, 1, 1), (3, 2, 2, 2), (3, 2, 1, 2)]
 
 
 def source(edit=lambda text: text):
@@ -68,3 +68,16 @@ def test_no_two_accesses_are_unordered(case):
 @pytest.mark.parametrize("case", CASES)
 def test_no_waiter_is_overtaken(case):
     assert run(*case).phases() == set()
+
+
+@pytest.mark.parametrize("now,then,NC,what", [
+    ("{E_Z, E_PART, C5,", "{E_Z, kNo, C5,", 3, "races"),                                # a product that waits for less
+    ("wait(F_ZG);", "", 3, "races"),                                                    # an epilogue
+    ("need = steps_before(g - 1) + own + 1;", "need = steps_before(g - 1) + own;", 9, "races"),      # a slot taken early
+    ("w2 + 3 * 65536 + BIG;", "w2 + 2 * 65536 + BIG;", 5, "provenance"),                # arrays that share a slot's place
+    ("BGROUP + (g & 1)", "BGROUP", 5, "phases"),                                        # one barrier for all groups
+])
+def test_the_model_sees_a_mistake(now, then, NC, what):
+    src = source(lambda text: text.replace(now, then))
+    assert src.text != source().text
+    assert getattr(walk(src, NC, 2 if NC == 3 else 4), what)()
