@@ -52,3 +52,39 @@ def test_operator_kernels_report_a_lost_load_and_the_context_survives():
                          capture_output=True, text=True, timeout=600)
     assert res.returncode == 0, res.stdout[-2000:] + res.stderr[-3000:]
     assert "LOST_LOAD_OK" in res.stdout
+
+
+# groups whose recompute alone takes several milliseconds: MLP backward with two CTAs per stream, TTT-Linear backward
+LONG_GROUPS = """
+import hashlib, torch
+import test_cluster_backward_gpu as bwd
+import test_linear_backward_gpu as lin
+from ttt_tk_b200 import take_status
+h = hashlib.sha256()
+g = torch.Generator().manual_seed(0)
+def put(res):
+    assert take_status() == 0
+    for k in sorted(res):
+        h.update(res[k].contiguous().view(torch.uint8).numpy().tobytes())
+cgs = 600
+d = bwd.inputs(1, 1, 2 * cgs, seed=3, eta_scale=0.01)
+ck = {k: 0.02 * torch.randn(1, 1, 2, *s, generator=g) for k, s in
+      zip(bwd.CHECKPOINT_NAMES, ((64, 256), (1, 256), (256, 64), (1, 64)))}
+put(bwd.run_backward(d, ck, cgs, 2))
+cgs = 1500
+d = lin.make(1, 1, 2 * cgs, seed=4)
+put(lin.run(d, cgs))
+print("DIGEST", h.hexdigest())
+"""
+
+
+def test_a_whole_groups_recompute_is_not_taken_for_a_lost_signal():
+    """A 1 ms wait limit, and groups that take longer to recompute: the same bits as with the default limit."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    digests = []
+    for ms in ("2000", "1"):
+        env = dict(os.environ, TTT_B200_WAIT_LIMIT_MS=ms, PYTHONPATH=os.pathsep.join([root, os.path.join(root, "tests")]))
+        res = subprocess.run([sys.executable, "-c", LONG_GROUPS], env=env, cwd=root, capture_output=True, text=True, timeout=600)
+        assert res.returncode == 0, res.stdout[-2000:] + res.stderr[-3000:]
+        digests.append([x for x in res.stdout.splitlines() if x.startswith("DIGEST")])
+    assert digests[0] and digests[0] == digests[1]

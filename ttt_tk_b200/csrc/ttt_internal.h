@@ -31,7 +31,8 @@ uint32_t ttt_take_status();
 // 128-byte swizzle (the layout every 64 x 64 token tile of the operator has in memory).
 int ttt_make_tile_map(CUtensorMap* map, const void* base, uint64_t rows);
 
-// Limit of the device-side bounded waits in nanoseconds (TTT_B200_WAIT_LIMIT_MS, default 2000 ms).
+// Limit of the device-side bounded waits in nanoseconds (TTT_B200_WAIT_LIMIT_MS, default 2000 ms).  The launcher adds to it
+// where a kernel waits for more than a few microseconds by design.
 uint64_t ttt_wait_limit_ns();
 
 // Read and clear the device status word of ttt_b200_backward_noalloc (0 = nothing reported).
