@@ -14,18 +14,20 @@ from ttt_tk_b200.buffers import alloc_backward_buffers, alloc_checkpoints, GRAD_
 
 def main():
     dev = "cuda"
-    B, H, NC, cgs = 1, 1, 3, 2
+    B, H, NC = 1, 1, 3
     d = orc.make_inputs(B, H, NC, seed=0, backward=True)
     t = {k: v.to(dev) for k, v in d.items()}
     eta5 = t["last_eta"].unsqueeze(-1).contiguous()
-    f = orc.ttt_forward(d["XQ"], d["XK"], d["XV"], d["last_eta"], d["ttt_norm_weight"], d["ttt_norm_bias"],
-                        d["W1"], d["b1"], d["W2"], d["b2"], cgs)
-    g = orc.ttt_backward(d["XQ"], d["XK"], d["XV"], d["last_eta"], d["ttt_norm_weight"], d["ttt_norm_bias"],
-                         f["W1_checkpoints"], f["b1_checkpoints"], f["W2_checkpoints"], f["b2_checkpoints"],
-                         d["grad_L_W1_last"], d["grad_L_b1_last"], d["grad_L_W2_last"], d["grad_L_b2_last"],
-                         d["grad_L_XQW_mini_batch"], cgs)
-    ckd = [f[k].to(dev).contiguous() for k in CHECKPOINT_NAMES]
-    for cluster in (1, 2, 4):
+    # (two CTAs per stream: a pair where there are groups to pipeline, else the hidden units split)
+    for cluster, cgs in ((1, 2), (2, 2), (2, 3), (4, 2)):
+        f = orc.ttt_forward(d["XQ"], d["XK"], d["XV"], d["last_eta"], d["ttt_norm_weight"], d["ttt_norm_bias"],
+                            d["W1"], d["b1"], d["W2"], d["b2"], cgs)
+        g = orc.ttt_backward(d["XQ"], d["XK"], d["XV"], d["last_eta"], d["ttt_norm_weight"], d["ttt_norm_bias"],
+                             f["W1_checkpoints"], f["b1_checkpoints"], f["W2_checkpoints"], f["b2_checkpoints"],
+                             d["grad_L_W1_last"], d["grad_L_b1_last"], d["grad_L_W2_last"], d["grad_L_b2_last"],
+                             d["grad_L_XQW_mini_batch"], cgs)
+        ckd = [f[k].to(dev).contiguous() for k in CHECKPOINT_NAMES]
+
         def fwd(lost):
             ck = alloc_checkpoints(B, H, NC, cgs, dev)
             out = torch.zeros_like(t["XQ"])
@@ -59,6 +61,7 @@ def main():
                     assert e <= 3e-2, (name, cluster, k, e)
             print(f"{name} cluster {cluster}: lost load reported, next launch correct", flush=True)
     # the TTT-Linear forward has the same hook
+    cgs = 2
     from oracle import ttt_linear as lin
     from ttt_tk_b200 import ttt_linear_forward
     dl = lin.make_inputs(B, H, NC, seed=1)

@@ -46,7 +46,7 @@ class Guarded:
 
 
 @pytest.mark.parametrize("cluster", [1, 2, 4])
-@pytest.mark.parametrize("B,H,NC,cgs", [(1, 2, 3, 2), (2, 1, 5, 4)])
+@pytest.mark.parametrize("B,H,NC,cgs", [(1, 2, 3, 2), (2, 1, 5, 4), (1, 2, 4, 4), (2, 1, 3, 1)])
 def test_forward_and_backward_stay_inside_their_buffers(cluster, B, H, NC, cgs):
     dev = "cuda"
     bf, f32 = torch.bfloat16, torch.float32

@@ -104,8 +104,8 @@ def test_cluster_forward_then_backward_against_autograd(cluster):
 
 def test_long_context_shape_with_the_launchers_own_cluster_choice():
     """The long-context configuration's structure (B = 1, few streams, many mini-batches, deep checkpoint
-    groups): with 2 streams the launcher gives every stream a cluster of 4 CTAs; forward and backward
-    against the oracle at a length it finishes quickly."""
+    groups): with 2 streams the launcher gives every stream a cluster of 4 CTAs in the forward and a pair in the
+    backward (three groups); forward and backward against the oracle at a length it finishes quickly."""
     B, H, NC, cgs = 1, 2, 96, 32
     d = orc.make_inputs(B, H, NC, seed=5, backward=True)
     dev = "cuda"
@@ -118,3 +118,26 @@ def test_long_context_shape_with_the_launchers_own_cluster_choice():
     assert orc.rel_l2(out.float().cpu(), f["Out"]) <= 1e-2
     ck = {k: v.cpu() for k, v in zip(CHECKPOINT_NAMES, ckd)}
     check(run_backward(d, ck, cgs, None), oracle_backward(d, ck, cgs), TOL, "launcher's choice")
+
+
+# Two CTAs split the hidden units only where there are no groups of several mini-batches to pipeline: one group, of any
+# length, or groups of one (elsewhere two CTAs are a pair, test_pair_backward_gpu.py).
+@pytest.mark.parametrize("B,H,NC,cgs", [(1, 1, 12, 12), (2, 2, 8, 8), (1, 3, 9, 1), (1, 2, 33, 64), (1, 1, 24, 1)])
+@pytest.mark.parametrize("eta_scale", [0.1, 1.0])
+def test_two_ctas_without_groups_to_pipeline_match_oracle(B, H, NC, cgs, eta_scale):
+    d = inputs(B, H, NC, seed=NC, eta_scale=eta_scale)
+    ck = oracle_forward(d, cgs)
+    check(run_backward(d, ck, cgs, 2), oracle_backward(d, ck, cgs), TOL, "hidden units over two CTAs")
+
+
+@pytest.mark.parametrize("B,H,NC,cgs", [(1, 34, 6, 6), (5, 12, 16, 16), (2, 37, 5, 1), (1, 74, 2, 2), (3, 50, 3, 3)])
+def test_two_ctas_without_groups_to_pipeline_at_every_stream_count(B, H, NC, cgs):
+    """34, 60 and 74 streams, which the launcher gives two CTAs by itself, and 150, more clusters than the device runs at once."""
+    d = inputs(B, H, NC, seed=H)
+    ck = oracle_forward(d, cgs)
+    one = run_backward(d, ck, cgs, 1)
+    a = run_backward(d, ck, cgs, 2)
+    b = run_backward(d, ck, cgs, 2 if B * H > 74 else None)
+    for k in GRAD_NAMES:
+        assert torch.equal(a[k], b[k]), f"{k} differs between two runs"
+    check(a, one, 1e-2, f"{B * H} streams against one CTA per stream")

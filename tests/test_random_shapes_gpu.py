@@ -23,7 +23,9 @@ def cases(seed, n):
              rnd.choice([1, 2, 3, 4, 8]), rnd.choice([1, 2, 4]), rnd.choice([0.01, 0.1, 1.0])) for i in range(n)]
 
 
-@pytest.mark.parametrize("it,B,H,NC,cgs,cluster,eta_scale", cases(1234, 12))
+# (the last three: two CTAs without groups to pipeline, which split the hidden units)
+@pytest.mark.parametrize("it,B,H,NC,cgs,cluster,eta_scale", cases(1234, 12) + [
+    (20, 1, 3, 7, 7, 2, 0.1), (21, 2, 2, 5, 1, 2, 1.0), (22, 1, 5, 12, 16, 2, 0.01)])
 def test_mlp_pair_on_a_random_shape(it, B, H, NC, cgs, cluster, eta_scale):
     dev = "cuda"
     d = orc.make_inputs(B, H, NC, seed=it, eta_scale=eta_scale, backward=True)
