@@ -71,7 +71,8 @@ def test_no_waiter_is_overtaken(case):
 
 
 @pytest.mark.parametrize("now,then,NC,what", [
-    ("{E_Z, E_PART, C5,", "{E_Z, kNo, C5,", 3, "races"),                                # a product that waits for less
+    ("{E_PART, kNo, kNo,", "{kNo, kNo, kNo,", 3, "races"),                              # a product that waits for less
+    ("{SGZ1, E_X, C2,", "{SGZ1, kNo, C2,", 3, "races"),
     ("wait(F_ZG);", "", 3, "races"),                                                    # an epilogue
     ("need = steps_before(g - 1) + own + 1;", "need = steps_before(g - 1) + own;", 9, "races"),      # a slot taken early
     ("w2 + 3 * 65536 + BIG;", "w2 + 2 * 65536 + BIG;", 5, "provenance"),                # arrays that share a slot's place

@@ -309,8 +309,8 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
 }
 __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
-enum : uint8_t { V_D, V_S2, V_C2, V_PART, V_C10, V_CB, V_C5, V_V, V_C3, V_C6, V_X, V_C7, V_COUNT };      // the sweep copies' events
-__constant__ const uint8_t kSweepEvent[V_COUNT] = {E_D, E_S2, C2, E_PART, C10, CB, C5, E_V, C3, C6, E_X, C7};
+enum : uint8_t { V_D, V_S2, V_C2, V_PART, V_C10, V_CB, V_C5, V_V, V_C3, V_C6, V_C7, V_COUNT };      // the sweep copies' events
+__constant__ const uint8_t kSweepEvent[V_COUNT] = {E_D, E_S2, C2, E_PART, C10, CB, C5, E_V, C3, C6, C7};
 constexpr int kSweepCopies = 19;
 __constant__ const CopyOp kSweepCopy[kSweepCopies] = {
     {V_D, K_LOAD, A_X2, SX2, R_Z, 0, 0, 0, 0, 0, BIG, BIG},
@@ -332,17 +332,19 @@ __constant__ const CopyOp kSweepCopy[kSweepCopies] = {
     {V_C6, K_TMA, M_V, SV, R_NONE, 1, 1, 0, S_V, 0, TILE, TILE},
     {V_C7, K_LOAD, A_W2, SW2, R_A, 1, 1, 0, 0, 0, BIG, BIG},
     {V_COUNT, K_NONE, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0}};
+// Two of these waits are not for an operand, they stand where the tensor pipe is busy or E4 runs: E_PART before G11b is for E5,
+// which overwrites gZ1 and adds to G_b1, and E_X before G8 for E4, which writes over the last step's addends to d_eta.
 constexpr int kSweepMmas = 13;
 __constant__ const MmaOp kSweepMma[kSweepMmas] = {
     {E_S1, SK, kNo, P_HID, R_S1, R_NONE, 0, 0, 0, S_K, TM_A},                  // G4
-    {SGZ1, kNo, C2, P_TOK, R_GZ, R_S1, 0, 0, 0, 0, TM_B},                     // G8
+    {SGZ1, E_X, C2, P_TOK, R_GZ, R_S1, 0, 0, 0, 0, TM_B},                     // G8
     {E_S2, SX2, kNo, P_TOK, R_Z, R_S2, 0, 0, 0, 0, TM_B + 64},                // G5
     {E_P, SW2, C4, P_TOK, R_S1, R_A, 0, 0, 0, 0, TM_A},                       // G6
     {SGZ2, kNo, C10, P_HID_MN, R_S1, R_NONE, 0, 0, 0, S_GZ2, TM_S2},          // G10
     {E_T, kNo, kNo, P_HID, R_A, R_NONE, 0, 0, 0, S_GZ2, TM_A},                // G12
-    {kNo, kNo, kNo, P_HID, R_S2, R_NONE, 0, 0, 0, S_Q, TM_B},                 // G11b
+    {E_PART, kNo, kNo, P_HID, R_S2, R_NONE, 0, 0, 0, S_Q, TM_B},              // G11b
     {SX2B, kNo, CB, P_HID_MN, R_GZ, R_NONE, 1, 0, 0, S_GZB, TM_S2},           // G2 of the next step
-    {E_Z, E_PART, C5, P_HID_ACC, R_A, R_NONE, 0, 0, 0, S_XF, TM_B},           // G11a (E5 overwrites gZ1 and adds to G_b1)
+    {E_Z, kNo, C5, P_HID_ACC, R_A, R_NONE, 0, 0, 0, S_XF, TM_B},              // G11a
     {kNo, kNo, kNo, P_HID_MN, R_Z, R_NONE, 0, 0, 0, S_XF, TM_S2},             // G14
     {SGZ1B, SQ, C3, P_HID_MN, R_S1, R_NONE, 1, 0, 0, S_Q, TM_S1},             // G3 of the next step
     {E_5, kNo, C6, P_HID_MN, R_GZ, R_NONE, 0, 0, 0, S_K, TM_S1},              // G15
@@ -1405,8 +1407,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
       // ---- E5: gZ1in^T = gX2^T gelu'(Z1^T) + R^T S^T
       wait_mma(C5);
-      // (over the first exchange: its last reader is behind E_Z, and E4 of the next step, which writes there again, needs the
-      // W2 that is loaded after E_X)
+      // (over the first exchange: its last reader is behind E_Z, and E4 of the next step, which writes there again, behind E_X)
       if (tm.l3 == 0) {
         float* xe = reinterpret_cast<float*>(smem + S_X1);
         xe[cq * 64 + tm.r0] = de0;
@@ -1579,7 +1580,10 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // d_eta; its fourth term, gZ1 G_b1, is summed over half of the hidden units by each of two warps: lane l takes the token pair (2 l, 2 l + 1)
   auto sweep_part = [&](int g, int half) {
     const int gsz = size_of(g);
-    if (g == 0 && !seen(E_5)) return;     // (the gradient state)
+    if (g == 0) {      // the gradient state is in place, and there are no addends yet
+      if (!seen(E_5)) return;
+      if (lane == 0) arrive(E_X);
+    }
     for (int j = gsz - 1; j >= 0; --j) {
       if (!seen(E_S1) || !seen(SGZ1)) return;
       const uint8_t* bg = smem + o_gz + half * 16384 + (lane & 3) * 4;      // (128 rows: the swizzle's phase is the same)
