@@ -53,16 +53,17 @@ WORKLOADS = {
 U_FLOP = 2 * 64 * 64 * 256            # one GEMM unit per mini-batch per (b,h)
 FWD_U, BWD_U = 7, 22                  # algorithmic GEMM units: forward; backward (7 recompute + 15 sweep)
 STATE_BYTES = 132352                  # fp32 W1 + b1 + W2 + b2 of one (b,h)
-# DRAM bytes per (stream, mini-batch) of the one-CTA backward from an ncu capture of the `prof` workload
-# (dram__bytes_read.sum + dram__bytes_write.sum over 128 streams x 16 mini-batches); the traffic grows in
-# proportion to the number of (stream, mini-batch) pairs, so a full-size launch is scaled from it.  The cluster kernels
-# ask for the same scratch bytes, but have no capture of their own that does not stay in L2.
-NCU_BWD_DRAM_BYTES_PER_MB = (583522304 + 587919104) / 2048
-# Scratch bytes the backward asks for per (stream, mini-batch): the recompute writes seven [256][64] bf16 images
-# (X2, Z1, dl/dZ1, gelu'(Z1_bar), X2_bar, W1^T, W2), three [64][64] bf16 tiles and two fp32[64] vectors; the sweep
-# reads the same back, X2 twice.
-SCRATCH_WRITE_PER_MB = 7 * 32768 + 3 * 8192 + 512
-SCRATCH_READ_PER_MB = 8 * 32768 + 3 * 8192 + 512
+# DRAM bytes per (stream, mini-batch) of a backward that gives a stream one CTA and of one that gives it a pair, from ncu
+# captures of the `prof` and `profc2` workloads (dram__bytes_read.sum + dram__bytes_write.sum over 128 and 64 streams x 16
+# mini-batches; profiles/); the traffic grows in proportion to the number of (stream, mini-batch) pairs, so a full-size
+# launch is scaled from it.  The kernels that split the hidden units ask for the same scratch bytes as one CTA, but have
+# no capture of their own that does not stay in L2.
+NCU_BWD_DRAM_BYTES_PER_MB = {"one": (583522304 + 587919104) / 2048, "pair": (267690496 + 272385536) / 1024}
+# Scratch bytes (written, read) per (stream, mini-batch).  The recompute writes seven [256][64] bf16 images (X2, Z1, dl/dZ1,
+# X2_bar, W1^T, W2 and gelu'(Z1_bar), as a pair dL/dZ1_bar), three [64][64] bf16 tiles and two fp32[64] vectors, as a pair
+# fp32[256] and three of 64; the sweep reads the same back, as one CTA X2 twice.
+SCRATCH_PER_MB = {"one": (7 * 32768 + 3 * 8192 + 512, 8 * 32768 + 3 * 8192 + 512),
+                  "pair": (7 * 32768 + 3 * 8192 + 1792, 7 * 32768 + 3 * 8192 + 1792)}
 
 
 def algorithmic_bytes(B, H, NC, cgs):
@@ -257,6 +258,7 @@ def run_ours(args, rank, world, local_rank):
     lib = _lib.lib()
     cl_fwd = lib.ttt_b200_launch_cluster(Bl * Hl, (cluster or 0) << 8, 0)
     cl_used = lib.ttt_b200_backward_ctas(Bl * Hl, NC, cgs, (cluster or 0) << 8)
+    pairs = lib.ttt_b200_backward_pairs(Bl * Hl, NC, cgs, (cluster or 0) << 8)
     bwd_launches = 2 if lib.ttt_b200_backward_tail(Bl * Hl, NC, cgs, (cluster or 0) << 8) else 1
 
     sampler = ClockSampler(local_rank)
@@ -415,10 +417,11 @@ def run_ours(args, rank, world, local_rank):
     bwd_tf = bwd_flop / (bwd_ms * 1e-3) / 1e12
     both_tf = (fwd_flop + bwd_flop) / ((fwd_ms + bwd_ms) * 1e-3) / 1e12
     n = -(-NC // cgs)
-    remat_bytes = Bl * Hl * (2 * n * STATE_BYTES + NC * (SCRATCH_WRITE_PER_MB + SCRATCH_READ_PER_MB))
-    dram_bwd = NCU_BWD_DRAM_BYTES_PER_MB * Bl * Hl * NC
+    per_mb = {"one": (Bl * Hl - pairs) * NC, "pair": pairs * NC}       # mini-batches by form
+    remat_bytes = Bl * Hl * 2 * n * STATE_BYTES + sum(m * sum(SCRATCH_PER_MB[k]) for k, m in per_mb.items())
+    dram_bwd = sum(m * NCU_BWD_DRAM_BYTES_PER_MB[k] for k, m in per_mb.items())
     bwd_kernel = "ttt_bwd_kernel" if cl_used == 1 else \
-        "ttt_bwd_pair_kernel" if cl_used == 2 and 1 < cgs < NC else f"ttt_bwd_cluster_kernel<{cl_used}>"
+        "ttt_bwd_pair_kernel" if pairs else f"ttt_bwd_cluster_kernel<{cl_used}>"
     res = {
         "metric": "ttt_mlp_fwd_bwd_tokens_per_s", "value": tokens_per_step / (ms_per_step * 1e-3),
         "unit": "tokens/s", "n_gpus": world, "steps": K, "warmup": W, "ms_per_step": ms_per_step,
@@ -449,8 +452,8 @@ def run_ours(args, rank, world, local_rank):
                      "unit": "TFLOP/s", "frac": bwd_tf / peak_tf,
                      "frac_of_burst": bwd_tf / burst, "frac_of_sustained": bwd_tf / sustained,
                      "traffic": dram_bwd,
-                     "traffic_note": "bytes per launch, scaled from an ncu capture of a smaller launch of the one-CTA "
-                                     "kernel by (streams x mini-batches); an estimate where a cluster kernel runs",
+                     "traffic_note": "bytes per launch, scaled from ncu captures of smaller launches (one CTA per stream, a "
+                                     "pair) by (streams x mini-batches); an estimate where the hidden units are split",
                      "peak_source": f"{pk_src}, " + ("burst cuBLAS bf16 (timed region under 1 s at full clock)" if use_burst
                                                      else "sustained cuBLAS bf16 (clock below maximum or a long region)")},
         "e2e": {"value": tokens_per_step / (e2e_ms * 1e-3), "unit": "tokens/s", "ms_per_step": e2e_ms,

@@ -298,6 +298,11 @@ int ttt_b200_backward_ctas(int streams, int NC, int checkpoint_group_size, uint3
  * gives two CTAs each.  0 if there is only one launch, -1 on error. */
 int ttt_b200_backward_tail(int streams, int NC, int checkpoint_group_size, uint32_t flags);
 
+/* How many of a backward's streams run as a pair of CTAs, one that recomputes and one that sweeps: all of them where
+ * ttt_b200_backward_ctas is two and there are groups of several mini-batches to pipeline (where there are not, the two CTAs
+ * take half of the hidden units each), those of ttt_b200_backward_tail, or none.  Returns -1 on error. */
+int ttt_b200_backward_pairs(int streams, int NC, int checkpoint_group_size, uint32_t flags);
+
 /* The widest cluster size whose capacity on the current device covers `streams`: four, else (forward only) two, else one.
  * TTT_B200_CLUSTER overrides.  Not what a launch runs between the two capacities: ttt_b200_launch_cluster is.  Returns
  * -1 on error. */

@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from oracle import ttt_mlp as orc
-from ttt_tk_b200 import ttt_forward, ttt_backward, take_status
+from ttt_tk_b200 import _lib, ttt_forward, ttt_backward, take_status
 from ttt_tk_b200.buffers import alloc_backward_buffers, alloc_checkpoints, GRAD_NAMES, CHECKPOINT_NAMES
 
 pytestmark = pytest.mark.gpu
@@ -125,6 +125,7 @@ def test_long_context_shape_with_the_launchers_own_cluster_choice():
 @pytest.mark.parametrize("B,H,NC,cgs", [(1, 1, 12, 12), (2, 2, 8, 8), (1, 3, 9, 1), (1, 2, 33, 64), (1, 1, 24, 1)])
 @pytest.mark.parametrize("eta_scale", [0.1, 1.0])
 def test_two_ctas_without_groups_to_pipeline_match_oracle(B, H, NC, cgs, eta_scale):
+    assert _lib.lib().ttt_b200_backward_pairs(B * H, NC, cgs, 2 << 8) == 0
     d = inputs(B, H, NC, seed=NC, eta_scale=eta_scale)
     ck = oracle_forward(d, cgs)
     check(run_backward(d, ck, cgs, 2), oracle_backward(d, ck, cgs), TOL, "hidden units over two CTAs")

@@ -38,6 +38,10 @@ def test_calls_that_pipeline_groups_take_two_ctas():
     c4, c2 = (_lib.lib().ttt_b200_cluster_capacity(c, 1) for c in (4, 2))
     assert [f(c4, 12, 4, 0), f(c4, 11, 4, 0), f(c4, 64, 3, 0), f(c4 + 1, 1, 1, 0), f(c2 + 1, 64, 8, 0)] == [2, 4, 4, 2, 1]
     assert [f(c4, 64, 8, c << 8) for c in (1, 2, 4, 3)] == [1, 2, 4, -1]
+    p = _lib.lib().ttt_b200_backward_pairs
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert [p(c4, 12, 4, 0), p(c4, 11, 4, 0), p(c2, 2, 1, 0), p(c2, 8, 8, 0), p(c2, 9, 8, 0), p(sms, 9, 8, 0), p(sms + 5, 9, 8, 0),
+            p(sms + 5, 8, 8, 0), p(c4, 64, 8, 3 << 8)] == [c4, 0, 0, 0, c2, 0, 5, 0, -1]
 
 
 @pytest.mark.parametrize("rest", [1, 2, 67, 74])

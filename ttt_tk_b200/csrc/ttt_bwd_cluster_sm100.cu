@@ -38,8 +38,9 @@
 // Bound by the chain: at four CTAs per stream the work of a phase is a few hundred cycles beside the latencies of MMA,
 // exchange, row sums and barriers.  Hence the epilogues work on packed fp32 pairs, take column sums from registers, and
 // leave the row sums that only the bias gradients need to the next MMA window.  Measured per mini-batch, 32 streams in
-// groups of 4: 15.5 -> 14.9 us (all rows' sums at once), -> 14.0 us (the rest); two CTAs per stream, 48 streams, 22.1 ->
-// 19.0-19.6 us.  Issue slots are used to 28-29 %, the tensor pipe to 9 % (four CTAs) and 14 % (two).
+// groups of 4: 15.5 -> 14.9 us (all rows' sums at once), -> 14.0 us (the rest).  Two CTAs per stream run here where there
+// are no groups to pipeline (else ttt_bwd_pair_sm100.cu), 48 streams x 32: 17.6 us in one group (one CTA: 20.7), 25.3 in
+// groups of one (31.4).  Issue slots are used to 28-29 %, the tensor pipe to 9 % (four CTAs) and 14 % (two).
 //
 // Every wait is bounded; a wait that runs out raises the abort flag of the whole cluster, the vote on
 // leaving a loop is taken CTA-wide at a barrier, and no CTA exits before its peers have reached the

@@ -16,7 +16,8 @@
 // "hidden-major" (hidden unit = TMEM lane), every 64x64 quantity "token-major" (token = TMEM lane, M = 64).  A CTA has
 // 16 epilogue warps and four helper warps that issue the MMAs and the bulk copies and wait for both, so that no epilogue
 // warp spends its issue slots on a product or sits on a buffer's barrier.  Epilogues and helpers hand each other work over
-// mbarriers; each completes once per mini-batch and everyone who waits for one waits for all its completions.
+// mbarriers; each completes once per mini-batch (E_5 and E_X once more, at the start) and everyone who waits for one waits for
+// all its completions.  tests/kernel_order.py derives the order of all accesses from this source and looks for gaps in it.
 //
 // Recompute (go = dL/dOut).  The chain group (warps 0..7) works a step ahead of the output group (warps 8..15):
 //   MMA1  Z1^T = W1^T K^T                     W2     bf16 copy of the new W2; b2

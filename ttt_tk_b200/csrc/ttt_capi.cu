@@ -103,7 +103,7 @@ int capacity(int cluster, bool backward) {
 // of 128 mini-batches in groups of 4 on a B200: forward 4.3 against 4.6 us per mini-batch with one CTA, backward 14.0
 // against 22.7; of the backward's longer calls: backward_ctas).  Where only clusters of two fit (34 to 74 streams), the
 // forward runs one CTA, whose output pass runs beside the chain in two groups of warps (4.6 us per mini-batch against 5.8
-// with two CTAs), and the backward two (60 streams in groups of 4: 14.3 us per mini-batch against 22.9 with one).  Beyond, one.
+// with two CTAs), and the backward two (60 streams in groups of 4: 13.3 us per mini-batch against 23.3 with one).  Beyond, one.
 static int ttt_launch_cluster(int streams, uint32_t flags, bool backward, int* cluster) {
   if (int rc = asked_cluster(flags, cluster)) return rc;
   if (*cluster != 0) return TTT_B200_OK;
@@ -116,14 +116,14 @@ static int ttt_launch_cluster(int streams, uint32_t flags, bool backward, int* c
 // A backward with two CTAs per stream gives them the recompute and the sweep (ttt_bwd_pair_sm100.cu) where there is
 // something to do side by side: groups of several mini-batches, and more than one of them.  Else each takes half of the
 // hidden units: a single group is within 4 % either way, groups of one mini-batch (one scratch slot, so that the two CTAs
-// take turns) 26 us per mini-batch against 28.
+// of a pair take turns) 26 us per mini-batch against 28.
 static bool runs_pair(int ctas, int NC, int cgs) { return ctas == 2 && cgs > 1 && NC > cgs; }
 
 // CTAs per stream of a backward.  Where four would fit, two are faster once a call has three groups of four mini-batches to
 // pipeline: the first group's recompute runs alone, and a group that has few slots to spare ends with a wait for the last of
 // the next (32 streams, pair against four CTAs, us per mini-batch: 256 mini-batches in groups of 16 9.3 / 13.2, 48 in groups
-// of 16 11.7 / 13.3, 24 in groups of 8 12.5 / 13.9, 12 in groups of 4 13.9 / 14.6; two groups: 16 in groups of 8 14.3 / 14.0,
-// 8 in groups of 4 15.5 / 14.7; small groups: 32 in groups of 3 14.8 / 14.7, in groups of 2 17.2 / 15.4).
+// of 16 11.7 / 13.3, 24 in groups of 8 12.5 / 13.8, 12 in groups of 4 14.0 / 14.5; two groups: 16 in groups of 8 14.1 / 14.0,
+// 8 in groups of 4 15.2 / 14.7; small groups: 32 in groups of 3 14.9 / 14.7, in groups of 2 17.2 / 15.4).
 static int backward_ctas(int streams, int NC, int cgs, uint32_t flags, int* ctas) {
   if (int rc = ttt_launch_cluster(streams, flags, true, ctas)) return rc;
   int asked = 0;
@@ -133,10 +133,11 @@ static int backward_ctas(int streams, int NC, int cgs, uint32_t flags, int* ctas
 
 // Streams of a backward with one CTA per stream that two CTAs per stream take, in a launch of their own after the others': those
 // beyond a multiple of the SMs, when the device runs them as pairs at once.  A turn over the SMs with one CTA per stream lasts
-// 21.7 us per mini-batch however few streams are in it, one of pairs 12.6 and some us of launch.  Backward, us, without and
-// with it: 176 streams x 64 in groups of 8 2798 / 2087, 192 x 37 in groups of 6 1700 / 1321, 312 x 52 in groups of 7 3480 /
-// 2918, 1536 x 16 in groups of 4 4312 / 4173; where pairs are most and have least to pipeline, 222 streams x 8 in groups of 2
-// 471 / 434, x 3 213 / 203, 370 x 3 313 / 307.
+// 21.7 us per mini-batch however few streams are in it, one of pairs 10 to 14 and some us of launch.  Backward, us, without
+// and with it: 176 streams x 64 in groups of 8 2786 / 2076, 192 x 37 in groups of 6 1686 / 1319, 312 x 52 in groups of 7 3476 /
+// 2927, 1536 x 16 in groups of 4 4310 / 4209; where pairs are most and have least to pipeline, 222 streams x 8 in groups of 2
+// 457 / 425, x 5 309 / 296, x 4 238 / 239, x 3 199 / 201, 370 x 3 300 / 304.  So it gains from five mini-batches on and is
+// within 2 % below (149 and 176 streams x 4 in groups of 2 236 / 233 and 235 / 229, x 3 196 / 198 and 195 / 194).
 static int backward_tail(int streams, int NC, int cgs, uint32_t flags, int ctas) {
   int asked = 0, dev = 0, sms = 0;
   if (ctas != 1 || !runs_pair(2, NC, cgs) || asked_cluster(flags, &asked) != TTT_B200_OK || asked != 0) return 0;
@@ -392,6 +393,12 @@ extern "C" int ttt_b200_backward_ctas(int streams, int NC, int checkpoint_group_
 extern "C" int ttt_b200_backward_tail(int streams, int NC, int checkpoint_group_size, uint32_t flags) {
   const int c = ttt_b200_backward_ctas(streams, NC, checkpoint_group_size, flags);
   return c < 0 ? -1 : backward_tail(streams, NC, checkpoint_group_size, flags, c);
+}
+
+extern "C" int ttt_b200_backward_pairs(int streams, int NC, int checkpoint_group_size, uint32_t flags) {
+  const int c = ttt_b200_backward_ctas(streams, NC, checkpoint_group_size, flags);
+  if (c < 0) return -1;
+  return runs_pair(c, NC, checkpoint_group_size) ? streams : backward_tail(streams, NC, checkpoint_group_size, flags, c);
 }
 
 extern "C" int ttt_b200_launch_cluster(int streams, uint32_t flags, int backward) {
