@@ -19,17 +19,17 @@ import re
 import numpy as np
 
 LANES = np.arange(32)
-SIZES = {"uint8_t": 1, "__nv_bfloat16": 2, "float": 4, "uint32_t": 4, "int": 4, "f32x2": 8, "float2": 8, "uint64_t": 8,
+SIZES = {"uint8_t": 1, "char": 1, "__nv_bfloat16": 2, "float": 4, "uint32_t": 4, "int": 4, "f32x2": 8, "float2": 8, "uint64_t": 8,
          "float4": 16, "uint4": 16}
 TYPES = set(SIZES) | {"bool", "long", "auto", "uint16_t", "TokFrag", "Frag16", "CopyOp", "MmaOp", "Product", "Lane", "unsigned", "void"}
 TEMPLATES = {"static_cast", "const_cast", "reinterpret_cast", "tma_wait_group_read", "tma_wait_group", "frag_allreduce2",
              "reg_take", "reg_give", "mma_hidden_lead", "mma_hidden_ta", "mma_lead", "mma_lead_ta"}
 # arithmetic on values, shuffles and fences: no access, no order
 PURE = set("""pk pk1 upk hsum add2 mul2 fma2 fmaf rsqrtf gelu_pair2 gelu_grad_h2 f32x2_to_f16x2 f16x2_to_f32x2 f32x2_to_bf16x2
-bf16x2_to_f32x2 bf16_lo bf16_hi pack_bf16 make_uint4 make_float2 __float_as_uint __uint_as_float __bfloat162float
+bf16x2_to_f32x2 bf16_lo bf16_hi pack_bf16 make_uint4 make_float2 make_float4 __float_as_uint __uint_as_float __bfloat162float
 __float2bfloat16 __shfl_xor_sync __syncwarp __threadfence fence_proxy_async_smem fence_proxy_async_all fence_mbar_init
 tc_fence_before_sync tc_fence_after_sync tmem_wait_ld tmem_wait_st tmem_alloc tmem_relinquish tmem_dealloc prefetch_tmap
-tma_commit_group globaltimer_ns atomicExch reg_take reg_give f16_pack""".split())
+prefetch_l2 tma_commit_group globaltimer_ns atomicExch reg_take reg_give f16_pack""".split())
 
 
 class Unknown:
@@ -272,7 +272,7 @@ class Block:
             q = closing(text, p)
             body = text[text.index("{", q) + 1:closing(text, text.index("{", q))]
             return ("lambda", m.group(1), params(text[p + 1:q]), Block(body).all())
-        if not text or word in ("using", "struct", "static_assert", "extern"):
+        if not text or word in ("using", "struct", "static_assert", "extern", "asm"):
             return ("block", [])
         if word == "return":
             return ("return", parse(text[6:]) if text[6:].strip() else None)
@@ -303,13 +303,35 @@ def params(text):
     return out
 
 
+def expand(text):
+    """Function-like macros, written out."""
+    for m in re.finditer(r"^#define (\w+)\(([^)]*)\)((?:.*\\\n)+.*\n)", text, re.M):
+        text = text.replace(m.group(0), "")
+        while True:
+            use = re.search(r"\b%s\(" % m.group(1), text)
+            if not use:
+                break
+            e, body, depth, args, start = closing(text, use.end() - 1), m.group(3).replace("\\\n", "\n"), 0, [], use.end()
+            for k in range(use.end(), e + 1):
+                depth += text[k] in "([{"
+                depth -= text[k] in ")]}"
+                if k == e or text[k] == "," and depth == 0:
+                    args.append(text[start:k])
+                    start = k + 1
+            for name, a in zip(split(m.group(2)), args):
+                body = re.sub(r"\b%s\b" % name, lambda _: a, body)
+            text = text[:use.start()] + body + text[e + 1:]
+    return text
+
+
 class Source:
     """Constants, enums, tables, helper functions and fragment maps of some files; and a kernel's body."""
 
     def __init__(self, *paths, edit=lambda text: text):
         text = "\n".join(edit(open(p).read()) for p in paths)
-        text = re.sub(r"/\*.*?\*/", "", re.sub(r"//[^\n]*", "", text), flags=re.S)
+        text = expand(re.sub(r"/\*.*?\*/", "", re.sub(r"//[^\n]*", "", text), flags=re.S))
         self.text = re.sub(r"^\s*#.*$", "", text, flags=re.M)
+        self.barriers = {}
         self.names, self.functions, self.maps = {"true": True, "false": False, "nullptr": 0, "T": True, "F": False}, {}, {}
         ev = lambda e: Walker.constant(self, e)                                                   # noqa: E731
         for m in re.finditer(r"\benum\b[^{;]*\{([^}]*)\}|constexpr (?:int|uint32_t|uint8_t|float) ([^;{}()]*=[^;]*);", self.text):
@@ -581,6 +603,8 @@ class Walker:
         leaf = getattr(self.leaf, "f_" + name, None)
         if leaf is not None:
             return leaf(self, *targs, *[self.ev(x, sc) for x in e[2]])
+        if name not in self.src.functions:
+            raise KeyError(f"{name}: neither here nor in the sources")
         prm, body = self.src.functions[name]
         if isinstance(body, str):
             body = Block(body).all()
@@ -750,6 +774,9 @@ class Agent:
     def f___all_sync(self, w, m, v): return bool(np.all(v))
     def f_mapa(self, w, addr, rank): return Ptr("s", addr, 1, cta=rank)
     def f_uniform(self, w, v): return v
+    def f_long(self, w, v): return v
+    def f_min(self, w, a, b): return min(a, b)
+    def f_smem_align_1024(self, w, p): return p
 
     # -- barriers
     def f_mbar_init(self, w, p, count): self.r.count[self.bar(p)] = int(count)
@@ -774,6 +801,8 @@ class Agent:
         b = np.unique(np.broadcast_to(b, 32)[w.mask])
         assert len(b) == 1
         return self.wait((self.cta, int(b[0])))
+
+    f_wait_bar = f_wait
 
     def f_bounded(self, w, b, parity):                  # with a parity of the caller's own: the last such phase of its kernel
         phase = self.r.bounded_phase
@@ -899,6 +928,7 @@ class Agent:
 
     def f_mma_lead(self, w, acc, d, a, b, idesc, lead): self.product(d, a, b, idesc)
     def f_mma_lead_rt(self, w, d, a, b, idesc, acc, lead): self.product(d, a, b, idesc)
+    def f_mma_issue_rt(self, w, d, a, b, idesc, acc): self.product(d, a, b, idesc)
     def f_mma_lead_ta(self, w, acc, d, a, b, idesc, lead): self.product(d, a, b, idesc, True)
     def f_umma_commit(self, w, p): self.arrive(self.bar(p), "products", [self.tensor[0]] if self.tensor else [])
 
@@ -924,7 +954,7 @@ class Run:
                 a = Agent(self, cta, warp)
                 w = Walker(source, a)
                 sc = Scope()
-                sc.v.update(params, smem=Ptr("s", 0, 1), threadIdx=Struct(x=warp * 32 + LANES), blockIdx=Struct(x=cta))
+                sc.v.update(params, smem=Ptr("s", 0, 1), smem_raw=Ptr("s", 0, 1), threadIdx=Struct(x=warp * 32 + LANES), blockIdx=Struct(x=cta))
                 inner = Scope(sc)
                 self.agent_scope = inner
                 try:

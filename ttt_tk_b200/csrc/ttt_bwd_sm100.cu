@@ -381,9 +381,9 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           }
         }
       }
+      if (tid == kProd && j > 0) tma_wait_group_read<0>();     // the previous mini-batch's x_hat_ln has left the U2 tile
       publish();
       if (tid == kProd) {
-        tma_wait_group_read<0>();     // the previous mini-batch's x_hat_ln has left the U2 tile (rewritten after MMA2)
         bulk_store_1d(p.sc_X2 + slot * BIG, bX2, BIG);
         bulk_store_1d(p.sc_Z1 + slot * BIG, bZ1, BIG);
         tma_commit_group();
