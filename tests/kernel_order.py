@@ -804,6 +804,9 @@ class Agent:
 
     f_wait_bar = f_wait
 
+    def f_skip_bar(self, w, b):
+        self.waits[self.cta, int(b)] = self.waits.get((self.cta, int(b)), 0) + 1
+
     def f_bounded(self, w, b, parity):                  # with a parity of the caller's own: the last such phase of its kernel
         phase = self.r.bounded_phase
         assert phase & 1 == parity

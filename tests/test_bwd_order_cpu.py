@@ -28,7 +28,7 @@ def run(NC, cgs):
         setattr(p, k, ko.Ptr("g", i + 1 << 40, 1))
     maps = {f"tm{k}": i for i, k in enumerate(["Q", "K", "V", "Go", "DQ", "DK", "DV"])}
     return ko.Run(src, "ttt_bwd_kernel", dict(maps, p=p), {i + 1: n * cgs for i, n in enumerate(SCRATCH.values())}, 1, 8,
-                  skip=("wait_bar",))
+                  skip=("wait_bar", "skip_bar"))
 
 
 @pytest.mark.parametrize("case", CASES)
@@ -40,3 +40,8 @@ def test_every_wait_ends_and_the_scratch_holds_what_was_stored(case):
 @pytest.mark.parametrize("case", CASES)
 def test_no_two_accesses_are_unordered(case):
     assert run(*case).races() == []
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_no_waiter_is_overtaken(case):
+    assert run(*case).phases() == set()

@@ -199,7 +199,7 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
 
-  // ---- barrier bookkeeping: every thread waits on every barrier use, in program order
+  // ---- barrier bookkeeping: every thread waits on every barrier use, in program order, or counts it (skip_bar)
   uint32_t ph = 0;        // expected parity per barrier
   uint32_t pending = 0;   // thread 0: loads issued and not yet waited for
   auto wait_bar = [&](int b) {
@@ -208,6 +208,7 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       pending &= ~(1u << b);
     }
   };
+  auto skip_bar = [&](int b) { ph ^= 1u << b; };      // a use that this warp need not wait for
   auto wait_mma = [&]() {
     wait_bar(BAR_MMA);
     __syncwarp();
@@ -827,7 +828,10 @@ ttt_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       }
       wait_bar(BAR_BIG + ib4);
       wait_bar(BAR_T + 4);
-      wait_bar(BAR_BIG + ib1);      // X2, requested two phases ago
+      // X2, requested two phases ago.  Only those who issue MMAs or the next load wait: nothing would hold that load, of W2
+      // into the same buffer, back until a warp without a part in them had seen this one.
+      if (warp <= kProd / 32) wait_bar(BAR_BIG + ib1);
+      else skip_bar(BAR_BIG + ib1);
       // G4 // G8 // G5
       TTT_ISSUE(mma_token_major(tmem + TM_B, smem_u32(big(ib4)), smem_u32(big(ib0))),
                 mma_token_major(tmem + TM_B + 64, smem_u32(big(ib1)), smem_u32(big(ib3))),
