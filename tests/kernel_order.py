@@ -23,13 +23,14 @@ SIZES = {"uint8_t": 1, "char": 1, "__nv_bfloat16": 2, "float": 4, "uint32_t": 4,
          "float4": 16, "uint4": 16}
 TYPES = set(SIZES) | {"bool", "long", "auto", "uint16_t", "TokFrag", "Frag16", "CopyOp", "MmaOp", "Product", "Lane", "unsigned", "void"}
 TEMPLATES = {"static_cast", "const_cast", "reinterpret_cast", "tma_wait_group_read", "tma_wait_group", "frag_allreduce2",
-             "reg_take", "reg_give", "mma_hidden_lead", "mma_hidden_ta", "mma_lead", "mma_lead_ta"}
+             "reg_take", "reg_give", "send_impl", "run_impl", "tok_row_allreduce", "mma_hid64", "mma_hidden_lead", "mma_hidden_ta", "mma_lead", "mma_lead_ta"}
 # arithmetic on values, shuffles and fences: no access, no order
 PURE = set("""pk pk1 upk hsum add2 mul2 fma2 fmaf rsqrtf gelu_pair2 gelu_grad_h2 f32x2_to_f16x2 f16x2_to_f32x2 f32x2_to_bf16x2
 bf16x2_to_f32x2 bf16_lo bf16_hi pack_bf16 make_uint4 make_float2 make_float4 __float_as_uint __uint_as_float __bfloat162float
 __float2bfloat16 __shfl_xor_sync __syncwarp __threadfence fence_proxy_async_smem fence_proxy_async_all fence_mbar_init
 tc_fence_before_sync tc_fence_after_sync tmem_wait_ld tmem_wait_st tmem_alloc tmem_relinquish tmem_dealloc prefetch_tmap
-prefetch_l2 tma_commit_group globaltimer_ns atomicExch reg_take reg_give f16_pack""".split())
+prefetch_l2 tma_commit_group globaltimer_ns atomicExch reg_take reg_give f16_pack
+gelu_half2 __shfl_down_sync RS_row_layernorm RS_row_sums griddep_launch griddep_wait""".split())
 
 
 class Unknown:
@@ -65,6 +66,23 @@ class Struct:
 
     def copy(self):
         return Struct(**self.__dict__)
+
+
+class Object:
+    """Of a class template that Source.template has read: members and methods share a scope."""
+
+    def __init__(self, walker, constants, methods):
+        scope = Scope()
+        scope.v.update(constants, n=0, nx=0)
+        scope.v.update({name: (scope, prm, body) for name, (prm, body) in methods.items()})
+        self.__dict__.update(off=None, scope=scope, walker=walker)
+
+    def __getattr__(self, name):
+        v = self.scope.v[name]
+        return (lambda *a: self.walker.run(v[1], v[2], list(a), Scope(v[0], self.walker.mask))) if isinstance(v, tuple) else v
+
+    def __setattr__(self, name, v):
+        self.scope.v[name] = v
 
 
 # ------------------------------------------------------------------------------------------------ expressions
@@ -244,7 +262,7 @@ class Block:
         word = re.match(r"\w+", s[self.i:])
         word = word.group(0) if word else ""
         if word == "if":
-            self.i += 2
+            self.i += re.match(r"if(\s+constexpr)?", s[self.i:]).end()
             c = parse(self.paren())
             a = self.one()
             self.ws()
@@ -279,7 +297,7 @@ class Block:
         if word == "break":
             return ("break",)
         m = DECL.match(text)
-        if m and m.group(1).split()[-1] in TYPES | {"TokMap", "TokMap16"}:
+        if m and (m.group(1).split()[-1] in TYPES | {"TokMap", "TokMap16"} or m.group(1).endswith("_object")):
             names = []
             for d in split(text[m.end():]):
                 n = re.match(r"[*&\s]*(\w+)", d)
@@ -295,11 +313,18 @@ class Block:
         return ("expr", parse(text))
 
 
+class Name(str):
+    default = None
+
+
 def params(text):
+    """(name, by reference) of each, the name with its default."""
     out = []
     for p in split(text):
-        m = re.search(r"(\w+)(?:\)?(?:\[\w*\])*)?$", p)
-        out.append((m.group(1), "&" in p or "*" in p))
+        head, _, default = p.partition("=")
+        name = Name(re.search(r"(\w+)(?:\)?(?:\[\w*\])*)?$", head.strip()).group(1))
+        name.default = default.strip()
+        out.append((name, "&" in head or "*" in head))
     return out
 
 
@@ -331,7 +356,7 @@ class Source:
         text = "\n".join(edit(open(p).read()) for p in paths)
         text = expand(re.sub(r"/\*.*?\*/", "", re.sub(r"//[^\n]*", "", text), flags=re.S))
         self.text = re.sub(r"^\s*#.*$", "", text, flags=re.M)
-        self.barriers = {}
+        self.barriers, self.classes = {}, {}
         self.names, self.functions, self.maps = {"true": True, "false": False, "nullptr": 0, "T": True, "F": False}, {}, {}
         ev = lambda e: Walker.constant(self, e)                                                   # noqa: E731
         for m in re.finditer(r"\benum\b[^{;]*\{([^}]*)\}|constexpr (?:int|uint32_t|uint8_t|float) ([^;{}()]*=[^;]*);", self.text):
@@ -364,7 +389,7 @@ class Source:
             b = self.text.index("{", q)
             body = self.text[b + 1:closing(self.text, b)]
             if "asm" not in body and m.group(2) not in PURE:
-                tp = [(x.split()[-1], False) for x in split(m.group(1) or "")]
+                tp = [(Name(x.split()[-1]), False) for x in split(m.group(1) or "")]
                 self.functions[m.group(2)] = (tp + params(self.text[m.end():q]), body)
         for m in re.finditer(r"struct (TokMap\w*) \{", self.text):
             body = self.text[m.end():closing(self.text, m.end() - 1)]
@@ -372,6 +397,24 @@ class Source:
             members = [(x[:x.index("(")], x[x.index("(") + 1:-1]) for x in split(init)]
             methods = re.findall(r"(\w+)\(([^)]*)\) const \{ return (.*?); \}", body)
             self.maps[m.group(1)] = (members, [(n, params(p), e) for n, p, e in methods])
+
+    def template(self, name, prefix, **args):
+        """A class template's constants and methods for these arguments; its static ones are also entered as <prefix>name."""
+        i = self.text.index("{", re.search(r"struct %s \{" % name, self.text).start())
+        body, consts, methods = self.text[i + 1:closing(self.text, i)], dict(args), {}
+        for m in re.finditer(r"static constexpr (?:int|uint32_t|bool) (\w+) = ([^;]*);", body):
+            sc = Scope()
+            sc.v.update(consts)
+            consts[m.group(1)] = Walker(self, None).ev(parse(m.group(2)), sc)
+        for m in re.finditer(r"(?:template <([^>]*)>\s*)?(?:static )?__device__ __forceinline__ [\w ]+?[\s&*]+(\w+)\(", body):
+            q = closing(body, m.end() - 1)
+            b = body.index("{", q)
+            code = Block(body[b + 1:closing(body, b)]).all()
+            methods[m.group(2)] = ([(x.split()[-1], False) for x in split(m.group(1) or "")] + params(body[m.end():q]), code)
+        self.names.update({prefix + k: v for k, v in consts.items()})
+        self.functions.update({prefix + k: v for k, v in methods.items()})
+        self.classes[prefix + "object"] = (consts, methods)
+        return consts
 
     def body(self, kernel):
         i = self.text.index("(", self.text.index(kernel))
@@ -560,7 +603,9 @@ class Walker:
             s.v[e[1]] = value if same else self.merge(value, s.v[e[1]])
         elif e[0] == "mem":
             a = self.ev(e[1], sc)
-            if isinstance(a, Struct):
+            if isinstance(a, Object):
+                setattr(a, e[2], value)
+            elif isinstance(a, Struct):
                 setattr(a, e[2], self.merge(value, getattr(a, e[2], U)))
         else:
             if e[0] == "idx" and isinstance(self.ev(e[1], sc), (Unknown, list)):
@@ -595,7 +640,7 @@ class Walker:
         s = sc.find(name)
         if s is not None and isinstance(s.v[name], tuple):
             scope, prm, body = s.v[name]
-            return self.run(prm, body, [self.ev(x, sc) for x in e[2]], Scope(scope, self.mask))
+            return self.run(prm, body, targs + [self.ev(x, sc) for x in e[2]], Scope(scope, self.mask))
         if name in PURE:
             for x in e[2]:
                 self.ev(x, sc)
@@ -612,6 +657,7 @@ class Walker:
         return self.run(prm, body, targs + [self.ev(x, sc) for x in e[2]], Scope(None, self.mask))
 
     def run(self, prm, body, args, scope):
+        args = args + [self.ev(parse(n.default), scope) for n, _ in prm[len(args):]]
         for (n, ref), a in zip(prm, args):
             scope.v[n] = a.copy() if isinstance(a, Struct) and not ref and not hasattr(a, "off") else a
         mask, gone, entry = self.mask, self.gone, self.entry
@@ -643,7 +689,8 @@ class Walker:
                     v = self.ev(init, sc)
                     sc.v[name] = v.copy() if isinstance(v, Struct) and not hasattr(v, "off") else v
                 else:
-                    sc.v[name] = Struct() if st[1] in ("Lane", "Product") else U
+                    sc.v[name] = Struct() if st[1] in ("Lane", "Product") else \
+                        Object(self, *self.src.classes[st[1]]) if st[1].endswith("_object") else U
         elif k == "if":
             c = self.truth(self.ev(st[1], sc))
             if c is True or c is False:
@@ -736,11 +783,14 @@ class Agent:
         return (self.cta if p.cta is None else p.cta, i)
 
     # -- accesses
+    def span(self, cta, addr, nbytes):
+        """The places of some bytes of shared memory: of 16, in the vectors of 4."""
+        grain = 16 if addr < self.r.vectors else 4
+        return {("s", cta, k * grain) for k in range(addr // grain, (addr + nbytes - 1) // grain + 1)}
+
     def keys(self, w, p, size):
         addr = np.broadcast_to(p.addr, 32)[w.mask]
-        cta = self.cta if p.cta is None else p.cta
-        return {("s", cta, int(k)) for k in np.unique(addr // 16)} if size <= 16 else \
-            {("s", cta, int(a) // 16 + k) for a in np.unique(addr) for k in range(size // 16)}
+        return set().union(*[self.span(self.cta if p.cta is None else p.cta, a, size) for a in np.unique(addr).tolist()])
 
     def touch(self, w, p, size, write):
         if p.space == "s":
@@ -765,6 +815,7 @@ class Agent:
     def f_tmem_st32(self, w, addr, v): return self.tmem(addr, 32, True)
     def f_tmem_ld_16x256b_x2(self, w, addr, v): return self.tmem(addr, 16, False)
     def f_tmem_ld_16x256b_x4(self, w, addr, v): return self.tmem(addr, 32, False)
+    def f_tmem_st_16x256b_x4(self, w, addr, v): return self.tmem(addr, 32, True)
 
     # -- plain helpers
     def f_smem_u32(self, w, p): return p.addr if p.cta is None else p
@@ -803,6 +854,25 @@ class Agent:
         return self.wait((self.cta, int(b[0])))
 
     f_wait_bar = f_wait
+
+    def f_mbar_wait_cl(self, w, p, parity, *_):
+        b = self.bar(Ptr("s", int(np.unique(np.broadcast_to(p.addr, 32)[w.mask])[0]), 8))
+        assert self.waits.get(b, 0) & 1 == parity, f"{self.name}: the use of {self.r.label(b)} that it waits for is not the next"
+        return self.wait(b)
+
+    def st_async(self, w, addr, bar, size):
+        addr, peer, bar = (np.broadcast_to(v, 32)[w.mask].tolist() for v in (addr.addr, addr.cta, bar.addr))
+        for c in sorted(set(peer)):
+            to = [(a, b) for a, b, q in zip(addr, bar, peer) if q == c]
+            n = self.issue(f"stores into cta {c}")
+            n.writes |= set().union(*[self.span(c, a, size) for a, _ in to])
+            # (a warp waits for every use of its own CTA's barrier, and sends for a use before it waits for it)
+            i = (to[0][1] - self.r.off_bar) // 8
+            self.r.loads.append(((c, i), size * len(to), n, self.waits.get((self.cta, i), 0)))
+
+    def f_st_async_f1(self, w, addr, bar, *v): self.st_async(w, addr, bar, 4)
+    def f_st_async_f2(self, w, addr, bar, *v): self.st_async(w, addr, bar, 8)
+    def f_st_async_f4(self, w, addr, bar, *v): self.st_async(w, addr, bar, 16)
 
     def f_skip_bar(self, w, b):
         self.waits[self.cta, int(b)] = self.waits.get((self.cta, int(b)), 0) + 1
@@ -856,9 +926,9 @@ class Agent:
         b = self.bar(Ptr("s", bar, 8))
         n = self.issue(f"load for {self.r.label(b)}")
         assert dst % 16 == 0 and 0 <= dst and dst + nbytes <= self.r.smem_bytes
-        n.writes |= {("s", self.cta, dst // 16 + k) for k in range(nbytes // 16)}
+        n.writes |= self.span(self.cta, dst, nbytes)
         n.reads |= reads
-        self.r.loads.append((b, nbytes, n, self))
+        self.r.loads.append((b, nbytes, n, None))
 
     def each(self, w, *vals):
         return zip(*[np.broadcast_to(v.addr if isinstance(v, Ptr) else v, 32)[w.mask].tolist() for v in vals])
@@ -869,16 +939,18 @@ class Agent:
 
     def scratch(self, addr, nbytes):
         base = addr >> 40
-        assert base in self.r.scratch and (addr & (1 << 40) - 1) + nbytes <= self.r.scratch[base] and nbytes % 256 == 0
+        if base not in self.r.scratch:
+            return set()
+        assert (addr & (1 << 40) - 1) + nbytes <= self.r.scratch[base] and nbytes % 256 == 0
         return {("g", (addr + k) >> 8) for k in range(0, nbytes, 256)}
 
     def f_bulk_load_1d(self, w, dst, src, nbytes, bar):
         for d, s, n, b in self.each(w, dst, src, nbytes, bar):
-            self.load_one(d, n, b, self.scratch(s, n) if s >> 40 in self.r.scratch else set())
+            self.load_one(d, n, b, self.scratch(s, n))
 
     def store(self, lane, src, nbytes, writes):
         read = self.issue(f"store from {src}")
-        read.reads |= {("s", self.cta, src // 16 + k) for k in range(nbytes // 16)}
+        read.reads |= self.span(self.cta, src, nbytes)
         done = self.r.node(f"{self.name} store's end", [read])
         done.writes |= writes
         self.stores.setdefault(lane, []).append([read, done])
@@ -923,9 +995,9 @@ class Agent:
         if a_tmem:
             t.reads |= {("t", self.cta, q, (a & 0xffff) // 8) for q in range(4)}
         else:
-            t.reads |= {("s", self.cta, int(k)) for k in self.rows(a, not idesc >> 15 & 1, m)}
+            t.reads |= {("s", self.cta, int(k) * 16) for k in self.rows(a, not idesc >> 15 & 1, m)}
         # (a product of 16 columns is a row sum: only its first column is used, the others multiply what happens to lie there)
-        t.reads |= {("s", self.cta, int(k)) for k in self.rows(b, not idesc >> 16 & 1, 1 if n == 16 else n)}
+        t.reads |= {("s", self.cta, int(k) * 16) for k in self.rows(b, not idesc >> 16 & 1, 1 if n == 16 else n)}
         t.writes |= {("t", self.cta, q, c) for q in range(4) for c in range((d & 0xffff) // 8, ((d & 0xffff) + n) // 8)}
         assert (d & 0xffff) + n <= 512
 
@@ -944,9 +1016,11 @@ class Run:
     """All warps of one cluster.  `params`: the kernel's argument struct and constants; `scratch`: allocations behind the
     scratch pointers (their addresses are (index << 40) + offset) and their sizes."""
 
-    def __init__(self, source, kernel, params, scratch, ctas, warps, skip=("bounded", "wait", "arm", "uniform")):
+    def __init__(self, source, kernel, params, scratch, ctas, warps, skip=("bounded", "wait", "arm", "uniform"), prefix="",
+                 vectors=None):
         self.src, self.ctas, self.warps, self.scratch = source, ctas, warps, scratch
-        self.off_bar, self.off_misc, self.smem_bytes = (source.names[k] for k in ("OFF_BAR", "OFF_MISC", "SMEM_BYTES"))
+        self.off_bar, self.off_misc, self.smem_bytes = (source.names[prefix + k] for k in ("OFF_BAR", "OFF_MISC", "SMEM_BYTES"))
+        self.vectors = self.smem_bytes if vectors is None else vectors      # where accesses are told apart by 4 bytes
         self.nodes, self.count, self.meets = [], {}, {}
         self.arrivals, self.expected, self.waiters, self.loads = {}, {}, [], []
         self.released, self.acquired = [], []
@@ -983,27 +1057,27 @@ class Run:
     # -- what orders what
     def link(self):
         self.problems = []
-        # an agent's k-th arrival belongs to phase k: each phase takes one of every agent that arrives there
+        # a phase takes the same share of every agent's arrivals
         self.phase = {}
         for b, by in self.arrivals.items():
-            if len(by) != self.count[b]:
-                self.problems.append(f"{self.label(b)}: {len(by)} warps arrive, {self.count[b]} are waited for")
+            phases, rest = divmod(sum(map(len, by.values())), self.count[b])
+            if rest or any(len(nodes) % max(phases, 1) for nodes in by.values()):
+                self.problems.append(f"{self.label(b)}: {[len(x) for x in by.values()]} arrivals, {self.count[b]} to a phase")
+                continue
             for nodes in by.values():
                 for k, n in enumerate(nodes):
-                    self.phase.setdefault(b, {}).setdefault(k, []).append(n)
+                    self.phase.setdefault(b, {}).setdefault(k * phases // len(nodes), []).append(n)
         arrived = {b: {k: len(v) for k, v in ph.items()} for b, ph in self.phase.items()}
-        tx = {}
-        for b, nbytes, n, a in self.loads:
-            k = tx.setdefault(b, [0, 0])                # phase, bytes so far
-            self.phase[b].setdefault(k[0], []).append(n)
-            k[1] += nbytes
-            if k[1] == self.expected[b][k[0]]:
-                tx[b] = [k[0] + 1, 0]
-            elif k[1] > self.expected[b][k[0]]:
-                self.problems.append(f"{n.what}: more bytes than {self.label(b)} expects")
-        for b, (k, got) in tx.items():
-            if got:
-                self.problems.append(f"{self.label(b)}: {got} bytes of {self.expected[b][k]}")
+        brought = {}
+        for b, nbytes, n, k in self.loads:              # k: the phase, of a CTA's own loads the first that is not complete
+            got, want = brought.setdefault(b, [0] * len(self.expected[b])), self.expected[b]
+            if k is None:
+                k = next((i for i, x in enumerate(got) if x < want[i]), len(got) - 1)
+            got[k] += nbytes
+            self.phase[b].setdefault(k, []).append(n)
+        for b, got in brought.items():
+            if got != self.expected[b]:
+                self.problems.append(f"{self.label(b)}: {got} bytes, expected {self.expected[b]}")
         for b, phase, n, a in self.waiters:
             by = self.phase.get(b, {}).get(phase, [])
             if arrived.get(b, {}).get(phase) != self.count[b]:

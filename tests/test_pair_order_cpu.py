@@ -49,7 +49,7 @@ def place(r, key):
     if key[0] != "s":
         return key[0]
     offs = [(v, k) for k, v in r.src.names.items() if isinstance(v, int) and
-            re.match("(OFF|%s)_" % ("S" if key[1] < r.ctas // 2 else "R"), k) and v <= key[2] * 16]
+            re.match("(OFF|%s)_" % ("S" if key[1] < r.ctas // 2 else "R"), k) and v <= key[2]]
     return max(offs)[1]
 
 

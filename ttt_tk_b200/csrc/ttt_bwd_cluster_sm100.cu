@@ -94,10 +94,10 @@ struct Cfg {
   static constexpr uint32_t OFF_SIGLN = OFF_DB + 256;
   static constexpr uint32_t OFF_SIGF = OFF_SIGLN + 256;
   static constexpr uint32_t OFF_GB1 = OFF_SIGF + 256;       // fp32[R] copy of the per-thread dL/db1
-  static constexpr uint32_t OFF_PART = OFF_GB1 + 1024;      // fp32[8][64] partial sums for d_eta (one row per warp)
+  static constexpr uint32_t OFF_PART = OFF_GB1 + 1024;      // fp32[4][64] partial sums for d_eta (one row per quadrant)
   // fp32[3][4][64] column-sum partials (the row-split form keeps the second-order stage's own-row partials,
   // 2 x [8][64], in the row-sum exchange area, which is not in use between that stage and their sum)
-  static constexpr uint32_t OFF_CSUM = OFF_PART + 2048;
+  static constexpr uint32_t OFF_CSUM = OFF_PART + 1024;
   static constexpr uint32_t OFF_ETA = OFF_CSUM + 3072;      // bf16[2][64]
   static constexpr uint32_t OFF_BAR = OFF_ETA + 256;
   static constexpr uint32_t OFF_MISC = OFF_BAR + 192;
@@ -1015,16 +1015,18 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                  mma_tok_partial(tmem + C::TM_B + 64, smem_u32(big(ib1)), smem_u32(big(ib3)), NB, lead),
                  HID_ONE(false, C::TM_A, big(ib0), t_k, 0u, 0),
                  if (NB > 1) HID_ONE(false, C::TM_A, big(ib0), t_k, 0u, NB - 1))
-      // ---- while the MMAs run: partial sums over this CTA's hidden units of gZ1 * G_b1 (fourth term of d_eta)
+      // ---- while the MMAs run: partial sums over this CTA's hidden units of gZ1 * G_b1 (fourth term of d_eta).  A warp takes
+      // the elements of gZ1 that its own fragment of P overwrites in E3: nothing holds another warp's E3 back until here.
       {
-        // warp w takes hidden units (R / 8) w .., lane l the token pair (2 l, 2 l + 1)
-        constexpr int RW = C::R / 8;
-        const uint8_t* bg = big(ib4) + (lane & 3) * 4;
-        const uint32_t chunk = lane >> 2;
+        // lane l takes the token pair l % 16 of the warp's 32 tokens and, of the quadrant's 16 rows of a block, 0..3 and
+        // 8..11 or, l >= 16, the others: the two half warps read opposite halves of the swizzled lines, without conflicts
+        const int sub = (lane >> 4) * 4, pair = lane & 15;
+        const uint8_t* bg = big(ib4) + (pair & 3) * 4;
+        const uint32_t chunk = tm.colhalf * 4 + (pair >> 2);
         float a0 = 0.f, a1 = 0.f, c0 = 0.f, c1 = 0.f;
 #pragma unroll
-        for (int hh = 0; hh < RW; hh += 4) {
-          const int h = warp * RW + hh;
+        for (int hh = 0; hh < 8 * NB; hh += 4) {
+          const int h = (hh >> 3) * 64 + tm.quad * 16 + (hh & 4) * 2 + sub;
           const float4 g = *reinterpret_cast<const float4*>(sGb1 + h);
           const uint32_t w0 = *reinterpret_cast<const uint32_t*>(bg + sw128_off(h, chunk));
           const uint32_t w1 = *reinterpret_cast<const uint32_t*>(bg + sw128_off(h + 1, chunk));
@@ -1035,7 +1037,11 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           a0 = fmaf(bf16_lo(w2), g.z, a0); a1 = fmaf(bf16_hi(w2), g.z, a1);
           c0 = fmaf(bf16_lo(w3), g.w, c0); c1 = fmaf(bf16_hi(w3), g.w, c1);
         }
-        *reinterpret_cast<float2*>(sPart + warp * 64 + 2 * lane) = make_float2(a0 + c0, a1 + c1);
+        a0 += c0;
+        a1 += c1;
+        a0 += __shfl_xor_sync(0xffffffffu, a0, 16);
+        a1 += __shfl_xor_sync(0xffffffffu, a1, 16);
+        if (lane < 16) *reinterpret_cast<float2*>(sPart + tm.quad * 64 + tm.colhalf * 32 + 2 * pair) = make_float2(a0, a1);
       }
       if constexpr (C::kRowSplit) {
         // finished inside E4's wait for its own sum
@@ -1118,9 +1124,9 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           }
           if (row_writer) {     // the partial sums over this CTA's hidden units of gZ1 * G_b1, once per row
 #pragma unroll
-            for (int w = 0; w < 8; ++w) {
-              de0 += sPart[w * 64 + tm.r0];
-              de1 += sPart[w * 64 + tm.r1];
+            for (int q = 0; q < 4; ++q) {
+              de0 += sPart[q * 64 + tm.r0];
+              de1 += sPart[q * 64 + tm.r1];
             }
           }
           a2_tag = rs.send_x(A2, de0, de1, tid, warp, lane);
@@ -1243,9 +1249,9 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           de1 = hsum(s1);
           if (row_writer) {     // the partial sums over this CTA's hidden units of gZ1 * G_b1, once per row
 #pragma unroll
-            for (int w = 0; w < 8; ++w) {
-              de0 += sPart[w * 64 + tm.r0];
-              de1 += sPart[w * 64 + tm.r1];
+            for (int q = 0; q < 4; ++q) {
+              de0 += sPart[q * 64 + tm.r0];
+              de1 += sPart[q * 64 + tm.r1];
             }
           }
           csum.run_with_extras(sum, de0, de1, tid, lane);
