@@ -58,3 +58,8 @@ def test_every_wait_ends_and_the_scratch_holds_what_was_stored(case):
 @pytest.mark.parametrize("case", CASES)
 def test_no_two_accesses_are_unordered(case):
     assert run(*case).races() == []
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_no_waiter_is_overtaken(case):
+    assert run(*case).phases() == set()

@@ -255,8 +255,8 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   constexpr int NR = C::RS::NR;
   using RSx = typename C::RS;
 
-  // ---- barrier bookkeeping: every thread waits on every barrier use, in program order
-  uint32_t ph = 0;        // expected parity per barrier (indices 0..15)
+  // ---- barrier bookkeeping: every thread waits on every barrier use, in program order, or counts it (skip_bar)
+  uint32_t ph = 0;        // expected parity per barrier
   uint32_t pending = 0;   // thread 0: loads issued and not yet waited for
   auto wait_bar = [&](int b) {
     if (mbar_wait_cl(&bars[b], (ph >> b) & 1u, abort_flag, limit, kC)) {
@@ -264,6 +264,7 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       pending &= ~(1u << b);
     }
   };
+  auto skip_bar = [&](int b) { ph ^= 1u << b; };      // a use that this warp need not wait for
   auto wait_mma = [&]() {
     wait_bar(BAR_MMA);
     __syncwarp();
@@ -1009,7 +1010,10 @@ ttt_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       publish();
       wait_bar(BAR_BIG + ib4);
       wait_bar(BAR_T + 4);
-      wait_bar(BAR_BIG + ib1);      // X2, requested two phases ago
+      // X2, requested two phases ago.  Only those who issue MMAs or the next load wait: nothing would hold that load, of W2
+      // into the same buffer, back until a warp without a part in them had seen this one.
+      if (warp <= kProd / 32) wait_bar(BAR_BIG + ib1);
+      else skip_bar(BAR_BIG + ib1);
       // G8 (partial T1) // G5 (partial acc1) // G4
       TTT_ISSUE4(mma_tok_partial(tmem + C::TM_B, smem_u32(big(ib4)), smem_u32(big(ib0)), NB, lead),
                  mma_tok_partial(tmem + C::TM_B + 64, smem_u32(big(ib1)), smem_u32(big(ib3)), NB, lead),
