@@ -23,14 +23,14 @@ SIZES = {"uint8_t": 1, "char": 1, "__nv_bfloat16": 2, "float": 4, "uint32_t": 4,
          "float4": 16, "uint4": 16}
 TYPES = set(SIZES) | {"bool", "long", "auto", "uint16_t", "TokFrag", "Frag16", "CopyOp", "MmaOp", "Product", "Lane", "unsigned", "void"}
 TEMPLATES = {"static_cast", "const_cast", "reinterpret_cast", "tma_wait_group_read", "tma_wait_group", "frag_allreduce2",
-             "reg_take", "reg_give", "send_impl", "run_impl", "tok_row_allreduce", "mma_hid64", "mma_hidden_lead", "mma_hidden_ta", "mma_lead", "mma_lead_ta"}
+             "reg_take", "reg_give", "send_impl", "run_impl", "tok_row_allreduce", "mma_hid64", "mma_64_lead", "mma_hidden_lead", "mma_hidden_ta", "mma_lead", "mma_lead_ta"}
 # arithmetic on values, shuffles and fences: no access, no order
 PURE = set("""pk pk1 upk hsum add2 mul2 fma2 fmaf rsqrtf gelu_pair2 gelu_grad_h2 f32x2_to_f16x2 f16x2_to_f32x2 f32x2_to_bf16x2
 bf16x2_to_f32x2 bf16_lo bf16_hi pack_bf16 make_uint4 make_float2 make_float4 __float_as_uint __uint_as_float __bfloat162float
 __float2bfloat16 __shfl_xor_sync __syncwarp __threadfence fence_proxy_async_smem fence_proxy_async_all fence_mbar_init
 tc_fence_before_sync tc_fence_after_sync tmem_wait_ld tmem_wait_st tmem_alloc tmem_relinquish tmem_dealloc prefetch_tmap
 prefetch_l2 tma_commit_group globaltimer_ns atomicExch reg_take reg_give f16_pack
-gelu_half2 __shfl_down_sync RS_row_layernorm RS_row_sums griddep_launch griddep_wait""".split())
+gelu_half2 atomicXor atomicOr __shfl_down_sync RS_row_layernorm RS_row_sums griddep_launch griddep_wait""".split())
 
 
 class Unknown:
@@ -834,7 +834,7 @@ class Agent:
 
     def arrive(self, b, what, pred=(), times=1):
         n = self.sync(f"arrives at {self.r.label(b)} ({what})", pred)
-        self.r.arrivals.setdefault(b, {}).setdefault(self, []).extend([n] * times)
+        self.r.arrivals.setdefault(b, {}).setdefault(self, []).append((n, times))
         return n
 
     def f_mbar_arrive(self, w, p): self.arrive(self.bar(p), "warp", times=int(w.mask.sum()))
@@ -853,12 +853,18 @@ class Agent:
         assert len(b) == 1
         return self.wait((self.cta, int(b[0])))
 
-    f_wait_bar = f_wait
+    def f_wait_bar(self, w, b, parity=None):
+        b = np.unique(np.broadcast_to(b, 32)[w.mask])
+        at = (self.cta, int(b[0]))
+        assert len(b) == 1 and (parity is None or self.waits.get(at, 0) & 1 == parity & 1), f"{self.name}: not {self.r.label(at)}'s next use"
+        return self.wait(at)
 
     def f_mbar_wait_cl(self, w, p, parity, *_):
         b = self.bar(Ptr("s", int(np.unique(np.broadcast_to(p.addr, 32)[w.mask])[0]), 8))
         assert self.waits.get(b, 0) & 1 == parity, f"{self.name}: the use of {self.r.label(b)} that it waits for is not the next"
         return self.wait(b)
+
+    f_mbar_wait_bounded = f_mbar_wait_cl
 
     def st_async(self, w, addr, bar, size):
         addr, peer, bar = (np.broadcast_to(v, 32)[w.mask].tolist() for v in (addr.addr, addr.cta, bar.addr))
@@ -1057,17 +1063,22 @@ class Run:
     # -- what orders what
     def link(self):
         self.problems = []
-        # a phase takes the same share of every agent's arrivals
-        self.phase = {}
+        # a phase takes the same share of every agent's arrivals; but one agent may complete the first by itself
+        self.phase, arrived = {}, {}
         for b, by in self.arrivals.items():
-            phases, rest = divmod(sum(map(len, by.values())), self.count[b])
-            if rest or any(len(nodes) % max(phases, 1) for nodes in by.values()):
-                self.problems.append(f"{self.label(b)}: {[len(x) for x in by.values()]} arrivals, {self.count[b]} to a phase")
+            count, ph = self.count[b], self.phase.setdefault(b, {})
+            whole = [n for x in by.values() for n, times in x[:1] if times == count > 1]
+            lists = [[n for n, times in x for _ in range(times) if n not in whole] for x in by.values()]
+            phases, rest = divmod(sum(map(len, lists)), count)
+            if rest or len(whole) > 1 or any(len(x) % max(phases, 1) for x in lists):
+                self.problems.append(f"{self.label(b)}: {[len(x) for x in lists]} arrivals, {count} to a phase")
                 continue
-            for nodes in by.values():
-                for k, n in enumerate(nodes):
-                    self.phase.setdefault(b, {}).setdefault(k * phases // len(nodes), []).append(n)
-        arrived = {b: {k: len(v) for k, v in ph.items()} for b, ph in self.phase.items()}
+            for x in lists:
+                for k, n in enumerate(x):
+                    ph.setdefault(k * phases // len(x) + len(whole), []).append(n)
+            arrived[b] = {k: len(v) for k, v in ph.items()}
+            if whole:
+                ph[0], arrived[b][0] = whole, count
         brought = {}
         for b, nbytes, n, k in self.loads:              # k: the phase, of a CTA's own loads the first that is not complete
             got, want = brought.setdefault(b, [0] * len(self.expected[b])), self.expected[b]
