@@ -69,7 +69,7 @@ constexpr int kThreads = 2 * kGroup;
 constexpr int kRegsChain = 152, kRegsOut = 104;
 static_assert(kRegsChain + kRegsOut <= 2 * 128, "the block is launched with 128 registers per thread");
 // named barriers: one per warp pair of each group, then one per group
-constexpr uint32_t kBarPairC = 1, kBarPairO = 5, kBarC = 9, kBarO = 10;
+constexpr uint32_t kBarPairC = 1, kBarPairO = 5, kBarC = 9, kBarO = 10, kBarBlk = 11;      // kBarBlk: + 128-row block of the chain
 
 constexpr uint32_t OFF_K = 0;
 constexpr uint32_t OFF_V = OFF_K + kStages * TILE;
@@ -101,8 +101,9 @@ constexpr int BAR_ACCB = 9;                             // two uses per mini-bat
 constexpr int BAR_W1READ = 10;
 constexpr int BAR_ZB = 11;
 constexpr int BAR_W2UPD = 12, BAR_W2RDY = 13, BAR_SREAD = 14, BAR_W1RDY = 15;
-constexpr int BAR_DRAIN = 16;                           // abort path only
-constexpr int kBars = 17;
+constexpr int BAR_U2RDY = 16, BAR_R = 17;
+constexpr int BAR_DRAIN = 18;                           // abort path only
+constexpr int kBars = 19;
 
 // tensor-memory columns: two 128-lane blocks of 64 fp32 (32 bf16-pair) columns per 256-row matrix
 constexpr uint32_t TM_W1 = 0;
@@ -172,13 +173,14 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_MISC);
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + OFF_MISC + 4);
   volatile uint32_t* never_flag = reinterpret_cast<volatile uint32_t*>(smem + OFF_MISC + 8);   // stays 0
+  volatile uint32_t* stop_flag = reinterpret_cast<volatile uint32_t*>(smem + OFF_MISC + 12);   // the chain group's copy of abort_flag
 
   const uint64_t limit = p.wait_limit_ns;
   const int NC = p.NC;
 
   if (tid == 0) {
     for (int i = 0; i < kBars; ++i)
-      mbar_init(&bars[i], i == BAR_SREAD ? 8 : i == BAR_W2RDY ? 3 : i == BAR_DRAIN ? 2 : 1);
+      mbar_init(&bars[i], i == BAR_SREAD ? 8 : i == BAR_W2RDY || i == BAR_DRAIN ? 3 : i == BAR_W1RDY || i == BAR_R ? 2 : 1);
     fence_mbar_init();
     *abort_flag = 0;
     *never_flag = 0;
@@ -247,6 +249,11 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       tc_fence_before_sync();
       named_bar_sync(kBarC, kGroup);
     };
+    auto publish_block = [&]() {     // the same, by and for the warps of one 128-row block
+      tc_fence_before_sync();
+      named_bar_sync(kBarBlk + wg, kGroup / 2);
+    };
+    const bool issuer = quad == 0;      // warps 0 and 4: each issues its block's products
     // ---- initial W1, b1: global fp32 -> tensor memory (master), shared memory (bf16 operand copy), checkpoint 0
     float b1v = p.b1[stream_id * 256 + hrow];
     {
@@ -275,8 +282,9 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       __syncwarp();
       tc_fence_after_sync();
     };
-    // The two 128-row blocks of a product are committed one by one: the warps of a block start when theirs is
-    // complete.
+    // The two 128-row blocks of a product are issued and committed one by one, each by the first of its four warps: the
+    // warps of a block start when theirs is complete, and where only a block's own rows are needed (U1, the bf16 W1) they
+    // wait for each other alone.
     for (; it < NC; ++it) {
       const int s = it & 1;
       const uint8_t* sK = smem + OFF_K + s * TILE;
@@ -286,14 +294,12 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       wait_bar(BAR_K + s, it >> 1);
 
       // ---- MMA1: Z1^T = W1^T K^T
-      if (cta_warp == 0) {
+      if (issuer) {
         tc_fence_after_sync();
-#pragma unroll
-        for (int blk = 0; blk < 2; ++blk) {
-          mma_hidden_ta<false, false>(tmem + TM_A + blk * 64, tmem + TM_W1B + blk * 32, smem_u32(sK), lead);
-          if (lead) umma_commit(&bars[BAR_ACCA + blk]);
-        }
+        mma_hidden_ta<false, false>(tmem + TM_A + wg * 64, tmem + TM_W1B + wg * 32, smem_u32(sK), lead);
+        if (lead) umma_commit(&bars[BAR_ACCA + wg]);
       }
+      if (it > 0) wait_bar(BAR_W2UPD, prev);             // the W2 update has read X2
       wait_acca();
       // ---- EPI1: X2^T = gelu(Z1^T + b1) -> smem; G' = gelu'(Z1^T + b1) stays in registers (the thread that needs it
       // in EPI3 is this one).  The next 16 columns are requested before these are processed.
@@ -320,7 +326,13 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           tmem_wait_ld();
         }
       }
+      if (gtid == 0) *stop_flag = *abort_flag;
       publish();
+      const bool stop = *stop_flag != 0;
+      if (loader && it > 0) {      // MMA4 of the last mini-batch has read K
+        load_k(it + 1);
+        issued = it + 2;
+      }
 
       // ---- MMA2: Z2 = X2 W2
       wait_bar(BAR_W2RDY, par);                          // also b2, written with it
@@ -377,14 +389,13 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       publish();
 
       // ---- MMA3: R^T = W2 U2^T
-      if (cta_warp == 0) {
+      if (issuer) {
         tc_fence_after_sync();
-#pragma unroll
-        for (int blk = 0; blk < 2; ++blk) {
-          mma_hidden_lead<false, false>(tmem + TM_A, smem_u32(sW2), smem_u32(sU2), blk, lead);
-          if (lead) umma_commit(&bars[BAR_ACCA + blk]);
-        }
+        mma_hidden_lead<false, false>(tmem + TM_A, smem_u32(sW2), smem_u32(sU2), wg, lead);
+        if (lead) umma_commit(&bars[BAR_ACCA + wg]);
+        if (lead) umma_commit(&bars[BAR_R]);
       }
+      if (gtid == 64) mbar_arrive(&bars[BAR_U2RDY]);     // the output group updates W2
       if (loader) load_tile(it + kStages, &tmV, OFF_V, BAR_V);      // V has been read
       wait_acca();
       // ---- EPI3: U1^T = R^T * G' (= -eta dl/dZ1), as bf16 over R in tensor memory; b1 += row sum
@@ -408,21 +419,15 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         sB1[prev * 256 + hrow] = b1v;      // b1 after this mini-batch
         tmem_wait_st();
       }
-      publish();
+      publish_block();
 
-      // ---- MMA4: W1^T += U1^T K ;  W2 += X2^T U2
-      if (cta_warp == 0) {
+      // ---- MMA4: W1^T += U1^T K
+      if (issuer) {
         if (it > 0) wait_bar(BAR_SREAD, prev);
         __syncwarp();
         tc_fence_after_sync();
-#pragma unroll
-        for (int blk = 0; blk < 2; ++blk) {
-          mma_hidden_ta<true, true>(tmem + TM_W1 + blk * 64, tmem + TM_A + blk * 64, smem_u32(sK), lead);
-          if (lead) umma_commit(&bars[BAR_ACCA + blk]);
-        }
-        mma_hidden_lead<true, true>(tmem + TM_W2, smem_u32(sX2), smem_u32(sU2), 0, lead);
-        mma_hidden_lead<true, true>(tmem + TM_W2, smem_u32(sX2), smem_u32(sU2), 1, lead);
-        if (lead) umma_commit(&bars[BAR_W2UPD]);
+        mma_hidden_ta<true, true>(tmem + TM_W1 + wg * 64, tmem + TM_A + wg * 64, smem_u32(sK), lead);
+        if (lead) umma_commit(&bars[BAR_ACCA + wg]);
       }
       if (it > 0) wait_bar(BAR_W1READ, prev);         // the last mini-batch's MMA5 has read the bf16 W1
       wait_acca();
@@ -435,14 +440,9 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         st_cols32_tmem(tmem + lane_base + TM_W1B + wg * 32 + half * 16, v);
       }
       tmem_wait_st();
-      tc_fence_before_sync();
-      const bool stop = named_bar_or(kBarC, kGroup, *abort_flag != 0);
-      if (gtid == 0) mbar_arrive(&bars[BAR_W1RDY]);
+      publish_block();
+      if (lane == 0 && quad == 1) mbar_arrive(&bars[BAR_W1RDY]);
       if (stop) break;
-      if (loader) {          // MMA4 has read K
-        load_k(it + kStages);
-        issued = it + kStages + 1;
-      }
     }
     if (loader && *abort_flag) {
       drain_loads(BAR_K, issued);
@@ -486,7 +486,17 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       const int s = it & 1;
       uint8_t* sQ = smem + OFF_Q + s * TILE;
       const uint32_t par = it & 1, next = par ^ 1u;
+      // ---- W2 += X2^T U2 (the group's reads of W2 for the last mini-batch's checkpoint are behind its barriers)
+      if (warp == 0) {
+        wait_bar(BAR_U2RDY, par);
+        __syncwarp();
+        tc_fence_after_sync();
+        mma_hidden_lead<true, true>(tmem + TM_W2, smem_u32(sX2), smem_u32(sU2), 0, lead);
+        mma_hidden_lead<true, true>(tmem + TM_W2, smem_u32(sX2), smem_u32(sU2), 1, lead);
+        if (lead) umma_commit(&bars[BAR_W2UPD]);
+      }
       wait_bar(BAR_W2UPD, par);
+      wait_bar(BAR_R, par);                              // MMA3 has read the bf16 W2
       __syncwarp();
       tc_fence_after_sync();
       // ---- b2 += column sums of U2 (bf16 values, the operand the W2 update sees), fp32 accumulate: a thread
@@ -662,7 +672,7 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   if (aborted) {
     // everything this CTA still has in flight is waited for (bounded, not cut short by the abort flag)
     // before its shared and tensor memory go away: the loads above, and the tensor-core work of both issuers
-    if (warp == 0 && lead) umma_commit(&bars[BAR_DRAIN]);
+    if ((cta_warp == 0 || cta_warp == 4 || cta_warp == 8) && lead) umma_commit(&bars[BAR_DRAIN]);
     if (tid == 0) {
       mbar_wait_bounded(&bars[BAR_DRAIN], 0, never_flag, limit);
       atomicExch(p.status, static_cast<uint32_t>(TTT_B200_ERR_TIMEOUT));
