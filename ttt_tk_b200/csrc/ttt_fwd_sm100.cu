@@ -13,17 +13,17 @@
 //
 // A mini-batch is a chain of dependent MMA -> epilogue round trips, and only a part of it is needed by the
 // next mini-batch: the output pass (the post-update product with Q, GELU, LayerNorm) is not.  So the CTA runs two
-// groups of eight warps, each with its own accumulator in tensor memory, one MMA issuer and its own barriers:
+// groups of eight warps, each with its own accumulator in tensor memory, its own MMA issuers and barriers:
 //
 //   chain group                                        output group
-//   MMA1  Z1^T = W1^T K^T        [256 x 64 tok]        (W2 updated:)  bf16 copy of the new W2 -> smem
-//   EPI1  X2^T = gelu(Z1^T + b1), G' = gelu'(.)                       b2 += colsum(U2); checkpoints
-//   MMA2  Z2 = X2 W2             [64 tok x 64]         (W1 copied:)   MMA5  Z1b^T = W1^T Q^T
+//   MMA1  Z1^T = W1^T K^T        [256 x 64 tok]        (U2 there:)    W2 += X2^T U2
+//   EPI1  X2^T = gelu(Z1^T + b1), G' = gelu'(.)                       bf16 copy of the new W2 -> smem; b2 += colsum(U2)
+//   MMA2  Z2 = X2 W2             [64 tok x 64]         (W1 copied:)   checkpoints;  MMA5  Z1b^T = W1^T Q^T
 //   LN    U2 = -eta * dl/dZ2 (fused LN + L2 gradient)  EPI5  X2b^T = gelu(Z1b^T + b1)
 //   MMA3  R^T = W2 U2^T                                MMA6  Z2b = X2b W2
 //   EPI3  U1^T = R^T * G';  b1 += rowsum               OUT   Q + gamma * LN(Z2b + b2) + beta -> TMA store
-//   MMA4  W1^T += U1^T K ;  W2 += X2^T U2
-//   EPI4  bf16 copy of the new W1^T -> smem
+//   MMA4  W1^T += U1^T K
+//   EPI4  bf16 copy of the new W1^T
 //
 // The output group works one step behind, on the state the chain group has just left: the chain is four round
 // trips per mini-batch instead of six, and each group's MMA latencies are filled with the other's epilogues (four
@@ -36,10 +36,16 @@
 // memory (G' in registers from EPI1 to EPI3, U1 and the bf16 W1 in tensor memory as A operands of their MMAs, which then
 // read 2 KB of shared memory instead of 6); and the MMAs are issued from warp-uniform code.  Measured (B200, 128 streams
 // of 128 mini-batches, one checkpoint in 8): 8.0 us per mini-batch as one group of 8 warps, 6.0 with the two groups, 4.6
-// with the rest; 1536 streams of 64 mini-batches 5.43 -> 3.23 ms.
+// with the rest, 4.3 with the products of a block issued by the block's own first warp and the W2 update by the output
+// group (before, one warp issued all sixteen MMAs of the state update and came 400 cycles late to EPI4, with everyone
+// waiting for it); 1536 streams of 64 mini-batches 5.43 -> 3.23 -> 2.95 ms.  A checkpoint costs about 2100 cycles (the
+// output group's 4200 for 132 KB of stores, of which half fit its slack); as bulk copies from a staging area it cost
+// more, since W1's turn of the area waits for W2 to leave.
 //
 // Hand-over between the groups (mbarriers, each completed once per mini-batch):
-//   w2upd   MMA4's W2 update has completed                     chain's tensor work -> output group
+//   u2rdy   U2 and X2 are in place                             chain -> output group (W2 update)
+//   r       MMA3 has read the bf16 W2                          chain's tensor work -> output group (its next copy)
+//   w2upd   the W2 update has completed                        output's tensor work -> output group; chain (EPI1: X2)
 //   w2rdy   bf16 W2 and b2 are refreshed                       output group -> chain (MMA2, LN)
 //   sread   the output group has read the state columns and
 //           taken note of w1rdy                                output group -> chain (MMA4)
@@ -460,6 +466,8 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       named_bar_sync(kBarO, kGroup);
     };
     uint8_t* stage = smem + OFF_STG + warp * 4096;
+    long ck = stream_id * p.nck + 1;                   // the next checkpoint, and the mini-batch that it precedes (0: none)
+    int next_ck = p.cgs < NC ? p.cgs : 0;
     // ---- initial W2: global fp32 -> tensor memory (master), shared memory (bf16 operand copy), checkpoint 0
     {
       const float4* W2g = reinterpret_cast<const float4*>(p.W2 + st_w + hrow * 64);
@@ -512,7 +520,7 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                               sU2 + sw128_off(warp * 8 + r, pr >> 2) + (pr & 3) * 4)));
         *reinterpret_cast<f32x2*>(part + warp * 64 + 2 * pr) = acc;
       }
-#pragma unroll 1
+#pragma unroll
       for (int half = 0; half < 2; ++half) {
         uint32_t v[32];
         tmem_ld32(tmem + lane_base + TM_W2 + wg * 64 + half * 32, v);
@@ -532,8 +540,10 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       wait_bar(BAR_W1RDY, par);
       __syncwarp();
       // ---- the state after this mini-batch is a checkpoint if the next one starts a group
-      if (it + 1 < NC && (it + 1) % p.cgs == 0) {
-        const long ckc = stream_id * p.nck + (it + 1) / p.cgs;
+      if (it + 1 == next_ck) {
+        const long ckc = ck;
+        ck += 1;
+        next_ck = it + 1 + p.cgs < NC ? it + 1 + p.cgs : 0;
         float* W1k = p.W1c + ckc * (64 * 256) + hrow;
         float* W2k = p.W2c + ckc * (256 * 64) + (hrow - lane) * 64;
 #pragma unroll 1
