@@ -256,7 +256,7 @@ def run_ours(args, rank, world, local_rank):
         step = DeviceStep(host, cgs, dev, cluster)
     Bl, Hl = b1 - b0, h1 - h0
     lib = _lib.lib()
-    cl_fwd = lib.ttt_b200_launch_cluster(Bl * Hl, (cluster or 0) << 8, 0)
+    cl_fwd = lib.ttt_b200_forward_ctas(Bl * Hl, NC, cgs, (cluster or 0) << 8)
     cl_used = lib.ttt_b200_backward_ctas(Bl * Hl, NC, cgs, (cluster or 0) << 8)
     pairs = lib.ttt_b200_backward_pairs(Bl * Hl, NC, cgs, (cluster or 0) << 8)
     bwd_launches = 2 if lib.ttt_b200_backward_tail(Bl * Hl, NC, cgs, (cluster or 0) << 8) else 1

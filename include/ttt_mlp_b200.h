@@ -43,7 +43,7 @@ enum {
    * runs out; the kernel reports code 3 through the status word and exits normally. */
   TTT_B200_FLAG_TEST_LOST_LOAD = 2u,
   /* Bits 8..11: how many CTAs (of a thread-block cluster) share one (batch, head) stream, each owning 256 / n hidden units
-   * or, in a backward with two, one recomputing and one sweeping; the reference fixes this at compile time (TP = 2 in kernels/ttt/ttt.cu:11-12,
+   * or, with two, one the chain and one the output pass (forward), one recomputing and one sweeping (backward); the reference fixes this at compile time (TP = 2 in kernels/ttt/ttt.cu:11-12,
    * 4 in kernels/ttt_backward/ttt.cu:12-16).  0 = chosen per launch from B*H and the number of clusters the GPU runs at once
    * (overridable with the environment variable TTT_B200_CLUSTER); 1, 2 or 4 = forced. */
   TTT_B200_FLAG_CLUSTER_SHIFT = 8,
@@ -285,10 +285,16 @@ int ttt_b200_version(void);
  * `flags` gives each (batch, head) stream of a problem with `streams` = B*H streams on the current device.  The size that
  * the flags name; else the one that TTT_B200_CLUSTER names (0 or empty: none); else four when the device runs that many
  * clusters of four at once (ttt_b200_cluster_capacity), else two in the backward when those fit, else one (measured
- * thresholds).  A backward long enough to pipeline its groups takes two where this says four: ttt_b200_backward_ctas.  The
+ * thresholds).  A call long enough to gain from it takes two where this says one or four: ttt_b200_forward_ctas,
+ * ttt_b200_backward_ctas.  The
  * reference fixes the split at compile time (kernels/ttt/ttt.cu:11-12,
  * kernels/ttt_backward/ttt.cu:12-16).  Returns -1 on error. */
 int ttt_b200_launch_cluster(int streams, uint32_t flags, int backward);
+
+/* The same for a forward of NC mini-batches in groups of checkpoint_group_size: without a size in the flags or the
+ * environment it is two where the device runs all streams as pairs of CTAs, one with the chain of the state and one with the
+ * output pass, and that is faster: instead of one from six mini-batches on, instead of four from 16 in groups of four on. */
+int ttt_b200_forward_ctas(int streams, int NC, int checkpoint_group_size, uint32_t flags);
 
 /* The same for a backward of NC mini-batches in groups of checkpoint_group_size: without a size in the flags or the
  * environment it is two instead of four from three groups of four mini-batches on. */

@@ -66,7 +66,7 @@ class BwdNoAllocArgs(ctypes.Structure):
 
 
 EXPORTS = ["ttt_b200_forward", "ttt_b200_linear_forward", "ttt_b200_linear_backward", "ttt_b200_linear_backward_scratch_bytes", "ttt_b200_backward", "ttt_b200_backward_noalloc", "ttt_b200_last_error", "ttt_b200_take_status",
-           "ttt_b200_version", "ttt_b200_pick_cluster", "ttt_b200_launch_cluster", "ttt_b200_backward_ctas", "ttt_b200_backward_tail", "ttt_b200_backward_pairs", "ttt_b200_cluster_capacity", "ttt_b200_umma_selftest", "ttt_b200_wait_selftest", "ttt_b200_pack_tokens",
+           "ttt_b200_version", "ttt_b200_pick_cluster", "ttt_b200_launch_cluster", "ttt_b200_forward_ctas", "ttt_b200_backward_ctas", "ttt_b200_backward_tail", "ttt_b200_backward_pairs", "ttt_b200_cluster_capacity", "ttt_b200_umma_selftest", "ttt_b200_wait_selftest", "ttt_b200_pack_tokens",
            "ttt_b200_unpack_tokens", "ttt_b200_eta_gate", "ttt_b200_eta_gate_backward", "ttt_b200_unpack_layernorm",
            "ttt_b200_pack_layernorm_backward"]
 
@@ -102,6 +102,8 @@ def load():
     lib.ttt_b200_pick_cluster.restype = ctypes.c_int
     lib.ttt_b200_launch_cluster.argtypes = [ctypes.c_int, c_uint32, ctypes.c_int]
     lib.ttt_b200_launch_cluster.restype = ctypes.c_int
+    lib.ttt_b200_forward_ctas.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, c_uint32]
+    lib.ttt_b200_forward_ctas.restype = ctypes.c_int
     lib.ttt_b200_backward_ctas.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, c_uint32]
     lib.ttt_b200_backward_ctas.restype = ctypes.c_int
     lib.ttt_b200_backward_tail.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, c_uint32]

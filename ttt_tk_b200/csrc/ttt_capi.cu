@@ -17,6 +17,8 @@
 
 int ttt_launch_forward(const ttt_b200_fwd_args* a, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
                        int drop_load);
+int ttt_launch_forward_pair(const ttt_b200_fwd_args* a, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
+                            int drop_load);
 int ttt_launch_backward(const ttt_b200_bwd_args* a, int streams, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
                         int drop_load);
 int ttt_launch_backward_pair(const ttt_b200_bwd_args* a, int first, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
@@ -31,6 +33,7 @@ uint64_t ttt_linear_backward_scratch_bytes(int B, int H, int cgs);
 int ttt_forward_cluster_capacity(int cluster);
 int ttt_backward_cluster_capacity(int cluster);
 int ttt_backward_pair_capacity();
+int ttt_forward_pair_capacity();
 int ttt_launch_forward_cluster(const ttt_b200_fwd_args* a, int cluster, cudaStream_t stream, uint32_t* status,
                                uint64_t limit_ns, int drop_load);
 
@@ -110,6 +113,24 @@ static int ttt_launch_cluster(int streams, uint32_t flags, bool backward, int* c
   if (streams <= capacity(4, backward)) *cluster = 4;
   else if (backward && streams <= capacity(2, backward)) *cluster = 2;
   else *cluster = 1;
+  return TTT_B200_OK;
+}
+
+// A forward with two CTAs per stream gives them the chain and the output pass (ttt_fwd_pair_sm100.cu) from four mini-batches
+// on.  Below, where only a caller asks for two, each takes half of the hidden units, and of the state's way in and out (12
+// streams, us, halves / chain and output: 1 mini-batch 10.9 / 14.5, 2 16.5 / 18.2, 3 23.1 / 23.3, 4 28.6 / 26.4).
+static bool forward_pair(int ctas, int NC) { return ctas == 2 && NC >= 4; }
+
+// CTAs per stream of a forward.  Two where the device runs all streams as pairs at once and that is the faster form: against
+// one CTA from six mini-batches on (us, one CTA / pair: 34 streams x 4 in groups of 2 27.6 / 27.5, x 6 in groups of 3 35.5 /
+// 34.9, x 16 in groups of 4 79 / 72; 48 x 32 in groups of 6 147 / 136, in groups of 1 203 / 177), against four, which share
+// the writing of the state, from 16 mini-batches in groups of four on (four / pair: 12 streams x 12 in groups of 4 54.8 /
+// 56.1, x 16 71.9 / 71.2; x 32 in groups of 6 138 / 131, x 16 in groups of 2 72.7 / 77.6; 32 x 128 in groups of 16 536 / 489).
+static int forward_ctas(int streams, int NC, int cgs, uint32_t flags, int* ctas) {
+  if (int rc = ttt_launch_cluster(streams, flags, false, ctas)) return rc;
+  int asked = 0;
+  if (asked_cluster(flags, &asked) != TTT_B200_OK || asked != 0 || streams > ttt_forward_pair_capacity()) return TTT_B200_OK;
+  if (*ctas == 4 ? NC >= 16 && cgs >= 4 : NC >= 6) *ctas = 2;
   return TTT_B200_OK;
 }
 
@@ -260,12 +281,17 @@ extern "C" int ttt_b200_forward(const ttt_b200_fwd_args* a, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   uint32_t* status = nullptr;
   if (int rc = pre_launch(&status)) return rc;
-  int cluster = 1;
-  if (int rc = ttt_launch_cluster(a->B * a->H, a->flags, false, &cluster)) return rc;
+  const int streams = a->B * a->H;
+  int ctas = 1;
+  if (int rc = forward_ctas(streams, a->NC, a->checkpoint_group_size, a->flags, &ctas)) return rc;
   const int drop = (a->flags & TTT_B200_FLAG_TEST_LOST_LOAD) ? (a->NC > 1 ? 1 : 0) : -1;
-  if (int rc = cluster == 1 ? ttt_launch_forward(a, stream, status, wait_limit_ns(), drop)
-                            : ttt_launch_forward_cluster(a, cluster, stream, status, wait_limit_ns(), drop))
+  if (ctas == 1) {
+    if (int rc = ttt_launch_forward(a, stream, status, wait_limit_ns(), drop)) return rc;
+  } else if (forward_pair(ctas, a->NC)) {
+    if (int rc = ttt_launch_forward_pair(a, stream, status, wait_limit_ns(), drop)) return rc;
+  } else if (int rc = ttt_launch_forward_cluster(a, ctas, stream, status, wait_limit_ns(), drop)) {
     return rc;
+  }
   if (a->flags & TTT_B200_FLAG_SYNC) return ttt_check_status(stream);
   return TTT_B200_OK;
 }
@@ -382,6 +408,12 @@ extern "C" int ttt_b200_pick_cluster(int streams, int backward) {
   if (c != 0) return c;
   if (streams <= capacity(4, backward != 0)) return 4;
   return !backward && streams <= capacity(2, false) ? 2 : 1;
+}
+
+extern "C" int ttt_b200_forward_ctas(int streams, int NC, int checkpoint_group_size, uint32_t flags) {
+  int c = 0;
+  if (streams < 1 || NC < 1 || checkpoint_group_size < 1) return -1;
+  return forward_ctas(streams, NC, checkpoint_group_size, flags, &c) == TTT_B200_OK ? c : -1;
 }
 
 extern "C" int ttt_b200_backward_ctas(int streams, int NC, int checkpoint_group_size, uint32_t flags) {
