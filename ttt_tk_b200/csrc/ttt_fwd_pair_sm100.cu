@@ -191,6 +191,10 @@ ttt_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     uint64_t t0 = 0;
     uint32_t spins = 0;
     while (!(b >= U_SENT ? mbar_try_wait_cluster(&bars[b], parity) : mbar_try_wait(&bars[b], parity))) {
+      if (warp < 16) {      // (whatever holds an epilogue warp up holds a helper warp up that waits for it: the clock is theirs)
+        if (*abort_flag) return false;
+        continue;
+      }
       if (++spins & 31u) continue;
       if (*abort_flag) return false;
       const uint64_t t = globaltimer_ns();
