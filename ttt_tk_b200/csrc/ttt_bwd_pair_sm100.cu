@@ -493,6 +493,7 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     return c;
   };
+  auto place = [&](const Lane& c, int slot) { return slot >= cgs ? c.far + (slot - cgs) * 262144L : c.mem + static_cast<long>(slot) * c.step; };
   // one copy, by the lanes for which `act` holds: mini-batch i, slot `slot`, shared-memory offset `off`, parity of its stage
   auto copy = [&](const Lane& c, bool act, int i, int slot, uint32_t off, uint32_t par, bool dropped) {
     if (!act || dropped) return;
@@ -972,6 +973,14 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     };
     if (g == 0) first(g);
     for (int j = -1; j < gsz; ++j) {
+      // this lane's copies of the mini-batch, put together before their events are waited for
+      uint8_t* const mem = place(c, slot_of(g, j + op.next));
+      const bool store = mine && op.kind == K_STORE && j + op.next < gsz;
+      const int ahead = is_v ? 1 : 2, i = i0 + j + ahead;      // the load's mini-batch
+      const bool load = (is_v || is_k) && j >= 0 && j + ahead < gsz && !dropped(i);
+      const uint32_t off = op.off + (is_k && (j & 1) ? op.par : 0u);
+      const int b = op.bar + (is_k ? j & 1 : 0);
+      const uint8_t* const src = c.mem + i * 128L;             // eta
 #pragma unroll 1
       for (int ev = j < 0 ? Y_W : Y_1; ev <= Y_W; ++ev) {      // j = -1: the checkpoint's W1
         if (!seen_all(j < 0 ? E_LD1 : ev == Y_1 ? E_1 : ev == Y_2 ? E_2 : ev == Y_3 ? E_3 : E_W1)) return;
@@ -981,11 +990,16 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           if (ev == Y_2 && lane == 0) arrive(F_ZG);
         }
         // V's tile is free after E_3 (x_hat_fused has left), K's stage after EPI4
-        const int ahead = ev == Y_3 ? 1 : 2;
-        const bool load = (ev == Y_3 && is_v) || (ev == Y_W && is_k && j >= 0);
-        copy(c, load && j + ahead < gsz, i0 + j + ahead, 0, op.off, is_k ? j & 1 : 0, dropped(i0 + j + ahead));
+        if (load && ev == (is_v ? Y_3 : Y_W)) {
+          if (op.arm) arm(b, op.arm);
+          if (op.kind == K_TMA) tma_load_2d(smem + off, c.map, &bars[b], 0, row_of(i));
+          else bulk_load_1d(smem + off, src, op.bytes, &bars[b]);
+        }
         if (ev == Y_W && j + 1 < gsz && !wait_slot(g, j + 1)) return;
-        copy(c, mine && op.kind == K_STORE && op.event == ev && j + op.next < gsz, 0, slot_of(g, j + op.next), op.off, 0, false);
+        if (store && op.event == ev) {
+          bulk_store_1d(mem, smem + op.off, op.bytes);
+          tma_commit_group();
+        }
         __syncwarp();
         if (ev == Y_3) {
           tma_wait_group_read<0>();
@@ -1004,6 +1018,9 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const bool mine = lane < kRecCopies;
     if (g == 0) copy(c, lane == kLaneQ || lane == kLaneGo, i0, 0, op.off, 0, dropped(i0));
     for (int j = -1; j < gsz; ++j) {
+      uint8_t* const mem = place(c, slot_of(g, j + op.next));
+      const bool store = mine && op.kind == K_STORE && j + op.next < gsz;
+      const int when = op.event == Y_W ? Y_LD : op.event;
 #pragma unroll 1
       for (int ev = Y_LD; ev <= Y_3; ++ev) {      // Y_LD: the W2 copy (j = -1: the checkpoint's W2)
         if (!seen_all(j < 0 ? E_LD2 : ev == Y_LD ? E_W2 : ev == Y_1 ? E_O5 : ev == Y_2 ? E_OS4 : E_OE1)) return;
@@ -1013,8 +1030,10 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           __syncwarp();
           if (lane == 0) arrive(F_XB);
         }
-        copy(c, mine && op.kind == K_STORE && op.event == (ev == Y_LD ? Y_W : ev) && j + op.next < gsz, 0,
-             slot_of(g, j + op.next), op.off, 0, false);
+        if (store && when == ev) {
+          bulk_store_1d(mem, smem + op.off, op.bytes);
+          tma_commit_group();
+        }
         __syncwarp();
         const bool dq = ev == Y_LD && j > 0;
         if (dq) {
@@ -1030,8 +1049,11 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           if (!dq && lane == 0) arrive(j < 0 ? F_XB : F_XB2);
         }
         // dL/dOut's tile is free when dQ has left it, Q's when gZ2b has
-        copy(c, (dq && lane == kLaneGo) || (ev == Y_3 && lane == kLaneQ && j + 1 < gsz), i0 + j + (dq ? 0 : 1), 0, op.off, 0,
-             dropped(i0 + j + (dq ? 0 : 1)));
+        const int i = i0 + j + (dq ? 0 : 1);
+        if (((dq && lane == kLaneGo) || (ev == Y_3 && lane == kLaneQ && j + 1 < gsz)) && !dropped(i)) {
+          arm(op.bar, op.arm);
+          tma_load_2d(smem + op.off, c.map, &bars[op.bar], 0, row_of(i));
+        }
         __syncwarp();
         if (j < 0) break;
       }
@@ -1458,12 +1480,18 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (!seen_all(C6) || !seen_all(C7)) return;
     }
     for (int j = gsz - 1; j >= 0; --j) {
+      // this lane's copy of the step, put together before its event is waited for
       const int i = i0 + j, par = nsw & 1;
+      const bool first = j == gsz - 1, more = j > 0;
+      const int slot = slot_of(g, j - op.next);
+      const bool act = !op.only_next || more;
+      const uint32_t off = op.off + role(op.role) + (par ? 0u : op.par);
+      uint8_t* const mem = op.src == A_ETA ? c.mem + (i - op.next) * 128L : place(c, slot);
 #pragma unroll 1
       for (int ev = 0; ev < V_COUNT; ++ev) {
         if (!seen_all(kSweepEvent[ev])) return;
         if (lane == 0) {
-          if ((ev == V_S2 && j < gsz - 1) || ev == V_V) {
+          if ((ev == V_S2 && !first) || ev == V_V) {
             const bool dk = ev == V_S2;
             tma_store_2d(dk ? &tmDK : &tmDV, smem + (dk ? S_K + (par ^ 1) * TILE : S_V), 0, row_of(dk ? i + 1 : i));
             tma_commit_group();
@@ -1472,8 +1500,11 @@ ttt_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           if (ev == V_C6) tma_wait_group_read<0>();     // dV has
         }
         __syncwarp();
-        copy(c, op.event == ev && (!op.only_next || j > 0), i - op.next, slot_of(g, j - op.next),
-             op.off + role(op.role), par ^ 1, false);
+        if (act && op.event == ev) {
+          if (op.arm) arm(op.bar, op.arm);
+          if (op.kind == K_TMA) tma_load_2d(smem + off, c.map, &bars[op.bar], 0, row_of(i - op.next));
+          else bulk_load_1d(smem + off, mem, op.bytes, &bars[op.bar]);
+        }
         __syncwarp();
       }
       turn();
