@@ -259,7 +259,7 @@ def run_ours(args, rank, world, local_rank):
     cl_fwd = lib.ttt_b200_forward_ctas(Bl * Hl, NC, cgs, (cluster or 0) << 8)
     cl_used = lib.ttt_b200_backward_ctas(Bl * Hl, NC, cgs, (cluster or 0) << 8)
     pairs = lib.ttt_b200_backward_pairs(Bl * Hl, NC, cgs, (cluster or 0) << 8)
-    bwd_launches = 2 if lib.ttt_b200_backward_tail(Bl * Hl, NC, cgs, (cluster or 0) << 8) else 1
+    bwd_launches = 2 if 0 < lib.ttt_b200_backward_tail(Bl * Hl, NC, cgs, (cluster or 0) << 8) < Bl * Hl else 1
 
     sampler = ClockSampler(local_rank)
     # warm-up happens inside timed_steps; the sampler is started just before so that most of its samples
@@ -420,7 +420,7 @@ def run_ours(args, rank, world, local_rank):
     per_mb = {"one": (Bl * Hl - pairs) * NC, "pair": pairs * NC}       # mini-batches by form
     remat_bytes = Bl * Hl * 2 * n * STATE_BYTES + sum(m * sum(SCRATCH_PER_MB[k]) for k, m in per_mb.items())
     dram_bwd = sum(m * NCU_BWD_DRAM_BYTES_PER_MB[k] for k, m in per_mb.items())
-    bwd_kernel = "ttt_bwd_kernel" if cl_used == 1 else \
+    bwd_kernel = "ttt_bwd_kernel" if cl_used == 1 and pairs < Bl * Hl else \
         "ttt_bwd_pair_kernel" if pairs else f"ttt_bwd_cluster_kernel<{cl_used}>"
     res = {
         "metric": "ttt_mlp_fwd_bwd_tokens_per_s", "value": tokens_per_step / (ms_per_step * 1e-3),
@@ -431,7 +431,7 @@ def run_ours(args, rank, world, local_rank):
                    "parallelism": (f"one problem, (batch x head) streams partitioned over {world} GPU(s): "
                                    f"{Bl} x {Hl} = {Bl * Hl} streams per GPU" if strong else
                                    f"one whole problem per GPU (replicas), {world} GPU(s)"),
-                   "ctas_per_stream": {"forward": cl_fwd, "backward": cl_used},
+                   "ctas_per_stream": {"forward": cl_fwd, "backward": 2 if pairs == Bl * Hl else cl_used},
                    "l2": "working set per step (~1.7 GB at c2 on one GPU) exceeds the 126 MB L2; no explicit flush"},
         "kernels": {"fwd_ms": fwd_ms, "bwd_ms": bwd_ms,
                     "fwd_tflops": fwd_flop / (fwd_ms * 1e-3) / 1e12, "bwd_tflops": bwd_tf,
@@ -440,7 +440,7 @@ def run_ours(args, rank, world, local_rank):
                     "fwd_bwd_frac_of_bf16_sustained_peak": both_tf / sustained,
                     "fwd_algorithmic_gbs": fwd_bytes / (fwd_ms * 1e-3) / 1e9,
                     "bwd_algorithmic_gbs": bwd_bytes / (bwd_ms * 1e-3) / 1e9,
-                    "streams_per_gpu": Bl * Hl, "ctas_per_stream_fwd": cl_fwd, "ctas_per_stream_bwd": cl_used},
+                    "streams_per_gpu": Bl * Hl, "ctas_per_stream_fwd": cl_fwd, "ctas_per_stream_bwd": 2 if pairs == Bl * Hl else cl_used},
         # checkpoint + recompute scratch traffic: checkpoints written by the forward and read by the backward,
         # scratch slots written by the recompute and read back by the sweep (bytes the kernels ask for)
         "remat_traffic": {"bytes_per_step": remat_bytes,

@@ -300,8 +300,9 @@ int ttt_b200_forward_ctas(int streams, int NC, int checkpoint_group_size, uint32
  * environment it is two instead of four from three groups of four mini-batches on. */
 int ttt_b200_backward_ctas(int streams, int NC, int checkpoint_group_size, uint32_t flags);
 
-/* Of a backward whose answer there is one: how many of its last streams (those beyond a multiple of the SMs) a second launch
- * gives two CTAs each.  0 if there is only one launch, -1 on error. */
+/* Of a backward whose answer there is one: how many of its last streams a launch after the others' gives two CTAs each: those
+ * beyond a multiple of the SMs, or, where two turns of pairs are faster than one of single CTAs, all of them.  0 if none, -1
+ * on error. */
 int ttt_b200_backward_tail(int streams, int NC, int checkpoint_group_size, uint32_t flags);
 
 /* How many of a backward's streams run as a pair of CTAs, one that recomputes and one that sweeps: all of them where

@@ -1700,6 +1700,8 @@ int clusters_at_once() {
 
 // How many streams the device runs at once with two CTAs each.
 int ttt_backward_pair_capacity() { return clusters_at_once<1>(); }
+// ... and with two streams to a cluster, the faster form.
+int ttt_backward_pairs_a_turn() { return 2 * clusters_at_once<2>(); }
 
 // The streams from `first` on, to the last.
 int ttt_launch_backward_pair(const ttt_b200_bwd_args* a, int first, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,

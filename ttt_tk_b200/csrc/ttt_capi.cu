@@ -33,6 +33,7 @@ uint64_t ttt_linear_backward_scratch_bytes(int B, int H, int cgs);
 int ttt_forward_cluster_capacity(int cluster);
 int ttt_backward_cluster_capacity(int cluster);
 int ttt_backward_pair_capacity();
+int ttt_backward_pairs_a_turn();
 int ttt_forward_pair_capacity();
 int ttt_launch_forward_cluster(const ttt_b200_fwd_args* a, int cluster, cudaStream_t stream, uint32_t* status,
                                uint64_t limit_ns, int drop_load);
@@ -152,19 +153,27 @@ static int backward_ctas(int streams, int NC, int cgs, uint32_t flags, int* ctas
   return TTT_B200_OK;
 }
 
-// Streams of a backward with one CTA per stream that two CTAs per stream take, in a launch of their own after the others': those
+// Streams of a call for one CTA per stream that two CTAs per stream take, in a launch of their own after the others': those
 // beyond a multiple of the SMs, when the device runs them as pairs at once.  A turn over the SMs with one CTA per stream lasts
 // 21.7 us per mini-batch however few streams are in it, one of pairs 10 to 14 and some us of launch.  Backward, us, without
 // and with it: 176 streams x 64 in groups of 8 2786 / 2076, 192 x 37 in groups of 6 1686 / 1319, 312 x 52 in groups of 7 3476 /
 // 2927, 1536 x 16 in groups of 4 4310 / 4209; where pairs are most and have least to pipeline, 222 streams x 8 in groups of 2
 // 457 / 425, x 5 309 / 296, x 4 238 / 239, x 3 199 / 201, 370 x 3 300 / 304.  So it gains from five mini-batches on and is
 // within 2 % below (149 and 176 streams x 4 in groups of 2 236 / 233 and 235 / 229, x 3 196 / 198 and 195 / 194).
+//
+// All of them, in two turns, where those hold them and are faster than one turn of single CTAs: per mini-batch two turns of
+// pairs take 18 to 20 us, one of single CTAs 21 to 22, but each turn starts with a recompute that nothing runs beside.  So it
+// takes groups to pipeline, and groups long enough that the sweep does not wait for the recompute.  Us, one CTA / pairs: 128
+// streams x 128 in groups of 8 2770 / 2458, x 64 1397 / 1295, x 64 in groups of 6 1435 / 1395, x 96 in groups of 12 2030 / 1869,
+// x 128 in groups of 20 2667 / 2457, 75 streams x 64 in groups of 8 1380 / 1244; 128 streams x 40 in groups of 5 921 / 938, x 64
+// in groups of 4 1517 / 1518, of 16 1344 / 1387, x 32 in groups of 6 735 / 769.
 static int backward_tail(int streams, int NC, int cgs, uint32_t flags, int ctas) {
   int asked = 0, dev = 0, sms = 0;
   if (ctas != 1 || !runs_pair(2, NC, cgs) || asked_cluster(flags, &asked) != TTT_B200_OK || asked != 0) return 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
     return 0;
+  if (streams <= 2 * ttt_backward_pairs_a_turn() && (cgs >= 8 ? NC >= 6 * cgs : cgs >= 6 && NC >= 10 * cgs)) return streams;
   const int rest = streams % sms;      // SMs hold one CTA each
   return streams > sms && rest <= ttt_backward_pair_capacity() ? rest : 0;
 }
@@ -374,7 +383,8 @@ extern "C" int ttt_b200_backward(const ttt_b200_bwd_args* a, void* stream_) {
   const uint64_t pair_limit = wait_limit_ns(a->checkpoint_group_size, a->NC);
   const int streams = a->B * a->H, tail = backward_tail(streams, a->NC, a->checkpoint_group_size, a->flags, cluster);
   if (cluster == 1) {
-    if (int rc = ttt_launch_backward(a, streams - tail, stream, status, wait_limit_ns(), drop)) return rc;
+    if (tail < streams)
+      if (int rc = ttt_launch_backward(a, streams - tail, stream, status, wait_limit_ns(), drop)) return rc;
     if (tail > 0)
       if (int rc = ttt_launch_backward_pair(a, streams - tail, stream, status, pair_limit, drop)) return rc;
   } else if (runs_pair(cluster, a->NC, a->checkpoint_group_size)) {
