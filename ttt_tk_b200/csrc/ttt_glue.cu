@@ -138,27 +138,50 @@ __global__ void __launch_bounds__(256, (kChunks <= 8 ? 4 : 2)) unpack_layernorm_
 // ---- backward of the output norm, fused with the token-major -> head-major turn of the gradient: the
 // result is the operator's grad_L_XQW_mini_batch.  With xhat = (x - mean) rstd and g = dy gamma:
 //   dx = rstd (g - mean(g) - xhat mean(g xhat)),   d_gamma[f] += sum over tokens of dy xhat,   d_beta[f] += sum of dy.
-// One pass over x and dy.  A lane owns 8 features (one 16-byte piece of a head row) for every token its CTA
-// works on: warp w takes the heads 4 w .. 4 w + 3 (and 4 (w + 8) .. when H > 32), so the parameter gradients
+// One pass over x and dy.  A token is the work of as many warps as it has groups of four heads (of eight warps with two groups
+// each when H > 32), and a CTA's eight warps take as many tokens side by side as that leaves room for: a lane owns 8 features
+// (one 16-byte piece of a head row) of every token its warps work on, so the parameter gradients
 // accumulate in 16 registers per head group with no traffic at all, and a token's two row means are put
-// together from the eight warps' partial sums through shared memory, kTokBatch tokens per CTA barrier.  When
-// the CTA has run out of tokens every lane adds its sums to the global ones with fp32 atomics (the order of
+// together from its warps' partial sums through shared memory, kTokBatch tokens per CTA barrier.  The next tokens' rows are
+// requested before these are worked on.  When
+// the CTA has run out of tokens its sums are added up and go to the global ones as fp32 atomics (the order of
 // the CTAs is not fixed: the last bits of the result can differ from run to run).
+// What bounds it: at small sizes the fp32 atomics, all CTAs' at the same addresses, so they are 16 bytes wide (a warp's eight
+// 4-byte ones touched 32 sectors each: 2048 tokens of 4 heads 40 us, now 8) and no more CTAs run than fit beside each other;
+// at large ones the round trip and barrier of a batch.  Before, with two tokens to a CTA whatever the number of heads and no
+// request ahead, and now: 8192 tokens of 12 heads 53 -> 23 us, of 32 heads 97 -> 42, 32768 of 32 184 -> 123 (3.3 TB/s).
 constexpr int kTokBatch = 2;
+// eight consecutive global sums += v, 16 bytes at a time where they are aligned for it
+__device__ __forceinline__ void add8(float* dst, const float (&v)[8]) {
+  if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+#pragma unroll
+    for (int k = 0; k < 8; k += 4)
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + k), "f"(v[k]), "f"(v[k + 1]), "f"(v[k + 2]),
+                   "f"(v[k + 3])
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) atomicAdd(dst + k, v[k]);
+  }
+}
 template <int kGroups>
-__global__ void __launch_bounds__(256, (kGroups == 1 ? 3 : 1))
+__global__ void __launch_bounds__(256, (kGroups == 1 ? 2 : 1))
 pack_layernorm_backward_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ x, const float* __restrict__ gamma,
                                const float2* __restrict__ stats, uint4* __restrict__ dx, float* __restrict__ d_gamma,
                                float* __restrict__ d_beta, long tokens, int T, int H) {
   __shared__ float2 part[2][kTokBatch][8];
+  __shared__ float sums[8][32][17];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane >> 3, piece = lane & 7;
   const float inv_n = 1.f / static_cast<float>(H * 64);
+  const int width = kGroups == 1 ? (H + 3) / 4 : 8;      // warps to a token
+  const int side = 8 / width;                            // tokens side by side
+  const int mine = warp / width, slot = warp - mine * width;
   int hh[kGroups];
   float gg[kGroups][8], ag[kGroups][8], ab[kGroups][8];
 #pragma unroll
   for (int g = 0; g < kGroups; ++g) {
-    hh[g] = 4 * (warp + 8 * g) + sub;
+    hh[g] = mine < side ? 4 * (slot + 8 * g) + sub : H;  // (a warp that is left over works on no head)
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       gg[g][k] = hh[g] < H ? gamma[hh[g] * 64 + piece * 8 + k] : 0.f;
@@ -166,30 +189,42 @@ pack_layernorm_backward_kernel(const uint4* __restrict__ dy, const uint4* __rest
       ab[g][k] = 0.f;
     }
   }
-  const long nbatch = (tokens + kTokBatch - 1) / kTokBatch;
-  int buf = 0;
-  for (long bt = blockIdx.x; bt < nbatch; bt += gridDim.x, buf ^= 1) {
-    uint4 rx[kTokBatch][kGroups], rg[kTokBatch][kGroups];
+  struct Rows {
+    uint4 x[kTokBatch][kGroups], g[kTokBatch][kGroups];
     float2 st[kTokBatch];
-    long xrow[kTokBatch];
+  };
+  const long per = static_cast<long>(kTokBatch) * side;
+  const long nbatch = (tokens + per - 1) / per;
+  auto token_of = [&](long bt, int q) { return bt * per + mine * kTokBatch + q; };
+  auto row_of = [&](long tok) {                          // of head 0; head h is h * T rows further
+    const long b = tok / T;
+    return b * H * T + (tok - b * T);
+  };
+  auto load = [&](long bt, Rows& r) {
 #pragma unroll
     for (int q = 0; q < kTokBatch; ++q) {
-      const long tok = bt * kTokBatch + q;
-      const bool live = tok < tokens;
-      const long b = live ? tok / T : 0, t = live ? tok - b * T : 0;
-      xrow[q] = b * H * T + t;                      // row of head 0; head h is h * T rows further
-      st[q] = live ? stats[tok] : make_float2(0.f, 0.f);
+      const long tok = token_of(bt, q);
+      const bool live = bt < nbatch && mine < side && tok < tokens;
+      const long xrow = live ? row_of(tok) : 0;
+      r.st[q] = live ? stats[tok] : make_float2(0.f, 0.f);
 #pragma unroll
       for (int g = 0; g < kGroups; ++g) {
         if (live && hh[g] < H) {
-          rx[q][g] = __ldcs(x + ((xrow[q] + static_cast<long>(hh[g]) * T) << 3) + piece);
-          rg[q][g] = __ldcs(dy + ((tok * H + hh[g]) << 3) + piece);
+          r.x[q][g] = __ldcs(x + ((xrow + static_cast<long>(hh[g]) * T) << 3) + piece);
+          r.g[q][g] = __ldcs(dy + ((tok * H + hh[g]) << 3) + piece);
         } else {
-          rx[q][g] = make_uint4(0u, 0u, 0u, 0u);    // dy = 0: no contribution to any sum
-          rg[q][g] = make_uint4(0u, 0u, 0u, 0u);
+          r.x[q][g] = make_uint4(0u, 0u, 0u, 0u);    // dy = 0: no contribution to any sum
+          r.g[q][g] = make_uint4(0u, 0u, 0u, 0u);
         }
       }
     }
+  };
+  Rows next;
+  load(blockIdx.x, next);
+  int buf = 0;
+  for (long bt = blockIdx.x; bt < nbatch; bt += gridDim.x, buf ^= 1) {
+    const Rows r = next;
+    load(bt + gridDim.x, next);
     float s1[kTokBatch], s2[kTokBatch];
 #pragma unroll
     for (int q = 0; q < kTokBatch; ++q) {
@@ -197,12 +232,12 @@ pack_layernorm_backward_kernel(const uint4* __restrict__ dy, const uint4* __rest
       s2[q] = 0.f;
 #pragma unroll
       for (int g = 0; g < kGroups; ++g) {
-        const __nv_bfloat162* vx = reinterpret_cast<const __nv_bfloat162*>(&rx[q][g]);
-        const __nv_bfloat162* vg = reinterpret_cast<const __nv_bfloat162*>(&rg[q][g]);
+        const __nv_bfloat162* vx = reinterpret_cast<const __nv_bfloat162*>(&r.x[q][g]);
+        const __nv_bfloat162* vg = reinterpret_cast<const __nv_bfloat162*>(&r.g[q][g]);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const float2 fx = __bfloat1622float2(vx[k]), fg = __bfloat1622float2(vg[k]);
-          const float x0 = (fx.x - st[q].x) * st[q].y, x1 = (fx.y - st[q].x) * st[q].y;
+          const float x0 = (fx.x - r.st[q].x) * r.st[q].y, x1 = (fx.y - r.st[q].x) * r.st[q].y;
           const float a0 = fg.x * gg[g][2 * k], a1 = fg.y * gg[g][2 * k + 1];
           s1[q] += a0 + a1;
           s2[q] = fmaf(a0, x0, fmaf(a1, x1, s2[q]));
@@ -233,23 +268,23 @@ pack_layernorm_backward_kernel(const uint4* __restrict__ dy, const uint4* __rest
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < kTokBatch; ++q) {
-      const long tok = bt * kTokBatch + q;
-      if (tok >= tokens) break;
+      const long tok = token_of(bt, q);
+      if (mine >= side || tok >= tokens) break;
       float m1 = 0.f, m2 = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) {
-        const float2 pw = part[buf][q][w];
+      for (int w = 0; w < width; ++w) {
+        const float2 pw = part[buf][q][mine * width + w];
         m1 += pw.x;
         m2 += pw.y;
       }
       m1 *= inv_n;
       m2 *= inv_n;
-      const float mean = st[q].x, rstd = st[q].y;
+      const float mean = r.st[q].x, rstd = r.st[q].y;
+      const long xrow = row_of(tok);
 #pragma unroll
       for (int g = 0; g < kGroups; ++g) {
         if (hh[g] < H) {
-          const __nv_bfloat162* vx = reinterpret_cast<const __nv_bfloat162*>(&rx[q][g]);
-          const __nv_bfloat162* vg = reinterpret_cast<const __nv_bfloat162*>(&rg[q][g]);
+          const __nv_bfloat162* vx = reinterpret_cast<const __nv_bfloat162*>(&r.x[q][g]);
+          const __nv_bfloat162* vg = reinterpret_cast<const __nv_bfloat162*>(&r.g[q][g]);
           uint4 o4;
           __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&o4);
 #pragma unroll
@@ -259,19 +294,32 @@ pack_layernorm_backward_kernel(const uint4* __restrict__ dy, const uint4* __rest
             o[k] = __floats2bfloat162_rn(rstd * (fmaf(fg.x, gg[g][2 * k], -m1) - x0 * m2),
                                          rstd * (fmaf(fg.y, gg[g][2 * k + 1], -m1) - x1 * m2));
           }
-          __stcs(dx + ((xrow[q] + static_cast<long>(hh[g]) * T) << 3) + piece, o4);
+          __stcs(dx + ((xrow + static_cast<long>(hh[g]) * T) << 3) + piece, o4);
         }
       }
     }
   }
+  if (kGroups == 1 && side > 1) {      // the tokens side by side have addends for the same features: the first warps' lanes sum them
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      sums[warp][lane][k] = ag[0][k];
+      sums[warp][lane][8 + k] = ab[0][k];
+    }
+    __syncthreads();
+    if (mine == 0)
+      for (int m = 1; m < side; ++m) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          ag[0][k] += sums[m * width + warp][lane][k];
+          ab[0][k] += sums[m * width + warp][lane][8 + k];
+        }
+      }
+  }
 #pragma unroll
   for (int g = 0; g < kGroups; ++g) {
-    if (hh[g] < H) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        atomicAdd(d_gamma + hh[g] * 64 + piece * 8 + k, ag[g][k]);
-        atomicAdd(d_beta + hh[g] * 64 + piece * 8 + k, ab[g][k]);
-      }
+    if (hh[g] < H && mine == 0) {
+      add8(d_gamma + hh[g] * 64 + piece * 8, ag[g]);
+      add8(d_beta + hh[g] * 64 + piece * 8, ab[g]);
     }
   }
 }
@@ -374,8 +422,9 @@ extern "C" int ttt_b200_pack_layernorm_backward(const void* grad_y, const void* 
   const long tokens = static_cast<long>(B) * T;
   // one wave of CTAs (as many as are resident at once), each looping over its token batches: every CTA ends
   // with 2 x 64 H atomic adds for the parameter gradients, so there should be no more of them than can run
-  long blocks = (tokens + kTokBatch - 1) / kTokBatch;
-  const long cap = static_cast<long>(sms) * (H <= 32 ? 3 : 1);
+  const long per = H <= 32 ? kTokBatch * (8 / ((H + 3) / 4)) : kTokBatch;
+  long blocks = (tokens + per - 1) / per;
+  const long cap = static_cast<long>(sms) * (H <= 32 ? 2 : 1);
   if (blocks > cap) blocks = cap;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
 #define TTT_LNB_LAUNCH(G)                                                                                        \
