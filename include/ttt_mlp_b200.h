@@ -297,7 +297,7 @@ int ttt_b200_launch_cluster(int streams, uint32_t flags, int backward);
 int ttt_b200_forward_ctas(int streams, int NC, int checkpoint_group_size, uint32_t flags);
 
 /* The same for a backward of NC mini-batches in groups of checkpoint_group_size: without a size in the flags or the
- * environment it is two instead of four from three groups of four mini-batches on. */
+ * environment it is two instead of four from three groups of four mini-batches or two of eight on. */
 int ttt_b200_backward_ctas(int streams, int NC, int checkpoint_group_size, uint32_t flags);
 
 /* Of a backward whose answer there is one: how many of its last streams a launch after the others' gives two CTAs each: those

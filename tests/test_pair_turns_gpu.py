@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from test_cluster_backward_gpu import inputs, oracle_forward, run_backward
+from test_cluster_backward_gpu import TOL, check, inputs, oracle_backward, oracle_forward, run_backward
 from ttt_tk_b200 import _lib
 from ttt_tk_b200.buffers import GRAD_NAMES
 
@@ -27,3 +27,17 @@ def test_two_turns_are_the_forced_form():
     now, two = run_backward(d, ck, cgs, None), run_backward(d, ck, cgs, 2)
     for k in GRAD_NAMES:
         assert torch.equal(now[k], two[k]), k
+
+
+@pytest.mark.parametrize("NC,cgs,ctas", [(16, 8, 2), (15, 8, 4), (14, 7, 4), (21, 7, 2)])
+def test_two_long_groups_take_a_pair(NC, cgs, ctas):
+    """Where four CTAs per stream would fit: the form it takes, against the oracle (3e-2: every gradient's gate)."""
+    lib = _lib.lib()
+    assert lib.ttt_b200_backward_ctas(lib.ttt_b200_cluster_capacity(4, 1), NC, cgs, 0) == ctas
+    d = inputs(1, 3, NC, seed=2)
+    ck = oracle_forward(d, cgs)
+    now = run_backward(d, ck, cgs, None)
+    check(now, oracle_backward(d, ck, cgs), TOL, "gradients")
+    for k, t in run_backward(d, ck, cgs, ctas).items():
+        if k in GRAD_NAMES:
+            assert torch.equal(now[k], t), k

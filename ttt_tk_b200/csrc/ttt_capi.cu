@@ -141,24 +141,27 @@ static int forward_ctas(int streams, int NC, int cgs, uint32_t flags, int* ctas)
 // of a pair take turns) 26 us per mini-batch against 28.
 static bool runs_pair(int ctas, int NC, int cgs) { return ctas == 2 && cgs > 1 && NC > cgs; }
 
-// CTAs per stream of a backward.  Where four would fit, two are faster once a call has three groups of four mini-batches to
-// pipeline: the first group's recompute runs alone, and a group that has few slots to spare ends with a wait for the last of
-// the next (32 streams, pair against four CTAs, us per mini-batch: 256 mini-batches in groups of 16 9.3 / 13.2, 48 in groups
-// of 16 11.7 / 13.3, 24 in groups of 8 12.5 / 13.8, 12 in groups of 4 14.0 / 14.5; two groups: 16 in groups of 8 14.1 / 14.0,
-// 8 in groups of 4 15.2 / 14.7; small groups: 32 in groups of 3 14.9 / 14.7, in groups of 2 17.2 / 15.4).
+// CTAs per stream of a backward.  Where four would fit, two are faster once a call has two groups of eight mini-batches or
+// three of four to pipeline: the first group's recompute runs alone, and a group that has few slots to spare ends with a wait
+// for the last of the next (32 streams, pair against four CTAs, us per mini-batch: 256 mini-batches in groups of 16 8.5 / 13.2,
+// 48 in groups of 16 10.4 / 13.5, 24 in groups of 8 11.4 / 14.0, 12 in groups of 4 13.0 / 14.8; two groups: 32 in groups of 16
+// 11.6 / 13.5, 16 in groups of 8 12.8 / 14.2, 12 streams 11.8 / 13.8, 8 in groups of 4 14.4 / 15.3; a short second group: 12 in
+// groups of 8 14.1 / 14.5, 20 in groups of 16 13.9 / 13.9, 9 in groups of 8 16.5 / 15.3; small groups: 32 in groups of 3 13.7 /
+// 14.8 and 6 16.4 / 15.7, 32 in groups of 2 16.0 / 15.5).
 static int backward_ctas(int streams, int NC, int cgs, uint32_t flags, int* ctas) {
   if (int rc = ttt_launch_cluster(streams, flags, true, ctas)) return rc;
   int asked = 0;
-  if (asked_cluster(flags, &asked) == TTT_B200_OK && asked == 0 && *ctas == 4 && cgs >= 4 && NC >= 3 * cgs) *ctas = 2;
+  if (asked_cluster(flags, &asked) == TTT_B200_OK && asked == 0 && *ctas == 4 && cgs >= 4 && NC >= (cgs >= 8 ? 2 : 3) * cgs)
+    *ctas = 2;
   return TTT_B200_OK;
 }
 
 // Streams of a call for one CTA per stream that two CTAs per stream take, in a launch of their own after the others': those
 // beyond a multiple of the SMs, when the device runs them as pairs at once.  A turn over the SMs with one CTA per stream lasts
-// 21.7 us per mini-batch however few streams are in it, one of pairs 10 to 14 and some us of launch.  Backward, us, without
-// and with it: 176 streams x 64 in groups of 8 2786 / 2076, 192 x 37 in groups of 6 1686 / 1319, 312 x 52 in groups of 7 3476 /
-// 2927, 1536 x 16 in groups of 4 4310 / 4209; where pairs are most and have least to pipeline, 222 streams x 8 in groups of 2
-// 457 / 425, x 5 309 / 296, x 4 238 / 239, x 3 199 / 201, 370 x 3 300 / 304.  So it gains from five mini-batches on and is
+// 21.7 us per mini-batch however few streams are in it, one of pairs 9 to 13 and some us of launch.  Backward, us, without
+// and with it: 176 streams x 64 in groups of 8 2783 / 2025, 192 x 37 in groups of 6 1681 / 1280, 312 x 52 in groups of 7 3454 /
+// 2860, 1536 x 16 in groups of 4 4272 / 4141; where pairs are most and have least to pipeline, 222 streams x 8 in groups of 2
+// 459 / 421, x 5 309 / 296, x 4 238 / 239, x 3 199 / 201, 370 x 3 300 / 304.  So it gains from five mini-batches on and is
 // within 2 % below (149 and 176 streams x 4 in groups of 2 236 / 233 and 235 / 229, x 3 196 / 198 and 195 / 194).
 //
 // All of them, in two turns, where those hold them and are faster than one turn of single CTAs: per mini-batch two turns of
