@@ -105,9 +105,10 @@ int capacity(int cluster, bool backward) {
 // streams than SMs the idle SMs can only help by taking a share of every stream's hidden units, and only while all
 // streams are resident at once.  Four CTAs per stream win whenever the device runs that many clusters of four (32 streams
 // of 128 mini-batches in groups of 4 on a B200: forward 4.3 against 4.6 us per mini-batch with one CTA, backward 14.0
-// against 22.7; of the backward's longer calls: backward_ctas).  Where only clusters of two fit (34 to 74 streams), the
-// forward runs one CTA, whose output pass runs beside the chain in two groups of warps (4.6 us per mini-batch against 5.8
-// with two CTAs), and the backward two (60 streams in groups of 4: 13.3 us per mini-batch against 23.3 with one).  Beyond, one.
+// against 22.7; of longer calls: forward_ctas, backward_ctas).  Where only clusters of two fit (34 to 74 streams), short
+// forwards run one CTA, whose output pass runs beside the chain in two groups of warps (4.6 us per mini-batch against 5.8
+// with half of the hidden units each), and the backward two (60 streams in groups of 5: 11.7 us per mini-batch against 23.3 with
+// one).  Beyond, one.
 static int ttt_launch_cluster(int streams, uint32_t flags, bool backward, int* cluster) {
   if (int rc = asked_cluster(flags, cluster)) return rc;
   if (*cluster != 0) return TTT_B200_OK;

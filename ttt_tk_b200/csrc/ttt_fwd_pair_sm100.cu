@@ -30,7 +30,7 @@
 // What bounds it: the chain.  Of its 6900 cycles, EPI1 has 1800 (the fp32 pipe alone needs 1150, the MUFU 1000), the LayerNorm
 // with its two exchanges 1250, the four products with their hand-overs 2800.  us per mini-batch, against one CTA per stream and
 // against four with a quarter of the hidden units each: 48 streams x 32 in groups of 4 4.75 -> 4.3, 32 x 128 in groups of 16
-// 4.6 / 4.19 -> 3.82, 4 x 32 in groups of 4 4.75 / 4.36 -> 4.1.  A checkpoint takes the output CTA 4900 cycles (132 KB at 27
+// 4.2 / 4.19 -> 3.73, 4 x 32 in groups of 4 4.65 / 4.36 -> 4.05.  A checkpoint takes the output CTA 4900 cycles (132 KB at 27
 // bytes a clock), of which the chain has to wait for about 2500.  Steps on the way, 32 x 128: 4.31 with everything in sixteen
 // warps, 4.12 with the LayerNorm in eight and X2 in two buffers, 3.84 with two streams to a cluster, 3.82 with W2's copy beside
 // MMA4 and all that needs no Z2 before its wait.  Not kept: G' in a pass of its own under MMA2 (that window is full: 3.94),

@@ -30,7 +30,7 @@
 // warps per scheduler).
 //
 // What bounds it: the chain's four round trips.  No pipe is full over a mini-batch (128 streams: issue slots 44 %, fp32
-// pipe 35 %, tensor pipe 20 %, DRAM 11 %), but within its epilogues the fp32 and MUFU pipes set the pace (EPI1 alone is
+// pipe 37 %, tensor pipe 21 %, DRAM 11 %), but within its epilogues the fp32 and MUFU pipes set the pace (EPI1 alone is
 // 1300 cycles of fp32 pipe at 9 packed operations and 2 conversions per pair of elements) and within its products the
 // shared-memory operands.  So the arithmetic runs on packed fp32 pairs; what only one thread needs stays out of shared
 // memory (G' in registers from EPI1 to EPI3, U1 and the bf16 W1 in tensor memory as A operands of their MMAs, which then
@@ -38,7 +38,7 @@
 // of 128 mini-batches, one checkpoint in 8): 8.0 us per mini-batch as one group of 8 warps, 6.0 with the two groups, 4.6
 // with the rest, 4.3 with the products of a block issued by the block's own first warp and the W2 update by the output
 // group (before, one warp issued all sixteen MMAs of the state update and came 400 cycles late to EPI4, with everyone
-// waiting for it); 1536 streams of 64 mini-batches 5.43 -> 3.23 -> 2.95 ms.  A checkpoint costs about 2100 cycles (the
+// waiting for it); 1536 streams of 64 mini-batches 5.43 -> 3.23 -> 2.98 ms.  A checkpoint costs about 2100 cycles (the
 // output group's 4200 for 132 KB of stores, of which half fit its slack); as bulk copies from a staging area it cost
 // more, since W1's turn of the area waits for W2 to leave.
 //
