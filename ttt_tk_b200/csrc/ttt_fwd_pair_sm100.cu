@@ -735,16 +735,16 @@ ttt_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, TM_COLS);
-  cluster_arrive();      // no CTA leaves while the other may still send to it
-  cluster_wait();
-  const bool any = *abort_flag != 0;      // of either CTA
-  if (any) {             // copies between the CTAs that an abort cut short may still be on their way: they take a few microseconds
+  if (aborted) {         // copies to the other CTA that the abort cut short may still be on their way: they take a few microseconds
     const uint64_t t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 50000) {}
     __syncthreads();
-    cluster_arrive();
-    cluster_wait();
   }
+  // No CTA leaves while another may still send to it.  One barrier for all of the cluster: whether a CTA aborted is its own
+  // affair, and with two streams to a cluster not the other stream's.  (A CTA that sent anything and did not abort has seen it
+  // used: X_FREE of the last mini-batch.)
+  cluster_arrive();
+  cluster_wait();
 }
 
 // Once per device: the kernel's dynamic shared memory limit.
