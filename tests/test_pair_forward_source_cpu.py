@@ -17,3 +17,14 @@ def test_every_cta_of_a_cluster_meets_the_same_number_of_barriers():
         if token not in "{}":
             found.append((token, depth))
     assert found == [("cluster_arrive()", 1), ("cluster_wait()", 1)] * 2
+
+
+def test_tensor_memory_is_read_by_whole_warps():
+    """A wait is left lane by lane.  Between it and a load from tensor memory the warp comes together: wait_mma, or done."""
+    epilogues = KERNEL[KERNEL.index("for (int it = 0;"):KERNEL.index("reg_give")]
+    last = None
+    for token in re.findall(r"\b(wait|wait_mma|done|done_tmem|frag_ld|tmem_ld\w+)\(", epilogues):
+        if token == "frag_ld" or token.startswith("tmem_ld"):
+            assert last != "wait"
+        else:
+            last = token

@@ -547,9 +547,9 @@ ttt_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
         done(E_5);
         // ---- OUT: Q + gamma * LN(Z2b + b2) + beta, over the Q tile (every thread rewrites what it has read)
+        if (tok) wait(OQ + s);
         wait_mma(OZ);
         if (tok) {
-          wait(OQ + s);
           TokFrag x;
           uint32_t q[8];
           frag_ld(tm, tmem + TM_ZB, x);
@@ -571,7 +571,8 @@ ttt_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           done(E_OUT + s);
         }
       }
-      if (p.W1f != nullptr && !idle && *abort_flag == 0) store_state(p.W1f + st_w, p.W2f + st_w, p.b1f + sid * 256, p.b2f + sid * 64);
+      if (p.W1f != nullptr && !idle && __all_sync(0xffffffffu, *abort_flag == 0))
+        store_state(p.W1f + st_w, p.W2f + st_w, p.b1f + sid * 256, p.b2f + sid * 64);
     }
   } else {
     reg_give<kRegsHelp>();
