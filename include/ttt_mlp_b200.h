@@ -42,10 +42,15 @@ enum {
    * of its second mini-batch (its only one when NC = 1), so that the kernel's bounded wait for them
    * runs out; the kernel reports code 3 through the status word and exits normally. */
   TTT_B200_FLAG_TEST_LOST_LOAD = 2u,
-  /* Bits 8..11: how many CTAs (of a thread-block cluster) share one (batch, head) stream, each owning 256 / n hidden units
-   * or, with two, one the chain and one the output pass (forward), one recomputing and one sweeping (backward); the reference fixes this at compile time (TP = 2 in kernels/ttt/ttt.cu:11-12,
-   * 4 in kernels/ttt_backward/ttt.cu:12-16).  0 = chosen per launch from B*H and the number of clusters the GPU runs at once
-   * (overridable with the environment variable TTT_B200_CLUSTER); 1, 2 or 4 = forced. */
+  /* Bits 8..11: how many CTAs (of a thread-block cluster) share one (batch, head) stream: four with a quarter of the hidden
+   * units each; two, one with the chain and one with the output pass (forward), one recomputing and one sweeping (backward; with
+   * half of the hidden units each where that has no groups to pipeline: a single one, or groups of one mini-batch); or one.  The
+   * reference fixes this at compile time (TP = 2 in kernels/ttt/ttt.cu:11-12, 4 in kernels/ttt_backward/ttt.cu:12-16).  0 =
+   * chosen per launch from B*H, NC, checkpoint_group_size and the number of clusters the GPU runs at once (overridable with the
+   * environment variable TTT_B200_CLUSTER); 1, 2 or 4 = forced.
+   * Calls of different forms agree within rounding, not bit for bit, and 0 can choose one form for a long call and another for a
+   * short one.  For a sequence in chunks to have the bits of one long call, name the size: 1 and 4 are one form each; 2 is one
+   * form in the forward, and in the backward as long as every chunk is longer than a group of at least two mini-batches. */
   TTT_B200_FLAG_CLUSTER_SHIFT = 8,
   TTT_B200_FLAG_CLUSTER_MASK = 0xFu << 8
 };

@@ -35,8 +35,8 @@ int ttt_backward_cluster_capacity(int cluster);
 int ttt_backward_pair_capacity();
 int ttt_backward_pairs_a_turn();
 int ttt_forward_pair_capacity();
-int ttt_launch_forward_cluster(const ttt_b200_fwd_args* a, int cluster, cudaStream_t stream, uint32_t* status,
-                               uint64_t limit_ns, int drop_load);
+int ttt_launch_forward_cluster(const ttt_b200_fwd_args* a, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
+                               int drop_load);
 
 namespace {
 
@@ -118,16 +118,14 @@ static int ttt_launch_cluster(int streams, uint32_t flags, bool backward, int* c
   return TTT_B200_OK;
 }
 
-// A forward with two CTAs per stream gives them the chain and the output pass (ttt_fwd_pair_sm100.cu) from four mini-batches
-// on.  Below, where only a caller asks for two, each takes half of the hidden units, and of the state's way in and out (12
-// streams, us, halves / chain and output: 1 mini-batch 10.9 / 14.5, 2 16.5 / 18.2, 3 23.1 / 23.3, 4 28.6 / 26.4).
-static bool forward_pair(int ctas, int NC) { return ctas == 2 && NC >= 4; }
-
 // CTAs per stream of a forward.  Two where the device runs all streams as pairs at once and that is the faster form: against
 // one CTA from six mini-batches on (us, one CTA / pair: 34 streams x 4 in groups of 2 27.6 / 27.5, x 6 in groups of 3 35.5 /
 // 34.9, x 16 in groups of 4 79 / 72; 48 x 32 in groups of 6 147 / 136, in groups of 1 203 / 177), against four, which share
 // the writing of the state, from 16 mini-batches in groups of four on (four / pair: 12 streams x 12 in groups of 4 54.8 /
 // 56.1, x 16 71.9 / 71.2; x 32 in groups of 6 138 / 131, x 16 in groups of 2 72.7 / 77.6; 32 x 128 in groups of 16 536 / 489).
+// Two are always the chain and the output pass (ttt_fwd_pair_sm100.cu), whatever the call's length: a sequence in chunks, with
+// the size named, then has the bits of one call.  (Half of the hidden units each is faster up to three mini-batches, 12 streams
+// x 1 10.9 / 14.5 us, but no rule takes two there.)
 static int forward_ctas(int streams, int NC, int cgs, uint32_t flags, int* ctas) {
   if (int rc = ttt_launch_cluster(streams, flags, false, ctas)) return rc;
   int asked = 0;
@@ -300,9 +298,9 @@ extern "C" int ttt_b200_forward(const ttt_b200_fwd_args* a, void* stream_) {
   const int drop = (a->flags & TTT_B200_FLAG_TEST_LOST_LOAD) ? (a->NC > 1 ? 1 : 0) : -1;
   if (ctas == 1) {
     if (int rc = ttt_launch_forward(a, stream, status, wait_limit_ns(), drop)) return rc;
-  } else if (forward_pair(ctas, a->NC)) {
+  } else if (ctas == 2) {
     if (int rc = ttt_launch_forward_pair(a, stream, status, wait_limit_ns(), drop)) return rc;
-  } else if (int rc = ttt_launch_forward_cluster(a, ctas, stream, status, wait_limit_ns(), drop)) {
+  } else if (int rc = ttt_launch_forward_cluster(a, stream, status, wait_limit_ns(), drop)) {
     return rc;
   }
   if (a->flags & TTT_B200_FLAG_SYNC) return ttt_check_status(stream);

@@ -368,14 +368,6 @@ __device__ __forceinline__ void tok_st_tile(const TokMap& m, uint8_t* tile, cons
     *reinterpret_cast<uint32_t*>(tile + m.off(m.r1, j)) = pack_bf16(v[4 * j + 2], v[4 * j + 3]);
   }
 }
-// per-column vector (fp32[64] in shared memory) -> the thread's 8 columns: c[2j], c[2j+1]
-__device__ __forceinline__ void tok_ld_cols(const TokMap& m, const float* vec, float (&c)[8]) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 f = *reinterpret_cast<const float2*>(vec + m.col(j));
-    c[2 * j] = f.x; c[2 * j + 1] = f.y;
-  }
-}
 // All-reduce N per-row partial sums over the 8 threads that share each row.  a[] belongs to row
 // r0, b[] to row r1.  xch: fp32[2][64][8] in shared memory; the call uses columns kSlot .. kSlot+N-1
 // of it.  There is no barrier after the read-back: the all-reduces of one epilogue phase must use
@@ -404,31 +396,6 @@ __device__ __forceinline__ void tok_row_allreduce(const TokMap& m, float (&a)[N]
     b[i] += xch[((m.colhalf ^ 1) * 64 + m.r1) * 8 + kSlot + i];
   }
 }
-// LayerNorm statistics of the thread's two rows: centres z in place, returns 1/std per row.  Uses the
-// exchange columns 0 and 1.
-__device__ __forceinline__ void tok_layernorm(const TokMap& m, float (&z)[16], float eps, float* xch, float& rstd0,
-                                              float& rstd1) {
-  float s0[1] = {0.f}, s1[1] = {0.f};
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    s0[0] += z[4 * j] + z[4 * j + 1];
-    s1[0] += z[4 * j + 2] + z[4 * j + 3];
-  }
-  tok_row_allreduce<1, 0>(m, s0, s1, xch);
-  const float mu0 = s0[0] * (1.f / 64.f), mu1 = s1[0] * (1.f / 64.f);
-  s0[0] = 0.f; s1[0] = 0.f;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    z[4 * j] -= mu0; z[4 * j + 1] -= mu0;
-    z[4 * j + 2] -= mu1; z[4 * j + 3] -= mu1;
-    s0[0] = fmaf(z[4 * j], z[4 * j], fmaf(z[4 * j + 1], z[4 * j + 1], s0[0]));
-    s1[0] = fmaf(z[4 * j + 2], z[4 * j + 2], fmaf(z[4 * j + 3], z[4 * j + 3], s1[0]));
-  }
-  tok_row_allreduce<1, 1>(m, s0, s1, xch);
-  rstd0 = rsqrtf(s0[0] * (1.f / 64.f) + eps);
-  rstd1 = rsqrtf(s1[0] * (1.f / 64.f) + eps);
-}
-
 // ---- The same fragments as packed fp32 pairs, for kernels whose CTA runs several groups of 8 warps: a[j] is
 // the column pair col(j), col(j) + 1 of row r0, b[j] that of row r1.  `bar` = the group's first of four named
 // barriers (one per warp pair), `xch` the group's exchange area (kXchBytes).

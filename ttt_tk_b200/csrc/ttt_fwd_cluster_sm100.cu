@@ -1,4 +1,4 @@
-// TTT-MLP forward for sm_100a, cluster-sharded: one thread-block cluster of kC = 2 or 4 CTAs per
+// TTT-MLP forward for sm_100a, cluster-sharded: one thread-block cluster of kC = 4 CTAs per
 // (batch, head) stream, each CTA owning 256 / kC of the hidden units.
 //
 // Replaces the reference's fwd_ttt_mlp_ker with its hidden dimension split over a cluster
@@ -43,9 +43,7 @@ struct Cfg {
   static constexpr int NB = 4 / kC;                  // 64-row blocks of hidden units per CTA
   static constexpr int R = 64 * NB;                  // hidden units per CTA
   static constexpr uint32_t HB = NB * TILE;          // bytes of an [R][64] bf16 tile
-  using RS = RowSplit<kC>;                     // kC = 4: row-split LayerNorm stages
-  using Sum = ClusterSum<kC, 16384>;           // kC = 2: all-reduce, stages on the whole tile in both CTAs
-  static constexpr bool kRowSplit = kC == 4;   // measured: at kC = 2 the second hop costs more than the halved stage saves
+  using RS = RowSplit<kC>;
   static constexpr uint32_t OFF_K = 0;
   static constexpr uint32_t OFF_V = OFF_K + kStages * TILE;
   static constexpr uint32_t OFF_Q = OFF_V + kStages * TILE;
@@ -56,7 +54,7 @@ struct Cfg {
   static constexpr uint32_t OFF_X2 = OFF_W2 + HB;
   static constexpr uint32_t OFF_GP = OFF_X2 + HB;
   static constexpr uint32_t OFF_SUM = OFF_GP + HB;                 // cluster exchange area
-  static constexpr uint32_t OFF_ETA = OFF_SUM + (kRowSplit ? RS::kBytes : Sum::kBytes);
+  static constexpr uint32_t OFF_ETA = OFF_SUM + RS::kBytes;
   static constexpr uint32_t OFF_B2 = OFF_ETA + kStages * 128;
   static constexpr uint32_t OFF_GAMMA = OFF_B2 + 256;
   static constexpr uint32_t OFF_BETA = OFF_GAMMA + 256;
@@ -144,7 +142,7 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   if (tid == kProd) {
     for (int s = 0; s < kStages; ++s) mbar_init(&full[s], 1);
     mbar_init(mma_bar, 4);
-    for (int i = 0; i < C::RS::kBufs; ++i) mbar_init(&sum_bars[i], C::kRowSplit ? C::RS::kBarCount : C::Sum::kArrivals);
+    for (int i = 0; i < C::RS::kBufs; ++i) mbar_init(&sum_bars[i], C::RS::kBarCount);
     mbar_init(drain_bar, 4);
     mbar_init(ag_bar, 1);
     fence_mbar_init();
@@ -228,14 +226,6 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   rs.limit = limit;
   constexpr int NR = C::RS::NR;                     // rows per thread in the row-split stages
   uint32_t ag_phase = 0;
-  typename C::Sum csum;
-  csum.bufp = smem + C::OFF_SUM;
-  csum.bars = sum_bars;
-  csum.n = 0;
-  csum.rank = rank;
-  csum.abort_flag = abort_flag;
-  csum.limit = limit;
-
   auto store_w1_block = [&](float* W1o, int b) {
     float w1[16];
     tok_ld(tm, tmem + C::TM_W1 + b * 64, w1);
@@ -312,37 +302,6 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   // that one waits for its own Z2 sum.
   uint32_t zo_tag = 0;
   int zo_it = -1;
-  float zo[16];          // kC = 2: the partial tile between the send and the receive of its reduce-scatter
-  auto finish_out_whole = [&]() {
-    const bool mine = csum.reduce_scatter_recv(zo, tid, zo_tag);
-    if (mine) {       // whole warp pairs (the two warps of a fragment quadrant) take this branch together
-      const uint8_t* sQp = smem + C::OFF_Q + (zo_it % kStages) * TILE;
-      float b2c[8], gam[8], bet[8], q[16];
-      tok_ld_cols(tm, sB2, b2c);
-      tok_ld_cols(tm, sGamma, gam);
-      tok_ld_cols(tm, sBeta, bet);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        zo[4 * j] += b2c[2 * j]; zo[4 * j + 1] += b2c[2 * j + 1];
-        zo[4 * j + 2] += b2c[2 * j]; zo[4 * j + 3] += b2c[2 * j + 1];
-      }
-      float rs0, rs1;
-      tok_ld_tile(tm, sQp, q);
-      tok_layernorm(tm, zo, TTT_LN_EPS, sXch, rs0, rs1);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i0 = 4 * j + e, i1 = 4 * j + 2 + e, c = 2 * j + e;
-          q[i0] += fmaf(gam[c], zo[i0] * rs0, bet[c]);
-          q[i1] += fmaf(gam[c], zo[i1] * rs1, bet[c]);
-        }
-      }
-      tok_st_global(tm, p.out + (stream_id * NC + zo_it) * 4096, q);
-    }
-    zo_it = -1;
-  };
-
   auto finish_out = [&]() {
     const uint8_t* sQp = smem + C::OFF_Q + (zo_it % kStages) * TILE;
     const float2 b2c = *reinterpret_cast<const float2*>(sB2 + 2 * lane);
@@ -391,9 +350,6 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       store_b1(p.b1c + ckc * 256);
       if (rank == 0 && tid < 64) p.b2c[ckc * 64 + tid] = sB2[tid];   // before this mini-batch's column sums reach b2
     }
-    if constexpr (!C::kRowSplit) {
-      if (zo_it >= 0) finish_out_whole();    // the previous mini-batch's output, with the b2 it saw
-    }
     wait_mma();
     // ---- EPI1: X2^T = gelu(Z1^T + b1), G' = gelu'(Z1^T + b1)
 #pragma unroll
@@ -424,7 +380,6 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // ---- LN: the partial Z2 tiles are summed by reduce-scatter; every CTA runs the fused LayerNorm + L2
     // gradient, U2 = -eta * dl/dZ2, on the token rows it owns (all 256 threads, CPT columns of one row each)
     // and hands its rows of U2 to the other CTAs' shared memories.
-    if constexpr (C::kRowSplit) {
     {
       float frag[16];
       tok_ld(tm, tmem + C::TM_Z, frag);
@@ -466,53 +421,6 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     }
     mbar_wait_cl(ag_bar, ag_phase, abort_flag, limit, kC);
     ag_phase ^= 1u;
-    } else {
-    {
-      float xh[16], b2c[8], gam[8], bet[8];
-      tok_ld(tm, tmem + C::TM_Z, xh);
-      csum.run(xh, tid, lane);
-      tok_ld_cols(tm, sB2, b2c);
-      tok_ld_cols(tm, sGamma, gam);
-      tok_ld_cols(tm, sBeta, bet);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        xh[4 * j] += b2c[2 * j]; xh[4 * j + 1] += b2c[2 * j + 1];
-        xh[4 * j + 2] += b2c[2 * j]; xh[4 * j + 3] += b2c[2 * j + 1];
-      }
-      float rs0, rs1;
-      float kk[16], vv[16], g[16];
-      tok_ld_tile(tm, sK, kk);
-      tok_ld_tile(tm, sV, vv);
-      tok_layernorm(tm, xh, TTT_LN_EPS, sXch, rs0, rs1);
-      float a[2] = {0.f, 0.f}, bb[2] = {0.f, 0.f};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i0 = 4 * j + e, i1 = 4 * j + 2 + e, c = 2 * j + e;
-          xh[i0] *= rs0;
-          xh[i1] *= rs1;
-          g[i0] = (fmaf(gam[c], xh[i0], bet[c]) - (vv[i0] - kk[i0])) * gam[c];
-          g[i1] = (fmaf(gam[c], xh[i1], bet[c]) - (vv[i1] - kk[i1])) * gam[c];
-          a[0] += g[i0]; a[1] = fmaf(g[i0], xh[i0], a[1]);
-          bb[0] += g[i1]; bb[1] = fmaf(g[i1], xh[i1], bb[1]);
-        }
-      }
-      tok_row_allreduce<2, 2>(tm, a, bb, sXch);
-      const float sc0 = -__bfloat162float(sEta[tm.r0]) * rs0 * (1.f / 64.f);
-      const float sc1 = -__bfloat162float(sEta[tm.r1]) * rs1 * (1.f / 64.f);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i0 = 4 * j + e, i1 = 4 * j + 2 + e;
-          g[i0] = (64.f * g[i0] - a[0] - xh[i0] * a[1]) * sc0;
-          g[i1] = (64.f * g[i1] - bb[0] - xh[i1] * bb[1]) * sc1;
-        }
-      }
-      tok_st_tile(tm, sU2, g);
-    }
-    }
     publish();
     // the previous mini-batch's Q tile has been read by every warp (its output is finished): its stage takes
     // the loads of the mini-batch two ahead
@@ -611,13 +519,10 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // ---- OUT: Q + gamma * LN(Z2b + b2) + beta.  Z2b is an output only: its partial tiles are summed by
     // reduce-scatter, and every CTA normalises and stores the token rows it owns.  The partial tile is
     // sent now; it is received, normalised and stored inside the first MMA window of the next mini-batch.
-    if constexpr (C::kRowSplit) {
+    {
       float frag[16];
       tok_ld(tm, tmem + C::TM_Z, frag);
       zo_tag = rs.send(frag, tid, warp, lane);
-    } else {
-      tok_ld(tm, tmem + C::TM_Z, zo);
-      zo_tag = csum.reduce_scatter_send(zo, tid);
     }
     zo_it = it;
     // the last CTA barrier of the mini-batch also takes the vote on leaving the loop: a peer can raise
@@ -628,10 +533,7 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     if (aborted) break;
   }
 #undef TTT_ISSUE4
-  if (!aborted && zo_it >= 0) {                  // the last mini-batch's output
-    if constexpr (C::kRowSplit) finish_out();
-    else finish_out_whole();
-  }
+  if (!aborted && zo_it >= 0) finish_out();      // the last mini-batch's output
 
   // ---- epilogue: optional final state, then teardown
   if (!aborted && p.W1f != nullptr) {
@@ -668,82 +570,64 @@ ttt_fwd_cluster_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   if (warp == 0) tmem_dealloc(tmem, C::TM_COLS);
 }
 
+// Four CTAs to a stream.  (Two, each with half of the hidden units, are no form of the forward: two are the chain and the
+// output pass, ttt_fwd_pair_sm100.cu, which is faster from four mini-batches on.)
+constexpr int kCtas = 4;
+using Launched = Cfg<kCtas>;
+
 // Once per device: the kernel's dynamic shared memory limit.
-template <int kC>
 int prepare_kernel() {
-  using C = Cfg<kC>;
   static std::once_flag once[64];
   static cudaError_t attr_err[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return ttt_set_error(TTT_B200_ERR_LAUNCH, "device index out of range");
   std::call_once(once[dev], [&] {
-    attr_err[dev] = cudaFuncSetAttribute(ttt_fwd_cluster_kernel<kC>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+    attr_err[dev] = cudaFuncSetAttribute(ttt_fwd_cluster_kernel<kCtas>, cudaFuncAttributeMaxDynamicSharedMemorySize, Launched::SMEM_BYTES);
   });
   if (attr_err[dev] != cudaSuccess) return ttt_set_error(TTT_B200_ERR_LAUNCH, cudaGetErrorString(attr_err[dev]));
   return TTT_B200_OK;
 }
 
-// How many clusters of kC CTAs the device runs at once (a cluster lives inside one GPC, and the GPCs' SM counts
-// are not all multiples of kC: fewer than SMs / kC).  0 if the query fails.
-template <int kC>
-int cluster_capacity() {
-  using C = Cfg<kC>;
-  static std::once_flag once[64];
-  static int cap[64];
-  if (prepare_kernel<kC>()) return 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::call_once(once[dev], [&] {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kC * 64);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = C::SMEM_BYTES;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kC;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, ttt_fwd_cluster_kernel<kC>, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
-    }
-    cap[dev] = n;
-  });
-  return cap[dev];
-}
-
-template <int kC>
-int launch_cluster(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmOut,
-                   const FwdClParams& p, int streams, cudaStream_t stream) {
-  using C = Cfg<kC>;
-  if (int rc = prepare_kernel<kC>()) return rc;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(streams) * kC);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = C::SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = kC;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, ttt_fwd_cluster_kernel<kC>, tmQ, tmK, tmV, tmOut, p);
-  if (e != cudaSuccess) return ttt_set_error(TTT_B200_ERR_LAUNCH, cudaGetErrorString(e));
-  return TTT_B200_OK;
+void cluster_attribute(cudaLaunchAttribute* attr, unsigned n) {
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = n;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
 }
 
 }  // namespace
 
-int ttt_launch_forward_cluster(const ttt_b200_fwd_args* a, int cluster, cudaStream_t stream, uint32_t* status,
-                               uint64_t limit_ns, int drop_load) {
+// How many clusters of two or four of these CTAs, of which an SM holds one, the device runs at once (a cluster lives inside one
+// GPC, and the GPCs' SM counts are not all multiples of it: fewer than SMs / cluster).  0 for other sizes or if the query fails.
+int ttt_forward_cluster_capacity(int cluster) {
+  static std::once_flag once[2][64];
+  static int cap[2][64];
+  if ((cluster != 2 && cluster != 4) || prepare_kernel()) return 0;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const int k = cluster == 4;
+  std::call_once(once[k][dev], [&] {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cluster * 64);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = Launched::SMEM_BYTES;
+    cudaLaunchAttribute attr[1];
+    cluster_attribute(attr, cluster);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, ttt_fwd_cluster_kernel<kCtas>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    cap[k][dev] = n;
+  });
+  return cap[k][dev];
+}
+
+int ttt_launch_forward_cluster(const ttt_b200_fwd_args* a, cudaStream_t stream, uint32_t* status, uint64_t limit_ns,
+                               int drop_load) {
   const uint64_t rows = static_cast<uint64_t>(a->B) * a->H * a->NC * 64;
   CUtensorMap tmQ, tmK, tmV, tmOut;
   if (int rc = ttt_make_tile_map(&tmQ, a->XQ, rows)) return rc;
@@ -764,12 +648,19 @@ int ttt_launch_forward_cluster(const ttt_b200_fwd_args* a, int cluster, cudaStre
   p.drop_load = drop_load;
   p.status = status;
   p.wait_limit_ns = limit_ns;
-  const int streams = a->B * a->H;
-  if (cluster == 2) return launch_cluster<2>(tmQ, tmK, tmV, tmOut, p, streams, stream);
-  if (cluster == 4) return launch_cluster<4>(tmQ, tmK, tmV, tmOut, p, streams, stream);
-  return ttt_set_error(TTT_B200_ERR_BAD_ARGS, "cluster size must be 2 or 4");
-}
-
-int ttt_forward_cluster_capacity(int cluster) {
-  return cluster == 2 ? cluster_capacity<2>() : cluster == 4 ? cluster_capacity<4>() : 0;
+  if (int rc = prepare_kernel()) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(a->B * a->H) * kCtas);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = Launched::SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  cluster_attribute(attr, kCtas);
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, ttt_fwd_cluster_kernel<kCtas>, tmQ, tmK, tmV, tmOut, p);
+  if (e != cudaSuccess) return ttt_set_error(TTT_B200_ERR_LAUNCH, cudaGetErrorString(e));
+  return TTT_B200_OK;
 }

@@ -37,7 +37,7 @@ def _host():
 
 def _flags(sync, cluster, lost_load=False):
     """Flag word of the C ABI: bit 0 synchronise, bit 1 the failure-path test hook, bits 8..11 the number
-    of CTAs (1, 2 or 4) that share one stream (0 / None: chosen from B*H and the SM count)."""
+    of CTAs (1, 2 or 4) that share one stream (0 / None: chosen per call)."""
     cluster = 0 if cluster is None else int(cluster)
     _check(cluster in (0, 1, 2, 4), "cluster must be None, 1, 2 or 4")
     return (_lib.FLAG_SYNC if sync else 0) | (_lib.FLAG_TEST_LOST_LOAD if lost_load else 0) | (cluster << 8)
@@ -52,7 +52,9 @@ def ttt_forward(XQ, XK, XV, last_eta, ttt_norm_weight, ttt_norm_bias, W1, b1, W2
     Keyword-only extras (not in the reference): `final_state` = (W1, b1, W2, b2) fp32 tensors
     that receive the state after the last mini-batch; `sync` blocks until the result is ready
     and raises on a device-side failure; `cluster` forces how many CTAs share one (batch, head)
-    stream (1, 2 or 4; default: chosen from B*H and the GPU's SM count).
+    stream (1, 2 or 4; default: chosen from B*H, the length, the group size and the GPU's SM count).
+    A sequence in chunks, each call's `final_state` the next one's initial state, agrees with one
+    long call within rounding; with `cluster` named it has its bits.
     """
     _host().forward(XQ, XK, XV, last_eta, ttt_norm_weight, ttt_norm_bias, W1, b1, W2, b2, W1_checkpoints,
                     b1_checkpoints, W2_checkpoints, b2_checkpoints, Out, checkpoint_group_size, final_state,
@@ -107,7 +109,8 @@ def ttt_backward(XQ, XK, XV, last_eta, ttt_norm_weight, ttt_norm_bias,
     Positional arguments: exactly the reference's 42 tensors + int
     (kernels/ttt_backward/ttt.cu:1451-1495).  grad_L_ttt_norm_weight / bias hold one row per
     batch element ([B, H, 1, 64]); the caller sums over dim 0 as with the reference
-    (kernels/ttt_backward/matching.py:522-523).
+    (kernels/ttt_backward/matching.py:522-523).  `cluster` as in `ttt_forward`; chunks have the bits of one
+    call with 1 or 4 named, or with 2 where every chunk is longer than a group of at least two mini-batches.
     """
     _host().backward(XQ, XK, XV, last_eta, ttt_norm_weight, ttt_norm_bias, W1_checkpoints, b1_checkpoints,
                      W2_checkpoints, b2_checkpoints, Out, W1_init_group, b1_init_group, W2_init_group, b2_init_group,
