@@ -1,0 +1,34 @@
+"""Waits of the one-CTA MLP forward (csrc/ttt_fwd_sm100.cu): with any one of its hand-overs' waits or signals left out, the
+order of accesses that kernel_order.py derives from the source shows it."""
+import os
+
+import pytest
+
+import kernel_order as ko
+from test_pair_order_cpu import CSRC, FILES
+
+
+def walk(edit, NC=4, cgs=2):
+    src = ko.Source(*[os.path.join(CSRC, f) for f in FILES[:-1] + ["ttt_fwd_sm100.cu"]], edit=edit)
+    src.barriers = {v: k for k, v in src.names.items() if k.startswith("BAR_")}
+    p = ko.Struct(H=1, NC=NC, cgs=cgs, nck=-(-NC // cgs), drop_load=-1, wait_limit_ns=0, eta=ko.Ptr("x", 100 << 40, 2))
+    for k in "gamma beta W1 b1 W2 b2 W1c b1c W2c b2c W1f b1f W2f b2f status".split():
+        setattr(p, k, ko.Ptr("x", 100 << 40, 4))
+    maps = {f"tm{k}": i for i, k in enumerate(["Q", "K", "V", "Out"])}
+    return ko.Run(src, "ttt_fwd_kernel", dict(maps, p=p), {}, 1, 16, skip=("wait_bar",))
+
+
+@pytest.mark.parametrize("wait", [
+    "wait_bar(BAR_U2RDY, par);",                       # W2's update before U2 is there
+    "wait_bar(BAR_R, par);",                           # the bf16 W2 rewritten under MMA3
+    "if (it > 0) wait_bar(BAR_W2UPD, prev);",          # X2 rewritten under W2's update
+    "if (it > 0) wait_bar(BAR_W1READ, prev);",         # the bf16 W1 rewritten under MMA5
+    "if (it > 0) wait_bar(BAR_SREAD, prev);",          # W1 updated while a checkpoint is read
+    "wait_bar(BAR_W2RDY, par);",                       # MMA2 before the bf16 W2 is there
+    "wait_bar(BAR_W1RDY, par);",                       # MMA5 before the bf16 W1 is there
+])
+def test_each_wait_is_needed(wait):
+    seen = []
+    r = walk(lambda text: seen.append(text.count(wait)) or text.replace(wait, ""))
+    assert sum(seen) == 1
+    assert r.problems or r.races() or r.phases()
