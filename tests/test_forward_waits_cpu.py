@@ -1,6 +1,7 @@
 """Waits of the one-CTA MLP forward (csrc/ttt_fwd_sm100.cu): with any one of its hand-overs' waits or signals left out, the
 order of accesses that kernel_order.py derives from the source shows it."""
 import os
+import re
 
 import pytest
 
@@ -32,3 +33,10 @@ def test_each_wait_is_needed(wait):
     r = walk(lambda text: seen.append(text.count(wait)) or text.replace(wait, ""))
     assert sum(seen) == 1
     assert r.problems or r.races() or r.phases()
+
+
+def test_loads_come_from_warps_that_issue_no_products():
+    """The first warp of each 128-row block issues the chain group's products, the group's first warp the output group's."""
+    text = open(os.path.join(CSRC, "ttt_fwd_sm100.cu")).read()
+    chain, output = (int(n) // 32 for n in re.findall(r"const bool loader = gtid == (\d+);", text))
+    assert "const bool issuer = quad == 0;" in text and chain % 4 != 0 and output != 0

@@ -243,7 +243,7 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   if (chain) {
     // ================================================================================== chain group
     reg_take<kRegsChain>();
-    const bool loader = gtid == 128;      // not the MMA issuer: its bookkeeping stays off the issue path
+    const bool loader = gtid == 224;      // of a warp that issues no products: its bookkeeping stays off the issue path
     if (loader) {
       for (; issued < kStages; ++issued) {
         load_k(issued);
