@@ -222,6 +222,93 @@ struct BwdParams {
   uint64_t wait_limit_ns;
 };
 
+// ---- 64 x 64 token-major tiles spread over 16 warps: a warp takes the 16 rows of its quadrant and 16 of the 64 columns,
+// a thread rows r0 and r1 = r0 + 8 and the column pairs col(0), col(1) (the TokMap fragment, halved).
+struct TokMap16 {
+  int quad, cq, l3;
+  int r0, r1;
+  uint32_t taddr;
+  __device__ __forceinline__ TokMap16(int warp, int lane)
+      : quad(warp & 3), cq(warp >> 2), l3(lane & 3), r0((warp & 3) * 16 + (lane >> 2)), r1(r0 + 8),
+        taddr((static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>((warp >> 2) * 16)) {}
+  __device__ __forceinline__ int col(int j) const { return cq * 16 + j * 8 + l3 * 2; }
+  __device__ __forceinline__ uint32_t off(int r, int j) const { return sw128_off(r, cq * 2 + j) + l3 * 4; }
+};
+struct Frag16 {
+  f32x2 a[2], b[2];
+};
+__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ Frag16 f16_pack(const uint32_t (&u)[8]) {
+  Frag16 f;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    f.a[j] = pk(u[4 * j], u[4 * j + 1]);
+    f.b[j] = pk(u[4 * j + 2], u[4 * j + 3]);
+  }
+  return f;
+}
+// the raw bf16 pairs of a swizzled tile: w[2j] row r0, w[2j + 1] row r1
+__device__ __forceinline__ void f16_ld_raw(const TokMap16& m, const uint8_t* tile, uint32_t (&w)[4]) {
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    w[2 * j] = *reinterpret_cast<const uint32_t*>(tile + m.off(m.r0, j));
+    w[2 * j + 1] = *reinterpret_cast<const uint32_t*>(tile + m.off(m.r1, j));
+  }
+}
+__device__ __forceinline__ void f16_st_tile(const TokMap16& m, uint8_t* tile, const Frag16& f) {
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    *reinterpret_cast<uint32_t*>(tile + m.off(m.r0, j)) = f32x2_to_bf16x2(f.a[j]);
+    *reinterpret_cast<uint32_t*>(tile + m.off(m.r1, j)) = f32x2_to_bf16x2(f.b[j]);
+  }
+}
+__device__ __forceinline__ f32x2 f16_col(const TokMap16& m, const float* vec, int j) {
+  return *reinterpret_cast<const f32x2*>(vec + m.col(j));
+}
+// Column sums over a warp's 16 rows, the eight lanes that share a column pair halving the set at every exchange: every
+// lane ends with the total of column f16_colsum_col (lanes that differ in bit 2 with the same one).
+__device__ __forceinline__ float f16_colsum(f32x2 v0, f32x2 v1, int lane) {
+  float k[4];
+  upk(v0, k[0], k[1]);
+  upk(v1, k[2], k[3]);
+  const bool u4 = lane & 16, u3 = lane & 8;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float send = u4 ? k[i] : k[2 + i], keep = u4 ? k[2 + i] : k[i];
+    k[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+  const float s = (u3 ? k[1] : k[0]) + __shfl_xor_sync(0xffffffffu, u3 ? k[0] : k[1], 8);
+  return s + __shfl_xor_sync(0xffffffffu, s, 4);
+}
+__device__ __forceinline__ int f16_colsum_col(const TokMap16& m, int lane) {
+  return m.cq * 16 + ((lane >> 4) & 1) * 8 + m.l3 * 2 + ((lane >> 3) & 1);
+}
+// two sums per row over the row's four lanes and four warps; xch: float2[4][64], bar: the first of four named barriers
+__device__ __forceinline__ void f16_row_sums(const TokMap16& m, float (&a)[2], float (&b)[2], float2* xch, uint32_t bar) {
+#pragma unroll
+  for (int s = 1; s <= 2; s <<= 1) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      a[i] += __shfl_xor_sync(0xffffffffu, a[i], s);
+      b[i] += __shfl_xor_sync(0xffffffffu, b[i], s);
+    }
+  }
+  if (m.l3 == 0) {
+    xch[m.cq * 64 + m.r0] = make_float2(a[0], a[1]);
+    xch[m.cq * 64 + m.r1] = make_float2(b[0], b[1]);
+  }
+  named_bar_sync(bar + m.quad, 128);
+  const float2 a0 = xch[m.r0], a1 = xch[64 + m.r0], a2 = xch[128 + m.r0], a3 = xch[192 + m.r0];
+  const float2 b0 = xch[m.r1], b1 = xch[64 + m.r1], b2 = xch[128 + m.r1], b3 = xch[192 + m.r1];
+  a[0] = (a0.x + a1.x) + (a2.x + a3.x); a[1] = (a0.y + a1.y) + (a2.y + a3.y);
+  b[0] = (b0.x + b1.x) + (b2.x + b3.x); b[1] = (b0.y + b1.y) + (b2.y + b3.y);
+}
+
 // D[128 x 16] = A B^T with A in tensor memory (as in mma_hidden_ta) and B 16 rows of 64 bf16 from `b_smem` on (K-major)
 __device__ __forceinline__ void mma_rowsum_ta(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_smem, uint32_t lead) {
   constexpr uint32_t idesc = umma_idesc_bf16(128, 16, false, false, false);

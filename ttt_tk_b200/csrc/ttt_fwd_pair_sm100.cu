@@ -113,14 +113,6 @@ struct FwdParams {
   uint64_t wait_limit_ns;
 };
 
-// 32 fp32 accumulator columns as bf16 pairs to 16 columns of tensor memory (an A operand of the MMAs)
-__device__ __forceinline__ void st_cols32_tmem(uint32_t taddr, const uint32_t (&v)[32]) {
-  uint32_t w[16];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) w[k] = pack_bf16(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
-  tmem_st16(taddr, w);
-}
-
 // Streams to a cluster, whose first CTAs are the chains and whose others the output passes: the SMs of a TPC, which share an
 // instruction cache, then run the same program (48 streams x 32: 176 -> 141 us; with a stream to a cluster 74 would run at
 // once, but at 5.2 us per mini-batch against 4.3 with one CTA each).

@@ -141,14 +141,6 @@ struct FwdParams {
   uint64_t wait_limit_ns;
 };
 
-// 32 fp32 accumulator columns as bf16 pairs to 16 columns of tensor memory (an A operand of the MMAs)
-__device__ __forceinline__ void st_cols32_tmem(uint32_t taddr, const uint32_t (&v)[32]) {
-  uint32_t w[16];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) w[k] = pack_bf16(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
-  tmem_st16(taddr, w);
-}
-
 __global__ void __launch_bounds__(kThreads, 1)
 ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmOut,
