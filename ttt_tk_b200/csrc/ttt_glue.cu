@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256, (kChunks <= 8 ? 4 : 2)) unpack_layernorm_
 // result is the operator's grad_L_XQW_mini_batch.  With xhat = (x - mean) rstd and g = dy gamma:
 //   dx = rstd (g - mean(g) - xhat mean(g xhat)),   d_gamma[f] += sum over tokens of dy xhat,   d_beta[f] += sum of dy.
 // One pass over x and dy.  A token is the work of as many warps as it has groups of four heads (of eight warps with two groups
-// each when H > 32), and a CTA's eight warps take as many tokens side by side as that leaves room for: a lane owns 8 features
+// each when H > 32), and a CTA's eight warps take up to as many tokens side by side (`side`) as that leaves room for: a lane owns 8 features
 // (one 16-byte piece of a head row) of every token its warps work on, so the parameter gradients
 // accumulate in 16 registers per head group with no traffic at all, and a token's two row means are put
 // together from its warps' partial sums through shared memory, kTokBatch tokens per CTA barrier.  The next tokens' rows are
@@ -168,14 +168,13 @@ template <int kGroups>
 __global__ void __launch_bounds__(256, (kGroups == 1 ? 2 : 1))
 pack_layernorm_backward_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ x, const float* __restrict__ gamma,
                                const float2* __restrict__ stats, uint4* __restrict__ dx, float* __restrict__ d_gamma,
-                               float* __restrict__ d_beta, long tokens, int T, int H) {
+                               float* __restrict__ d_beta, long tokens, int T, int H, int side) {
   __shared__ float2 part[2][kTokBatch][8];
   __shared__ float sums[8][32][17];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane >> 3, piece = lane & 7;
   const float inv_n = 1.f / static_cast<float>(H * 64);
   const int width = kGroups == 1 ? (H + 3) / 4 : 8;      // warps to a token
-  const int side = 8 / width;                            // tokens side by side
   const int mine = warp / width, slot = warp - mine * width;
   int hh[kGroups];
   float gg[kGroups][8], ag[kGroups][8], ab[kGroups][8];
@@ -422,7 +421,11 @@ extern "C" int ttt_b200_pack_layernorm_backward(const void* grad_y, const void* 
   const long tokens = static_cast<long>(B) * T;
   // one wave of CTAs (as many as are resident at once), each looping over its token batches: every CTA ends
   // with 2 x 64 H atomic adds for the parameter gradients, so there should be no more of them than can run
-  const long per = H <= 32 ? kTokBatch * (8 / ((H + 3) / 4)) : kTokBatch;
+  // tokens side by side in a CTA: as many as its warps have room for, while that leaves 32 CTAs (one mini-batch, us, all / this: 1
+  // head 3.65 / 3.03, 4 heads 3.90 / 3.34, 12 heads 3.91 / 3.55; 512 tokens of 4 heads 4.02 / 4.00)
+  int side = H <= 32 ? 8 / ((H + 3) / 4) : 1;
+  while (side > 1 && tokens < 32L * kTokBatch * side) --side;
+  const long per = static_cast<long>(kTokBatch) * side;
   long blocks = (tokens + per - 1) / per;
   const long cap = static_cast<long>(sms) * (H <= 32 ? 2 : 1);
   if (blocks > cap) blocks = cap;
@@ -430,7 +433,7 @@ extern "C" int ttt_b200_pack_layernorm_backward(const void* grad_y, const void* 
 #define TTT_LNB_LAUNCH(G)                                                                                        \
   pack_layernorm_backward_kernel<G><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(                          \
       static_cast<const uint4*>(grad_y), static_cast<const uint4*>(x), gamma, reinterpret_cast<const float2*>(stats), \
-      static_cast<uint4*>(grad_x), grad_gamma, grad_beta, tokens, T, H)
+      static_cast<uint4*>(grad_x), grad_gamma, grad_beta, tokens, T, H, side)
   if (H <= 32) TTT_LNB_LAUNCH(1);
   else TTT_LNB_LAUNCH(2);
 #undef TTT_LNB_LAUNCH
