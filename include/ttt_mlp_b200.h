@@ -286,22 +286,21 @@ int ttt_b200_take_status(void);
 /* Library / ABI version (major * 1000 + minor). */
 int ttt_b200_version(void);
 
-/* How many CTAs (1, 2 or 4) a call of ttt_b200_forward (backward = 0) or ttt_b200_backward (backward != 0) with these
+/* How many CTAs (1, 2 or 4) a short call of ttt_b200_forward (backward = 0) or ttt_b200_backward (backward != 0) with these
  * `flags` gives each (batch, head) stream of a problem with `streams` = B*H streams on the current device.  The size that
  * the flags name; else the one that TTT_B200_CLUSTER names (0 or empty: none); else four when the device runs that many
  * clusters of four at once (ttt_b200_cluster_capacity), else two in the backward when those fit, else one (measured
- * thresholds).  A call long enough to gain from it takes two where this says one or four: ttt_b200_forward_ctas,
- * ttt_b200_backward_ctas.  The
- * reference fixes the split at compile time (kernels/ttt/ttt.cu:11-12,
- * kernels/ttt_backward/ttt.cu:12-16).  Returns -1 on error. */
+ * thresholds).  Not always what a call runs: one that is long enough to gain from it takes two where this says one or four, which
+ * ttt_b200_forward_ctas and ttt_b200_backward_ctas know.  The reference fixes the split at compile time
+ * (kernels/ttt/ttt.cu:11-12, kernels/ttt_backward/ttt.cu:12-16).  Returns -1 on error. */
 int ttt_b200_launch_cluster(int streams, uint32_t flags, int backward);
 
-/* The same for a forward of NC mini-batches in groups of checkpoint_group_size: without a size in the flags or the
+/* What a forward of NC mini-batches in groups of checkpoint_group_size runs: without a size in the flags or the
  * environment it is two where the device runs all streams as pairs of CTAs, one with the chain of the state and one with the
  * output pass, and that is faster: instead of one from six mini-batches on, instead of four from 16 in groups of four on. */
 int ttt_b200_forward_ctas(int streams, int NC, int checkpoint_group_size, uint32_t flags);
 
-/* The same for a backward of NC mini-batches in groups of checkpoint_group_size: without a size in the flags or the
+/* What a backward of NC mini-batches in groups of checkpoint_group_size runs: without a size in the flags or the
  * environment it is two instead of four from three groups of four mini-batches or two of eight on. */
 int ttt_b200_backward_ctas(int streams, int NC, int checkpoint_group_size, uint32_t flags);
 
@@ -316,8 +315,8 @@ int ttt_b200_backward_tail(int streams, int NC, int checkpoint_group_size, uint3
 int ttt_b200_backward_pairs(int streams, int NC, int checkpoint_group_size, uint32_t flags);
 
 /* The widest cluster size whose capacity on the current device covers `streams`: four, else (forward only) two, else one.
- * TTT_B200_CLUSTER overrides.  Not what a launch runs between the two capacities: ttt_b200_launch_cluster is.  Returns
- * -1 on error. */
+ * TTT_B200_CLUSTER overrides.  Not what a call runs: ttt_b200_forward_ctas and ttt_b200_backward_ctas are.  Returns -1 on
+ * error. */
 int ttt_b200_pick_cluster(int streams, int backward);
 
 /* How many clusters of `cluster` (2 or 4) CTAs of the forward (backward = 0) or backward kernel the current

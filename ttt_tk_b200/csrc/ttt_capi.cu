@@ -106,8 +106,7 @@ int capacity(int cluster, bool backward) {
 // streams are resident at once.  Four CTAs per stream win whenever the device runs that many clusters of four (32 streams
 // of 128 mini-batches in groups of 4 on a B200: forward 4.3 against 4.6 us per mini-batch with one CTA, backward 14.0
 // against 22.7; of longer calls: forward_ctas, backward_ctas).  Where only clusters of two fit (34 to 74 streams), short
-// forwards run one CTA, whose output pass runs beside the chain in two groups of warps (4.6 us per mini-batch against 5.8
-// with half of the hidden units each), and the backward two (60 streams in groups of 5: 11.7 us per mini-batch against 23.3 with
+// forwards run one CTA, whose output pass runs beside the chain in two groups of warps, and the backward two (60 streams in groups of 5: 11.7 us per mini-batch against 23.3 with
 // one).  Beyond, one.
 static int ttt_launch_cluster(int streams, uint32_t flags, bool backward, int* cluster) {
   if (int rc = asked_cluster(flags, cluster)) return rc;
@@ -120,9 +119,9 @@ static int ttt_launch_cluster(int streams, uint32_t flags, bool backward, int* c
 
 // CTAs per stream of a forward.  Two where the device runs all streams as pairs at once and that is the faster form: against
 // one CTA from six mini-batches on (us, one CTA / pair: 34 streams x 4 in groups of 2 27.6 / 27.5, x 6 in groups of 3 35.5 /
-// 34.9, x 16 in groups of 4 79 / 72; 48 x 32 in groups of 6 147 / 136, in groups of 1 203 / 177), against four, which share
+// 34.9, x 16 in groups of 4 79 / 72; 66 streams x 6 in one group 34.6 / 34.6; 48 x 32 in groups of 6 147 / 136, in groups of 1 203 / 177), against four, which share
 // the writing of the state, from 16 mini-batches in groups of four on (four / pair: 12 streams x 12 in groups of 4 54.8 /
-// 56.1, x 16 71.9 / 71.2; x 32 in groups of 6 138 / 131, x 16 in groups of 2 72.7 / 77.6; 32 x 128 in groups of 16 536 / 489).
+// 56.1, x 16 71.9 / 70.5, 33 streams x 16 72.1 / 71.1; x 32 in groups of 6 138 / 131, x 16 in groups of 2 72.7 / 77.6; 32 x 128 in groups of 16 536 / 489).
 // Two are always the chain and the output pass (ttt_fwd_pair_sm100.cu), whatever the call's length: a sequence in chunks, with
 // the size named, then has the bits of one call.  (Half of the hidden units each is faster up to three mini-batches, 12 streams
 // x 1 10.9 / 14.5 us, but no rule takes two there.)
@@ -168,7 +167,9 @@ static int backward_ctas(int streams, int NC, int cgs, uint32_t flags, int* ctas
 // takes groups to pipeline, and groups long enough that the sweep does not wait for the recompute.  Us, one CTA / pairs: 128
 // streams x 128 in groups of 8 2770 / 2458, x 64 1397 / 1295, x 64 in groups of 6 1435 / 1395, x 96 in groups of 12 2030 / 1869,
 // x 128 in groups of 20 2667 / 2457, 75 streams x 64 in groups of 8 1380 / 1244; 128 streams x 40 in groups of 5 921 / 938, x 64
-// in groups of 4 1517 / 1518, of 16 1344 / 1387, x 32 in groups of 6 735 / 769.
+// in groups of 4 1517 / 1518, of 16 1344 / 1387, x 32 in groups of 6 735 / 769.  On the line itself, 75 / 96 / 112 / 128 / 132
+// streams (132 is two full turns): six groups of eight 1043 / 975, 1046 / 993, 1048 / 1007, 1053 / 1015, 1055 / 1023; of nine 1163 /
+// 1072, 1166 / 1099, 1167 / 1107, 1172 / 1123, 1174 / 1142; ten of six 1331 / 1279, 1333 / 1290, 1337 / 1309, 1345 / 1335, 1349 / 1353.
 static int backward_tail(int streams, int NC, int cgs, uint32_t flags, int ctas) {
   int asked = 0, dev = 0, sms = 0;
   if (ctas != 1 || !runs_pair(2, NC, cgs) || asked_cluster(flags, &asked) != TTT_B200_OK || asked != 0) return 0;
@@ -413,7 +414,7 @@ extern "C" int ttt_b200_cluster_capacity(int cluster, int backward) {
 }
 
 // The widest size whose capacity covers the streams (two in the forward only): a property of the device, kept for its
-// callers.  What a launch runs is ttt_b200_launch_cluster's answer.
+// callers.  What a call runs is the answer of ttt_b200_forward_ctas and ttt_b200_backward_ctas.
 extern "C" int ttt_b200_pick_cluster(int streams, int backward) {
   int c = 0;
   if (streams < 1 || asked_cluster(0u, &c) != TTT_B200_OK) return -1;

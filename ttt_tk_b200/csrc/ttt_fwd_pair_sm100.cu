@@ -314,7 +314,7 @@ ttt_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (lane == 0) mbar_arrive(&bars[E_4 + blk]);
         if (lane == 0 && ch == 1) mbar_arrive(&bars[E_W2]);
       } else {
-        // (through U1 and the bf16 W2, which nothing uses yet)
+        // (through X2b and the bf16 W2, which nothing uses yet)
         store_rows_own(p.W2c + sid * p.nck * (64 * 256) + (hrow - lane) * 64 + ch * 32, v,
                        smem + (tok ? OFF_X2B : OFF_W2) + (warp & 7) * 4096, lane);
         if (ch == 0) p.b1c[sid * p.nck * 256 + hrow] = b1v;

@@ -38,7 +38,7 @@
 // of 128 mini-batches, one checkpoint in 8): 8.0 us per mini-batch as one group of 8 warps, 6.0 with the two groups, 4.6
 // with the rest, 4.3 with the products of a block issued by the block's own first warp and the W2 update by the output
 // group (before, one warp issued all sixteen MMAs of the state update and came 400 cycles late to EPI4, with everyone
-// waiting for it); 1536 streams of 64 mini-batches 5.43 -> 3.23 -> 2.98 ms.  A checkpoint costs about 2100 cycles (the
+// waiting for it); 1536 streams of 64 mini-batches 5.43 -> 3.23 -> 3.00 ms.  A checkpoint costs about 2100 cycles (the
 // output group's 4200 for 132 KB of stores, of which half fit its slack); as bulk copies from a staging area it cost
 // more, since W1's turn of the area waits for W2 to leave.
 //
@@ -228,7 +228,7 @@ ttt_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   };
   const long st_w = stream_id * (64 * 256);
   const bool chain = cta_warp < 8;
-  const uint32_t lead = elect_one() ? 1u : 0u;      // the lane that issues the MMAs (warp 0 of each group)
+  const uint32_t lead = elect_one() ? 1u : 0u;      // the lane that issues the MMAs (warps 0 and 4 of the chain group, warp 0 of the output group)
   int it = 0;
   int issued = 0;       // loads of this group issued so far (its loading thread), for the abort path
 
