@@ -9,7 +9,7 @@ import kernel_order as ko
 from test_pair_order_cpu import CSRC, FILES
 
 
-def walk(edit, NC=4, cgs=2):
+def walk(edit, NC, cgs):
     src = ko.Source(*[os.path.join(CSRC, f) for f in FILES[:-1] + ["ttt_fwd_sm100.cu"]], edit=edit)
     src.barriers = {v: k for k, v in src.names.items() if k.startswith("BAR_")}
     p = ko.Struct(H=1, NC=NC, cgs=cgs, nck=-(-NC // cgs), drop_load=-1, wait_limit_ns=0, eta=ko.Ptr("x", 100 << 40, 2))
@@ -19,18 +19,27 @@ def walk(edit, NC=4, cgs=2):
     return ko.Run(src, "ttt_fwd_kernel", dict(maps, p=p), {}, 1, 16, skip=("wait_bar",))
 
 
-@pytest.mark.parametrize("wait", [
+@pytest.mark.parametrize("NC,cgs", [(1, 1), (3, 1), (5, 3), (5, 2), (2, 2)])
+def test_every_wait_ends_and_all_accesses_are_ordered(NC, cgs):
+    r = walk(lambda text: text, NC, cgs)
+    assert r.problems == [] and r.races() == [] and r.phases() == set()
+
+
+WAITS = [
     "wait_bar(BAR_U2RDY, par);",                       # W2's update before U2 is there
     "wait_bar(BAR_R, par);",                           # the bf16 W2 rewritten under MMA3
     "if (it > 0) wait_bar(BAR_W2UPD, prev);",          # X2 rewritten under W2's update
     "if (it > 0) wait_bar(BAR_W1READ, prev);",         # the bf16 W1 rewritten under MMA5
-    "if (it > 0) wait_bar(BAR_SREAD, prev);",          # W1 updated while a checkpoint is read
+    "if (it > 0) wait_bar(BAR_SREAD, prev);",          # the state updated while a checkpoint is read
     "wait_bar(BAR_W2RDY, par);",                       # MMA2 before the bf16 W2 is there
     "wait_bar(BAR_W1RDY, par);",                       # MMA5 before the bf16 W1 is there
-])
-def test_each_wait_is_needed(wait):
+]
+
+
+@pytest.mark.parametrize("wait,cgs", [(w, c) for w in WAITS for c in (2, 3)])
+def test_each_wait_is_needed(wait, cgs):
     seen = []
-    r = walk(lambda text: seen.append(text.count(wait)) or text.replace(wait, ""))
+    r = walk(lambda text: seen.append(text.count(wait)) or text.replace(wait, ""), 5, cgs)
     assert sum(seen) == 1
     assert r.problems or r.races() or r.phases()
 

@@ -38,7 +38,10 @@
 // of 128 mini-batches, one checkpoint in 8): 8.0 us per mini-batch as one group of 8 warps, 6.0 with the two groups, 4.6
 // with the rest, 4.3 with the products of a block issued by the block's own first warp and the W2 update by the output
 // group (before, one warp issued all sixteen MMAs of the state update and came 400 cycles late to EPI4, with everyone
-// waiting for it); 1536 streams of 64 mini-batches 5.43 -> 3.23 -> 3.00 ms.  A checkpoint costs about 2100 cycles (the
+// waiting for it); 1536 streams of 64 mini-batches 5.43 -> 3.23 -> 3.00 ms.  In groups of two, where the output group is the
+// longer one on average, that made calls of 16 and more mini-batches 1.1 to 1.6 % slower (128 x 32 169.1 -> 171.4 us; in groups
+// of one and three as before); with W2's update left to the chain there (167.6) the kernel's other calls lost up to 0.9 %.  A
+// checkpoint costs about 2100 cycles (the
 // output group's 4200 for 132 KB of stores, of which half fit its slack); as bulk copies from a staging area it cost
 // more, since W1's turn of the area waits for W2 to leave.
 //
