@@ -63,7 +63,8 @@
 // slots freed when their last load has landed (groups of 4: 12.0 -> 11.7).  12.1 with the sweep's products written out and the
 // clock left to the helpers (32 streams in groups of 16 9.9 -> 9.4, 4 in groups of 4 11.7 -> 11.0): the issuing warp took 1200
 // cycles a product, of which the tensor pipe needs 320 to 500, and with thirteen of them was busy all of a step's 15700; the
-// epilogues' waits carried a clock's worth of instructions each (11 KB in all).  11.7 with a copy's addresses and sizes put
+// epilogues' waits carried a clock's worth of instructions each (11 KB in all; with them again, and all else as it is, 60 streams x
+// 37 430 -> 448 us, 32 x 128 1138 -> 1187, 4 x 32 339 -> 349).  11.7 with a copy's addresses and sizes put
 // together before the events that it waits for (8.5 at 32 streams, 10.7 at 4).  Not kept: the sweep running on into the next
 // group (64 x 64 in groups of 8 654 -> 679 us for both passes: the recompute is as slow, and the sweep then waits in mid-step);
 // the recompute's chain starting a group under the output pass of the last (32 x 128 in groups of 16 1136 -> 1167 us, 128 x 64

@@ -40,10 +40,10 @@
 // group (before, one warp issued all sixteen MMAs of the state update and came 400 cycles late to EPI4, with everyone
 // waiting for it); 1536 streams of 64 mini-batches 5.43 -> 3.23 -> 3.00 ms.  In groups of two, where the output group is the
 // longer one on average, that made calls of 16 and more mini-batches 1.1 to 1.6 % slower (128 x 32 169.1 -> 171.4 us; in groups
-// of one and three as before); with W2's update left to the chain there (167.6) the kernel's other calls lost up to 0.9 %.  A
-// checkpoint costs about 2100 cycles (the
-// output group's 4200 for 132 KB of stores, of which half fit its slack); as bulk copies from a staging area it cost
-// more, since W1's turn of the area waits for W2 to leave.
+// of one and three as before); with W2's update left to the chain there (167.6) the kernel's other calls lost up to 0.9 %.  The
+// copy of W2 rolled again, 1536 x 64 2946 -> 3023 us; checkpoints divided for instead of counted, 2949.  A checkpoint costs about
+// 2100 cycles (the output group's 4200 for 132 KB of stores, of which half fit its slack); as bulk copies from a staging area
+// it cost more, since W1's turn of the area waits for W2 to leave.
 //
 // Hand-over between the groups (mbarriers, each completed once per mini-batch):
 //   u2rdy   U2 and X2 are in place                             chain -> output group (W2 update)

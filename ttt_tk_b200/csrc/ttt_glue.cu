@@ -149,7 +149,9 @@ __global__ void __launch_bounds__(256, (kChunks <= 8 ? 4 : 2)) unpack_layernorm_
 // What bounds it: at small sizes the fp32 atomics, all CTAs' at the same addresses, so they are 16 bytes wide (a warp's eight
 // 4-byte ones touched 32 sectors each: 2048 tokens of 4 heads 40 us, now 8) and no more CTAs run than fit beside each other;
 // at large ones the round trip and barrier of a batch.  Before, with two tokens to a CTA whatever the number of heads and no
-// request ahead, and now: 8192 tokens of 12 heads 53 -> 23 us, of 32 heads 97 -> 42, 32768 of 32 184 -> 123 (3.3 TB/s).
+// request ahead, and now: 8192 tokens of 12 heads 53 -> 23 us, of 32 heads 97 -> 42, 32768 of 32 184 -> 123 (3.3 TB/s).  Each of
+// the three taken out again, in a row of calls: 8192 tokens of 12 heads 20.1 us, 4-byte atomics 39.3, one token at a time 29.9, no
+// request ahead 20.1; 32768 of 32 116, 138, 116, 174.
 constexpr int kTokBatch = 2;
 // eight consecutive global sums += v, 16 bytes at a time where they are aligned for it
 __device__ __forceinline__ void add8(float* dst, const float (&v)[8]) {
